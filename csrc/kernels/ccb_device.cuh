@@ -120,6 +120,7 @@ __device__ __forceinline__ void trace_mark(const CommDev& c, int k) {
 }
 
 // ------------------------------------------------------ element load/store --
+template <int N> struct Int { static constexpr int value = N; };
 template <class T> struct Elem;
 template <> struct Elem<float> {
   static __device__ __forceinline__ float to_f(float x) { return x; }
@@ -300,6 +301,201 @@ __device__ __forceinline__ void store16(T* base, size_t idx, size_t limit, const
     for (int i = 0; i < 16; ++i)
       if (idx + i < limit) p[i] = Elem<T>::from_f(v[i]);
   }
+}
+
+// ------------------------------------------- 32-byte element load/store --
+// The same 16 elements of a lane in 32-byte accesses (256 bits, sm_100): one access in 16-bit
+// types and two in fp32, so that every access of a warp covers whole 32-byte sectors, where
+// 16-byte accesses at the lanes' 32- or 64-byte stride touch half of each. Their operands are
+// eight consecutive registers: for kernels that have registers to spare (exchange, solo,
+// lossless). The ring kernel, at its limit of 64, spilled 64 bytes with them and took 242 us
+// instead of 212 (four ranks, 64 MiB of bf16 each, fp8).
+__device__ __forceinline__ void ldg_stream32(const void* p, uint32_t* w) {
+  asm volatile("ld.global.cs.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7]) : "l"(p));
+}
+__device__ __forceinline__ void stg_stream32(void* p, const uint32_t* w) {
+  asm volatile("st.global.cs.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]),
+               "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7]) : "memory");
+}
+
+
+template <class T> struct Wide16 { uint32_t w[4 * sizeof(T)]; };
+
+// The first W words of w are those `mis` elements of T further on. `mis` (0 .. 32 bytes - 1
+// element) is the same in all lanes of a warp, so the branches are uniform.
+template <class T, int N>
+__device__ __forceinline__ void shift_down(uint32_t (&w)[N], uint32_t mis) {
+  uint32_t words = mis;
+  if constexpr (sizeof(T) == 2) {
+    words = mis >> 1;
+    if (mis & 1u) {
+#pragma unroll
+      for (int k = 0; k < N - 1; ++k) w[k] = __byte_perm(w[k], w[k + 1], 0x5432);
+    }
+  }
+  if (words & 1u) {
+#pragma unroll
+    for (int k = 0; k < N - 1; ++k) w[k] = w[k + 1];
+  }
+  if (words & 2u) {
+#pragma unroll
+    for (int k = 0; k < N - 2; ++k) w[k] = w[k + 2];
+  }
+  if (words & 4u) {
+#pragma unroll
+    for (int k = 0; k < N - 4; ++k) w[k] = w[k + 4];
+  }
+}
+// Rotation of the warp's 32 * W words (one lane's follow the other's) by `mis` elements of T
+// towards higher lanes; the last `mis` come round to lane 0. At most eight shuffles.
+template <class T>
+__device__ __forceinline__ void rotate_up(uint32_t (&w)[4 * sizeof(T)], uint32_t mis, int lane) {
+  constexpr int W = 4 * (int)sizeof(T);
+  const int from = (lane + 31) & 31;
+  uint32_t words = mis;
+  if constexpr (sizeof(T) == 2) {
+    words = mis >> 1;
+    if (mis & 1u) {
+      const uint32_t edge = __shfl_sync(0xffffffffu, w[W - 1], from);
+#pragma unroll
+      for (int k = W - 1; k >= 1; --k) w[k] = __byte_perm(w[k - 1], w[k], 0x5432);
+      w[0] = __byte_perm(edge, w[0], 0x5432);
+    }
+  }
+  auto by = [&](auto step) {
+    constexpr int s = decltype(step)::value;
+    if (!(words & (uint32_t)s)) return;
+    uint32_t edge[s];
+#pragma unroll
+    for (int k = 0; k < s; ++k) edge[k] = __shfl_sync(0xffffffffu, w[W - s + k], from);
+#pragma unroll
+    for (int k = W - 1; k >= s; --k) w[k] = w[k - s];
+#pragma unroll
+    for (int k = 0; k < s; ++k) w[k] = edge[k];
+  };
+  by(Int<1>{});
+  by(Int<2>{});
+  by(Int<4>{});
+}
+
+// `idx` is a multiple of 512 plus 16 times the lane; elements at or beyond `limit` read as 0.
+// 32-byte accesses at a 32-byte boundary, 16-byte ones at a 16-byte boundary. At any other
+// address kAnyOffset reads 32 bytes at a time from the boundary below to the boundary above and
+// shifts them into place (each such access holds at least one byte of the lane's elements, so it
+// stays inside their allocation); without it the elements come one by one.
+template <class T, bool kAnyOffset = false>
+__device__ __forceinline__ void load16_wide(const T* base, size_t idx, size_t limit, Wide16<T>& raw) {
+  constexpr int W = 4 * (int)sizeof(T);
+  const T* p = base + idx;
+  const uint32_t off = (uint32_t)(reinterpret_cast<uintptr_t>(p) & 31);
+  const bool inside = idx + 16 <= limit;
+  if (inside && off == 0) {
+#pragma unroll
+    for (int k = 0; k < W; k += 8) ldg_stream32(reinterpret_cast<const char*>(p) + 4 * k, raw.w + k);
+  } else if (inside && off == 16) {
+#pragma unroll
+    for (int k = 0; k < W; k += 4) {
+      const uint4 u = ldg_stream(reinterpret_cast<const char*>(p) + 4 * k);
+      raw.w[k] = u.x; raw.w[k + 1] = u.y; raw.w[k + 2] = u.z; raw.w[k + 3] = u.w;
+    }
+  } else if (kAnyOffset && inside) {
+    uint32_t w[W + 8];
+#pragma unroll
+    for (int k = 0; k < W + 8; k += 8) ldg_stream32(reinterpret_cast<const char*>(p) - off + 4 * k, w + k);
+    shift_down<T>(w, off / (uint32_t)sizeof(T));
+#pragma unroll
+    for (int k = 0; k < W; ++k) raw.w[k] = w[k];
+  } else {
+#pragma unroll
+    for (int i = 0; i < W; ++i) {
+      if constexpr (sizeof(T) == 4) {
+        raw.w[i] = (idx + i < limit) ? elem_bits(p[i]) : 0u;
+      } else {
+        const uint32_t lo = (idx + 2 * i < limit) ? elem_bits(p[2 * i]) : 0u;
+        const uint32_t hi = (idx + 2 * i + 1 < limit) ? elem_bits(p[2 * i + 1]) : 0u;
+        raw.w[i] = lo | (hi << 16);
+      }
+    }
+  }
+}
+template <class T>
+__device__ __forceinline__ void wide16_to_f(const Wide16<T>& raw, float (&v)[16]) {
+  if constexpr (sizeof(T) == 4) {
+#pragma unroll
+    for (int i = 0; i < 16; ++i) v[i] = bits_to_f<T>(raw.w[i]);
+  } else {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      v[2 * i] = bits_to_f<T>(raw.w[i] & 0xffffu);
+      v[2 * i + 1] = bits_to_f<T>(raw.w[i] >> 16);
+    }
+  }
+}
+// The counterpart. With kAnyOffset a whole unit (all 512 elements of the warp inside the limit,
+// so that all lanes are here) at an address that is no multiple of 16 bytes is rotated up to the
+// 32-byte boundaries across the warp and stored in 32-byte accesses, but for its first elements
+// and its last, which come to lie in lane 0. One element a store, as it was before, touches a
+// sector for every element: an eight-rank all-gather of 1,638,401 bf16 values a rank (blocks at
+// odd offsets, fp8) took 673 us, and takes 100.
+template <class T, bool kAnyOffset = false>
+__device__ __forceinline__ void store16_wide(T* base, size_t idx, size_t limit, const Wide16<T>& raw) {
+  constexpr int W = 4 * (int)sizeof(T);
+  T* p = base + idx;
+  const uint32_t off = (uint32_t)(reinterpret_cast<uintptr_t>(p) & 31);
+  const bool inside = idx + 16 <= limit;
+  if (inside && off == 0) {
+#pragma unroll
+    for (int k = 0; k < W; k += 8) stg_stream32(reinterpret_cast<char*>(p) + 4 * k, raw.w + k);
+    return;
+  }
+  if (inside && off == 16) {
+#pragma unroll
+    for (int k = 0; k < W; k += 4)
+      stg_stream(reinterpret_cast<char*>(p) + 4 * k, make_uint4(raw.w[k], raw.w[k + 1], raw.w[k + 2], raw.w[k + 3]));
+    return;
+  }
+  uint32_t w[W];
+#pragma unroll
+  for (int k = 0; k < W; ++k) w[k] = raw.w[k];
+  T* first = p;      // element i goes to first + i for i < mis, to p + i otherwise
+  uint32_t mis = 0;
+  const uint32_t n = inside ? 16u : idx < limit ? (uint32_t)(limit - idx) : 0u;
+  if constexpr (kAnyOffset) {
+    const uint32_t lane = threadIdx.x & 31;
+    if ((off & 15) && idx - lane * kLaneElems + kWarpElems <= limit) {   // the same in all lanes
+      mis = off / (uint32_t)sizeof(T);
+      rotate_up<T>(w, mis, (int)lane);
+      p -= mis;
+      if (lane) {
+#pragma unroll
+        for (int k = 0; k < W; k += 8) stg_stream32(reinterpret_cast<char*>(p) + 4 * k, w + k);
+        return;
+      }
+      first = p + kWarpElems;
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 16; ++i) {
+    if ((uint32_t)i < n) {
+      T* at = (kAnyOffset && (uint32_t)i < mis ? first : p) + i;
+      if constexpr (sizeof(T) == 4) *reinterpret_cast<uint32_t*>(at) = w[i];
+      else *reinterpret_cast<unsigned short*>(at) = (unsigned short)(w[(i >> 1) & (W - 1)] >> (16 * (i & 1)));
+    }
+  }
+}
+template <class T, bool kAnyOffset = false>
+__device__ __forceinline__ void store16_wide(T* base, size_t idx, size_t limit, const float (&v)[16]) {
+  Wide16<T> raw;
+  if constexpr (sizeof(T) == 4) {
+#pragma unroll
+    for (int i = 0; i < 16; ++i) raw.w[i] = __float_as_uint(v[i]);
+  } else {
+    // one packed conversion per pair of values
+#pragma unroll
+    for (int i = 0; i < 8; ++i) raw.w[i] = pack2<T>(v[2 * i], v[2 * i + 1]);
+  }
+  store16_wide<T, kAnyOffset>(base, idx, limit, raw);
 }
 
 // fp32 side buffers (error-feedback residuals) use the same lane shape.

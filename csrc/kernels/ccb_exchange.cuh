@@ -43,61 +43,83 @@ __global__ void __launch_bounds__(kThreads, 2) exchange_kernel(const __grid_cons
     if (a.cnt[r][p] != a.cnt[r][f] || a.send_off[r][p] != a.send_off[r][f]) same = false;
   }
 
-  if (dstmask && same) {
-    const int f = __ffs(dstmask) - 1;
-    const size_t valid = a.cnt[r][f];
-    const T* src = send + a.send_off[r][f];
-    for (size_t t = b; t * tile_elems < valid; t += G) {
-      if (!active_warp || t * tile_elems + warp_off >= valid) continue;
+  // A rank's own block never goes through its arena: the packet is decoded where it was encoded.
+  // One tile is requested ahead of the one in work, so that a warp waits for memory once per
+  // tile and not once per access. (All-gather among 8 ranks of 1,638,401 bf16 values each
+  // in fp8: 673 us before, most of it element-wise stores at odd offsets, 100 after.)
+  // (In fp32 a tile ahead is 16 registers more than the kernel has: there the load stays where it is used.)
+  constexpr bool kAhead = sizeof(T) == 2, kPacketAhead = sizeof(typename C::Packet) <= 32;
+  auto encode_block = [&](const T* src, size_t valid, auto&& deliver) {
+    size_t t = b;
+    Wide16<T> raw;
+    bool have = active_warp && t * tile_elems + warp_off < valid;
+    if (have && kAhead) load16_wide<T, true>(src, t * tile_elems + lane_off, valid, raw);
+    while (have) {
       const size_t idx = t * tile_elems + lane_off;
+      if (!kAhead) load16_wide<T, true>(src, idx, valid, raw);
       float v[16];
-      load16<T>(src, idx, valid, v);
+      wide16_to_f<T>(raw, v);
+      t += G;
+      have = t * tile_elems + warp_off < valid;
+      if (have && kAhead) load16_wide<T, true>(src, t * tile_elems + lane_off, valid, raw);
       typename C::Packet pk;
       C::encode(v, pk);
-      for (int j = 0; j < n; ++j) {
-        const int p = (r + j) % n;
-        if ((dstmask >> p) & 1u) C::store(c.arena[p] + area + (size_t)r * a.slot_bytes, pad, idx, pk);
-      }
+      deliver(idx, pk);
     }
-  } else if (dstmask) {
-    for (int j = 0; j < n; ++j) {
-      const int p = (r + j) % n;
-      const size_t valid = a.cnt[r][p];
-      if (valid == 0) continue;
-      const T* src = send + a.send_off[r][p];
-      char* dst = c.arena[p] + area + (size_t)r * a.slot_bytes;
-      for (size_t t = b; t * tile_elems < valid; t += G) {
-        if (!active_warp || t * tile_elems + warp_off >= valid) continue;
-        const size_t idx = t * tile_elems + lane_off;
-        float v[16];
-        load16<T>(src, idx, valid, v);
-        typename C::Packet pk;
-        C::encode(v, pk);
-        C::store(dst, pad, idx, pk);
+  };
+  auto keep_own = [&](size_t idx, const typename C::Packet& pk) {
+    float d[16];
+    C::decode(pk, d);
+    store16_wide<T, true>(recv + a.recv_off[r][r], idx, a.cnt[r][r], d);
+  };
+  const uint32_t peers = dstmask & ~(1u << r);
+  const bool own = (dstmask >> r) & 1u;
+  if (dstmask && same) {
+    const int f = __ffs(dstmask) - 1;
+    encode_block(send + a.send_off[r][f], a.cnt[r][f], [&](size_t idx, const typename C::Packet& pk) {
+      for (int j = 1; j < n; ++j) {
+        const int p = r + j < n ? r + j : r + j - n;
+        if ((peers >> p) & 1u) C::store(c.arena[p] + area + (size_t)r * a.slot_bytes, pad, idx, pk);
       }
+      if (own) keep_own(idx, pk);
+    });
+  } else if (peers) {
+    for (int j = 1; j < n; ++j) {
+      const int p = r + j < n ? r + j : r + j - n;
+      if (!((peers >> p) & 1u)) continue;
+      char* dst = c.arena[p] + area + (size_t)r * a.slot_bytes;
+      encode_block(send + a.send_off[r][p], a.cnt[r][p], [&](size_t idx, const typename C::Packet& pk) { C::store(dst, pad, idx, pk); });
     }
   }
   __syncthreads();
-  if (threadIdx.x < n && threadIdx.x != r && ((dstmask >> threadIdx.x) & 1u))
-    signal_flag(flag_ptr(c.arena[threadIdx.x], 0, r, b), c.epoch);
+  if (threadIdx.x == 0 && peers) signal_peers(c, peers, 0, r, b);
+  // The own block of an exchange with several different blocks comes after the others have
+  // been read (its place in recv may be another block's place in send), while they travel.
+  if (own && !same) encode_block(send + a.send_off[r][r], a.cnt[r][r], keep_own);
 
   uint32_t srcmask = 0;
   for (int q = 0; q < n; ++q)
-    if (a.cnt[q][r]) srcmask |= 1u << q;
-  if (!cta_wait_sources(sync, c, my, 0, r, srcmask, 0x30)) return;
-  for (int j = 0; j < n; ++j) {
-    const int q = (r + j) % n;
+    if (q != r && a.cnt[q][r]) srcmask |= 1u << q;
+  if (srcmask && !cta_wait_sources(sync, c, my, 0, r, srcmask, 0x30)) return;
+  for (int j = 1; j < n; ++j) {
+    const int q = r + j < n ? r + j : r + j - n;
     const size_t valid = a.cnt[q][r];
-    if (valid == 0) continue;
+    const char* slot = my + area + (size_t)q * a.slot_bytes;
     T* dst = recv + a.recv_off[r][q];
-    for (size_t t = b; t * tile_elems < valid; t += G) {
-      if (!active_warp || t * tile_elems + warp_off >= valid) continue;
+    size_t t = b;
+    typename C::Packet nxt;
+    bool have = active_warp && t * tile_elems + warp_off < valid;
+    if (have && kPacketAhead) C::load(slot, pad, t * tile_elems + lane_off, nxt);
+    while (have) {
       const size_t idx = t * tile_elems + lane_off;
-      typename C::Packet pk;
-      C::load(my + area + (size_t)q * a.slot_bytes, pad, idx, pk);
+      if (!kPacketAhead) C::load(slot, pad, idx, nxt);
+      const typename C::Packet pk = nxt;
+      t += G;
+      have = t * tile_elems + warp_off < valid;
+      if (have && kPacketAhead) C::load(slot, pad, t * tile_elems + lane_off, nxt);
       float d[16];
       C::decode(pk, d);
-      store16<T>(dst, idx, valid, d);
+      store16_wide<T, true>(dst, idx, valid, d);
     }
   }
   if (a.ack) end_handshake(sync, c, r);

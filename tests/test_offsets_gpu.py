@@ -1,0 +1,45 @@
+"""Blocks at odd offsets of a buffer: the addresses at which the 32-byte accesses have to
+shift, rotate or give way."""
+import pytest
+import torch
+
+from ccbench_b200 import Communicator
+from ccbench_b200.ops import codecs as C
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("codec", ["none", "int8", "fp8"])
+def test_exchange_at_every_offset_in_a_32_byte_line(dtype, codec):
+    n, count = 2, 2 * 512 + 37      # two whole units, which are rotated, and a partial one
+    per_line = 32 // torch.empty((), dtype=dtype).element_size()
+    comm = Communicator.local(n, arena_bytes=16 << 20)
+    stride = count + per_line
+    xs = [torch.randn(stride * n, generator=torch.Generator().manual_seed(r)).to(dtype) for r in range(n)]
+    xg = [x.cuda() for x in xs]
+    for shift in range(per_line):
+        send_off = [[shift + d * (count + 1) for d in range(n)] for _ in range(n)]
+        recv_off = [[(per_line - shift) + s * (count + 3) for s in range(n)] for _ in range(n)]
+        out = [torch.full((2 * stride + 64,), 7.0, dtype=dtype, device="cuda") for _ in range(n)]
+        comm.exchange(xg, out, [[count] * n for _ in range(n)], send_off, recv_off, codec=codec)
+        torch.cuda.synchronize()
+        for d in range(n):
+            want = torch.full((2 * stride + 64,), 7.0, dtype=dtype)
+            for s in range(n):
+                block = xs[s][send_off[s][d]:send_off[s][d] + count]
+                want[recv_off[d][s]:recv_off[d][s] + count] = C.roundtrip(block.float(), codec, dtype).to(dtype)
+            assert torch.equal(out[d].cpu(), want), (shift, d)
+    comm.close()
+
+
+def test_exchange_in_place_all_to_all_of_odd_blocks():
+    n, count = 4, 3 * 512 + 1
+    comm = Communicator.local(n, arena_bytes=16 << 20)
+    xs = [torch.randn(n * count, generator=torch.Generator().manual_seed(r)) for r in range(n)]
+    bufs = [x.cuda() for x in xs]
+    comm.all_to_all(bufs, bufs, codec="none")
+    torch.cuda.synchronize()
+    for d in range(n):
+        assert torch.equal(bufs[d].cpu(), torch.cat([x[d * count:(d + 1) * count] for x in xs]))
+    comm.close()
