@@ -32,6 +32,7 @@
 
 #include "../rt/ccb_rt_internal.h"
 #include "ccb_device.cuh"
+#include "ccb_bits.cuh"
 
 namespace ccb {
 
@@ -43,170 +44,153 @@ constexpr int kLlHeader = 32;
 
 template <class T> struct LlTraits;
 template <> struct LlTraits<float> {
-  static constexpr int kExpBits = 8, kRestBytesPerTile = 3 * kLlTileElems;
-  static __device__ __forceinline__ uint32_t key(uint32_t b) { return (b >> 23) & 0xffu; }
-  static __device__ __forceinline__ uint32_t rest(uint32_t b) { return (b & 0x7fffffu) | ((b >> 31) << 23); }
-  static __device__ __forceinline__ uint32_t join(uint32_t k, uint32_t r) { return ((r >> 23) << 31) | (k << 23) | (r & 0x7fffffu); }
+  static constexpr int kExpShift = 23, kExpBits = 8, kRestBytesPerTile = 3 * kLlTileElems;
 };
 template <> struct LlTraits<__nv_bfloat16> {
-  static constexpr int kExpBits = 8, kRestBytesPerTile = kLlTileElems;
-  static __device__ __forceinline__ uint32_t key(uint32_t b) { return (b >> 7) & 0xffu; }
-  static __device__ __forceinline__ uint32_t rest(uint32_t b) { return (b & 0x7fu) | ((b >> 15) << 7); }
-  static __device__ __forceinline__ uint32_t join(uint32_t k, uint32_t r) { return ((r >> 7) << 15) | (k << 7) | (r & 0x7fu); }
+  static constexpr int kExpShift = 7, kExpBits = 8, kRestBytesPerTile = kLlTileElems;
 };
 template <> struct LlTraits<__half> {
-  static constexpr int kExpBits = 5, kRestBytesPerTile = kLlTileElems + 3 * kLlTileElems / 8;
-  static __device__ __forceinline__ uint32_t key(uint32_t b) { return (b >> 10) & 0x1fu; }
-  static __device__ __forceinline__ uint32_t rest(uint32_t b) { return (b & 0x3ffu) | ((b >> 15) << 10); }
-  static __device__ __forceinline__ uint32_t join(uint32_t k, uint32_t r) { return ((r >> 10) << 15) | (k << 10) | (r & 0x3ffu); }
+  static constexpr int kExpShift = 10, kExpBits = 5, kRestBytesPerTile = kLlTileElems + 3 * kLlTileElems / 8;
 };
 
 template <class T> __host__ __device__ constexpr size_t ll_slot_bytes() { return 32 + (size_t)kLlTileElems * sizeof(T); }
 
-// The 16 values of a lane as bit patterns (zero beyond `limit`), and back.
-template <class T>
-__device__ __forceinline__ void ll_load_bits(const T* base, size_t idx, size_t limit, uint32_t (&b)[16]) {
-  Raw16<T> raw;
-  load16_raw<T>(base, idx, limit, raw);
-#pragma unroll
-  for (int k = 0; k < (int)sizeof(T); ++k) {
-    const uint32_t w[4] = {raw.q[k].x, raw.q[k].y, raw.q[k].z, raw.q[k].w};
-    if constexpr (sizeof(T) == 4) {
-#pragma unroll
-      for (int i = 0; i < 4; ++i) b[4 * k + i] = w[i];
-    } else {
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        b[8 * k + 2 * i] = w[i] & 0xffffu;
-        b[8 * k + 2 * i + 1] = w[i] >> 16;
-      }
-    }
-  }
+// Byte `k` of four words as one word.
+__device__ __forceinline__ uint32_t bytes_of(uint32_t a, uint32_t b, uint32_t c, uint32_t d, int k) {
+  const uint32_t pair = (uint32_t)k | ((uint32_t)(k + 4) << 4);
+  return __byte_perm(__byte_perm(a, b, pair), __byte_perm(c, d, pair), 0x5410);
 }
-template <class T>
-__device__ __forceinline__ void ll_store_bits(T* base, size_t idx, size_t limit, const uint32_t (&b)[16]) {
-  T* p = base + idx;
-  if (idx + 16 <= limit && (reinterpret_cast<uintptr_t>(p) & 15) == 0) {
-    if constexpr (sizeof(T) == 4) {
+
+// Bit planes of the 16 small values (8 bits at most) of each lane of a warp. The values 4 r + g
+// (r = 0..3) of a lane share the word u[g], value 4 r + g in byte r; a 32 x 32 bit-matrix
+// transpose of u[g] across the warp leaves plane p of value 4 r + g in lane 8 r + p. The four
+// words of a lane are then the words 16 p + 4 r .. + 3 of the plane section: ONE 16-byte store
+// by the lanes whose plane exists. Four transposes of five shuffles replace 16 ballots and 16
+// selects of the storing lane per plane; the encoder issued about 700 instructions per block of
+// 512 values for four planes and issues about 180 now.
+__device__ __forceinline__ void store_planes(uint32_t* section, uint32_t (&u)[4], int planes, int lane) {
 #pragma unroll
-      for (int k = 0; k < 4; ++k) stg_stream(reinterpret_cast<char*>(p) + 16 * k, make_uint4(b[4 * k], b[4 * k + 1], b[4 * k + 2], b[4 * k + 3]));
-    } else {
+  for (int g = 0; g < 4; ++g) u[g] = transpose32(u[g], lane);
+  const int r = lane >> 3, p = lane & 7;
+  if (p < planes) *reinterpret_cast<uint4*>(section + 16 * p + 4 * r) = make_uint4(u[0], u[1], u[2], u[3]);
+}
+__device__ __forceinline__ void load_planes(const uint32_t* section, uint32_t (&u)[4], int planes, int lane) {
+  const int r = lane >> 3, p = lane & 7;
+  const uint4 q = p < planes ? *reinterpret_cast<const uint4*>(section + 16 * p + 4 * r) : make_uint4(0u, 0u, 0u, 0u);
+  u[0] = transpose32(q.x, lane);
+  u[1] = transpose32(q.y, lane);
+  u[2] = transpose32(q.z, lane);
+  u[3] = transpose32(q.w, lane);
+}
+// The words u[] of values held in pairs (value 2 k in the low half of w[k], byte `at` of each half), and back.
+__device__ __forceinline__ void planes_of_pairs(const uint32_t (&w)[8], int at, uint32_t (&u)[4]) {
+  u[0] = bytes_of(w[0], w[2], w[4], w[6], at);
+  u[1] = bytes_of(w[0], w[2], w[4], w[6], at + 2);
+  u[2] = bytes_of(w[1], w[3], w[5], w[7], at);
+  u[3] = bytes_of(w[1], w[3], w[5], w[7], at + 2);
+}
+__device__ __forceinline__ void pairs_of_planes(const uint32_t (&u)[4], uint32_t (&w)[8]) {
 #pragma unroll
-      for (int k = 0; k < 2; ++k)
-        stg_stream(reinterpret_cast<char*>(p) + 16 * k,
-                   make_uint4(b[8 * k] | (b[8 * k + 1] << 16), b[8 * k + 2] | (b[8 * k + 3] << 16),
-                              b[8 * k + 4] | (b[8 * k + 5] << 16), b[8 * k + 6] | (b[8 * k + 7] << 16)));
-    }
-  } else {
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      if (idx + i < limit) {
-        if constexpr (sizeof(T) == 4) reinterpret_cast<uint32_t*>(p)[i] = b[i];
-        else reinterpret_cast<unsigned short*>(p)[i] = (unsigned short)b[i];
-      }
-    }
+  for (int r = 0; r < 4; ++r) {   // bytes r of u[0], u[1] are the values 4 r, 4 r + 1
+    w[2 * r] = __byte_perm(u[0], u[1], (uint32_t)r | ((uint32_t)(r + 4) << 8)) & 0x00ff00ffu;
+    w[2 * r + 1] = __byte_perm(u[2], u[3], (uint32_t)r | ((uint32_t)(r + 4) << 8)) & 0x00ff00ffu;
   }
 }
 
-__device__ __forceinline__ uint4 pack16_bytes(const uint32_t (&v)[16], int shift) {
-  uint32_t w[4];
-#pragma unroll
-  for (int k = 0; k < 4; ++k)
-    w[k] = ((v[4 * k] >> shift) & 0xffu) | (((v[4 * k + 1] >> shift) & 0xffu) << 8) | (((v[4 * k + 2] >> shift) & 0xffu) << 16) |
-           (((v[4 * k + 3] >> shift) & 0xffu) << 24);
-  return make_uint4(w[0], w[1], w[2], w[3]);
-}
-__device__ __forceinline__ void unpack16_bytes(uint4 q, int shift, uint32_t (&v)[16]) {
-  const uint32_t w[4] = {q.x, q.y, q.z, q.w};
-#pragma unroll
-  for (int k = 0; k < 4; ++k)
-#pragma unroll
-    for (int i = 0; i < 4; ++i) v[4 * k + i] |= ((w[k] >> (8 * i)) & 0xffu) << shift;
-}
-
-// Word `idx` of a run of ballot words: every lane gets the same `word`; lane idx % 32
-// keeps it in hold[idx / 32], so that the run is written with one coalesced store per 32 words.
-template <int N>
-__device__ __forceinline__ void keep_word(uint32_t (&hold)[N], int idx, uint32_t word, int lane) {
-#pragma unroll
-  for (int h = 0; h < N; ++h)
-    if ((idx >> 5) == h && (idx & 31) == lane) hold[h] = word;
-}
-
+// The encoder is bound by memory once the planes come out of transposes: a tile's values are
+// requested while the tile before is packed, and one barrier per tile passes the widths round.
+// 32 Mi bf16 gradients through encode and decode: 177 us with ballots, 60 us so (B200; 235 MB
+// have to move, 35 us at 6.65 TB/s).
 template <class T>
 __global__ void __launch_bounds__(kLlThreads) lossless_encode_kernel(const T* __restrict__ in, size_t count, char* out, size_t ntiles) {
   using Tr = LlTraits<T>;
-  __shared__ uint32_t widths[kLlBlocksPerTile], kmins[kLlBlocksPerTile];
+  __shared__ uint2 info[2][kLlBlocksPerTile];   // (width, minimum) of each block, by parity of the tile
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  unsigned long long* total = reinterpret_cast<unsigned long long*>(out + 16);
-  for (size_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
+  const size_t lane_at = (size_t)warp * kWarpElems + (size_t)lane * kLaneElems;
+  unsigned long long produced = 0;
+  size_t t = blockIdx.x;
+  Wide16<T> next;
+  if (t < ntiles) load16_wide<T>(in, t * kLlTileElems + lane_at, count, next);
+  for (int parity = 0; t < ntiles; t += gridDim.x, parity ^= 1) {
     char* slot = out + kLlHeader + t * ll_slot_bytes<T>();
-    const size_t idx = t * kLlTileElems + (size_t)warp * kWarpElems + (size_t)lane * kLaneElems;
-    uint32_t b[16], key[16], rest[16];
-    ll_load_bits<T>(in, idx, count, b);
-    uint32_t kmin = 0xffu, kmax = 0u;
-#pragma unroll
-    for (int j = 0; j < 16; ++j) {
-      key[j] = Tr::key(b[j]);
-      rest[j] = Tr::rest(b[j]);
-      kmin = min(kmin, key[j]);
-      kmax = max(kmax, key[j]);
-    }
-    kmin = __reduce_min_sync(0xffffffffu, kmin);
-    kmax = __reduce_max_sync(0xffffffffu, kmax);
-    const int w = kmax == kmin ? 0 : 32 - __clz(kmax - kmin);
-    if (lane == 0) {
-      widths[warp] = (uint32_t)w;
-      kmins[warp] = kmin;
-    }
-    // sign and mantissa: raw byte planes (and for f16 three ballot planes)
-    char* restp = slot + 32;
+    const Wide16<T> raw = next;
+    if (t + gridDim.x < ntiles) load16_wide<T>(in, (t + gridDim.x) * kLlTileElems + lane_at, count, next);
+    char* restp = slot + 32 + warp * kWarpElems + lane * 16;
+    uint32_t u[4], kmin, kmax;
+    // sign and mantissa: raw byte planes (and for f16 three bit planes); then the exponents
     if constexpr (sizeof(T) == 4) {
+      uint32_t key[16], rest[16];
+      kmin = 0xffu, kmax = 0u;
 #pragma unroll
-      for (int p = 0; p < 3; ++p) stg(restp + (size_t)p * kLlTileElems + warp * kWarpElems + lane * 16, pack16_bytes(rest, 8 * p));
-    } else {
-      stg(restp + warp * kWarpElems + lane * 16, pack16_bytes(rest, 0));
-      if constexpr (Tr::kExpBits == 5) {
-        uint32_t hold[2] = {0u, 0u};
-#pragma unroll
-        for (int p = 0; p < 3; ++p)
-#pragma unroll
-          for (int j = 0; j < 16; ++j) keep_word(hold, p * 16 + j, __ballot_sync(0xffffffffu, (rest[j] >> (8 + p)) & 1u), lane);
-        uint32_t* hp = reinterpret_cast<uint32_t*>(restp + kLlTileElems) + warp * 48;
-        hp[lane] = hold[0];
-        if (lane < 16) hp[32 + lane] = hold[1];
+      for (int j = 0; j < 16; ++j) {
+        key[j] = (raw.w[j] >> 23) & 0xffu;
+        rest[j] = (raw.w[j] & 0x7fffffu) | ((raw.w[j] >> 8) & 0x800000u);
+        kmin = min(kmin, key[j]);
+        kmax = max(kmax, key[j]);
       }
-    }
-    __syncthreads();
-    uint32_t off = 0, all = 0;
 #pragma unroll
-    for (int k = 0; k < kLlBlocksPerTile; ++k) {
-      if (k < warp) off += widths[k];
-      all += widths[k];
+      for (int p = 0; p < 3; ++p)
+        stg(restp + (size_t)p * kLlTileElems, make_uint4(bytes_of(rest[0], rest[1], rest[2], rest[3], p), bytes_of(rest[4], rest[5], rest[6], rest[7], p),
+                                                         bytes_of(rest[8], rest[9], rest[10], rest[11], p), bytes_of(rest[12], rest[13], rest[14], rest[15], p)));
+      kmin = __reduce_min_sync(0xffffffffu, kmin);
+      kmax = __reduce_max_sync(0xffffffffu, kmax);
+#pragma unroll
+      for (int g = 0; g < 4; ++g) u[g] = bytes_of(key[g] - kmin, key[4 + g] - kmin, key[8 + g] - kmin, key[12 + g] - kmin, 0);
+    } else {
+      constexpr uint32_t kKey = ((1u << Tr::kExpBits) - 1u) * 0x00010001u;
+      constexpr uint32_t kMan = ((1u << Tr::kExpShift) - 1u) * 0x00010001u;
+      uint32_t key[8], rest[8], lo = kKey, hi = 0u;
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {   // two values at a time
+        key[k] = (raw.w[k] >> Tr::kExpShift) & kKey;
+        rest[k] = (raw.w[k] & kMan) | ((raw.w[k] >> (15 - Tr::kExpShift)) & (0x00010001u << Tr::kExpShift));
+        lo = __vminu2(lo, key[k]);
+        hi = __vmaxu2(hi, key[k]);
+      }
+      stg(restp, make_uint4(__byte_perm(rest[0], rest[1], 0x6420), __byte_perm(rest[2], rest[3], 0x6420),
+                            __byte_perm(rest[4], rest[5], 0x6420), __byte_perm(rest[6], rest[7], 0x6420)));
+      if constexpr (Tr::kExpBits == 5) {
+        uint32_t high[4];
+        planes_of_pairs(rest, 1, high);
+        store_planes(reinterpret_cast<uint32_t*>(slot + 32 + kLlTileElems) + warp * 48, high, 3, lane);
+      }
+      kmin = __reduce_min_sync(0xffffffffu, min(lo & 0xffffu, lo >> 16));
+      kmax = __reduce_max_sync(0xffffffffu, max(hi & 0xffffu, hi >> 16));
+#pragma unroll
+      for (int k = 0; k < 8; ++k) key[k] -= kmin * 0x00010001u;
+      planes_of_pairs(key, 0, u);
     }
+    const int w = 32 - __clz((int)(kmax - kmin));   // 0 when all exponents are equal
+    if (lane == 0) info[parity][warp] = make_uint2((uint32_t)w, kmin);
+    __syncthreads();   // the other parity's words were read before this barrier's predecessor
+    const uint2 mine = info[parity][lane & (kLlBlocksPerTile - 1)];
+    const uint32_t off = __reduce_add_sync(0xffffffffu, lane < warp ? mine.x : 0u);
     // exponent planes of this block, behind those of the blocks before it
-    uint32_t* ep = reinterpret_cast<uint32_t*>(slot + 32 + Tr::kRestBytesPerTile) + off * 16;
-    uint32_t hold[4] = {0u, 0u, 0u, 0u};
-    for (int p = 0; p < w; ++p) {
-#pragma unroll
-      for (int j = 0; j < 16; ++j) keep_word(hold, p * 16 + j, __ballot_sync(0xffffffffu, ((key[j] - kmin) >> p) & 1u), lane);
-    }
-#pragma unroll
-    for (int h = 0; h < 4; ++h)
-      if (h * 32 + lane < w * 16) ep[h * 32 + lane] = hold[h];
+    store_planes(reinterpret_cast<uint32_t*>(slot + 32 + Tr::kRestBytesPerTile) + off * 16, u, w, lane);
     if (warp == 0) {
+      const uint32_t all = __reduce_add_sync(0xffffffffu, lane < kLlBlocksPerTile ? mine.x : 0u);
       const uint32_t used = 32u + (uint32_t)Tr::kRestBytesPerTile + all * 64u;
       if (lane == 0) {
         *reinterpret_cast<uint32_t*>(slot) = used;
-        atomicAdd(total, (unsigned long long)used);
+        produced += used;
       }
       if (lane < kLlBlocksPerTile) {
-        reinterpret_cast<unsigned char*>(slot)[4 + lane] = (unsigned char)widths[lane];
-        reinterpret_cast<unsigned char*>(slot)[12 + lane] = (unsigned char)kmins[lane];
+        reinterpret_cast<unsigned char*>(slot)[4 + lane] = (unsigned char)mine.x;
+        reinterpret_cast<unsigned char*>(slot)[12 + lane] = (unsigned char)mine.y;
       }
       if (lane < 3) reinterpret_cast<uint32_t*>(slot)[5 + lane] = 0u;
     }
-    __syncthreads();  // widths[] is rewritten by the next tile
+  }
+  // The container's header was cleared before the launch; the byte count is summed over the
+  // CTAs (one atomic each, not one per tile), block 0 adds the header's own bytes and the rest.
+  if (threadIdx.x == 0) {
+    if (blockIdx.x == 0) {
+      reinterpret_cast<uint32_t*>(out)[0] = kLlMagic;
+      reinterpret_cast<uint32_t*>(out)[1] = sizeof(T) == 4 ? CCB_F32 : Tr::kExpBits == 8 ? CCB_BF16 : CCB_F16;
+      reinterpret_cast<unsigned long long*>(out)[1] = count;
+      produced += kLlHeader;
+    }
+    atomicAdd(reinterpret_cast<unsigned long long*>(out + 16), produced);
   }
 }
 
@@ -219,44 +203,59 @@ __global__ void __launch_bounds__(kLlThreads) lossless_decode_kernel(const char*
     const char* slot = in + kLlHeader + t * ll_slot_bytes<T>();
     const size_t idx = t * kLlTileElems + (size_t)warp * kWarpElems + (size_t)lane * kLaneElems;
     if (t * kLlTileElems + (size_t)warp * kWarpElems >= count) continue;
-    const unsigned char* hdr = reinterpret_cast<const unsigned char*>(slot);
-    uint32_t off = 0;
-    for (int k = 0; k < warp; ++k) off += hdr[4 + k];
-    const int w = hdr[4 + warp];
-    const uint32_t kmin = hdr[12 + warp];
-    uint32_t rest[16], key[16];
+    const uint4 head = *reinterpret_cast<const uint4*>(slot);       // used, widths 0-3, widths 4-7, minima 0-3
+    const uint32_t high_min = *reinterpret_cast<const uint32_t*>(slot + 16);
+    const char* restp = slot + 32 + warp * kWarpElems + lane * 16;
+    uint4 rq[sizeof(T) == 4 ? 3 : 1];
 #pragma unroll
-    for (int j = 0; j < 16; ++j) rest[j] = 0u, key[j] = 0u;
-    const char* restp = slot + 32;
+    for (int p = 0; p < (sizeof(T) == 4 ? 3 : 1); ++p) rq[p] = *reinterpret_cast<const uint4*>(restp + (size_t)p * kLlTileElems);
+    const uint32_t wsel = warp < 4 ? head.y : head.z, sh = 8 * (warp & 3);
+    const int w = (int)((wsel >> sh) & 0xffu);
+    const uint32_t kmin = ((warp < 4 ? head.w : high_min) >> sh) & 0xffu;
+    const uint32_t off = __dp4a(wsel & ((1u << sh) - 1u), 0x01010101u, warp < 4 ? 0u : __dp4a(head.y, 0x01010101u, 0u));
+    uint32_t u[4];
+    load_planes(reinterpret_cast<const uint32_t*>(slot + 32 + Tr::kRestBytesPerTile) + off * 16, u, w, lane);
+    Wide16<T> raw;
     if constexpr (sizeof(T) == 4) {
+      const uint32_t p0[4] = {rq[0].x, rq[0].y, rq[0].z, rq[0].w}, p1[4] = {rq[1].x, rq[1].y, rq[1].z, rq[1].w},
+                     p2[4] = {rq[2].x, rq[2].y, rq[2].z, rq[2].w};
 #pragma unroll
-      for (int p = 0; p < 3; ++p)
-        unpack16_bytes(*reinterpret_cast<const uint4*>(restp + (size_t)p * kLlTileElems + warp * kWarpElems + lane * 16), 8 * p, rest);
-    } else {
-      unpack16_bytes(*reinterpret_cast<const uint4*>(restp + warp * kWarpElems + lane * 16), 0, rest);
-      if constexpr (Tr::kExpBits == 5) {
-        const uint32_t* hp = reinterpret_cast<const uint32_t*>(restp + kLlTileElems) + warp * 48;
-#pragma unroll
-        for (int p = 0; p < 3; ++p)
-#pragma unroll
-          for (int j = 0; j < 16; ++j) rest[j] |= ((hp[p * 16 + j] >> lane) & 1u) << (8 + p);
+      for (int j = 0; j < 16; ++j) {
+        const uint32_t r = j & 3, low = __byte_perm(p0[j >> 2], p1[j >> 2], r | ((r + 4) << 4));    // bytes 0, 1
+        const uint32_t rest = __byte_perm(low, p2[j >> 2], 0x10u | ((r + 4) << 8)) & 0xffffffu;
+        const uint32_t key = ((u[j & 3] >> (8 * (j >> 2))) & 0xffu) + kmin;
+        raw.w[j] = ((rest << 8) & 0x80000000u) | (key << 23) | (rest & 0x7fffffu);
       }
-    }
-    const uint32_t* ep = reinterpret_cast<const uint32_t*>(slot + 32 + Tr::kRestBytesPerTile) + off * 16;
-    for (int p = 0; p < w; ++p) {
+    } else {
+      uint32_t key[8], rest[8];
+      pairs_of_planes(u, key);
+      const uint32_t q[4] = {rq[0].x, rq[0].y, rq[0].z, rq[0].w};
 #pragma unroll
-      for (int j = 0; j < 16; ++j) key[j] |= ((ep[p * 16 + j] >> lane) & 1u) << p;
-    }
-    uint32_t b[16];
+      for (int k = 0; k < 8; ++k) rest[k] = __byte_perm(q[k >> 1], 0u, k & 1 ? 0x4342 : 0x4140);
+      if constexpr (Tr::kExpBits == 5) {
+        uint32_t high[4], hp[8];
+        load_planes(reinterpret_cast<const uint32_t*>(slot + 32 + kLlTileElems) + warp * 48, high, 3, lane);
+        pairs_of_planes(high, hp);
 #pragma unroll
-    for (int j = 0; j < 16; ++j) b[j] = Tr::join(key[j] + kmin, rest[j]);
+        for (int k = 0; k < 8; ++k) rest[k] |= hp[k] << 8;
+      }
+      constexpr uint32_t kMan = ((1u << Tr::kExpShift) - 1u) * 0x00010001u;
+#pragma unroll
+      for (int k = 0; k < 8; ++k)
+        raw.w[k] = (((rest[k] << (15 - Tr::kExpShift)) & 0x80008000u) | (rest[k] & kMan)) | ((key[k] + kmin * 0x00010001u) << Tr::kExpShift);
+    }
     if constexpr (MODE == 1) {
-      uint32_t have[16];
-      ll_load_bits<T>(out, idx, count, have);
+      Wide16<T> have;
+      load16_wide<T>(out, idx, count, have);
+      float x[16], y[16];
+      wide16_to_f<T>(raw, x);
+      wide16_to_f<T>(have, y);
 #pragma unroll
-      for (int j = 0; j < 16; ++j) b[j] = elem_bits(Elem<T>::from_f(bits_to_f<T>(b[j]) + bits_to_f<T>(have[j])));
+      for (int j = 0; j < 16; ++j) x[j] += y[j];
+      store16_wide<T>(out, idx, count, x);
+    } else {
+      store16_wide<T>(out, idx, count, raw);
     }
-    ll_store_bits<T>(out, idx, count, b);
   }
 }
 
@@ -285,18 +284,18 @@ extern "C" int ccb_lossless_encode(int dtype, const void* in, uint64_t count, vo
     return CCB_ERR_ARG;
   }
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  struct { uint32_t magic, dtype; uint64_t count, used, zero; } h = {kLlMagic, (uint32_t)dtype, count, (uint64_t)kLlHeader, 0};
-  if (cudaMemcpyAsync(out, &h, sizeof(h), cudaMemcpyHostToDevice, s) != cudaSuccess) {
-    set_error("ccb_lossless_encode: header copy failed: %s", cudaGetErrorString(cudaGetLastError()));
+  if (dtype != CCB_F32 && dtype != CCB_BF16 && dtype != CCB_F16) return CCB_ERR_UNSUPPORTED;
+  // the kernel writes the header (a copy from the host would be a staged transfer per call) and
+  // adds up its byte count, which has to start at zero
+  if (cudaMemsetAsync(out, 0, kLlHeader, s) != cudaSuccess) {
+    set_error("ccb_lossless_encode: clearing the header failed: %s", cudaGetErrorString(cudaGetLastError()));
     return CCB_ERR_CUDA;
   }
   const size_t nt = ll_tiles(count);
-  if (nt == 0) return CCB_OK;
   const int g = ll_grid(nt);
   if (dtype == CCB_F32) lossless_encode_kernel<float><<<g, kLlThreads, 0, s>>>((const float*)in, count, (char*)out, nt);
   else if (dtype == CCB_BF16) lossless_encode_kernel<__nv_bfloat16><<<g, kLlThreads, 0, s>>>((const __nv_bfloat16*)in, count, (char*)out, nt);
-  else if (dtype == CCB_F16) lossless_encode_kernel<__half><<<g, kLlThreads, 0, s>>>((const __half*)in, count, (char*)out, nt);
-  else return CCB_ERR_UNSUPPORTED;
+  else lossless_encode_kernel<__half><<<g, kLlThreads, 0, s>>>((const __half*)in, count, (char*)out, nt);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {
     set_error("ccb_lossless_encode: %s", cudaGetErrorString(e));

@@ -46,6 +46,7 @@
 #include "../rt/ccb_rt_internal.h"
 #include "ccb/ccb_sz.h"
 #include "ccb_fastdiv.h"
+#include "ccb_bits.cuh"
 #include "ccb_reduce.cuh"
 
 namespace cg = cooperative_groups;
@@ -141,20 +142,6 @@ __device__ __forceinline__ TileCoord tile_coord(const SzArgs& a, unsigned int ti
 // words 8 * threadIdx.x .. +7 of the tile in shared memory (two 16-byte accesses). A packing
 // row is element e of all 32 lanes of a warp: row index 8 z + e.
 
-// Transposes the 32 x 32 bit matrix whose row i is the word held by lane i: afterwards
-// lane j holds column j (bit i of the result = bit j of lane i's input). Five exchange steps.
-__device__ __forceinline__ uint32_t transpose32(uint32_t x, int lane) {
-#pragma unroll
-  for (int s = 16; s >= 1; s >>= 1) {
-    const uint32_t m = s == 16 ? 0x0000ffffu : s == 8 ? 0x00ff00ffu : s == 4 ? 0x0f0f0f0fu : s == 2 ? 0x33333333u : 0x55555555u;
-    const uint32_t p = __shfl_xor_sync(0xffffffffu, x, s);
-    const bool up = (lane & s) != 0;
-    const uint32_t moved = up ? (p >> s) : (p << s);
-    const uint32_t keep = up ? ~m : m;
-    x = (x & keep) | (moved & ~keep);
-  }
-  return x;
-}
 __device__ __forceinline__ uint32_t bytesum(uint32_t v) { return __dp4a(v, 0x01010101u, 0u); }
 // True when every byte of w (each at most 32) is at most 8 / at most 16.
 __device__ __forceinline__ bool bytes_le8(uint32_t w) { return ((w + 0x77777777u) & 0x80808080u) == 0; }
