@@ -21,6 +21,9 @@ def _decl():
     L.ccb_sz_capacity.restype = ctypes.c_uint64
     L.ccb_sz_compress.argtypes = [c_vp, c_int, c_int, c_int, c_f, c_vp, c_vp, c_vp]
     L.ccb_sz_decompress.argtypes = [c_vp, c_int, c_int, c_int, c_f, c_vp, c_vp]
+    L.ccb_sz_container_scan.argtypes = [c_vp, c_vp, ctypes.c_uint64, c_vp, c_vp]
+    L.ccb_sz_container_pack.argtypes = [c_vp, c_vp, c_int, c_int, c_int, c_f, ctypes.c_uint64, c_vp, c_vp]
+    L.ccb_sz_container_unpack.argtypes = [c_vp, c_vp, ctypes.c_uint64, c_vp, c_vp]
     L.ccb_sz_collective.argtypes = [c_vp, ctypes.POINTER(c_vp), ctypes.POINTER(c_vp), c_int, c_int, c_int, c_f, c_int, c_vp, c_vp]
     return L
 
@@ -87,11 +90,25 @@ MAGIC, VERSION = 0x5A534343, 2
 GROUP_STRIDE, GROUP_HEADER, HEADER_BYTES = 66112, 32, 40
 
 
+def _by_kernel(t: torch.Tensor, align: int) -> bool:
+    return t.is_cuda and t.dtype == torch.uint8 and t.is_contiguous() and t.data_ptr() % align == 0
+
+
 def to_container(buf: torch.Tensor, shape, eb: float) -> torch.Tensor:
     """Packs the group slots of `buf` (as returned by compress) into one contiguous uint8
-    tensor on the same device. Plain tensor operations, no extra kernel."""
+    tensor on the same device: a scan and a copy kernel for a GPU buffer (with one read-back
+    of the total between them), plain tensor operations for a host buffer."""
     nz, ny, nx = shape
     ngroups = buf.numel() // GROUP_STRIDE
+    if _by_kernel(buf, 16) and ngroups and buf.numel() == ngroups * GROUP_STRIDE:
+        with torch.cuda.device(buf.device):
+            L = _decl()
+            offsets = torch.empty(ngroups + 2, dtype=torch.int64, device=buf.device)
+            _check(L.ccb_sz_container_scan(buf.data_ptr(), None, ngroups, offsets.data_ptr(), _stream()))
+            total = int(offsets[ngroups].item())
+            blob = torch.empty(HEADER_BYTES + 4 * ngroups + total, dtype=torch.uint8, device=buf.device)
+            _check(L.ccb_sz_container_pack(buf.data_ptr(), offsets.data_ptr(), nx, ny, nz, eb, ngroups, blob.data_ptr(), _stream()))
+        return blob
     slots = buf.view(ngroups, GROUP_STRIDE)
     sizes = slots[:, :GROUP_HEADER].contiguous().view(torch.int32).to(torch.int64).sum(dim=1) + GROUP_HEADER
     keep = torch.arange(GROUP_STRIDE, device=buf.device).unsqueeze(0) < sizes.unsqueeze(1)
@@ -116,6 +133,19 @@ def from_container(blob: torch.Tensor):
     nbytes = head[32:40].view(torch.int64).item()
     if ngroups * GROUP_STRIDE != capacity((nz, ny, nx)):
         raise ValueError("container header does not match its dimensions")
+    if _by_kernel(blob, 4) and ngroups and blob.numel() >= HEADER_BYTES + 4 * ngroups:
+        if blob.numel() - HEADER_BYTES - 4 * ngroups != nbytes:
+            raise ValueError("container payload is damaged")
+        with torch.cuda.device(blob.device):
+            L = _decl()
+            offsets = torch.empty(ngroups + 2, dtype=torch.int64, device=blob.device)
+            _check(L.ccb_sz_container_scan(None, blob.data_ptr() + HEADER_BYTES, ngroups, offsets.data_ptr(), _stream()))
+            total, largest = offsets[ngroups:].tolist()
+            if total != nbytes or largest > GROUP_STRIDE:
+                raise ValueError("container payload is damaged")
+            buf = torch.empty(ngroups * GROUP_STRIDE, dtype=torch.uint8, device=blob.device)
+            _check(L.ccb_sz_container_unpack(blob.data_ptr() + HEADER_BYTES + 4 * ngroups, offsets.data_ptr(), ngroups, buf.data_ptr(), _stream()))
+        return buf, (nz, ny, nx), eb
     sizes = blob[HEADER_BYTES:HEADER_BYTES + 4 * ngroups].contiguous().view(torch.int32).to(torch.int64)
     payload = blob[HEADER_BYTES + 4 * ngroups:]
     if payload.numel() != nbytes or int(sizes.sum().item()) != nbytes or int(sizes.max().item()) > GROUP_STRIDE:

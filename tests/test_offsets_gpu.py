@@ -1,10 +1,11 @@
-"""Blocks at odd offsets of a buffer: the addresses at which the 32-byte accesses have to
-shift, rotate or give way."""
+"""Blocks at odd offsets of a buffer, and the packed container by kernels: the addresses at
+which the 32-byte accesses have to shift, rotate or give way."""
 import pytest
 import torch
 
 from ccbench_b200 import Communicator
 from ccbench_b200.ops import codecs as C
+from ccbench_b200.ops import sz
 
 pytestmark = pytest.mark.gpu
 
@@ -43,3 +44,28 @@ def test_exchange_in_place_all_to_all_of_odd_blocks():
     for d in range(n):
         assert torch.equal(bufs[d].cpu(), torch.cat([x[d * count:(d + 1) * count] for x in xs]))
     comm.close()
+
+
+@pytest.mark.parametrize("shape", [(1, 1, 1), (9, 7, 33), (17, 40, 130), (64, 64, 72)])
+@pytest.mark.parametrize("shift", [0, 4, 8, 12])
+def test_container_by_kernel_is_the_container_of_the_host_codec(shape, shift):
+    g = torch.Generator().manual_seed(sum(shape))
+    f = torch.randn(shape, generator=g).cumsum(2)
+    eb = 1e-3
+    buf, _ = sz.compress(f.cuda(), eb)
+    blob = sz.to_container(buf, shape, eb)
+    assert torch.equal(blob.cpu(), torch.from_numpy(sz.encode_cpu(f.numpy(), eb)))
+    # a container that starts at another alignment (part of a larger message), and one on the host
+    room = torch.zeros(blob.numel() + 16, dtype=torch.uint8, device="cuda")
+    room[shift:shift + blob.numel()] = blob
+    for view in (room[shift:shift + blob.numel()], blob.cpu()):
+        again, s2, e2 = sz.from_container(view)
+        assert tuple(s2) == shape and e2 == torch.tensor(eb, dtype=torch.float32).item()
+        slots = buf.view(-1, sz.GROUP_STRIDE).cpu()
+        for got, had in zip(again.view(-1, sz.GROUP_STRIDE).cpu(), slots):
+            used = int(had[:32].view(torch.int32).sum()) + 32
+            assert torch.equal(got[:used], had[:used]) and not got[used:].any()
+    bad = blob.clone()
+    bad[sz.HEADER_BYTES:sz.HEADER_BYTES + 4].view(torch.int32).add_(16)
+    with pytest.raises(ValueError):
+        sz.from_container(bad)
