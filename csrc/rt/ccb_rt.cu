@@ -14,7 +14,9 @@
 #include <unistd.h>
 
 #include <atomic>
+#include <map>
 #include <mutex>
+#include <tuple>
 #include <string>
 #include <vector>
 
@@ -236,14 +238,27 @@ uint32_t next_epoch(ccb_comm* c) {
   return c->epoch;
 }
 
-// How many CTAs per rank may be launched so that every CTA of every local rank is
-// resident at once (CTAs spin on flags written by same-numbered CTAs elsewhere).
-int grid_cap(ccb_comm* c, const void* kernel, int threads) {
+// The occupancy of a kernel does not change, and asking for it costs more than the rest of a
+// small call's host work: it is asked once per kernel, block size and device of the process.
+static int resident_ctas(const void* kernel, int threads, int device) {
+  static std::mutex lock;
+  static std::map<std::tuple<const void*, int, int>, int> known;
+  std::lock_guard<std::mutex> hold(lock);
+  auto at = known.find(std::make_tuple(kernel, threads, device));
+  if (at != known.end()) return at->second;
   int per_sm = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, 0) != cudaSuccess || per_sm < 1) {
     (void)cudaGetLastError();
-    per_sm = 1;
+    return 1;   // not kept: the next call asks again
   }
+  known[std::make_tuple(kernel, threads, device)] = per_sm;
+  return per_sm;
+}
+
+// How many CTAs per rank may be launched so that every CTA of every local rank is
+// resident at once (CTAs spin on flags written by same-numbered CTAs elsewhere).
+int grid_cap(ccb_comm* c, const void* kernel, int threads) {
+  int per_sm = resident_ctas(kernel, threads, c->device);
   if (per_sm > 2) per_sm = 2;
   int cap = per_sm * c->num_sms / c->nlocal;
   if (cap > CCB_MAX_CTAS) cap = CCB_MAX_CTAS;
@@ -891,6 +906,10 @@ static const void* reduce_fn(int dtype, int codec, int shape) {
   if (shape == kOneShot) return CCB_DISPATCH_TC(dtype, codec, (reinterpret_cast<const void*>(&reduce_kernel<TT, CC, kOneShot>)));
   return CCB_DISPATCH_TC(dtype, codec, (reinterpret_cast<const void*>(&reduce_kernel<TT, CC, kTwoShot>)));
 }
+static const void* solo_fn(int dtype, int codec, bool ef) {
+  if (ef) return CCB_DISPATCH_TC(dtype, codec, (reinterpret_cast<const void*>(&solo_kernel<TT, CC, true>)));
+  return CCB_DISPATCH_TC(dtype, codec, (reinterpret_cast<const void*>(&solo_kernel<TT, CC, false>)));
+}
 static const void* exchange_fn(int dtype, int codec) {
   return CCB_DISPATCH_TC(dtype, codec, (reinterpret_cast<const void*>(&exchange_kernel<TT, CC>)));
 }
@@ -987,6 +1006,34 @@ static int reduce_launch(ccb_comm* c, const void* const* send, void* const* recv
   return launch(c, fn, ctas, &a, stream);
 }
 
+// An all-reduce of one rank (see solo_kernel): as many CTAs as are resident at once.
+static int solo_launch(ccb_comm* c, const void* const* send, void* const* recv, float* const* ef, uint64_t count, int dtype, int codec,
+                       cudaStream_t stream) {
+  const void* fn = solo_fn(dtype, codec, ef && ef[0]);
+  if (!fn) {
+    set_error("unsupported dtype %d / codec %d", dtype, codec);
+    return CCB_ERR_UNSUPPORTED;
+  }
+  ReduceArgs a;
+  memset(&a, 0, sizeof(a));
+  a.c.nranks = 1;
+  a.send[0] = send[0];
+  a.recv[0] = recv[0];
+  a.ef[0] = ef ? ef[0] : nullptr;
+  a.count = count;
+  const size_t blocks = (count + (size_t)kSoloThreads * kLaneElems - 1) / ((size_t)kSoloThreads * kLaneElems);
+  size_t cap = (size_t)c->num_sms * resident_ctas(fn, kSoloThreads, c->device);
+  if (c->max_ctas > 0 && cap > (size_t)c->max_ctas) cap = (size_t)c->max_ctas;
+  void* params[] = {&a};
+  cudaError_t e = cudaLaunchKernel(fn, dim3((unsigned)(blocks < cap ? blocks : cap)), dim3(kSoloThreads), params, 0, stream);
+  if (e != cudaSuccess) {
+    set_error("kernel launch failed: %s", cudaGetErrorString(e));
+    return CCB_ERR_CUDA;
+  }
+  count_launch();
+  return CCB_OK;
+}
+
 int nvls_all_reduce(ccb_comm* c, const void* const* send, void* const* recv, uint64_t count, int dtype, int op,
                     cudaStream_t stream) {
   if (!c->mc_arena || c->nlocal != 1) {
@@ -1052,6 +1099,7 @@ extern "C" int ccb_all_reduce(ccb_comm* c, const void* const* send, void* const*
   }
   const int n = c->nranks;
   const size_t es = elem_size(dtype);
+  if (n == 1 && algo != CCB_ALGO_NVLS) return solo_launch(c, send, recv, ef, count, dtype, codec, stream);
   if (algo == CCB_ALGO_AUTO) {
     // One-shot has one exchange instead of two (about 10 us less latency) but every rank
     // sends its whole message to every peer: (n-1) * S wire bytes against 2(n-1)/n * S.

@@ -1,0 +1,50 @@
+"""An all-reduce of one rank (its own kernel) against the restated algorithms: partial and whole
+units, more units than resident warps, views at odd offsets, with and without error feedback."""
+import os
+
+import pytest
+import torch
+
+from ccbench_b200 import Communicator
+from ccbench_b200.ops import codecs as C
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def comm():
+    c = Communicator.create(0, 1, f"solo{os.getpid()}", arena_bytes=32 << 20)
+    yield c
+    c.close()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("codec", ["int8", "int8_g256", "fp8", "int4", "none"])
+@pytest.mark.parametrize("count", [1, 511, 512, 4096 + 17, 148 * 5 * 8 * 512 + 512 * 3 + 5])
+def test_one_rank_matches_the_restatement(comm, dtype, codec, count):
+    x = (torch.randn(count + 3, generator=torch.Generator().manual_seed(count)) * 3).to(dtype)
+    xg = x.cuda()
+    for algo, shift in (("twoshot", 0), ("oneshot", 1), ("ring", 0), ("tree", 3)):
+        send = xg[shift:shift + count]
+        out = torch.zeros(count + 2, dtype=dtype, device="cuda")
+        comm.all_reduce(send, out[1:1 + count], codec=codec, algo=algo)
+        torch.cuda.synchronize()
+        want = C.simulate_all_reduce([x[shift:shift + count]], codec, algo, dtype)
+        assert torch.equal(out[1:1 + count].float().cpu(), want), (algo, shift)
+        assert out[0] == 0 and out[-1] == 0
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("codec", ["int8", "fp8"])
+def test_one_rank_error_feedback_in_place(comm, dtype, codec):
+    count = 3 * 512 + 40
+    x = torch.randn(count, generator=torch.Generator().manual_seed(5)).to(dtype)
+    buf, ef = x.cuda(), torch.zeros(count, device="cuda")
+    want_ef = [torch.zeros(count)]
+    for _ in range(3):
+        buf.copy_(x)
+        comm.all_reduce(buf, codec=codec, error_feedback=ef)
+        want = C.simulate_all_reduce([x], codec, "twoshot", dtype, ef=want_ef)
+        torch.cuda.synchronize()
+        assert torch.equal(buf.float().cpu(), want)
+        assert torch.equal(ef.cpu(), want_ef[0])
