@@ -8,6 +8,7 @@ AlltoAll serves in MoE training, with per-destination fp8 compression."""
 from __future__ import annotations
 
 import ctypes
+import functools
 from dataclasses import dataclass
 
 import torch
@@ -42,6 +43,7 @@ def plan_route(expert_ids: torch.Tensor, gates: torch.Tensor, nranks: int) -> Ro
                  gates.reshape(-1).float().contiguous(), counts, k)
 
 
+@functools.cache   # the declarations once, not on every call
 def _decl():
     L = lib()
     vp, pp, up = ctypes.c_void_p, ctypes.POINTER(ctypes.c_void_p), ctypes.POINTER(ctypes.c_uint64)
