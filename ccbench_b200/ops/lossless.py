@@ -10,6 +10,7 @@ measurement of scripts/intermediate/test_dietgpu_compress.py."""
 from __future__ import annotations
 
 import ctypes
+import functools
 
 import numpy as np
 
@@ -135,12 +136,13 @@ def used_bytes_np(buf: np.ndarray) -> int:
 
 
 # ------------------------------------------------------------------ GPU entry points --
+@functools.cache   # the declarations once, not on every call
 def _gpu():
     import torch
 
     from .. import constants as K
     from .._lib import lib
-    from ..comm import _DTYPES, _check
+    from ..comm import _DTYPES, _check, current_stream_ptr
 
     L = lib()
     L.ccb_lossless_max_bytes.restype = ctypes.c_uint64
@@ -148,29 +150,29 @@ def _gpu():
     L.ccb_lossless_encode.argtypes = [ctypes.c_int, ctypes.c_void_p, ctypes.c_uint64, ctypes.c_void_p, ctypes.c_void_p]
     L.ccb_lossless_decode.argtypes = [ctypes.c_int, ctypes.c_void_p, ctypes.c_uint64, ctypes.c_void_p, ctypes.c_int, ctypes.c_void_p]
     L.ccb_lossless_used_bytes.argtypes = [ctypes.c_void_p, ctypes.POINTER(ctypes.c_uint64), ctypes.c_void_p]
-    return torch, L, _DTYPES, _check
+    return torch, L, _DTYPES, _check, current_stream_ptr
 
 
 def encode(x):
     """x: contiguous CUDA tensor (float32, bfloat16 or float16) -> container (uint8 CUDA tensor)."""
-    torch, L, DT, check = _gpu()
+    torch, L, DT, check, stream = _gpu()
     out = torch.empty(int(L.ccb_lossless_max_bytes(DT[x.dtype], x.numel())), dtype=torch.uint8, device=x.device)
-    check(L.ccb_lossless_encode(DT[x.dtype], x.data_ptr(), x.numel(), out.data_ptr(), torch.cuda.current_stream().cuda_stream))
+    check(L.ccb_lossless_encode(DT[x.dtype], x.data_ptr(), x.numel(), out.data_ptr(), stream()))
     return out
 
 
 def decode(comp, count: int, dtype, out=None, accumulate: bool = False):
-    torch, L, DT, check = _gpu()
+    torch, L, DT, check, stream = _gpu()
     out = torch.empty(count, dtype=dtype, device=comp.device) if out is None else out
     check(L.ccb_lossless_decode(DT[dtype], comp.data_ptr(), count, out.data_ptr(), 1 if accumulate else 0,
-                                torch.cuda.current_stream().cuda_stream))
+                                stream()))
     return out
 
 
 def used_bytes(comp) -> int:
-    torch, L, DT, check = _gpu()
+    torch, L, DT, check, stream = _gpu()
     v = ctypes.c_uint64(0)
-    check(L.ccb_lossless_used_bytes(comp.data_ptr(), ctypes.byref(v), torch.cuda.current_stream().cuda_stream))
+    check(L.ccb_lossless_used_bytes(comp.data_ptr(), ctypes.byref(v), stream()))
     return int(v.value)
 
 

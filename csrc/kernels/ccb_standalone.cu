@@ -19,6 +19,7 @@ namespace ccb {
 
 constexpr int kSaThreads = 256;
 
+// User values go in 32-byte accesses, at whatever offset a chunk starts (chunks of an odd count).
 // blockIdx.y selects one of several equal chunks: chunk c reads in + c * in_stride elements
 // and writes wire + c * wire_stride bytes, so that a chunked buffer is one launch.
 template <class T, class C>
@@ -31,8 +32,10 @@ __global__ void __launch_bounds__(kSaThreads) encode_kernel(const T* __restrict_
   const int lane = threadIdx.x & 31;
   for (size_t u = warp; u < units; u += nwarps) {
     const size_t idx = u * kWarpElems + (size_t)lane * kLaneElems;
+    Wide16<T> raw;
+    load16_wide<T, true>(in, idx, count, raw);
     float v[16];
-    load16<T>(in, idx, count, v);
+    wide16_to_f<T>(raw, v);
     typename C::Packet pk;
     C::encode(v, pk);
     C::store(wire, pad, idx, pk);
@@ -56,12 +59,14 @@ __global__ void __launch_bounds__(kSaThreads) decode_kernel(const char* wire, si
     float d[16];
     C::decode(pk, d);
     if (MODE == 1) {
+      Wide16<T> raw;
+      load16_wide<T, true>(out, idx, count, raw);
       float a[16];
-      load16<T>(out, idx, count, a);
+      wide16_to_f<T>(raw, a);
 #pragma unroll
       for (int i = 0; i < 16; ++i) d[i] += a[i];
     }
-    store16<T>(out, idx, count, d);
+    store16_wide<T, true>(out, idx, count, d);
   }
 }
 
@@ -75,12 +80,15 @@ __global__ void __launch_bounds__(kSaThreads) accumulate_kernel(const T* __restr
   for (size_t u = warp; u < units; u += nwarps) {
     const size_t idx = u * kWarpElems + (size_t)lane * kLaneElems;
     if (idx >= count) continue;
+    Wide16<T> ra, rb;
+    load16_wide<T>(src, idx, count, ra);
+    load16_wide<T>(inout, idx, count, rb);
     float a[16], b[16];
-    load16<T>(src, idx, count, a);
-    load16<T>(inout, idx, count, b);
+    wide16_to_f<T>(ra, a);
+    wide16_to_f<T>(rb, b);
 #pragma unroll
     for (int i = 0; i < 16; ++i) b[i] += a[i];
-    store16<T>(inout, idx, count, b);
+    store16_wide<T>(inout, idx, count, b);
   }
 }
 
