@@ -4,16 +4,18 @@ must match the kernel's exactly."""
 from __future__ import annotations
 
 import ctypes
+import functools
 
 import numpy as np
 import torch
 
 from .._lib import lib
-from ..comm import Communicator, _check
+from ..comm import Communicator, _check, current_stream_ptr
 
 TX, TY, TZ = 32, 8, 8
 
 
+@functools.cache   # the declarations once, not on every call
 def _decl():
     L = lib()
     c_vp, c_int, c_f = ctypes.c_void_p, ctypes.c_int, ctypes.c_float
@@ -29,7 +31,7 @@ def _decl():
 
 
 def _stream():
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    return current_stream_ptr()
 
 
 def capacity(shape) -> int:

@@ -43,6 +43,10 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include <map>
+#include <mutex>
+#include <utility>
+
 #include "../rt/ccb_rt_internal.h"
 #include "ccb/ccb_sz.h"
 #include "ccb_fastdiv.h"
@@ -120,6 +124,30 @@ __device__ __forceinline__ void tma_load_3d(void* smem_dst, const CUtensorMap* m
       ::"r"(smem_u32(smem_dst)), "l"(map), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar)) : "memory");
 }
 
+// One word into the shared memory of CTA `rank` of the cluster, at the place that `dst` has in
+// this CTA's; its arrival counts 4 bytes on that CTA's mbarrier.
+__device__ __forceinline__ void st_async_u32(uint32_t* dst, uint64_t* bar, uint32_t rank, uint32_t v) {
+  asm volatile(
+      "{\n.reg .b32 a, b;\n"
+      "mapa.shared::cluster.u32 a, %0, %2;\n"
+      "mapa.shared::cluster.u32 b, %1, %2;\n"
+      "st.async.shared::cluster.mbarrier::complete_tx::bytes.u32 [a], %3, [b];\n}\n"
+      ::"r"(smem_u32(dst)), "r"(smem_u32(bar)), "r"(rank), "r"(v) : "memory");
+}
+// mbar_wait for words that other CTAs of the cluster wrote.
+__device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity) {
+  for (uint32_t spin = 0; spin < (1u << 26); ++spin) {
+    uint32_t done;
+    asm volatile(
+        "{\n.reg .pred p;\n"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
+        "selp.u32 %0, 1, 0, p;\n}\n"
+        : "=r"(done) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+    if (done) return true;
+  }
+  return false;
+}
+
 struct TileCoord { int x0, y0, z0; };
 __device__ __forceinline__ TileCoord tile_coord(const SzArgs& a, unsigned int tile) {
   TileCoord t;
@@ -147,12 +175,12 @@ __device__ __forceinline__ uint32_t bytesum(uint32_t v) { return __dp4a(v, 0x010
 __device__ __forceinline__ bool bytes_le8(uint32_t w) { return ((w + 0x77777777u) & 0x80808080u) == 0; }
 __device__ __forceinline__ bool bytes_le16(uint32_t w) { return ((w + 0x6f6f6f6fu) & 0x80808080u) == 0; }
 
-// Bit-planes of four rows: `W` holds their widths (one byte each), `off` is the word offset
-// of the first row's planes. With all widths <= 8 the four rows share ONE bit-matrix
-// transpose (lane 8 r + j ends up with plane j of row r); widths up to 16 take two, wider
-// rows one transpose each. The byte layout does not depend on which way was taken.
+// Bit-planes of four rows with widths of up to 32 bits: `W` holds the widths (one byte each),
+// `off` is the word offset of the first row's planes. Widths up to 16 take two bit-matrix
+// transposes, wider rows one each. (Up to 8 bits, by far the most common, the four rows share
+// one transpose: see the callers.) The byte layout does not depend on which way was taken.
 template <bool kStore>
-__device__ __forceinline__ void planes4(uint32_t (&u)[4], uint32_t W, uint32_t off, uint32_t* words, int lane) {
+__device__ __forceinline__ void wide_planes4(uint32_t (&u)[4], uint32_t W, uint32_t off, uint32_t* words, int lane) {
   auto pass = [&](int bits, int first_row, int rows) {   // rows * bits == 32
     const int rr = lane / bits, jj = lane % bits, row = first_row + rr;
     const uint32_t w = (W >> (8 * row)) & 0xffu;
@@ -168,9 +196,7 @@ __device__ __forceinline__ void planes4(uint32_t (&u)[4], uint32_t W, uint32_t o
       for (int r2 = 0; r2 < rows; ++r2) u[first_row + r2] = bits == 32 ? U : (U >> (bits * r2)) & ((1u << bits) - 1u);
     }
   };
-  if (bytes_le8(W)) {
-    pass(8, 0, 4);
-  } else if (bytes_le16(W)) {
+  if (bytes_le16(W)) {
     pass(16, 0, 2);
     pass(16, 2, 2);
   } else {
@@ -186,7 +212,8 @@ constexpr float kRoundMagic = 12582912.f;   // 1.5 * 2^23: adding and subtractin
 // With `recon` set, the decoder's view of the tile (q * step, or the raw values of a raw
 // tile) is also written to its place in that field: the sender's own copy of what every
 // receiver will decode, without a decode pass.
-__device__ __forceinline__ uint32_t pack_tile(float* vals, unsigned char* pk, int* s_tot, const SzArgs& a,
+// `failed` (any thread, with sync.fail set): the tile's copy never came; every thread gets 0.
+__device__ __forceinline__ uint32_t pack_tile(float* vals, unsigned char* pk, int* s_tot, const SzArgs& a, bool failed, const CtaSync& sync,
                                               float* recon = nullptr, TileCoord tc = TileCoord{0, 0, 0}) {
   const int lane = threadIdx.x & 31, z = threadIdx.x >> 5;
   int4* q4 = reinterpret_cast<int4*>(vals) + 2 * threadIdx.x;
@@ -196,28 +223,45 @@ __device__ __forceinline__ uint32_t pack_tile(float* vals, unsigned char* pk, in
     x[0] = v0.x; x[1] = v0.y; x[2] = v0.z; x[3] = v0.w; x[4] = v1.x; x[5] = v1.y; x[6] = v1.z; x[7] = v1.w;
   }
   int q[8];
-  bool bad = false;
   const float half = 0.5f * a.two_eb;
+  // s = x / step; adding 1.5 * 2^23 rounds it to nearest even and leaves the integer in the low
+  // mantissa bits, subtracting it again gives it as a float; diff = x - q * step with the very
+  // product that the decoder computes (every operation rounded by itself: no fused multiply-add).
+  // (As packed pairs, mul.rn.f32x2 and add.rn.f32x2, the operations came out fused all the same.)
+  float smax = 0.f;
+  bool far = false;
 #pragma unroll
   for (int e = 0; e < 8; ++e) {
-    const float s = __fmul_rn(x[e], a.inv_two_eb);
-    bad |= !(fabsf(s) < kQMax);  // also catches NaN / Inf
-    float rf = __fadd_rn(__fadd_rn(s, kRoundMagic), -kRoundMagic);
-    const float diff = __fsub_rn(x[e], __fmul_rn(rf, a.two_eb));  // against the decoder's own product (no FMA)
-    // Nearly always |diff| <= step / 2 < eb: the value sits on the nearest grid point and the
-    // bound holds, nothing to correct or to re-check. The correction runs only when some lane
-    // of the warp needs it (NaN counts as needing it), with the same result either way.
-    if (__any_sync(0xffffffffu, !(fabsf(diff) <= half))) {
+    const float s = __fmul_rn(x[e], a.inv_two_eb), r = __fadd_rn(s, kRoundMagic);
+    const float diff = __fsub_rn(x[e], __fmul_rn(__fadd_rn(r, -kRoundMagic), a.two_eb));
+    smax = fmaxf(smax, fabsf(s));
+    far |= !(fabsf(diff) <= half);
+    q[e] = __float_as_int(r) - __float_as_int(kRoundMagic);
+  }
+  bool bad = failed || !(smax < kQMax);   // infinities too; a NaN is caught below (its difference is NaN)
+  // Nearly always |diff| <= step / 2 < eb: the value sits on the nearest grid point and the
+  // bound holds, nothing to correct or to re-check. The correction runs only when some lane
+  // of the warp needs it (NaN counts as needing it), with the same result either way.
+  if (__any_sync(0xffffffffu, far)) {
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      const float s = __fmul_rn(x[e], a.inv_two_eb);
+      bad |= !(fabsf(s) < kQMax);
+      float rf = __fadd_rn(__fadd_rn(s, kRoundMagic), -kRoundMagic);
+      const float diff = __fsub_rn(x[e], __fmul_rn(rf, a.two_eb));
       rf += diff > half ? 1.f : 0.f;                              // fp32 rounding picked the farther grid point
       rf -= -diff > half ? 1.f : 0.f;
       // The grid step is a shade under 2 eb, which absorbs the rounding of q * step for
       // |q| < 2^13. Beyond that a value can fall between two grid points that are both more
       // than eb away: such a tile is stored raw, so the bound always holds.
       bad |= fabsf(__fsub_rn(x[e], __fmul_rn(rf, a.two_eb))) > a.eb;
+      q[e] = (int)rf;
     }
-    q[e] = (int)rf;
   }
-  const bool raw_tile = __syncthreads_or(bad);
+  q4[0] = make_int4(q[0], q[1], q[2], q[3]);
+  q4[1] = make_int4(q[4], q[5], q[6], q[7]);
+  const bool raw_tile = __syncthreads_or(bad);   // and the barrier between the codes and their readers
+  if (raw_tile && sync.fail) return 0;           // the tile never arrived
   if (recon) {
     const int gx = tc.x0 + 8 * (lane & 3), gy = tc.y0 + (lane >> 2), gz = tc.z0 + z;
     if (gy < a.ny && gz < a.nz) {
@@ -235,16 +279,14 @@ __device__ __forceinline__ uint32_t pack_tile(float* vals, unsigned char* pk, in
       }
     }
   }
-  if (raw_tile) {  // raw tile: marker + the fp32 values
+  if (raw_tile) {  // raw tile: marker + the fp32 values, each thread its own eight
     for (int i = threadIdx.x; i < kRows; i += kSzThreads) pk[i] = (i == 0) ? 255 : 0;
-    float* raw = reinterpret_cast<float*>(pk + kRows);
-    for (int i = threadIdx.x; i < kTileVals; i += kSzThreads) raw[i] = vals[i];
+    float4* raw = reinterpret_cast<float4*>(pk + kRows) + 2 * threadIdx.x;
+    raw[0] = make_float4(x[0], x[1], x[2], x[3]);
+    raw[1] = make_float4(x[4], x[5], x[6], x[7]);
     __syncthreads();
     return kRows + kTileVals * 4;
   }
-  q4[0] = make_int4(q[0], q[1], q[2], q[3]);
-  q4[1] = make_int4(q[4], q[5], q[6], q[7]);
-  __syncthreads();
   // Lorenzo residual = the three first differences, in any order: z through shared memory
   // (plane z - 1 belongs to the warp below), y through the lane four below, x in registers.
   if (z > 0) {
@@ -258,43 +300,68 @@ __device__ __forceinline__ uint32_t pack_tile(float* vals, unsigned char* pk, in
   }
   int left = __shfl_up_sync(0xffffffffu, q[7], 1);
   if ((lane & 3) == 0) left = 0;
-  uint32_t u[8], W[2] = {0u, 0u};
+  uint32_t u[8];
 #pragma unroll
   for (int e = 7; e >= 0; --e) {
     const int d = q[e] - (e ? q[e - 1] : left);
     u[e] = ((uint32_t)d << 1) ^ (uint32_t)(d >> 31);
   }
-#pragma unroll
-  for (int e = 0; e < 8; ++e) {
-    const uint32_t any = __reduce_or_sync(0xffffffffu, u[e]);
-    W[e >> 2] |= (uint32_t)(32 - __clz(any)) << (8 * (e & 3));
-  }
-  const uint32_t tot_lo = bytesum(W[0]), tot = tot_lo + bytesum(W[1]);
-  if (lane == 0) {
-    reinterpret_cast<uint2*>(pk)[z] = make_uint2(W[0], W[1]);   // the eight width bytes of this plane
-    s_tot[z] = (int)tot;
-  }
-  __syncthreads();
-  uint32_t base = 0, total = 0;
-#pragma unroll
-  for (int zz = 0; zz < kTZ; ++zz) {
-    const uint32_t t = (uint32_t)s_tot[zz];
-    base += zz < z ? t : 0u;
-    total += t;
-  }
   uint32_t* words = reinterpret_cast<uint32_t*>(pk + kRows);
-  uint32_t ua[4] = {u[0], u[1], u[2], u[3]}, ub[4] = {u[4], u[5], u[6], u[7]};
-  planes4<true>(ua, W[0], base, words, lane);
-  planes4<true>(ub, W[1], base + tot_lo, words, lane);
+  // Rows of at most 8 bits: four rows share one transpose, after which lane 8 r + j holds bit
+  // plane j of row r. Which planes exist is then one vote: the planes up to each row's highest
+  // nonzero one (its bits smeared downwards), and a lane's place is the count of those before
+  // it. This replaced a warp-wide OR, a count of leading zeros and byte sums for every row
+  // (packing a 512^3 field: 459 us before, 419 after, with one barrier of the tile less).
+  const bool narrow = !__any_sync(0xffffffffu, (u[0] | u[1] | u[2] | u[3] | u[4] | u[5] | u[6] | u[7]) > 0xffu);
+  uint32_t W0 = 0u, W1 = 0u;   // narrow: the planes that exist, one bit a lane; otherwise the widths, one byte a row
+  uint32_t tot_lo, tot;        // words of the first four rows, of all eight
+  if (narrow) {
+    u[0] = transpose32(__byte_perm(__byte_perm(u[0], u[1], 0x0040), __byte_perm(u[2], u[3], 0x0040), 0x5410), lane);
+    u[1] = transpose32(__byte_perm(__byte_perm(u[4], u[5], 0x0040), __byte_perm(u[6], u[7], 0x0040), 0x5410), lane);
+    W0 = __ballot_sync(0xffffffffu, u[0] != 0u);
+    W1 = __ballot_sync(0xffffffffu, u[1] != 0u);
+    W0 |= (W0 >> 1) & 0x7f7f7f7fu;
+    W1 |= (W1 >> 1) & 0x7f7f7f7fu;
+    W0 |= (W0 >> 2) & 0x3f3f3f3fu;
+    W1 |= (W1 >> 2) & 0x3f3f3f3fu;
+    W0 |= (W0 >> 4) & 0x0f0f0f0fu;
+    W1 |= (W1 >> 4) & 0x0f0f0f0fu;
+    if (lane < 8) pk[8 * z + lane] = (unsigned char)__popc(((lane < 4 ? W0 : W1) >> (8 * (lane & 3))) & 0xffu);
+    tot_lo = __popc(W0);
+    tot = tot_lo + __popc(W1);
+  } else {
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      const uint32_t w = 32 - __clz((int)__reduce_or_sync(0xffffffffu, u[e]));
+      if (e < 4) W0 |= w << (8 * e);
+      else W1 |= w << (8 * (e - 4));
+    }
+    tot_lo = bytesum(W0);
+    tot = tot_lo + bytesum(W1);
+    if (lane == 0) reinterpret_cast<uint2*>(pk)[z] = make_uint2(W0, W1);   // the eight width bytes of this plane
+  }
+  if (lane == 0) s_tot[z] = (int)tot;
+  __syncthreads();
+  const uint32_t t = lane < kTZ ? (uint32_t)s_tot[lane] : 0u;
+  const uint32_t total = __reduce_add_sync(0xffffffffu, t), base = __reduce_add_sync(0xffffffffu, lane < z ? t : 0u);
+  if (narrow) {
+    const uint32_t before = (1u << lane) - 1u;
+    if ((W0 >> lane) & 1u) words[base + __popc(W0 & before)] = u[0];
+    if ((W1 >> lane) & 1u) words[base + tot_lo + __popc(W1 & before)] = u[1];
+  } else {
+    uint32_t ua[4] = {u[0], u[1], u[2], u[3]}, ub[4] = {u[4], u[5], u[6], u[7]};
+    wide_planes4<true>(ua, W0, base, words, lane);
+    wide_planes4<true>(ub, W1, base + tot_lo, words, lane);
+  }
   const uint32_t bytes = kRows + 4u * total;
   const uint32_t padded = (bytes + 15u) & ~15u;
-  for (uint32_t i = bytes + threadIdx.x; i < padded; i += kSzThreads) pk[i] = 0;
+  if (threadIdx.x < (padded - bytes) / 4) words[total + threadIdx.x] = 0u;
   __syncthreads();
   return padded;
 }
 
 // Decodes a packed tile at `src` (global or arena memory) and writes it to its place in `out`;
-// `qs` is 8 KB of shared scratch.
+// `qs` is 8 KB of shared scratch, another one than the call before it had.
 __device__ __forceinline__ void unpack_tile(const unsigned char* src, int* qs, const SzArgs& a, float* out, const TileCoord& t) {
   const int lane = threadIdx.x & 31, z = threadIdx.x >> 5;
   // the 16 words of row widths, one per lane, and their running word count
@@ -306,21 +373,42 @@ __device__ __forceinline__ void unpack_tile(const unsigned char* src, int* qs, c
       if (gx < a.nx && gy < a.ny && gz < a.nz)
         out[((size_t)gz * a.ny + gy) * a.nx + gx] = __uint_as_float(ldg_cg_u32(raw + i));
     }
+    __syncthreads();   // the scratch of the tile before is free when the one after this takes it
     return;
   }
-  const uint32_t mine = bytesum(hw);
-  uint32_t incl = mine;
-#pragma unroll
-  for (int d = 1; d < 16; d <<= 1) {
-    const uint32_t v = __shfl_up_sync(0xffffffffu, incl, d);
-    if (lane >= d) incl += v;
-  }
+  const uint32_t base = __reduce_add_sync(0xffffffffu, lane < 2 * z ? bytesum(hw) : 0u);
   const uint32_t W0 = __shfl_sync(0xffffffffu, hw, 2 * z), W1 = __shfl_sync(0xffffffffu, hw, 2 * z + 1);
-  const uint32_t base = __shfl_sync(0xffffffffu, incl - mine, 2 * z);
   uint32_t* words = reinterpret_cast<uint32_t*>(const_cast<unsigned char*>(src) + kRows);
   uint32_t ua[4], ub[4];
-  planes4<false>(ua, W0, base, words, lane);
-  planes4<false>(ub, W1, base + bytesum(W0), words, lane);
+  // Unpacking a 512^3 field took 373 us with the row offsets by a scan, the longer transpose and
+  // a third barrier, and takes 276 (B200).
+  if (bytes_le8(W0) && bytes_le8(W1)) {   // lane 8 r + j fetches plane j of row r: one transpose for four rows
+    const int sh = lane & 24, j = lane & 7;
+    const uint32_t before = (1u << sh) - 1u;
+    const uint32_t w0 = (W0 >> sh) & 0xffu, w1 = (W1 >> sh) & 0xffu;
+    const uint32_t at0 = base + bytesum(W0 & before) + j, at1 = base + bytesum(W0) + bytesum(W1 & before) + j;
+    const uint32_t X0 = (uint32_t)j < w0 ? ldg_cg_u32(words + at0) : 0u, X1 = (uint32_t)j < w1 ? ldg_cg_u32(words + at1) : 0u;
+    const uint32_t U0 = transpose32(X0, lane), U1 = transpose32(X1, lane);
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      ua[r] = (U0 >> (8 * r)) & 0xffu;
+      ub[r] = (U1 >> (8 * r)) & 0xffu;
+    }
+  } else {
+    auto four = [&](uint32_t (&u)[4], uint32_t W, uint32_t off) {
+      if (bytes_le8(W)) {
+        const int sh = lane & 24, j = lane & 7;
+        const uint32_t at = off + bytesum(W & ((1u << sh) - 1u)) + j;
+        const uint32_t U = transpose32((uint32_t)j < ((W >> sh) & 0xffu) ? ldg_cg_u32(words + at) : 0u, lane);
+#pragma unroll
+        for (int r = 0; r < 4; ++r) u[r] = (U >> (8 * r)) & 0xffu;
+      } else {
+        wide_planes4<false>(u, W, off, words, lane);
+      }
+    };
+    four(ua, W0, base);
+    four(ub, W1, base + bytesum(W0));
+  }
   int p[8];
 #pragma unroll
   for (int e = 0; e < 8; ++e) {
@@ -357,16 +445,29 @@ __device__ __forceinline__ void unpack_tile(const unsigned char* src, int* qs, c
   {
     const int y = z;  // this warp now owns line y of every plane
     const int gx = t.x0 + lane, gy = t.y0 + y;
-    const bool ok = gx < a.nx && gy < a.ny;
+    const size_t plane = (size_t)a.ny * a.nx;
+    float* at = out + (size_t)t.z0 * plane + (size_t)gy * a.nx + gx;
+    const int planes = gx < a.nx && gy < a.ny ? a.nz - t.z0 : 0;   // planes of the tile that this thread writes
+    const int* from = qs + y * kTX + lane;
     int run = 0;
+    if (planes >= kTZ) {
 #pragma unroll
-    for (int zz = 0; zz < kTZ; ++zz) {
-      run += qs[(zz * kTY + y) * kTX + lane];
-      const int gz = t.z0 + zz;
-      if (ok && gz < a.nz) out[((size_t)gz * a.ny + gy) * a.nx + gx] = __fmul_rn((float)run, a.two_eb);
+      for (int zz = 0; zz < kTZ; ++zz) {
+        run += from[zz * kTY * kTX];
+        *at = __fmul_rn((float)run, a.two_eb);
+        at += plane;
+      }
+    } else {
+#pragma unroll
+      for (int zz = 0; zz < kTZ; ++zz) {
+        run += from[zz * kTY * kTX];
+        if (zz < planes) *at = __fmul_rn((float)run, a.two_eb);
+        at += plane;
+      }
     }
   }
-  __syncthreads();   // the scratch is free for the next tile
+  // No barrier: the caller alternates between two scratch buffers, and a thread that writes
+  // this one again has passed the two barriers of the tile between.
 }
 
 __device__ __forceinline__ void load_tile_plain(const float* in, float* vals, const TileCoord& t, const SzArgs& a) {
@@ -404,6 +505,8 @@ __global__ void __launch_bounds__(kSzThreads, kKind == 1 ? 6 : kKind == 2 ? 5 : 
   __shared__ int s_tot[kTZ];
   __shared__ uint32_t s_size[2];         // this CTA's packed size per group parity, read by the cluster
   __shared__ __align__(8) uint64_t mbar[2];
+  __shared__ uint32_t s_sizes[2][kClusterSize];     // compress: the cluster's sizes, sent by their CTAs
+  __shared__ __align__(8) uint64_t size_bar[2];     // counts their arrival, per group parity
   __shared__ CtaSync sync;
 
   cg::cluster_group cluster = cg::this_cluster();
@@ -419,9 +522,14 @@ __global__ void __launch_bounds__(kSzThreads, kKind == 1 ? 6 : kKind == 2 ? 5 : 
     sync.fail = 0;
     mbar_init(&mbar[0], 1);
     mbar_init(&mbar[1], 1);
+    if (kKind == 0) {
+      mbar_init(&size_bar[0], 1);
+      mbar_init(&size_bar[1], 1);
+    }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncthreads();
+  if (kKind == 0) cluster.sync();   // the mbarriers exist before anybody counts on them
   uint32_t phases = 0u;     // bit s: parity the next wait on mbarrier s expects
   auto landed = [&](int slot) {   // bounded wait for the copy into buffer `slot`; reports a copy that never came
     const bool ok = mbar_wait(&mbar[slot], (phases >> slot) & 1u);
@@ -430,6 +538,7 @@ __global__ void __launch_bounds__(kSzThreads, kKind == 1 ? 6 : kKind == 2 ? 5 : 
       if (threadIdx.x == 0 && a.c.status) atomicOr(a.c.status + CCB_STATUS_FLAGS, CCB_ST_TIMEOUT);
       sync.fail = 1;
     }
+    return ok;
   };
 
   if (collective) trace_mark(a.c, 0);
@@ -488,12 +597,33 @@ __global__ void __launch_bounds__(kSzThreads, kKind == 1 ? 6 : kKind == 2 ? 5 : 
       prefetch(g + ncl, slot ^ 1);   // that buffer was released by the __syncthreads ending the previous pack
       if (tile < ntiles) {
         float* cur = vals2[slot];
-        if (a.use_tma) landed(slot);
+        // No barrier here: every thread waits for the copy itself, and the plain load leaves a
+        // plane of the tile to the warp that packs it.
+        bool ok = true;
+        if (a.use_tma) ok = landed(slot);
         else load_tile_plain(in, cur, tile_coord(a, tile), a);
-        __syncthreads();
-        size = sync.fail ? 0 : pack_tile(cur, pk2[slot], s_tot, a, own_out, tile_coord(a, tile));
+        __syncwarp();
+        size = pack_tile(cur, pk2[slot], s_tot, a, !ok, sync, own_out, tile_coord(a, tile));
       } else {
         __syncthreads();   // keeps one CTA barrier per iteration between a copy-out and its signal
+      }
+      if constexpr (kKind == 0) {
+        // Compressing into a local buffer the CTAs exchange nothing but their sizes: each sends
+        // its own to the eight and waits for eight words. A cluster barrier's release waited
+        // for the copy-out's global stores as well, a fifth of the stall cycles: packing a 512^3
+        // field took 419 us with it and takes 344 (B200).
+        // The words of this parity are written again two groups on, by a CTA that has this
+        // CTA's size of the next group, sent after all its threads read the words here.
+        if (threadIdx.x == 0) mbar_expect_tx(&size_bar[slot], 4 * kClusterSize);
+        if (threadIdx.x < kClusterSize) st_async_u32(&s_sizes[slot][k], &size_bar[slot], threadIdx.x, size);
+        if (pend) emit(pend_g, pend_off, pend_size, pk2[slot ^ 1]);
+        const bool ok = mbar_wait_cluster(&size_bar[slot], (it >> 1) & 1u);
+        const int ln = threadIdx.x & 31;
+        uint32_t off = __reduce_add_sync(0xffffffffu, ok && ln < k ? s_sizes[slot][ln] : 0u);
+        if (!ok) sync.fail = 1;
+        pend = true; pend_g = g; pend_off = off; pend_size = size;
+        produced += size;
+        continue;
       }
       if (threadIdx.x == 0) s_size[slot] = size;
       // One cluster barrier per group, split in two so that the copy-out of the PREVIOUS
@@ -556,6 +686,7 @@ __global__ void __launch_bounds__(kSzThreads, kKind == 1 ? 6 : kKind == 2 ? 5 : 
   if (collective) trace_mark(a.c, 2);
   auto dwave_end = [&](unsigned int w) { return (unsigned int)(((unsigned long long)per_src * (w + 1)) / kBcastWaves); };
   unsigned int dwave = 0;
+  int scratch = 0;
   uint32_t sz_next = (mode == 1) ? sizes_of(0) : 0u;
   for (unsigned int f = 0; f < nitems; ++f) {
     if (collective && per_src && f == per_src) trace_mark(a.c, 3);   // first received field decoded
@@ -587,8 +718,9 @@ __global__ void __launch_bounds__(kSzThreads, kKind == 1 ? 6 : kKind == 2 ? 5 : 
       if (threadIdx.x == 0 && a.c.status) atomicOr(a.c.status + CCB_STATUS_FLAGS, CCB_ST_TIMEOUT);
     }
     const int q = mode == 2 ? (r + 1 + (int)(f / per_src)) % n : a.root;
+    scratch ^= 1;
     float* out = a.f[lr].out + (mode == 2 ? (size_t)q * a.nx * a.ny * a.nz : 0);
-    unpack_tile(reinterpret_cast<const unsigned char*>(group_of(f)) + kGroupHeader + off, reinterpret_cast<int*>(vals2[0]), a,
+    unpack_tile(reinterpret_cast<const unsigned char*>(group_of(f)) + kGroupHeader + off, reinterpret_cast<int*>(vals2[scratch]), a,
                 out, tile_coord(a, (cl + (f % per_src) * ncl) * kClusterSize + k));
   }
   if (collective) trace_mark(a.c, 4);
@@ -769,6 +901,23 @@ static void fill_geometry(SzArgs& a, int nx, int ny, int nz, float eb) {
 // launched with the cluster attribute alone (co-residency then rests on the occupancy bound).
 static int g_sz_launch_path = 0;
 
+// Asking for the occupancy of a cluster launch costs more than the launch: once per kernel and device.
+static int resident_clusters(void (*kernel)(const SzArgs), const cudaLaunchConfig_t& cfg, int num_sms) {
+  static std::mutex lock;
+  static std::map<std::pair<void (*)(const SzArgs), int>, int> known;
+  int dev = 0, clusters = 0;
+  cudaGetDevice(&dev);
+  std::lock_guard<std::mutex> hold(lock);
+  auto at = known.find(std::make_pair(kernel, dev));
+  if (at != known.end()) return at->second;
+  if (cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) != cudaSuccess || clusters < 1) {
+    (void)cudaGetLastError();
+    return num_sms / kClusterSize;   // not kept: the next call asks again
+  }
+  known[std::make_pair(kernel, dev)] = clusters;
+  return clusters;
+}
+
 // Launch with a cluster of 8 CTAs; cooperative when the kernel waits on peers.
 static int sz_launch(SzArgs& a, int nlocal, int num_sms, bool waits, cudaStream_t stream) {
   void (*kernel)(const SzArgs) = a.mode == 0 ? sz_kernel<0> : a.mode == 1 ? sz_kernel<1> : sz_kernel<2>;
@@ -785,11 +934,7 @@ static int sz_launch(SzArgs& a, int nlocal, int num_sms, bool waits, cudaStream_
   cfg.attrs = attrs;
   cfg.numAttrs = 1;
   cfg.gridDim = dim3(kClusterSize, 1, 1);
-  int max_clusters = 0;
-  if (cudaOccupancyMaxActiveClusters(&max_clusters, kernel, &cfg) != cudaSuccess || max_clusters < 1) {
-    (void)cudaGetLastError();
-    max_clusters = num_sms / kClusterSize;
-  }
+  const int max_clusters = resident_clusters(kernel, cfg, num_sms);
   // CTAs that wait on peers must all be resident: stay within the resident clusters
   unsigned int clusters = a.ngroups;
   const unsigned int cap = (unsigned)(max_clusters / nlocal > 0 ? max_clusters / nlocal : 1);

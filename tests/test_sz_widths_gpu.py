@@ -1,0 +1,42 @@
+"""Packed bytes of the error-bounded codec where its packer and unpacker branch: planes with rows
+of at most 8, at most 16 and more bits side by side in a tile, values off the nearest grid point,
+raw tiles between packed ones."""
+import numpy as np
+import pytest
+import torch
+
+from ccbench_b200.ops import sz
+
+pytestmark = pytest.mark.gpu
+
+
+def _field(kind, shape):
+    g = torch.Generator().manual_seed(11)
+    f = torch.randn(shape, generator=g)
+    if kind == "mixed":      # the scale changes from plane to plane: 3 to 22 bits
+        f *= (4.0 ** (torch.arange(shape[0]) % 8)).view(-1, 1, 1)
+    elif kind == "rows":     # and inside a plane from one element of eight to the next
+        f *= 8.0 ** (torch.arange(shape[2]) % 8 // 2).view(1, 1, -1)
+    elif kind == "far":      # large multiples of the step: fp32 rounding picks the farther grid point now and then
+        f = f * 0.5 + 8000.0
+    elif kind == "raw":      # infinities, NaN and values beyond the integer range, each in a tile of its own
+        f[0, 0, 0] = float("inf")
+        f[-1, 3, 40] = float("nan")
+        f[1, -1, -1] = -3e38
+    elif kind == "flat":
+        f = torch.zeros(shape)
+        f[2] = 1.0
+    return f
+
+
+@pytest.mark.parametrize("kind", ["mixed", "rows", "far", "raw", "flat"])
+@pytest.mark.parametrize("shape", [(16, 16, 64), (19, 21, 99), (9, 40, 132), (41, 9, 160)])
+def test_bytes_and_values_are_those_of_the_host_codec(kind, shape):
+    f = _field(kind, shape)
+    eb = 1e-2 if kind != "far" else 1e-3
+    buf, used = sz.compress(f.cuda(), eb)
+    blob = sz.to_container(buf, shape, eb).cpu().numpy()
+    want = sz.encode_cpu(f.numpy(), eb)
+    assert np.array_equal(blob, want)
+    back = sz.decompress(buf, shape, eb).cpu().numpy()
+    assert np.array_equal(back, sz.decode_cpu(want), equal_nan=True)
