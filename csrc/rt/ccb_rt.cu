@@ -954,7 +954,12 @@ static int reduce_launch(ccb_comm* c, const void* const* send, void* const* recv
     const size_t chunks = (per + kPipeChunkElems - 1) / kPipeChunkElems;
     const size_t ctas = chunks < (size_t)cap ? chunks : (size_t)cap;
     const size_t per_cta = ctas ? chunks / ctas : 0;
-    if (pfn && (per_cta >= (size_t)c->pipe_min_chunks || c->pipe_mode == 2)) {
+    // Several ranks on one GPU have no link whose stores could overlap with the decode, and every
+    // wave still costs its fences and flags. With 21 and 22 chunks per CTA the plain kernel is the
+    // faster one there (25 MiB buckets: all-reduce of 4 ranks with error feedback 200 us
+    // pipelined, 158 plain; reduce-scatter of 8 ranks 134 and 109); from 24 it stays as it was.
+    const size_t least = (size_t)c->pipe_min_chunks * (c->nlocal > 1 ? 6 : 1);
+    if (pfn && (per_cta >= least || c->pipe_mode == 2)) {
       // Measured at 256 MiB: two ranks are fastest with 6 waves (272 us against 283 with 8; a
       // wave is then a quarter of the data and each costs two fence-and-flag rounds), four
       // ranks with 8 (386 against 392 with 4).
