@@ -902,8 +902,9 @@ namespace ccb {
     default: return nullptr;                                                         \
   }
 
-static const void* reduce_fn(int dtype, int codec, int shape) {
+static const void* reduce_fn(int dtype, int codec, int shape, bool ef) {
   if (shape == kOneShot) return CCB_DISPATCH_TC(dtype, codec, (reinterpret_cast<const void*>(&reduce_kernel<TT, CC, kOneShot>)));
+  if (!ef) return CCB_DISPATCH_TC(dtype, codec, (reinterpret_cast<const void*>(&reduce_kernel<TT, CC, kTwoShotPlain>)));
   return CCB_DISPATCH_TC(dtype, codec, (reinterpret_cast<const void*>(&reduce_kernel<TT, CC, kTwoShot>)));
 }
 static const void* solo_fn(int dtype, int codec, bool ef) {
@@ -939,7 +940,9 @@ static int ctas_for(ccb_comm* c, const void* fn, size_t elems, int* tile_warps) 
 static int reduce_launch(ccb_comm* c, const void* const* send, void* const* recv, float* const* ef, size_t base,
                          size_t recv_base, size_t count, size_t shard_elems, int dtype, int op, int codec, int mode,
                          int root, int shape, cudaStream_t stream) {
-  const void* fn = reduce_fn(dtype, codec, shape);
+  bool any_ef = false;
+  for (int i = 0; i < c->nlocal; ++i) any_ef = any_ef || (ef && ef[i]);
+  const void* fn = reduce_fn(dtype, codec, shape, any_ef);
   if (!fn) {
     set_error("unsupported dtype %d / codec %d", dtype, codec);
     return CCB_ERR_UNSUPPORTED;
