@@ -27,6 +27,15 @@ int ccb_sz_launch_path(void);
 int ccb_sz_compress(const float* in, int nx, int ny, int nz, float eb, void* out, unsigned long long* d_used,
                     ccb_stream_t stream);
 int ccb_sz_decompress(const void* in, int nx, int ny, int nz, float eb, float* out, ccb_stream_t stream);
+/* The packed container (docs/formats.md) of a compressed buffer, all pointers device memory.
+ * scan: offsets[g] = used bytes before group g, offsets[ngroups] their total, offsets[ngroups + 1]
+ * the largest group's (ngroups + 2 words); from the groups' own headers (slots) or from a list of
+ * sizes, exactly one of the two given. pack writes 40 + 4 * ngroups + offsets[ngroups] bytes;
+ * unpack takes the payload behind a container's size list and fills ngroups whole slots. */
+int ccb_sz_container_scan(const void* slots, const uint32_t* sizes, uint64_t ngroups, unsigned long long* offsets, ccb_stream_t stream);
+int ccb_sz_container_pack(const void* slots, const unsigned long long* offsets, int nx, int ny, int nz, float eb, uint64_t ngroups, void* out,
+                          ccb_stream_t stream);
+int ccb_sz_container_unpack(const void* payload, const unsigned long long* offsets, uint64_t ngroups, void* slots, ccb_stream_t stream);
 /* root < 0: AllGather (recv holds nranks fields in rank order); root >= 0: Broadcast.
  * One fused kernel: compress, store into the peers' arenas, decode on arrival.
  * `d_used`: optional device counters, one per local rank, of the compressed bytes a
