@@ -27,7 +27,8 @@ int ccb_sz_launch_path(void);
 int ccb_sz_compress(const float* in, int nx, int ny, int nz, float eb, void* out, unsigned long long* d_used,
                     ccb_stream_t stream);
 int ccb_sz_decompress(const void* in, int nx, int ny, int nz, float eb, float* out, ccb_stream_t stream);
-/* The packed container (docs/formats.md) of a compressed buffer, all pointers device memory.
+/* The packed container of a compressed buffer: a 40-byte header, the used bytes of each group as u32,
+ * then the used bytes of every group. All pointers device memory.
  * scan: offsets[g] = used bytes before group g, offsets[ngroups] their total, offsets[ngroups + 1]
  * the largest group's (ngroups + 2 words); from the groups' own headers (slots) or from a list of
  * sizes, exactly one of the two given. pack writes 40 + 4 * ngroups + offsets[ngroups] bytes;
