@@ -13,7 +13,12 @@
 
 namespace ccb {
 
-template <class T, class C>
+// kOwnDirect: a rank's own block need not go through its arena, the packet is decoded where it was
+// encoded. Where buffers of the ranks of one process lie in one another (see the host) it is not
+// so: then a rank's own block too is read before its flag and written after the others'. Two
+// instantiations, because the choice as an argument cost up to 2 % of an all-gather at odd
+// offsets (registers: 8 ranks, 2,097,153 fp32 values in int8, 173 against 176 us).
+template <class T, class C, bool kOwnDirect>
 __global__ void __launch_bounds__(kThreads, 2) exchange_kernel(const __grid_constant__ ExchangeArgs a) {
   __shared__ CtaSync sync;
   const CommDev& c = a.c;
@@ -43,7 +48,6 @@ __global__ void __launch_bounds__(kThreads, 2) exchange_kernel(const __grid_cons
     if (a.cnt[r][p] != a.cnt[r][f] || a.send_off[r][p] != a.send_off[r][f]) same = false;
   }
 
-  // A rank's own block never goes through its arena: the packet is decoded where it was encoded.
   // One tile is requested ahead of the one in work, so that a warp waits for memory once per
   // tile and not once per access. (All-gather among 8 ranks of 1,638,401 bf16 values each
   // in fp8: 673 us before, most of it element-wise stores at odd offsets, 100 after.)
@@ -72,26 +76,28 @@ __global__ void __launch_bounds__(kThreads, 2) exchange_kernel(const __grid_cons
     C::decode(pk, d);
     store16_wide<T, true>(recv + a.recv_off[r][r], idx, a.cnt[r][r], d);
   };
-  const uint32_t peers = dstmask & ~(1u << r);
-  const bool own = (dstmask >> r) & 1u;
+  const uint32_t staged = kOwnDirect ? dstmask & ~(1u << r) : dstmask;   // blocks that go through an arena
+  const bool own = kOwnDirect && ((dstmask >> r) & 1u);
+  constexpr int kFirst = kOwnDirect ? 1 : 0;
   if (dstmask && same) {
     const int f = __ffs(dstmask) - 1;
     encode_block(send + a.send_off[r][f], a.cnt[r][f], [&](size_t idx, const typename C::Packet& pk) {
-      for (int j = 1; j < n; ++j) {
+      for (int j = kFirst; j < n; ++j) {
         const int p = r + j < n ? r + j : r + j - n;
-        if ((peers >> p) & 1u) C::store(c.arena[p] + area + (size_t)r * a.slot_bytes, pad, idx, pk);
+        if ((staged >> p) & 1u) C::store(c.arena[p] + area + (size_t)r * a.slot_bytes, pad, idx, pk);
       }
       if (own) keep_own(idx, pk);
     });
-  } else if (peers) {
-    for (int j = 1; j < n; ++j) {
+  } else if (staged) {
+    for (int j = kFirst; j < n; ++j) {
       const int p = r + j < n ? r + j : r + j - n;
-      if (!((peers >> p) & 1u)) continue;
+      if (!((staged >> p) & 1u)) continue;
       char* dst = c.arena[p] + area + (size_t)r * a.slot_bytes;
       encode_block(send + a.send_off[r][p], a.cnt[r][p], [&](size_t idx, const typename C::Packet& pk) { C::store(dst, pad, idx, pk); });
     }
   }
   __syncthreads();
+  const uint32_t peers = dstmask & ~(1u << r);
   if (threadIdx.x == 0 && peers) signal_peers(c, peers, 0, r, b);
   // The own block of an exchange with several different blocks comes after the others have
   // been read (its place in recv may be another block's place in send), while they travel.
@@ -99,9 +105,9 @@ __global__ void __launch_bounds__(kThreads, 2) exchange_kernel(const __grid_cons
 
   uint32_t srcmask = 0;
   for (int q = 0; q < n; ++q)
-    if (q != r && a.cnt[q][r]) srcmask |= 1u << q;
+    if (q != r && a.cnt[q][r]) srcmask |= 1u << q;   // what this CTA put into its own arena it reads back itself
   if (srcmask && !cta_wait_sources(sync, c, my, 0, r, srcmask, 0x30)) return;
-  for (int j = 1; j < n; ++j) {
+  for (int j = kFirst; j < n; ++j) {
     const int q = r + j < n ? r + j : r + j - n;
     const size_t valid = a.cnt[q][r];
     const char* slot = my + area + (size_t)q * a.slot_bytes;

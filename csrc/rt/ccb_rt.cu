@@ -13,6 +13,7 @@
 #include <string.h>
 #include <unistd.h>
 
+#include <algorithm>
 #include <atomic>
 #include <map>
 #include <mutex>
@@ -911,8 +912,9 @@ static const void* solo_fn(int dtype, int codec, bool ef) {
   if (ef) return CCB_DISPATCH_TC(dtype, codec, (reinterpret_cast<const void*>(&solo_kernel<TT, CC, true>)));
   return CCB_DISPATCH_TC(dtype, codec, (reinterpret_cast<const void*>(&solo_kernel<TT, CC, false>)));
 }
-static const void* exchange_fn(int dtype, int codec) {
-  return CCB_DISPATCH_TC(dtype, codec, (reinterpret_cast<const void*>(&exchange_kernel<TT, CC>)));
+static const void* exchange_fn(int dtype, int codec, bool own_direct) {
+  if (!own_direct) return CCB_DISPATCH_TC(dtype, codec, (reinterpret_cast<const void*>(&exchange_kernel<TT, CC, false>)));
+  return CCB_DISPATCH_TC(dtype, codec, (reinterpret_cast<const void*>(&exchange_kernel<TT, CC, true>)));
 }
 static const void* ring_fn(int dtype, int codec) {
   return CCB_DISPATCH_TC(dtype, codec, (reinterpret_cast<const void*>(&ring_kernel<TT, CC>)));
@@ -933,6 +935,24 @@ static int ctas_for(ccb_comm* c, const void* fn, size_t elems, int* tile_warps) 
   size_t tiles = (units + tw - 1) / tw;
   if (tiles < 1) tiles = 1;
   return tiles < (size_t)cap ? (int)tiles : cap;
+}
+
+// Address range of a buffer, or of the part of it that a call touches; empty when lo >= hi.
+struct Span { uintptr_t lo, hi; };
+static Span span_of(const void* p, size_t from, size_t to) {
+  const uintptr_t b = reinterpret_cast<uintptr_t>(p);
+  return Span{b + from, b + to};
+}
+// Several ranks of one process may be given buffers that lie in one another (every rank's result
+// in the first rank's buffer, two buffers exchanged by an all-to-all). The kernels read what a rank
+// sends before its flag and write what it receives after the others' flags, so such calls work;
+// a rank may go around that order for its own block only where no other rank's receive buffer
+// meets its send buffer.
+static bool ranks_apart(const Span* send, const Span* recv, int nlocal) {
+  for (int i = 0; i < nlocal; ++i)
+    for (int j = 0; j < nlocal; ++j)
+      if (i != j && send[i].lo < recv[j].hi && recv[j].lo < send[i].hi) return false;
+  return true;
 }
 
 // One launch of the reduce family on `count` elements starting at element `base`
@@ -986,6 +1006,14 @@ static int reduce_launch(ccb_comm* c, const void* const* send, void* const* recv
     a.send[i] = static_cast<const char*>(send[i]) + base * es;
     a.recv[i] = static_cast<char*>(recv[i]) + recv_base * es;
     a.ef[i] = (ef && ef[i]) ? ef[i] + base : nullptr;
+  }
+  if (shape == kOneShot) {
+    Span out[CCB_MAX_RANKS], in[CCB_MAX_RANKS];
+    for (int i = 0; i < c->nlocal; ++i) {
+      in[i] = span_of(a.send[i], 0, count * es);
+      out[i] = span_of(a.recv[i], 0, count * es);
+    }
+    a.own_direct = ranks_apart(in, out, c->nlocal) ? 1 : 0;
   }
   a.count = count;
   a.shard_elems = shard_elems;
@@ -1250,7 +1278,7 @@ extern "C" int ccb_exchange(ccb_comm* c, const void* const* send, void* const* r
   int rc = check_alive(c);
   if (rc) return rc;
   const int n = c->nranks;
-  const void* fn = exchange_fn(dtype, codec);
+  const void* fn = exchange_fn(dtype, codec, true);
   if (!fn) {
     set_error("unsupported dtype %d / codec %d", dtype, codec);
     return CCB_ERR_UNSUPPORTED;
@@ -1283,6 +1311,30 @@ extern "C" int ccb_exchange(ccb_comm* c, const void* const* send, void* const* r
   a.rank0 = c->rank0;
   a.nlocal = c->nlocal;
   a.ack = full ? 0 : 1;
+  Span out[CCB_MAX_RANKS], in[CCB_MAX_RANKS];
+  const size_t es = elem_size(dtype);
+  bool own_direct = true;
+  for (int i = 0; i < c->nlocal; ++i) {
+    const int r = c->rank0 + i;
+    size_t s0 = SIZE_MAX, s1 = 0, r0 = SIZE_MAX, r1 = 0;
+    for (int p = 0; p < n; ++p) {
+      if (a.cnt[r][p]) {
+        s0 = std::min<size_t>(s0, a.send_off[r][p]);
+        s1 = std::max<size_t>(s1, a.send_off[r][p] + a.cnt[r][p]);
+      }
+      if (a.cnt[p][r]) {
+        r0 = std::min<size_t>(r0, a.recv_off[r][p]);
+        r1 = std::max<size_t>(r1, a.recv_off[r][p] + a.cnt[p][r]);
+      }
+    }
+    in[i] = s1 ? span_of(send[i], s0 * es, s1 * es) : Span{0, 0};
+    out[i] = r1 ? span_of(recv[i], r0 * es, r1 * es) : Span{0, 0};
+    // a rank's own buffers may meet too, if its own block stays where it is (the calls in place)
+    if (a.cnt[r][r] && in[i].lo < out[i].hi && out[i].lo < in[i].hi &&
+        span_of(send[i], a.send_off[r][r] * es, 0).lo != span_of(recv[i], a.recv_off[r][r] * es, 0).lo)
+      own_direct = false;
+  }
+  if (!own_direct || !ranks_apart(in, out, c->nlocal)) fn = exchange_fn(dtype, codec, false);
   const int ctas = ctas_for(c, fn, maxcnt, &a.tile_warps);
   return launch(c, fn, ctas, &a, static_cast<cudaStream_t>(stream_));
 }
