@@ -107,12 +107,16 @@ def to_container(buf: torch.Tensor, shape, eb: float) -> torch.Tensor:
             L = _decl()
             offsets = torch.empty(ngroups + 2, dtype=torch.int64, device=buf.device)
             _check(L.ccb_sz_container_scan(buf.data_ptr(), None, ngroups, offsets.data_ptr(), _stream()))
-            total = int(offsets[ngroups].item())
+            total, largest = offsets[ngroups:].tolist()
+            if largest > GROUP_STRIDE:
+                raise ValueError("a group of the buffer was given up in compression, or is damaged")
             blob = torch.empty(HEADER_BYTES + 4 * ngroups + total, dtype=torch.uint8, device=buf.device)
             _check(L.ccb_sz_container_pack(buf.data_ptr(), offsets.data_ptr(), nx, ny, nz, eb, ngroups, blob.data_ptr(), _stream()))
         return blob
     slots = buf.view(ngroups, GROUP_STRIDE)
     sizes = slots[:, :GROUP_HEADER].contiguous().view(torch.int32).to(torch.int64).sum(dim=1) + GROUP_HEADER
+    if ngroups and int(sizes.max()) > GROUP_STRIDE:
+        raise ValueError("a group of the buffer was given up in compression, or is damaged")
     keep = torch.arange(GROUP_STRIDE, device=buf.device).unsqueeze(0) < sizes.unsqueeze(1)
     payload = slots[keep]
     step = torch.tensor(2.0 * eb, dtype=torch.float32) * (1 - 2.0 ** -10)

@@ -63,6 +63,7 @@ constexpr int kRows = kTY * kTZ;                  // 64
 constexpr int kSzThreads = 256;                   // warp = z plane, lane = x
 constexpr int kClusterSize = 8;
 constexpr int kTileCap = kRows + kTileVals * 4;   // 8256 bytes, worst case (w = 32 everywhere)
+constexpr uint32_t kLostTile = 1u << 24;          // size word of the tiles of a group that could not be packed: more than a group can hold
 constexpr int kGroupHeader = 32;
 constexpr int kGroupStride = kGroupHeader + kClusterSize * kTileCap + 32;  // 66112, multiple of 16
 static_assert(kGroupStride % 16 == 0, "slots must keep 16-byte alignment");
@@ -211,9 +212,9 @@ constexpr float kRoundMagic = 12582912.f;   // 1.5 * 2^23: adding and subtractin
 // The codes overwrite the values in shared memory (each thread its own eight words).
 // With `recon` set, the decoder's view of the tile (q * step, or the raw values of a raw
 // tile) is also written to its place in that field: the sender's own copy of what every
-// receiver will decode, without a decode pass.
-// `failed` (any thread, with sync.fail set): the tile's copy never came; every thread gets 0.
-__device__ __forceinline__ uint32_t pack_tile(float* vals, unsigned char* pk, int* s_tot, const SzArgs& a, bool failed, const CtaSync& sync,
+// receiver will decode, without a decode pass. `failed` (any thread): the tile's copy never came and
+// the values are NaN; the tile is stored raw.
+__device__ __forceinline__ uint32_t pack_tile(float* vals, unsigned char* pk, int* s_tot, const SzArgs& a, bool failed,
                                               float* recon = nullptr, TileCoord tc = TileCoord{0, 0, 0}) {
   const int lane = threadIdx.x & 31, z = threadIdx.x >> 5;
   int4* q4 = reinterpret_cast<int4*>(vals) + 2 * threadIdx.x;
@@ -261,7 +262,6 @@ __device__ __forceinline__ uint32_t pack_tile(float* vals, unsigned char* pk, in
   q4[0] = make_int4(q[0], q[1], q[2], q[3]);
   q4[1] = make_int4(q[4], q[5], q[6], q[7]);
   const bool raw_tile = __syncthreads_or(bad);   // and the barrier between the codes and their readers
-  if (raw_tile && sync.fail) return 0;           // the tile never arrived
   if (recon) {
     const int gx = tc.x0 + 8 * (lane & 3), gy = tc.y0 + (lane >> 2), gz = tc.z0 + z;
     if (gy < a.ny && gz < a.nz) {
@@ -499,7 +499,7 @@ __global__ void __launch_bounds__(kSzThreads, kKind == 1 ? 6 : kKind == 2 ? 5 : 
   const int mode = kKind == 2 ? a.mode : kKind;
   const unsigned int kBcastWaves = a.bcast_waves;
   // Two 8 KB buffers: compress lands the next tile in one while the other is packed;
-  // decompress prefixes in vals2[0].
+  // decompress prefixes one tile in one of them and the next in the other.
   __shared__ __align__(128) float vals2[2][kTileVals];
   __shared__ __align__(16) unsigned char pk2[2][kStage];
   __shared__ int s_tot[kTZ];
@@ -600,10 +600,13 @@ __global__ void __launch_bounds__(kSzThreads, kKind == 1 ? 6 : kKind == 2 ? 5 : 
         // No barrier here: every thread waits for the copy itself, and the plain load leaves a
         // plane of the tile to the warp that packs it.
         bool ok = true;
-        if (a.use_tma) ok = landed(slot);
-        else load_tile_plain(in, cur, tile_coord(a, tile), a);
+        if (!a.use_tma) {
+          load_tile_plain(in, cur, tile_coord(a, tile), a);
+        } else if (!(ok = landed(slot))) {   // a tile that never came goes out as NaN (this thread's eight values)
+          for (int e = 0; e < 8; ++e) cur[8 * threadIdx.x + e] = __int_as_float(0x7fffffff);
+        }
         __syncwarp();
-        size = pack_tile(cur, pk2[slot], s_tot, a, !ok, sync, own_out, tile_coord(a, tile));
+        size = pack_tile(cur, pk2[slot], s_tot, a, !ok, own_out, tile_coord(a, tile));
       } else {
         __syncthreads();   // keeps one CTA barrier per iteration between a copy-out and its signal
       }
@@ -620,7 +623,7 @@ __global__ void __launch_bounds__(kSzThreads, kKind == 1 ? 6 : kKind == 2 ? 5 : 
         const bool ok = mbar_wait_cluster(&size_bar[slot], (it >> 1) & 1u);
         const int ln = threadIdx.x & 31;
         uint32_t off = __reduce_add_sync(0xffffffffu, ok && ln < k ? s_sizes[slot][ln] : 0u);
-        if (!ok) sync.fail = 1;
+        if (!ok) sync.fail = 1;   // the tile may land in another's place, inside the slot: the whole group is given up below
         pend = true; pend_g = g; pend_off = off; pend_size = size;
         produced += size;
         continue;
@@ -655,6 +658,13 @@ __global__ void __launch_bounds__(kSzThreads, kKind == 1 ? 6 : kKind == 2 ? 5 : 
           if (wave_end(wave) > (wave ? wave_end(wave - 1) : 0u)) signal_peers(a.c, ((1u << n) - 1u) & ~(1u << r), (int)wave, r, b);
     }
     cluster.sync();      // nobody leaves while a neighbour may still read its sizes
+    if (kKind == 0 && sync.fail && threadIdx.x == 0) {
+      // A wait above gave up: none of these groups is to be trusted. Their size words say so (a
+      // container is refused, unpacking stays inside the slot), and the top bit of the byte count.
+      for (unsigned int g = cl; g < a.ngroups; g += ncl)
+        for (int j = 0; j < kClusterSize; ++j) reinterpret_cast<uint32_t*>(a.local_out + (size_t)g * kGroupStride)[j] = kLostTile;
+      if (a.used_bytes) atomicOr(a.used_bytes + lr, 1ull << 63);
+    }
     if (a.used_bytes && threadIdx.x == 0 && produced) atomicAdd(a.used_bytes + lr, produced + 0ull);
   }
   if (mode == 0) return;

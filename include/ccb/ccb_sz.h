@@ -23,7 +23,9 @@ uint64_t ccb_sz_capacity(int nx, int ny, int nz);
  * launched with the cluster attribute alone (grid bounded by the resident-cluster count). */
 int ccb_sz_launch_path(void);
 /* |in - decompress(compress(in))| <= eb for every finite element. `d_used` (device
- * memory, optional) receives the number of compressed bytes produced. */
+ * memory, optional) receives the number of compressed bytes produced. Should a bounded wait of the
+ * kernel ever give up, its top bit is set, a tile that never arrived is NaN, and the size words of
+ * the groups concerned are larger than a group can be, so that no container is made of them. */
 int ccb_sz_compress(const float* in, int nx, int ny, int nz, float eb, void* out, unsigned long long* d_used,
                     ccb_stream_t stream);
 int ccb_sz_decompress(const void* in, int nx, int ny, int nz, float eb, float* out, ccb_stream_t stream);

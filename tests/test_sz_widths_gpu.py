@@ -40,3 +40,25 @@ def test_bytes_and_values_are_those_of_the_host_codec(kind, shape):
     assert np.array_equal(blob, want)
     back = sz.decompress(buf, shape, eb).cpu().numpy()
     assert np.array_equal(back, sz.decode_cpu(want), equal_nan=True)
+
+
+@pytest.mark.parametrize("shape", [(41, 9, 160), (64, 64, 64)])
+@pytest.mark.parametrize("tiles", [[0], [7], list(range(8))])
+def test_a_group_given_up_makes_no_container_and_harms_no_other(shape, tiles):
+    f = _field("mixed", shape).cuda()
+    buf, used = sz.compress(f, 1e-2)
+    assert 0 < int(used) < buf.numel()
+    back = sz.decompress(buf, shape, 1e-2)
+    for t in tiles:
+        word = sz.GROUP_STRIDE + 4 * t
+        buf[word:word + 4].view(torch.int32).fill_(1 << 24)
+    got = sz.decompress(buf, shape, 1e-2)
+    tx, ty = -(-shape[2] // sz.TX), -(-shape[1] // sz.TY)
+    for t in range(8, 16):   # the tiles of that group may be anything
+        z, y, x = t // (tx * ty) * sz.TZ, t // tx % ty * sz.TY, t % tx * sz.TX
+        for v in (got, back):
+            v[z:z + sz.TZ, y:y + sz.TY, x:x + sz.TX] = 0
+    assert torch.equal(got, back)
+    for where in (buf, buf.cpu()):
+        with pytest.raises(ValueError):
+            sz.to_container(where, shape, 1e-2)
