@@ -62,3 +62,28 @@ def test_a_group_given_up_makes_no_container_and_harms_no_other(shape, tiles):
     for where in (buf, buf.cpu()):
         with pytest.raises(ValueError):
             sz.to_container(where, shape, 1e-2)
+
+
+@pytest.mark.parametrize("shape", [(192, 192, 256), (190, 191, 255)])
+def test_raw_tiles_between_packed_ones_over_several_turns(shape):
+    """4608 tiles, 576 groups: more than three a cluster. Runs of raw tiles of every length from none
+    to a few groups lie between packed ones, so both scratch buffers of the unpacker and both
+    parities of the packer's size exchange are used again around them."""
+    g = torch.Generator().manual_seed(3)
+    f = torch.randn(shape, generator=g)
+    tiles = [-(-shape[0] // 8), -(-shape[1] // 8), -(-shape[2] // 32)]
+    hit = (torch.rand(tiles, generator=g) < torch.rand(tiles[0], 1, 1, generator=g)).repeat_interleave(8, 0).repeat_interleave(8, 1).repeat_interleave(32, 2)
+    f[hit[:shape[0], :shape[1], :shape[2]]] *= 1e9
+    eb = 1e-2
+    buf, _ = sz.compress(f.cuda(), eb)
+    want = sz.encode_cpu(f.numpy(), eb)
+    assert np.array_equal(sz.to_container(buf, shape, eb).cpu().numpy(), want)
+    again, s2, e2 = sz.from_container(torch.from_numpy(want).cuda())
+    for b in (buf, again):
+        back = sz.decompress(b, shape, eb).cpu()
+        assert (back - f).abs().max().item() <= eb32(eb)
+        assert torch.equal(back, torch.from_numpy(sz.decode_cpu(want)))
+
+
+def eb32(eb):
+    return float(np.float32(eb))
