@@ -908,9 +908,10 @@ static const void* reduce_fn(int dtype, int codec, int shape, bool ef) {
   if (!ef) return CCB_DISPATCH_TC(dtype, codec, (reinterpret_cast<const void*>(&reduce_kernel<TT, CC, kTwoShotPlain>)));
   return CCB_DISPATCH_TC(dtype, codec, (reinterpret_cast<const void*>(&reduce_kernel<TT, CC, kTwoShot>)));
 }
+template <bool kTrace>
 static const void* solo_fn(int dtype, int codec, bool ef) {
-  if (ef) return CCB_DISPATCH_TC(dtype, codec, (reinterpret_cast<const void*>(&solo_kernel<TT, CC, true>)));
-  return CCB_DISPATCH_TC(dtype, codec, (reinterpret_cast<const void*>(&solo_kernel<TT, CC, false>)));
+  if (ef) return CCB_DISPATCH_TC(dtype, codec, (reinterpret_cast<const void*>(&solo_kernel<TT, CC, true, kTrace>)));
+  return CCB_DISPATCH_TC(dtype, codec, (reinterpret_cast<const void*>(&solo_kernel<TT, CC, false, kTrace>)));
 }
 static const void* exchange_fn(int dtype, int codec, bool own_direct) {
   if (!own_direct) return CCB_DISPATCH_TC(dtype, codec, (reinterpret_cast<const void*>(&exchange_kernel<TT, CC, false>)));
@@ -1045,7 +1046,7 @@ static int reduce_launch(ccb_comm* c, const void* const* send, void* const* recv
 // An all-reduce of one rank (see solo_kernel): as many CTAs as are resident at once.
 static int solo_launch(ccb_comm* c, const void* const* send, void* const* recv, float* const* ef, uint64_t count, int dtype, int codec,
                        cudaStream_t stream) {
-  const void* fn = solo_fn(dtype, codec, ef && ef[0]);
+  const void* fn = c->trace ? solo_fn<true>(dtype, codec, ef && ef[0]) : solo_fn<false>(dtype, codec, ef && ef[0]);
   if (!fn) {
     set_error("unsupported dtype %d / codec %d", dtype, codec);
     return CCB_ERR_UNSUPPORTED;
@@ -1053,12 +1054,14 @@ static int solo_launch(ccb_comm* c, const void* const* send, void* const* recv, 
   ReduceArgs a;
   memset(&a, 0, sizeof(a));
   a.c.nranks = 1;
+  a.c.trace = c->trace;
   a.send[0] = send[0];
   a.recv[0] = recv[0];
   a.ef[0] = ef ? ef[0] : nullptr;
   a.count = count;
   const size_t blocks = (count + (size_t)kSoloThreads * kLaneElems - 1) / ((size_t)kSoloThreads * kLaneElems);
   size_t cap = (size_t)c->num_sms * resident_ctas(fn, kSoloThreads, c->device);
+  if (cap > CCB_MAX_CTAS) cap = CCB_MAX_CTAS;   // a trace has a column for so many
   if (c->max_ctas > 0 && cap > (size_t)c->max_ctas) cap = (size_t)c->max_ctas;
   void* params[] = {&a};
   cudaError_t e = cudaLaunchKernel(fn, dim3((unsigned)(blocks < cap ? blocks : cap)), dim3(kSoloThreads), params, 0, stream);

@@ -81,7 +81,8 @@ int ccb_comm_set_pipeline(ccb_comm* c, int mode, int link_warps, int mc);
 int ccb_comm_status(ccb_comm* c, uint32_t* words);
 /* Device-side phase tracing: when on, every CTA of the two-shot kernels records
  * globaltimer nanoseconds at its phase boundaries (slots: 0 start, 1 first phase-1
- * done, 2 first phase-2 done, 3 all phase-2 done, 4 end). */
+ * done, 2 first phase-2 done, 3 all phase-2 done, 4 end); so does the kernel of a
+ * communicator of one rank, where 1 follows 0 and 2, 3, 4 mark the end. */
 int ccb_comm_set_trace(ccb_comm* c, int on);
 int ccb_comm_read_trace(ccb_comm* c, unsigned long long* out, int ctas);
 /* Wire bytes a call moves per rank for `count` elements (for ratio reporting). */

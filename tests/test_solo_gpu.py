@@ -1,6 +1,9 @@
 """An all-reduce of one rank (its own kernel) against the restated algorithms: partial and whole
 units, more units than resident warps, views at odd offsets, with and without error feedback."""
 import os
+import subprocess
+import sys
+from pathlib import Path
 
 import pytest
 import torch
@@ -48,3 +51,30 @@ def test_one_rank_error_feedback_in_place(comm, dtype, codec):
         torch.cuda.synchronize()
         assert torch.equal(buf.float().cpu(), want)
         assert torch.equal(ef.cpu(), want_ef[0])
+
+
+@pytest.mark.parametrize("algo", ["auto", "twoshot"])
+@pytest.mark.parametrize("count,ef", [(100, False), (8 << 20, False), (8 << 20, True)])
+def test_one_rank_trace(comm, algo, count, ef):
+    x = torch.randn(count, device="cuda")
+    res = torch.zeros(count, device="cuda") if ef else None
+    comm.set_trace(True)
+    try:
+        comm.all_reduce(x, torch.empty_like(x), codec="int8", algo=algo, error_feedback=res)
+        torch.cuda.synchronize()
+        tr = comm.read_trace(1024)
+    finally:
+        comm.set_trace(False)
+    tr = tr[tr[:, 0] > 0]
+    assert 1 <= tr.shape[0] <= -(-count // 4096)
+    assert (tr[:, 0] <= tr[:, 1]).all()
+    assert (tr[:, 1] <= tr[:, 2]).all() and (tr[:, 2] <= tr[:, 3]).all() and (tr[:, 3] <= tr[:, 4]).all()
+    assert int(tr[:, 4].max() - tr[:, 0].min()) < 1_000_000_000
+
+
+def test_phase_timeline_of_one_rank():
+    env = {k: v for k, v in os.environ.items() if k not in ("WORLD_SIZE", "RANK", "LOCAL_RANK")}
+    out = subprocess.run([sys.executable, "-m", "ccbench_b200.bench.phases", "--what", "allreduce"], capture_output=True, text=True, timeout=300,
+                         env=env, cwd=Path(__file__).resolve().parent.parent)
+    assert out.returncode == 0, out.stdout + out.stderr
+    assert out.stdout.count("mark 4") == 3
