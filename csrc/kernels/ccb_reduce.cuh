@@ -345,19 +345,22 @@ __global__ void __launch_bounds__(kThreads, 2) reduce_kernel(const __grid_consta
 // pass is bound by memory. The next unit is requested before the one in hand is encoded.
 // (256 MiB of bf16 in int8: 113 us in the two-shot kernel, 32 warps an SM that each waited for
 // one unit at a time in 16-byte accesses; 100.5 us here, 5.3 TB/s, B200.)
-// The phase marks are in an instantiation of their own: in the same kernel they take up to eight
-// registers, and 256 MiB of bf16 in fp8 went from 92.0 to 93.3 us.
+// kAny is the form with the phase marks and for other CTA sizes (a capped grid, see the host): in
+// the usual form they take up to eight registers, and 256 MiB of bf16 in fp8 went from 92.0 to
+// 93.5 us. Its launch bounds give the same registers a thread for larger CTAs.
 constexpr int kSoloThreads = 256;
-template <class T, class C, bool kEf, bool kTrace>
-__global__ void __launch_bounds__(kSoloThreads, kEf || sizeof(T) == 4 ? 3 : 5) solo_kernel(const __grid_constant__ ReduceArgs a) {
+template <class T, class C, bool kEf, bool kAny>
+__global__ void __launch_bounds__(kAny ? (kEf || sizeof(T) == 4 ? 768 : 640) : kSoloThreads,
+                                  kAny ? (kEf || sizeof(T) == 4 ? 1 : 2) : (kEf || sizeof(T) == 4 ? 3 : 5)) solo_kernel(const __grid_constant__ ReduceArgs a) {
   const T* send = static_cast<const T*>(a.send[0]);
   T* recv = static_cast<T*>(a.recv[0]);
   float* ef = kEf ? a.ef[0] : nullptr;
-  const size_t count = a.count, step = (size_t)gridDim.x * kSoloThreads * kLaneElems;
+  const unsigned int threads = kAny ? blockDim.x : kSoloThreads;
+  const size_t count = a.count, step = (size_t)gridDim.x * threads * kLaneElems;
   const size_t lane_at = (size_t)(threadIdx.x & 31) * kLaneElems;
-  size_t e0 = ((size_t)blockIdx.x * kSoloThreads + (threadIdx.x & ~31u)) * kLaneElems;   // the warp's unit
+  size_t e0 = ((size_t)blockIdx.x * threads + (threadIdx.x & ~31u)) * kLaneElems;   // the warp's unit
   Wide16<T> raw;
-  if constexpr (kTrace) {
+  if constexpr (kAny) {
     trace_mark(a.c, 0);
     trace_mark(a.c, 1);   // nothing goes to a peer
   }
@@ -385,7 +388,7 @@ __global__ void __launch_bounds__(kSoloThreads, kEf || sizeof(T) == 4 ? 3 : 5) s
       store16_wide<float>(ef, idx, count, d);
     }
   }
-  if constexpr (kTrace)
+  if constexpr (kAny)
     for (int k = 2; k <= 4; ++k) trace_mark(a.c, k);   // the CTA's own part is all there is
 }
 

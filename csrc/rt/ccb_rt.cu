@@ -908,10 +908,10 @@ static const void* reduce_fn(int dtype, int codec, int shape, bool ef) {
   if (!ef) return CCB_DISPATCH_TC(dtype, codec, (reinterpret_cast<const void*>(&reduce_kernel<TT, CC, kTwoShotPlain>)));
   return CCB_DISPATCH_TC(dtype, codec, (reinterpret_cast<const void*>(&reduce_kernel<TT, CC, kTwoShot>)));
 }
-template <bool kTrace>
+template <bool kAny>
 static const void* solo_fn(int dtype, int codec, bool ef) {
-  if (ef) return CCB_DISPATCH_TC(dtype, codec, (reinterpret_cast<const void*>(&solo_kernel<TT, CC, true, kTrace>)));
-  return CCB_DISPATCH_TC(dtype, codec, (reinterpret_cast<const void*>(&solo_kernel<TT, CC, false, kTrace>)));
+  if (ef) return CCB_DISPATCH_TC(dtype, codec, (reinterpret_cast<const void*>(&solo_kernel<TT, CC, true, kAny>)));
+  return CCB_DISPATCH_TC(dtype, codec, (reinterpret_cast<const void*>(&solo_kernel<TT, CC, false, kAny>)));
 }
 static const void* exchange_fn(int dtype, int codec, bool own_direct) {
   if (!own_direct) return CCB_DISPATCH_TC(dtype, codec, (reinterpret_cast<const void*>(&exchange_kernel<TT, CC, false>)));
@@ -1046,7 +1046,13 @@ static int reduce_launch(ccb_comm* c, const void* const* send, void* const* recv
 // An all-reduce of one rank (see solo_kernel): as many CTAs as are resident at once.
 static int solo_launch(ccb_comm* c, const void* const* send, void* const* recv, float* const* ef, uint64_t count, int dtype, int codec,
                        cudaStream_t stream) {
-  const void* fn = c->trace ? solo_fn<true>(dtype, codec, ef && ef[0]) : solo_fn<false>(dtype, codec, ef && ef[0]);
+  // A grid capped at a CTA an SM or less gets CTAs of 512 threads, the size that the other kernels
+  // have: 128 Mi bf16 values in fp8 under a cap of 148 took 145 us in the two-shot kernel, 152 in
+  // CTAs of 256 threads and 102 so (cap 16: 1085, 1077, 577). From two a SM the small ones are
+  // the faster (64 Mi fp32 values, cap 200: 97 against 106 us).
+  const int threads = c->max_ctas > 0 && c->max_ctas <= c->num_sms ? kThreads : kSoloThreads;
+  const bool any = c->trace || threads != kSoloThreads;
+  const void* fn = any ? solo_fn<true>(dtype, codec, ef && ef[0]) : solo_fn<false>(dtype, codec, ef && ef[0]);
   if (!fn) {
     set_error("unsupported dtype %d / codec %d", dtype, codec);
     return CCB_ERR_UNSUPPORTED;
@@ -1059,12 +1065,12 @@ static int solo_launch(ccb_comm* c, const void* const* send, void* const* recv, 
   a.recv[0] = recv[0];
   a.ef[0] = ef ? ef[0] : nullptr;
   a.count = count;
-  const size_t blocks = (count + (size_t)kSoloThreads * kLaneElems - 1) / ((size_t)kSoloThreads * kLaneElems);
-  size_t cap = (size_t)c->num_sms * resident_ctas(fn, kSoloThreads, c->device);
+  const size_t blocks = (count + (size_t)threads * kLaneElems - 1) / ((size_t)threads * kLaneElems);
+  size_t cap = (size_t)c->num_sms * resident_ctas(fn, threads, c->device);
   if (cap > CCB_MAX_CTAS) cap = CCB_MAX_CTAS;   // a trace has a column for so many
   if (c->max_ctas > 0 && cap > (size_t)c->max_ctas) cap = (size_t)c->max_ctas;
   void* params[] = {&a};
-  cudaError_t e = cudaLaunchKernel(fn, dim3((unsigned)(blocks < cap ? blocks : cap)), dim3(kSoloThreads), params, 0, stream);
+  cudaError_t e = cudaLaunchKernel(fn, dim3((unsigned)(blocks < cap ? blocks : cap)), dim3((unsigned)threads), params, 0, stream);
   if (e != cudaSuccess) {
     set_error("kernel launch failed: %s", cudaGetErrorString(e));
     return CCB_ERR_CUDA;

@@ -53,6 +53,30 @@ def test_one_rank_error_feedback_in_place(comm, dtype, codec):
         assert torch.equal(ef.cpu(), want_ef[0])
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("codec", ["int8", "fp8", "none"])
+@pytest.mark.parametrize("cap", [1, 3, 148, 149])
+@pytest.mark.parametrize("with_ef", [False, True])
+def test_one_rank_under_a_grid_cap(comm, dtype, codec, cap, with_ef):
+    """Several turns of the look-ahead loop in both CTA sizes (512 threads up to a CTA an SM, else
+    256), in place, the last unit partial."""
+    count = (3 if cap < 100 else 2) * cap * 16 * 512 + 5 * 512 + 21
+    x = (torch.randn(count, generator=torch.Generator().manual_seed(cap)) * 3).to(dtype)
+    ef = torch.zeros(count, device="cuda") if with_ef else None
+    want_ef = [torch.zeros(count)] if with_ef else None
+    buf = torch.zeros(count + 1, dtype=dtype, device="cuda")[1:]
+    comm.set_max_ctas(cap)
+    try:
+        for _ in range(2 if with_ef else 1):
+            buf.copy_(x)
+            comm.all_reduce(buf, codec=codec, algo="twoshot", error_feedback=ef)
+            torch.cuda.synchronize()
+            assert torch.equal(buf.float().cpu(), C.simulate_all_reduce([x], codec, "twoshot", dtype, ef=want_ef))
+            assert not with_ef or torch.equal(ef.cpu(), want_ef[0])
+    finally:
+        comm.set_max_ctas(0)
+
+
 @pytest.mark.parametrize("algo", ["auto", "twoshot"])
 @pytest.mark.parametrize("count,ef", [(100, False), (8 << 20, False), (8 << 20, True)])
 def test_one_rank_trace(comm, algo, count, ef):
