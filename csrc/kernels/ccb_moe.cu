@@ -26,11 +26,13 @@ struct MoeArgs {
   uint64_t cnt[CCB_MAX_RANKS][CCB_MAX_RANKS];   // rows [src][dst] (dispatch direction)
   uint64_t hidden, tokens;
   uint64_t slot_pad, slot_bytes;          // per (src,dst) slot, elements / bytes
-  int topk, combine;
+  int topk;
   int rank0, nlocal;
 };
 
-template <class T, class C>
+// One body, two instantiations: each direction has registers of its own (as one kernel, fp32
+// without a codec spilled 92 bytes with the unit ahead; so no more than 4 anywhere).
+template <class T, class C, bool kCombine>
 __global__ void __launch_bounds__(kThreads, 2) moe_kernel(const __grid_constant__ MoeArgs a) {
   __shared__ CtaSync sync;
   const CommDev& c = a.c;
@@ -59,14 +61,14 @@ __global__ void __launch_bounds__(kThreads, 2) moe_kernel(const __grid_constant_
   // ---- send: block (r -> p). Dispatch gathers rows through perm; combine sends the
   // ---- contiguous block of rows that came from origin p (transposed counts).
   // Destinations are visited starting with the next rank, (r + 1) % n, ..., r: at any moment
-  // every rank stores to a different peer, so no inbound link takes all the traffic. Everywhere
-  // below the next unit is requested before the one in hand is converted: a unit's address
-  // hangs on an index load, and a warp that did one unit at a time waited for both in turn.
-  // A dispatch decodes its own rows where it encoded them, after the peers have been told.
-  // (8 ranks, 8192 x 4096 bf16, top 2, fp8: dispatch and combine 1106 us before, 1059 after. The
-  // staged rows make it 5.4 GB, 810 us at 6.65 TB/s.)
+  // every rank stores to a different peer, so no inbound link takes all the traffic. In both send
+  // phases and in a dispatch's receive the next unit is requested before the one in hand is
+  // converted: a unit's address may hang on an index load, and a warp that did one unit at a time
+  // waited for both in turn. A dispatch decodes its own rows where it encoded them, after the
+  // peers have been told. (8 ranks, 8192 x 4096 bf16, top 2, fp8: dispatch 583 us one unit at a
+  // time, 517 so. With the combine's 508 that is 5.4 GB of staged rows, 820 us at 6.55 TB/s.)
   auto send_block = [&](int p, auto&& deliver) {
-    const size_t rows = a.combine ? a.cnt[p][r] : a.cnt[r][p];
+    const size_t rows = kCombine ? a.cnt[p][r] : a.cnt[r][p];
     size_t base_row = 0, send_row_off = 0;  // combine: first row of origin p; dispatch: offset into perm
     for (int s = 0; s < p; ++s) {
       base_row += a.cnt[s][r];
@@ -78,7 +80,7 @@ __global__ void __launch_bounds__(kThreads, 2) moe_kernel(const __grid_constant_
     auto request = [&]() {
       size_t col;
       const size_t j = row_of(u, col);
-      const size_t srow = a.combine ? base_row + j : (size_t)a.perm[lr][send_row_off + j];
+      const size_t srow = kCombine ? base_row + j : (size_t)a.perm[lr][send_row_off + j];
       load16_wide<T>(src + srow * H, col, H, raw);
       idx = j * H + col;
     };
@@ -94,7 +96,7 @@ __global__ void __launch_bounds__(kThreads, 2) moe_kernel(const __grid_constant_
       deliver(at, pk);
     }
   };
-  for (int jd = 1; jd <= (a.combine ? n : n - 1); ++jd) {
+  for (int jd = 1; jd <= (kCombine ? n : n - 1); ++jd) {
     const int p = r + jd < n ? r + jd : r + jd - n;
     char* slot = c.arena[p] + area + (size_t)r * a.slot_bytes;
     send_block(p, [&](size_t at, const typename C::Packet& pk) { C::store(slot, pad, at, pk); });
@@ -102,9 +104,9 @@ __global__ void __launch_bounds__(kThreads, 2) moe_kernel(const __grid_constant_
   __syncthreads();
   // the combine's receiver gathers rows written by any CTA, its own rank's included,
   // so there the flag goes to this rank's own arena as well
-  if (threadIdx.x == 0) signal_peers(c, a.combine ? (1u << n) - 1u : ((1u << n) - 1u) & ~(1u << r), 0, r, b);
+  if (threadIdx.x == 0) signal_peers(c, kCombine ? (1u << n) - 1u : ((1u << n) - 1u) & ~(1u << r), 0, r, b);
 
-  if (!a.combine) {
+  if constexpr (!kCombine) {
     // ---- dispatch receive: rows of source q land at recv row (sum_{s<q} cnt[s][r]) + j
     // own rows first (nothing to wait for), then each source as its flag arrives, in the
     // order in which the sources reach this rank
@@ -143,82 +145,52 @@ __global__ void __launch_bounds__(kThreads, 2) moe_kernel(const __grid_constant_
         store16_wide<T>(to, at, at + 16, d);
       }
     }
-    return;
-  }
-
-  // ---- combine receive: wait for every CTA of every source, then gather per token
-  for (int i = threadIdx.x; i < n * G; i += kThreads) {
-    const int q = i / G, cb = i % G;
-    if (!wait_flag(flag_ptr(my, 0, q, cb), c.epoch, c, my, 0xC0 | (q << 8))) sync.fail = 1;
-  }
-  __syncthreads();
-  if (sync.fail) {
-    if (threadIdx.x == 0) broadcast_abort(c, c.epoch);
-    return;
-  }
-  const size_t units = a.tokens * upr;
-  // The (unit, expert) pairs of this warp in one sequence: the packet of the next pair is
-  // requested before the one in hand is added, and the indices of the one after that.
-  struct Pair { int q, j; float g; };
-  size_t u = (size_t)b * kWarps + warp, col = 0, u_ix = u;
-  int k_ix = 0;
-  auto indices = [&]() -> Pair {
-    Pair m = {0, 0, 0.f};
-    if (u_ix < units && a.topk > 0) {
-      size_t cc;
-      const size_t i = row_of(u_ix, cc) * a.topk + k_ix;
-      m.q = a.dest_rank[lr][i];
-      m.j = a.pos[lr][i];
-      m.g = a.gate[lr][i];
+  } else {
+    // ---- combine receive: wait for every CTA of every source, then gather per token
+    for (int i = threadIdx.x; i < n * G; i += kThreads) {
+      const int q = i / G, cb = i % G;
+      if (!wait_flag(flag_ptr(my, 0, q, cb), c.epoch, c, my, 0xC0 | (q << 8))) sync.fail = 1;
     }
-    if (++k_ix == a.topk) k_ix = 0, u_ix += (size_t)G * kWarps;
-    return m;
-  };
-  typename C::Packet nxt;
-  auto request = [&](const Pair& m, size_t unit) {
-    row_of(unit, col);
-    C::load(my + area + (size_t)m.q * a.slot_bytes, pad, (size_t)m.j * H + col, nxt);
-  };
-  Pair ahead = indices();
-  float g = 0.f;
-  if (u < units && a.topk > 0) {
-    g = ahead.g;
-    request(ahead, u);
-    ahead = indices();
-  }
-  while (u < units) {
-    float acc[16];
+    __syncthreads();
+    if (sync.fail) {
+      if (threadIdx.x == 0) broadcast_abort(c, c.epoch);
+      return;
+    }
+    const size_t units = a.tokens * upr;
+    // One pair at a time: the 16 warps of a CTA hide the loads of one another, and an index sequence
+    // that ran ahead of the packets cost more than it hid (8 ranks of 2048 x 2048 bf16 in fp8: 138
+    // us with it and 131 without at top 4, 83 and 80 at top 2, 52 and 54 at top 1).
+    for (size_t u = (size_t)b * kWarps + warp; u < units; u += (size_t)G * kWarps) {
+      size_t col;
+      const size_t tok = row_of(u, col);
+      float acc[16];
 #pragma unroll
-    for (int i = 0; i < 16; ++i) acc[i] = 0.f;
-    const size_t un = u + (size_t)G * kWarps;
-    for (int k = 0; k < a.topk; ++k) {
-      const typename C::Packet pk = nxt;
-      const float gate = g;
-      const size_t of = k + 1 < a.topk ? u : un;
-      if (of < units) {
-        g = ahead.g;
-        request(ahead, of);
-        ahead = indices();
+      for (int i = 0; i < 16; ++i) acc[i] = 0.f;
+      for (int k = 0; k < a.topk; ++k) {
+        const int q = a.dest_rank[lr][tok * a.topk + k];
+        const size_t j = (size_t)a.pos[lr][tok * a.topk + k];
+        const float g = a.gate[lr][tok * a.topk + k];
+        typename C::Packet pk;
+        C::load(my + area + (size_t)q * a.slot_bytes, pad, j * H + col, pk);
+        float d[16];
+        C::decode(pk, d);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) acc[i] += g * d[i];
       }
-      float d[16];
-      C::decode(pk, d);
-#pragma unroll
-      for (int i = 0; i < 16; ++i) acc[i] += gate * d[i];
+      store16_wide<T>(dst + tok * H, col, H, acc);
     }
-    const size_t at = u * kWarpElems + (size_t)lane * kLaneElems;
-    store16_wide<T>(dst, at, at + 16, acc);
-    u = un;
   }
 }
 
+template <bool kCombine>
 static const void* moe_fn(int dtype, int codec) {
 #define CCB_MOE_CODEC(T)                                                                              \
   switch (codec) {                                                                                    \
-    case CCB_CODEC_NONE: return reinterpret_cast<const void*>(&moe_kernel<T, CodecNone<T>>);          \
-    case CCB_CODEC_INT8: return reinterpret_cast<const void*>(&moe_kernel<T, CodecInt8<128>>);        \
-    case CCB_CODEC_INT8_G256: return reinterpret_cast<const void*>(&moe_kernel<T, CodecInt8<256>>);   \
-    case CCB_CODEC_FP8: return reinterpret_cast<const void*>(&moe_kernel<T, CodecFp8>);               \
-    case CCB_CODEC_INT4: return reinterpret_cast<const void*>(&moe_kernel<T, CodecInt4>);             \
+    case CCB_CODEC_NONE: return reinterpret_cast<const void*>(&moe_kernel<T, CodecNone<T>, kCombine>);          \
+    case CCB_CODEC_INT8: return reinterpret_cast<const void*>(&moe_kernel<T, CodecInt8<128>, kCombine>);        \
+    case CCB_CODEC_INT8_G256: return reinterpret_cast<const void*>(&moe_kernel<T, CodecInt8<256>, kCombine>);   \
+    case CCB_CODEC_FP8: return reinterpret_cast<const void*>(&moe_kernel<T, CodecFp8, kCombine>);               \
+    case CCB_CODEC_INT4: return reinterpret_cast<const void*>(&moe_kernel<T, CodecInt4, kCombine>);             \
     default: return nullptr;                                                                          \
   }
   switch (dtype) {
@@ -230,8 +202,7 @@ static const void* moe_fn(int dtype, int codec) {
   return nullptr;
 }
 
-static int moe_launch(ccb_comm* c, MoeArgs& a, int dtype, int codec, uint64_t max_rows, uint64_t work_rows, cudaStream_t stream) {
-  const void* fn = moe_fn(dtype, codec);
+static int moe_launch(ccb_comm* c, const void* fn, MoeArgs& a, int dtype, int codec, uint64_t max_rows, uint64_t work_rows, cudaStream_t stream) {
   if (!fn) {
     set_error("unsupported dtype %d / codec %d", dtype, codec);
     return CCB_ERR_UNSUPPORTED;
@@ -286,8 +257,7 @@ extern "C" int ccb_moe_dispatch(ccb_comm* c, const void* const* x, void* const* 
     a.perm[i] = perm[i];
   }
   a.hidden = hidden;
-  a.combine = 0;
-  return moe_launch(c, a, dtype, codec, mx, mx, static_cast<cudaStream_t>(stream));
+  return moe_launch(c, moe_fn<false>(dtype, codec), a, dtype, codec, mx, mx, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int ccb_moe_combine(ccb_comm* c, const void* const* y, void* const* out, const int32_t* const* dest_rank,
@@ -314,6 +284,5 @@ extern "C" int ccb_moe_combine(ccb_comm* c, const void* const* y, void* const* o
   a.hidden = hidden;
   a.tokens = tokens;
   a.topk = topk;
-  a.combine = 1;
-  return moe_launch(c, a, dtype, codec, mx, tokens > mx ? tokens : mx, static_cast<cudaStream_t>(stream));
+  return moe_launch(c, moe_fn<true>(dtype, codec), a, dtype, codec, mx, tokens > mx ? tokens : mx, static_cast<cudaStream_t>(stream));
 }
