@@ -157,6 +157,7 @@ struct ccb_comm {
   int noncoop_ctas = 0;     // grids of at most this many CTAs are launched without the cooperative attribute
   int pipe_mode = 1;        // 0 = never use the pipelined two-shot kernel, 1 = when large enough, 2 = always
   int pipe_min_chunks = 4;  // chunks (4096 elements) per CTA from which it is used
+  bool pipe_min_given = false;          // it came from the environment
   int pipe_link_warps = 20; // of the 31 data warps of a CTA, how many store over NVLink
   int pipe_mc = 0;          // phase 2 through the NVLS multicast mapping (measured slower at 2 and 4 GPUs: off)
   unsigned long long* trace = nullptr;  // device buffer, CCB_MAX_CTAS * nlocal * CCB_TRACE_SLOTS
@@ -192,6 +193,7 @@ static int finish_common(ccb_comm* c) {
   c->noncoop_ctas = (int)env_u64("CCB_NONCOOP_CTAS", 0);
   c->pipe_mode = (int)env_u64("CCB_PIPE", 1);
   c->pipe_min_chunks = (int)env_u64("CCB_PIPE_MIN_CHUNKS", 4);
+  c->pipe_min_given = env_u64("CCB_PIPE_MIN_CHUNKS", 0) != 0;
   c->pipe_link_warps = (int)env_u64("CCB_PIPE_LINK_WARPS", 20);
   if (c->pipe_link_warps < 1) c->pipe_link_warps = 1;
   if (c->pipe_link_warps > 30) c->pipe_link_warps = 30;
@@ -979,11 +981,21 @@ static int reduce_launch(ccb_comm* c, const void* const* send, void* const* recv
     const size_t ctas = chunks < (size_t)cap ? chunks : (size_t)cap;
     const size_t per_cta = ctas ? chunks / ctas : 0;
     // Several ranks on one GPU have no link whose stores could overlap with the decode, and every
-    // wave still costs its fences and flags. With 21 and 22 chunks per CTA the plain kernel is the
-    // faster one there (25 MiB buckets: all-reduce of 4 ranks with error feedback 200 us
-    // pipelined, 158 plain; reduce-scatter of 8 ranks 134 and 109); from 24 it stays as it was.
-    const size_t least = (size_t)c->pipe_min_chunks * (c->nlocal > 1 ? 6 : 1);
-    if (pfn && (per_cta >= least || c->pipe_mode == 2)) {
+    // wave still costs its fences and flags. Measured there with 2 to 8 ranks, int8, fp8, int4 and
+    // no codec, bf16 and fp32, 2 to 192 chunks a CTA: from 7 chunks the plain kernel is the faster
+    // one everywhere, by most around 24 (4 ranks, bf16 in int8: 8 chunks 48 against 55 us, 24: 97
+    // and 134, 48: 173 and 198, 192: 624 and 679), in reduce-scatters from 4. At 4 to 6 chunks the
+    // pipelined one gains where a residual adds to a 16-bit message (8 ranks: 86 against 78 us at
+    // 4 chunks, 115 against 111 at 6). From 24 chunks it is kept all the same, though it is the
+    // slower one: such a communicator stands in for one over several GPUs, and large messages
+    // (those that a small arena cuts into slices of this size among them) are to take the kernel that
+    // they take there. A smallest size that the environment gives holds as it is given.
+    bool pays = per_cta >= (size_t)c->pipe_min_chunks;
+    if (c->nlocal > 1 && !c->pipe_min_given) {
+      const bool small_ef = per_cta <= 6 && any_ef && mode == CCB_MODE_ALLREDUCE && elem_size(dtype) == 2;
+      pays = pays && (small_ef || per_cta >= 24);
+    }
+    if (pfn && (pays || c->pipe_mode == 2)) {
       // Measured at 256 MiB: two ranks are fastest with 6 waves (272 us against 283 with 8; a
       // wave is then a quarter of the data and each costs two fence-and-flag rounds), four
       // ranks with 8 (386 against 392 with 4).

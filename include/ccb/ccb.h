@@ -73,7 +73,9 @@ int ccb_comm_set_waves(ccb_comm* c, int waves);
  * current value, default 20; the rest decode); mc != 0 lets its second phase store once to the
  * NVLS multicast address when the communicator has one (off by default: measured slower than
  * per-peer stores at 2 and 4 GPUs). Also CCB_PIPE,
- * CCB_PIPE_LINK_WARPS, CCB_PIPE_MC, CCB_PIPE_MIN_CHUNKS in the environment. */
+ * CCB_PIPE_LINK_WARPS, CCB_PIPE_MC, CCB_PIPE_MIN_CHUNKS (the smallest number of chunks of 4096
+ * elements a CTA, 4 unless given; a communicator that plays several ranks on one GPU takes the
+ * pipelined kernel in mode 1 from 24, unless it is given) in the environment. */
 int ccb_comm_set_pipeline(ccb_comm* c, int mode, int link_warps, int mc);
 /* Copies the CCB_STATUS_WORDS status words; returns CCB_ERR_TIMEOUT when a kernel of
  * this communicator gave up a wait (the communicator must then be destroyed). Only

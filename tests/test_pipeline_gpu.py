@@ -207,3 +207,39 @@ def test_link_probe_methods_run_and_reject_bad_arguments():
                 _check(lib().ccb_link_probe(comm._h, bad[0], bad[1], ctypes.c_uint64(bad[2]), stream))
     finally:
         comm.close()
+
+
+@pytest.mark.parametrize("given,chunks,ef,piped", [
+    (None, 3, True, False), (None, 4, True, True), (None, 6, True, True), (None, 7, True, False), (None, 5, False, False),
+    (None, 23, True, False), (None, 24, False, True),
+    ("8", 7, False, False), ("8", 8, False, True), ("60", 59, False, False), ("1", 2, True, True),
+])
+def test_kernel_choice_of_ranks_on_one_gpu(monkeypatch, given, chunks, ef, piped):
+    """The lines between the plain and the pipelined kernel, and CCB_PIPE_MIN_CHUNKS as it is given;
+    values equal up to a flipped code in a thousand either way."""
+    n, ctas = 2, torch.cuda.get_device_properties(0).multi_processor_count // 2
+    if given:
+        monkeypatch.setenv("CCB_PIPE_MIN_CHUNKS", given)
+    else:
+        monkeypatch.delenv("CCB_PIPE_MIN_CHUNKS", raising=False)
+    count = n * chunks * ctas * 4096
+    comm = Communicator.local(n, arena_bytes=4 * count + (64 << 20))
+    try:
+        g = torch.Generator(device="cuda").manual_seed(chunks)
+        xg = [torch.randn(count, device="cuda", generator=g).to(torch.bfloat16) for _ in range(n)]
+        out = [torch.empty_like(x) for x in xg]
+        res = [torch.zeros(count, device="cuda") for _ in range(n)] if ef else None
+        comm.set_trace(True)
+        comm.all_reduce(xg, out, codec="int8", algo="twoshot", error_feedback=res)
+        torch.cuda.synchronize()
+        tr = comm.read_trace(4)
+        comm.set_trace(False)
+        assert comm.status()[0] == 0
+        assert (int(tr[0, 5]) > 0) == piped   # slot 5 is written by the pipelined kernel only
+        plain = [torch.empty_like(x) for x in xg]
+        comm.set_pipeline(0)
+        comm.all_reduce(xg, plain, codec="int8", algo="twoshot")
+        torch.cuda.synchronize()
+        assert (out[0] != plain[0]).float().mean().item() < 1e-3 and torch.equal(out[0], out[1])
+    finally:
+        comm.close()
