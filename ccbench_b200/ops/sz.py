@@ -66,9 +66,9 @@ def broadcast(comm: Communicator, send, recv, eb: float, root: int = 0, used: to
 
 
 def launch_path() -> int:
-    """How the last collective launch went: 1 = cluster + cooperative attributes accepted
-    together, 2 = the driver refused the pair and the cluster attribute was used alone, 0 =
-    no collective launched yet."""
+    """How the last collective launch went: 1 = the kernel's clusters and the cooperative attribute
+    accepted together, 2 = the driver refused the pair and the kernel was launched plainly, 0 = no
+    collective launched yet."""
     return int(_decl().ccb_sz_launch_path())
 
 

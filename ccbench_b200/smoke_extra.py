@@ -27,7 +27,9 @@ def run() -> None:
         recv = [torch.empty((n,) + tuple(f[0].shape), device=dev) for _ in range(n)]
         sz.all_gather(comm, f, recv, eb)
         torch.cuda.synchronize()
-        assert torch.equal(recv[3][0], back)
+        wrong = [(d, q, (recv[d][q] != b).nonzero().tolist()[:3]) for d, q, b in ((3, 0, back), (0, 0, back), (1, 2, recv[2][2]))
+                 if not torch.equal(recv[d][q], b)]
+        assert not wrong, f"all-gather (rank, field, first places): {wrong}, status {comm.status()}, launch path {sz.launch_path()}"
         assert max((recv[1][q] - f[q]).abs().max().item() for q in range(n)) <= eb32
 
         # MoE dispatch with fp8 rows, then combine with identity experts

@@ -498,8 +498,11 @@ constexpr unsigned int kMaxBcastWaves = 8;   // most progress steps of a broadca
 // kKind: 0 compress into a local buffer, 1 decompress from one, 2 the collectives (mode 2
 // all-gather, 3 broadcast). One body, three instantiations, so that each direction gets its
 // own register allocation and occupancy.
+// The cluster shape belongs to the kernel, not to the launch: as a launch attribute it was lost where
+// a profiler took over the collectives' cooperative launch, every CTA took itself for tile 0 of
+// its group, and seven tiles of eight were never written.
 template <int kKind>
-__global__ void __launch_bounds__(kSzThreads, kKind == 1 ? 6 : kKind == 2 ? 5 : 4) sz_kernel(const __grid_constant__ SzArgs a) {
+__global__ void __cluster_dims__(kClusterSize, 1, 1) __launch_bounds__(kSzThreads, kKind == 1 ? 6 : kKind == 2 ? 5 : 4) sz_kernel(const __grid_constant__ SzArgs a) {
   const int mode = kKind == 2 ? a.mode : kKind;
   const unsigned int kBcastWaves = a.bcast_waves;
   // Two 8 KB buffers: compress lands the next tile in one while the other is packed;
@@ -910,8 +913,8 @@ static void fill_geometry(SzArgs& a, int nx, int ny, int nz, float eb) {
   a.inv_two_eb = 1.f / a.two_eb;
 }
 
-// How the last waiting launch went: 1 = cluster + cooperative accepted, 2 = refused and
-// launched with the cluster attribute alone (co-residency then rests on the occupancy bound).
+// How the last waiting launch went: 1 = cooperative launch of the clusters accepted, 2 = refused
+// and launched plainly (co-residency then rests on the occupancy bound).
 static int g_sz_launch_path = 0;
 
 // Asking for the occupancy of a cluster launch costs more than the launch: once per kernel and device.
@@ -931,21 +934,15 @@ static int resident_clusters(void (*kernel)(const SzArgs), const cudaLaunchConfi
   return clusters;
 }
 
-// Launch with a cluster of 8 CTAs; cooperative when the kernel waits on peers.
+// Launch of clusters of 8 CTAs (__cluster_dims__); cooperative when the kernel waits on peers.
 static int sz_launch(SzArgs& a, int nlocal, int num_sms, bool waits, cudaStream_t stream) {
   void (*kernel)(const SzArgs) = a.mode == 0 ? sz_kernel<0> : a.mode == 1 ? sz_kernel<1> : sz_kernel<2>;
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof(cfg));
-  cudaLaunchAttribute attrs[2];
-  attrs[0].id = cudaLaunchAttributeClusterDimension;
-  attrs[0].val.clusterDim.x = kClusterSize;
-  attrs[0].val.clusterDim.y = 1;
-  attrs[0].val.clusterDim.z = 1;
+  cudaLaunchAttribute attr;
   cfg.blockDim = dim3(kSzThreads, 1, 1);
   cfg.dynamicSmemBytes = 0;
   cfg.stream = stream;
-  cfg.attrs = attrs;
-  cfg.numAttrs = 1;
   cfg.gridDim = dim3(kClusterSize, 1, 1);
   const int max_clusters = resident_clusters(kernel, cfg, num_sms);
   // CTAs that wait on peers must all be resident: stay within the resident clusters
@@ -955,15 +952,16 @@ static int sz_launch(SzArgs& a, int nlocal, int num_sms, bool waits, cudaStream_
   if (clusters * kClusterSize > CCB_MAX_CTAS) clusters = CCB_MAX_CTAS / kClusterSize;
   cfg.gridDim = dim3(clusters * kClusterSize, (unsigned)nlocal, 1);
   if (waits) {
-    attrs[1].id = cudaLaunchAttributeCooperative;
-    attrs[1].val.cooperative = 1;
-    cfg.numAttrs = 2;
+    attr.id = cudaLaunchAttributeCooperative;
+    attr.val.cooperative = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
   }
   cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, a);
   if (waits) g_sz_launch_path = 1;
   if (e != cudaSuccess && waits) {  // some drivers refuse cluster + cooperative: the bounded grid still fits
     (void)cudaGetLastError();
-    cfg.numAttrs = 1;
+    cfg.numAttrs = 0;
     g_sz_launch_path = 2;
     e = cudaLaunchKernelEx(&cfg, kernel, a);
   }
