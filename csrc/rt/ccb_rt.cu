@@ -1447,7 +1447,7 @@ extern "C" int ccb_test_partial_all_reduce(ccb_comm* c, const void* send, void* 
     set_error("arena too small for this call");
     return CCB_ERR_CAPACITY;
   }
-  const void* fn = reinterpret_cast<const void*>(&reduce_kernel<float, CodecNone<float>, kTwoShot>);
+  const void* fn = reinterpret_cast<const void*>(&reduce_kernel<float, CodecNone<float>, kTwoShotPlain>);
   ReduceArgs a;
   memset(&a, 0, sizeof(a));
   a.c = comm_dev(c, next_epoch(c));

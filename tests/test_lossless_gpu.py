@@ -51,6 +51,28 @@ def test_container_matches_the_restatement_and_round_trips(dtype, count):
     assert np.array_equal(LL.np_decode(got), _bits(x))
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+def test_more_than_three_tiles_a_cta(dtype):
+    """The encoder passes the widths round by the parity of the tile and holds a tile ahead: a CTA
+    (eight an SM) meets both parities twice here, and the last tile is partial. Bytes of every slot,
+    both ways of decoding."""
+    count = (4 * 8 * torch.cuda.get_device_properties(0).multi_processor_count + 3) * LL.TILE - 1000
+    x = _data(count, dtype, seed=11)
+    comp = LL.encode(x.cuda())
+    want = LL.np_encode(_bits(x), CODES[dtype])
+    got = comp.cpu().numpy()
+    assert np.array_equal(got[:32], want[:32])
+    sb = LL.slot_bytes(CODES[dtype])
+    a, b = got[32:].reshape(-1, sb), want[32:].reshape(-1, sb)
+    used = np.ascontiguousarray(b[:, :4]).view(np.uint32)
+    inside = np.arange(sb)[None, :] < used
+    assert np.array_equal(a[inside], b[inside])
+    assert np.array_equal(_bits(LL.decode(comp, count, dtype)), _bits(x))
+    acc = torch.full((count,), 1.5, dtype=dtype, device="cuda")
+    LL.decode(comp, count, dtype, out=acc, accumulate=True)
+    assert torch.equal(acc.cpu().nan_to_num(), (x.float() + 1.5).to(dtype).nan_to_num())
+
+
 def test_decode_add_and_ratio_on_gradient_like_data():
     from ccbench_b200.models.workloads import gradient_like
 

@@ -34,6 +34,33 @@ def test_exchange_at_every_offset_in_a_32_byte_line(dtype, codec):
     comm.close()
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("codec", ["none", "int8", "int4"])
+@pytest.mark.parametrize("ctas", [1, 2])
+def test_exchange_at_odd_offsets_over_several_tiles_a_cta(dtype, codec, ctas):
+    """One or two CTAs a rank: the tile ahead is requested, shifted and stored several times, in
+    blocks that differ (an all-to-all) and in one block for all (an all-gather)."""
+    n, count = 3, 4 * 16 * 512 * ctas + 3 * 512 + 11
+    comm = Communicator.local(n, arena_bytes=32 << 20)
+    comm.set_max_ctas(ctas)
+    xs = [torch.randn(n * (count + 3), generator=torch.Generator().manual_seed(r)).to(dtype) for r in range(n)]
+    xg = [x.cuda() for x in xs]
+    through = lambda v: C.roundtrip(v.float(), codec, dtype).to(dtype)
+    for shift in (1, 3, 6):
+        send_off = [[shift + d * (count + 1) for d in range(n)] for _ in range(n)]
+        recv_off = [[5 - shift % 2 + s * (count + 3) for s in range(n)] for _ in range(n)]
+        for off in (send_off, [[o[0]] * n for o in send_off]):
+            out = [torch.full((n * (count + 3) + 16,), 7.0, dtype=dtype, device="cuda") for _ in range(n)]
+            comm.exchange(xg, out, [[count] * n for _ in range(n)], off, recv_off, codec=codec)
+            torch.cuda.synchronize()
+            for d in range(n):
+                want = torch.full(out[d].shape, 7.0, dtype=dtype)
+                for s in range(n):
+                    want[recv_off[d][s]:recv_off[d][s] + count] = through(xs[s][off[s][d]:off[s][d] + count])
+                assert torch.equal(out[d].cpu(), want), (shift, d)
+    comm.close()
+
+
 def test_exchange_in_place_all_to_all_of_odd_blocks():
     n, count = 4, 3 * 512 + 1
     comm = Communicator.local(n, arena_bytes=16 << 20)
