@@ -336,15 +336,19 @@ static ncclResult_t byte_exchange(ncclComm_t comm, const char *send, const size_
 }
 
 /* ------------------------------------------------------------ collectives --- */
-/* Movement collectives see their payload as the widest element the byte count allows. */
-static int move_dtype(size_t bytes_per_block, size_t *count) {
+/* Movement collectives see their payload as fp32 words, which pass through the kernels bit by bit,
+ * where the byte count allows. An odd number of 16-bit floats goes as that type: the kernels
+ * convert it to fp32 and back, which keeps every value but not every pattern of a NaN, so no
+ * other payload may go that way (two bytes 0xff of an int8 buffer would arrive as 0x7fff). */
+static int move_dtype(size_t bytes_per_block, ncclDataType_t t, size_t *count) {
+    const int dt = fused_dtype(t);
     if (bytes_per_block % 4 == 0) {
         *count = bytes_per_block / 4;
         return CCB_F32;
     }
-    if (bytes_per_block % 2 == 0) {
+    if (dt == CCB_F16 || dt == CCB_BF16) {
         *count = bytes_per_block / 2;
-        return CCB_F16;
+        return dt;
     }
     return -1;
 }
@@ -358,7 +362,7 @@ ncclResult_t ncclAllGather(const void *sendbuff, void *recvbuff, size_t sendcoun
     if (bytes == 0) return ncclSuccess;
     const int codec = move_codec(datatype);
     size_t cnt = sendcount;
-    const int dt = codec != CCB_CODEC_NONE ? fused_dtype(datatype) : move_dtype(bytes, &cnt);
+    const int dt = codec != CCB_CODEC_NONE ? fused_dtype(datatype) : move_dtype(bytes, datatype, &cnt);
     if (dt >= 0 && comm->n > 1) {
         const void *s[1] = {sendbuff};
         void *r[1] = {recvbuff};
@@ -382,7 +386,7 @@ static ncclResult_t all_to_all(const void *sendbuff, void *recvbuff, size_t coun
     if (bytes == 0) return ncclSuccess;
     const int codec = move_codec(datatype);
     size_t cnt = count;
-    const int dt = codec != CCB_CODEC_NONE ? fused_dtype(datatype) : move_dtype(bytes, &cnt);
+    const int dt = codec != CCB_CODEC_NONE ? fused_dtype(datatype) : move_dtype(bytes, datatype, &cnt);
     if (dt >= 0 && comm->n > 1 && sendbuff != recvbuff) {
         const void *s[1] = {sendbuff};
         void *r[1] = {recvbuff};
@@ -413,7 +417,7 @@ ncclResult_t ncclBroadcast(const void *sendbuff, void *recvbuff, size_t count, n
     if (bytes == 0) return ncclSuccess;
     const int codec = move_codec(datatype);
     size_t cnt = count;
-    const int dt = codec != CCB_CODEC_NONE ? fused_dtype(datatype) : move_dtype(bytes, &cnt);
+    const int dt = codec != CCB_CODEC_NONE ? fused_dtype(datatype) : move_dtype(bytes, datatype, &cnt);
     if (dt >= 0 && comm->n > 1) {
         const void *s[1] = {sendbuff};
         void *r[1] = {recvbuff};

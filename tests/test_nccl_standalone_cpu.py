@@ -184,6 +184,18 @@ def test_collectives_choose_the_fused_kernels_the_byte_exchange_or_gather_and_fo
     assert log() == [(3, 0, 3000, 256)]
 
 
+def test_payloads_that_are_no_whole_words(provider):
+    """Three 16-bit floats travel as their type (an infinity of bf16 is a NaN pattern of fp16), six
+    bytes of anything else as bytes."""
+    L, comm, log = provider
+    s, r = 0x10000, 0x20000
+    for dtype, code in ((6, 2), (9, 1)):   # ncclFloat16, ncclBfloat16
+        assert L.ncclAllGather(s, r, 3, dtype, comm, None) == 0
+        assert log() == [(3, code, 3000, 3)]
+    assert L.ncclAllGather(s, r, 6, NCCL_INT8, comm, None) == 0
+    assert sorted(log()) == sorted([(1, p, d, 6) for p in (0, 2, 3) for d in (0, 1)] + [(2, 0, 0, 6)])
+
+
 def test_entry_points_that_are_not_served_say_so(provider):
     import ctypes
 
