@@ -383,17 +383,18 @@ __device__ __forceinline__ void rotate_up(uint32_t (&w)[4 * sizeof(T)], uint32_t
 // 32-byte accesses at a 32-byte boundary, 16-byte ones at a 16-byte boundary. At any other
 // address kAnyOffset reads 32 bytes at a time from the boundary below to the boundary above and
 // shifts them into place (each such access holds at least one byte of the lane's elements, so it
-// stays inside their allocation); without it the elements come one by one.
-template <class T, bool kAnyOffset = false>
+// stays inside their allocation); without it the elements come one by one. With kBy16 no access
+// at a 16-byte boundary is wider than that.
+template <class T, bool kAnyOffset = false, bool kBy16 = false>
 __device__ __forceinline__ void load16_wide(const T* base, size_t idx, size_t limit, Wide16<T>& raw) {
   constexpr int W = 4 * (int)sizeof(T);
   const T* p = base + idx;
   const uint32_t off = (uint32_t)(reinterpret_cast<uintptr_t>(p) & 31);
   const bool inside = idx + 16 <= limit;
-  if (inside && off == 0) {
+  if (!kBy16 && inside && off == 0) {
 #pragma unroll
     for (int k = 0; k < W; k += 8) ldg_stream32(reinterpret_cast<const char*>(p) + 4 * k, raw.w + k);
-  } else if (inside && off == 16) {
+  } else if (inside && (off & 15) == 0) {
 #pragma unroll
     for (int k = 0; k < W; k += 4) {
       const uint4 u = ldg_stream(reinterpret_cast<const char*>(p) + 4 * k);

@@ -19,10 +19,11 @@ namespace ccb {
 
 constexpr int kSaThreads = 256;
 
-// User values go in 32-byte accesses, at whatever offset a chunk starts (chunks of an odd count).
+// User values go in 32-byte accesses, at whatever offset a chunk starts (chunks of an odd count);
+// with kBy16 the encoder reads aligned ones 16 bytes at a time (see encode_t).
 // blockIdx.y selects one of several equal chunks: chunk c reads in + c * in_stride elements
 // and writes wire + c * wire_stride bytes, so that a chunked buffer is one launch.
-template <class T, class C>
+template <class T, class C, bool kBy16>
 __global__ void __launch_bounds__(kSaThreads) encode_kernel(const T* __restrict__ in, size_t count, char* wire, size_t pad,
                                                             size_t in_stride, size_t wire_stride) {
   in += (size_t)blockIdx.y * in_stride;
@@ -33,7 +34,7 @@ __global__ void __launch_bounds__(kSaThreads) encode_kernel(const T* __restrict_
   for (size_t u = warp; u < units; u += nwarps) {
     const size_t idx = u * kWarpElems + (size_t)lane * kLaneElems;
     Wide16<T> raw;
-    load16_wide<T, true>(in, idx, count, raw);
+    load16_wide<T, true, kBy16>(in, idx, count, raw);
     float v[16];
     wide16_to_f<T>(raw, v);
     typename C::Packet pk;
@@ -184,19 +185,35 @@ static dim3 sa_grid2(size_t units, size_t nchunks) {
   return dim3((unsigned)gx, (unsigned)nchunks, 1);
 }
 
+// Sixteen-byte reads are the faster ones for the integer codecs of 16-bit values and for fp32 up to
+// 32 Mi values (aligned input, B200, with them / with 32-byte ones: 64 Mi bf16 values in int4 41.0 /
+// 43.4 us, in int8 44.1 / 45.2; 16 Mi fp32 values in int4 19.9 / 21.0). The wide ones are faster for
+// more fp32 values (64 Mi in int8 67.8 / 61.2 us, 128 Mi 129.6 / 110.6), for fp8 of 16-bit values,
+// which has 32 registers with them and 37 without (64 Mi 42.8 / 40.2), and where nothing is
+// compressed (16 Mi bf16 18.0 / 17.0). Other addresses take the same path in both.
 template <class T>
 static int encode_t(int codec, const void* in, size_t count, void* wire, size_t pad, cudaStream_t s, size_t nchunks = 1,
                     size_t in_stride = 0, size_t wire_stride = 0) {
   const dim3 g = sa_grid2(pad / kWarpElems, nchunks);
-#define CCB_ENC(C) encode_kernel<T, C><<<g, kSaThreads, 0, s>>>((const T*)in, count, (char*)wire, pad, in_stride, wire_stride)
+  const bool by16 = sizeof(T) == 2 || count * nchunks < ((size_t)32 << 20);
+#define CCB_ENC(C, BY16) encode_kernel<T, C, BY16><<<g, kSaThreads, 0, s>>>((const T*)in, count, (char*)wire, pad, in_stride, wire_stride)
+#define CCB_ENC_CODEC(C)                              \
+  do {                                                \
+    if (by16) CCB_ENC(C, true);                       \
+    else CCB_ENC(C, sizeof(T) == 2); /* fp32 alone */ \
+  } while (0)
   switch (codec) {
-    case CCB_CODEC_NONE: CCB_ENC(CodecNone<T>); break;
-    case CCB_CODEC_INT8: CCB_ENC(CodecInt8<128>); break;
-    case CCB_CODEC_INT8_G256: CCB_ENC(CodecInt8<256>); break;
-    case CCB_CODEC_FP8: CCB_ENC(CodecFp8); break;
-    case CCB_CODEC_INT4: CCB_ENC(CodecInt4); break;
+    case CCB_CODEC_NONE: CCB_ENC(CodecNone<T>, false); break;
+    case CCB_CODEC_INT8: CCB_ENC_CODEC(CodecInt8<128>); break;
+    case CCB_CODEC_INT8_G256: CCB_ENC_CODEC(CodecInt8<256>); break;
+    case CCB_CODEC_FP8:
+      if (by16) CCB_ENC(CodecFp8, sizeof(T) == 4);
+      else CCB_ENC(CodecFp8, false);
+      break;
+    case CCB_CODEC_INT4: CCB_ENC_CODEC(CodecInt4); break;
     default: return CCB_ERR_UNSUPPORTED;
   }
+#undef CCB_ENC_CODEC
 #undef CCB_ENC
   return CCB_OK;
 }
@@ -266,8 +283,7 @@ extern "C" int ccb_decode_reduce(int codec, int dtype, const void* wire, uint64_
 // The same three operations on `nchunks` equal chunks in ONE launch: chunk c holds
 // chunk_count elements at element offset c * chunk_count of the plain buffer and its wire at
 // byte offset c * wire_stride (wire_stride >= ccb_wire_bytes(codec, dtype, chunk_count), a
-// multiple of 16). chunk_count must keep every chunk 16-byte aligned for the fast path;
-// other counts work through the element-wise path.
+// multiple of 16). Chunks that do not start on 16 bytes cost a little more (shifted loads).
 extern "C" int ccb_encode_chunks(int codec, int dtype, const void* in, uint64_t chunk_count, uint64_t nchunks, void* wire,
                                  uint64_t wire_stride, void* stream) {
   if (!chunk_count || !nchunks) return CCB_OK;

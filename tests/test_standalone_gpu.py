@@ -49,3 +49,22 @@ def test_reference_wire_layout(group):
     assert torch.equal(wire[ng * 4:].view(torch.int8), q)
     back = S.refwire_decode(wire.cuda(), count, torch.float32, group).cpu()
     assert torch.allclose(back, q.float() / inv.repeat_interleave(group)[:count], rtol=1e-6, atol=0)
+
+
+@pytest.mark.parametrize("dt", ["f32", "bf16", "f16"])
+@pytest.mark.parametrize("codec", ["int8", "int4", "fp8", "none"])
+@pytest.mark.parametrize("count,shift", [((32 << 20) - 512, 0), ((32 << 20) + 512 + 3, 0), (4 * 512 + 7, 4), (4 * 512 + 7, 3)])
+def test_encoder_with_either_access_width(codec, dt, count, shift):
+    """Both sides of the size at which fp32 goes to the wider reads, and starts at 0, 16 and other
+    bytes of a 32-byte line. First and last whole units bit by bit; everything within the codec's
+    step (half of it, or for fp8 a sixteenth of the value) and the type's rounding."""
+    dtype = DT[dt]
+    g = torch.Generator(device="cuda").manual_seed(count % 1000 + shift)
+    x = torch.randn(count + shift, device="cuda", generator=g).to(dtype)[shift:]
+    back = S.decode(S.encode(x, codec), codec, count, dtype)
+    last = count // 512 * 512 - 512
+    for part in (slice(0, 1024), slice(last, count)):
+        assert torch.equal(back[part].cpu(), C.roundtrip(x[part].cpu().float(), codec, dtype).to(dtype))
+    step = {"int8": 1 / 127, "int4": 1 / 7, "fp8": 1 / 8, "none": 0.0}[codec] * x.abs().max().float()
+    ulp = {"f32": 0.0, "bf16": 2.0 ** -8, "f16": 2.0 ** -11}[dt] if codec != "none" else 0.0
+    assert ((back.float() - x.float()).abs() <= step + ulp * x.float().abs()).all()
