@@ -749,7 +749,7 @@ __global__ void __cluster_dims__(kClusterSize, 1, 1) __launch_bounds__(kSzThread
 // one copy of the used bytes. As tensor operations (a mask over the group slots, a boolean
 // index into them) they passed over the slots' whole capacity, eight times the payload,
 // several times: a field of 130 x 201 x 258 took 819 us through compress, pack, unpack and
-// decompress, 208 us since (B200).
+// decompress, 159 us since (B200).
 
 // offsets[g] = sum of the (clipped) sizes before group g; offsets[ngroups] = their total,
 // offsets[ngroups + 1] = the largest size as it stands. `sizes` (u32 each) or, without them, the
