@@ -212,29 +212,29 @@ __global__ void __launch_bounds__(kThreads, 2) reduce_kernel(const __grid_consta
             C::encode(v, pk);
             C::store(dst, pad, idx, pk);
           }
-          continue;
-        }
-        for (size_t k = kb; k < ke; ++k) {
-          const size_t t = b + k * G;
-          if (!active_warp || t * tile_elems + warp_off >= valid) continue;
-          const size_t idx = t * tile_elems + lane_off;
-          float v[16];
-          load16<T>(src, idx, valid, v);
-          if (efs) {
-            float e[16];
-            load16f_plain(efs, idx, valid, e);
+        } else {
+          for (size_t k = kb; k < ke; ++k) {
+            const size_t t = b + k * G;
+            if (!active_warp || t * tile_elems + warp_off >= valid) continue;
+            const size_t idx = t * tile_elems + lane_off;
+            float v[16];
+            load16<T>(src, idx, valid, v);
+            if (efs) {
+              float e[16];
+              load16f_plain(efs, idx, valid, e);
 #pragma unroll
-            for (int i = 0; i < 16; ++i) v[i] += e[i];
-          }
-          typename C::Packet pk;
-          C::encode(v, pk);
-          C::store(dst, pad, idx, pk);
-          if (efs) {
-            float d[16];
-            C::decode(pk, d);
+              for (int i = 0; i < 16; ++i) v[i] += e[i];
+            }
+            typename C::Packet pk;
+            C::encode(v, pk);
+            C::store(dst, pad, idx, pk);
+            if (efs) {
+              float d[16];
+              C::decode(pk, d);
 #pragma unroll
-            for (int i = 0; i < 16; ++i) d[i] = v[i] - d[i];
-            store16f_plain(efs, idx, valid, d);
+              for (int i = 0; i < 16; ++i) d[i] = v[i] - d[i];
+              store16f_plain(efs, idx, valid, d);
+            }
           }
         }
       }

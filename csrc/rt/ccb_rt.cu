@@ -193,7 +193,8 @@ static int finish_common(ccb_comm* c) {
   c->noncoop_ctas = (int)env_u64("CCB_NONCOOP_CTAS", 0);
   c->pipe_mode = (int)env_u64("CCB_PIPE", 1);
   c->pipe_min_chunks = (int)env_u64("CCB_PIPE_MIN_CHUNKS", 4);
-  c->pipe_min_given = env_u64("CCB_PIPE_MIN_CHUNKS", 0) != 0;
+  const char* given = getenv("CCB_PIPE_MIN_CHUNKS");
+  c->pipe_min_given = given && *given;
   c->pipe_link_warps = (int)env_u64("CCB_PIPE_LINK_WARPS", 20);
   if (c->pipe_link_warps < 1) c->pipe_link_warps = 1;
   if (c->pipe_link_warps > 30) c->pipe_link_warps = 30;

@@ -212,7 +212,7 @@ def test_link_probe_methods_run_and_reject_bad_arguments():
 @pytest.mark.parametrize("given,chunks,ef,piped", [
     (None, 3, True, False), (None, 4, True, True), (None, 6, True, True), (None, 7, True, False), (None, 5, False, False),
     (None, 23, True, False), (None, 24, False, True),
-    ("8", 7, False, False), ("8", 8, False, True), ("60", 59, False, False), ("1", 2, True, True),
+    ("8", 7, False, False), ("8", 8, False, True), ("60", 59, False, False), ("1", 2, True, True), ("0", 5, False, True),
 ])
 def test_kernel_choice_of_ranks_on_one_gpu(monkeypatch, given, chunks, ef, piped):
     """The lines between the plain and the pipelined kernel, and CCB_PIPE_MIN_CHUNKS as it is given;
