@@ -58,7 +58,7 @@ __device__ __forceinline__ void end_handshake(CtaSync& s, const CommDev& c, int 
   __syncthreads();
 }
 
-enum { kTwoShot = 0, kOneShot = 1, kTwoShotPlain = 2 };
+enum { kTwoShot = 0, kOneShot = 1, kTwoShotPlain = 2, kOneShotOwn = 3 };
 
 // SHAPE == kOneShot: every rank stores its whole (compressed) message into every
 // arena and reduces all n copies itself: one exchange, n times the bytes; for
@@ -89,7 +89,7 @@ __global__ void __launch_bounds__(kThreads, 2) reduce_kernel(const __grid_consta
   const bool active_warp = (int)(threadIdx.x >> 5) < a.tile_warps;
   const T* send = static_cast<const T*>(a.send[lr]);
   T* recv = static_cast<T*>(a.recv[lr]);
-  float* ef = SHAPE == kTwoShotPlain ? nullptr : a.ef[lr];
+  float* ef = SHAPE == kTwoShotPlain || SHAPE == kOneShotOwn ? nullptr : a.ef[lr];
   char* my = c.arena[r];
   const size_t half = CCB_DATA_OFFSET + (size_t)(c.epoch & 1u) * c.half_bytes;
   const size_t area1 = half, area2 = half + (size_t)n * a.slot_bytes;
@@ -105,14 +105,15 @@ __global__ void __launch_bounds__(kThreads, 2) reduce_kernel(const __grid_consta
     return left < a.shard_elems ? left : a.shard_elems;
   };
 
-  if constexpr (SHAPE == kOneShot) {
+  if constexpr (SHAPE == kOneShot || SHAPE == kOneShotOwn) {
     const size_t valid = shard_valid(0);
-    // Uncompressed, the own contribution is what lies in `send`: it is read there again (by the
-    // lane that will overwrite it, if the call is in place) and not passed through the arena.
-    // Not when another rank of this process receives into `send` (own_direct is 0): its result
-    // is written as soon as this rank's flag is up. (Two ranks, 5,000,011 fp32 values each:
-    // 39.9 us through the arena, 37.3 so.)
-    const bool own_in_place = C::kId == CCB_CODEC_NONE && ef == nullptr && a.own_direct;
+    // kOneShotOwn: uncompressed, the own contribution is what lies in `send`; it is read there again
+    // (by the lane that will overwrite it, if the call is in place) and not passed through the
+    // arena. Not when another rank of this process receives into `send`: its result is written as
+    // soon as this rank's flag is up. (Two ranks, 5,000,011 fp32 values each: 39.9 us through the
+    // arena, 36.7 so.) A shape of its own: as a choice at run time it cost the calls that go
+    // through the arena 3 % (8 ranks of 65,536 bf16 values: 15.7 and 16.2 us).
+    constexpr bool own_in_place = SHAPE == kOneShotOwn;
     for (size_t t = b; t * tile_elems < valid; t += G) {
       if (!active_warp || t * tile_elems + warp_off >= valid) continue;
       const size_t idx = t * tile_elems + lane_off;

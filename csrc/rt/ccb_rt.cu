@@ -1021,16 +1021,19 @@ static int reduce_launch(ccb_comm* c, const void* const* send, void* const* recv
     a.recv[i] = static_cast<char*>(recv[i]) + recv_base * es;
     a.ef[i] = (ef && ef[i]) ? ef[i] + base : nullptr;
   }
-  if (shape == kOneShot) {
+  // Below 8 MiB over the ranks played the arena's copy of a rank's own values comes from L2 sooner
+  // than the values themselves (8 ranks of 65,536 fp32 values: 23.2 us through it, 24.6 from
+  // send; 8 ranks of 1 Mi bf16 values, 16 MiB: 69.4 and 65.0).
+  if (shape == kOneShot && codec == CCB_CODEC_NONE && !any_ef && count * es * (size_t)c->nlocal >= ((size_t)8 << 20)) {
     Span out[CCB_MAX_RANKS], in[CCB_MAX_RANKS];
     for (int i = 0; i < c->nlocal; ++i) {
       in[i] = span_of(a.send[i], 0, count * es);
       out[i] = span_of(a.recv[i], 0, count * es);
     }
-    // Below 8 MiB over the ranks played the arena's copy comes from L2 sooner than the values
-    // themselves (8 ranks of 65,536 fp32 values: 23.2 us through it, 24.6 from send; 8 ranks of
-    // 1 Mi bf16 values, 16 MiB: 69.4 and 65.0).
-    a.own_direct = count * es * (size_t)c->nlocal >= ((size_t)8 << 20) && ranks_apart(in, out, c->nlocal) ? 1 : 0;
+    if (ranks_apart(in, out, c->nlocal))
+      fn = dtype == CCB_F32    ? reinterpret_cast<const void*>(&reduce_kernel<float, CodecNone<float>, kOneShotOwn>)
+           : dtype == CCB_BF16 ? reinterpret_cast<const void*>(&reduce_kernel<__nv_bfloat16, CodecNone<__nv_bfloat16>, kOneShotOwn>)
+                               : reinterpret_cast<const void*>(&reduce_kernel<__half, CodecNone<__half>, kOneShotOwn>);
   }
   a.count = count;
   a.shard_elems = shard_elems;

@@ -88,7 +88,6 @@ typedef struct ReduceArgs {
   int row_base;               /* pipelined two-shot: first flag row of this call (0, or 8 for odd epochs when calls may overlap) */
   int link_warps;             /* pipelined two-shot: warps that store over NVLink (the rest decode, one signals) */
   int use_mc;                 /* pipelined two-shot: phase 2 stores once to the NVLS multicast address */
-  int own_direct;             /* one-shot: the own values may be read from send again after the flags */
 } ReduceArgs;
 enum { CCB_MODE_ALLREDUCE = 0, CCB_MODE_REDUCESCATTER = 1, CCB_MODE_REDUCE = 2 };
 
