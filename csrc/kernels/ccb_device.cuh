@@ -309,9 +309,9 @@ __device__ __forceinline__ void store16(T* base, size_t idx, size_t limit, const
 // 16-byte accesses at the lanes' 32- or 64-byte stride touch half of each. Their operands are
 // eight consecutive registers, so a kernel at its limit of 64 pays for them in spills, and where
 // that is worth it was measured kernel by kernel: the ring kernel spilled 64 bytes and took 242 us
-// instead of 212 (four ranks, 64 MiB of bf16 each, fp8) and does without; the fp32 exchange
-// spills 24 to 52 bytes and is the faster one at every size from 1 MiB a rank, aligned blocks too
-// (all-gather of 8 ranks of 2 Mi fp32 values in int8: 214 us with 16-byte accesses, 165 so).
+// instead of 212 (four ranks, 64 MiB of bf16 each, fp8) and does without; the fp32 exchange at
+// any offset spills 24 to 52 bytes and takes 173 us where element accesses took 574 (all-gather
+// of 8 ranks of 2,097,153 fp32 values in int8).
 __device__ __forceinline__ void ldg_stream32(const void* p, uint32_t* w) {
   asm volatile("ld.global.cs.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
                : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7]) : "l"(p));

@@ -916,9 +916,10 @@ static const void* solo_fn(int dtype, int codec, bool ef) {
   if (ef) return CCB_DISPATCH_TC(dtype, codec, (reinterpret_cast<const void*>(&solo_kernel<TT, CC, true, kAny>)));
   return CCB_DISPATCH_TC(dtype, codec, (reinterpret_cast<const void*>(&solo_kernel<TT, CC, false, kAny>)));
 }
-static const void* exchange_fn(int dtype, int codec, bool own_direct) {
-  if (!own_direct) return CCB_DISPATCH_TC(dtype, codec, (reinterpret_cast<const void*>(&exchange_kernel<TT, CC, false>)));
-  return CCB_DISPATCH_TC(dtype, codec, (reinterpret_cast<const void*>(&exchange_kernel<TT, CC, true>)));
+static const void* exchange_fn(int dtype, int codec, bool own_direct, bool aligned) {
+  if (!own_direct) return CCB_DISPATCH_TC(dtype, codec, (reinterpret_cast<const void*>(&exchange_kernel<TT, CC, false, true>)));
+  if (aligned) return CCB_DISPATCH_TC(dtype, codec, (reinterpret_cast<const void*>(&exchange_kernel<TT, CC, true, false>)));
+  return CCB_DISPATCH_TC(dtype, codec, (reinterpret_cast<const void*>(&exchange_kernel<TT, CC, true, true>)));
 }
 static const void* ring_fn(int dtype, int codec) {
   return CCB_DISPATCH_TC(dtype, codec, (reinterpret_cast<const void*>(&ring_kernel<TT, CC>)));
@@ -1306,7 +1307,7 @@ extern "C" int ccb_exchange(ccb_comm* c, const void* const* send, void* const* r
   int rc = check_alive(c);
   if (rc) return rc;
   const int n = c->nranks;
-  const void* fn = exchange_fn(dtype, codec, true);
+  const void* fn = exchange_fn(dtype, codec, true, true);
   if (!fn) {
     set_error("unsupported dtype %d / codec %d", dtype, codec);
     return CCB_ERR_UNSUPPORTED;
@@ -1341,16 +1342,18 @@ extern "C" int ccb_exchange(ccb_comm* c, const void* const* send, void* const* r
   a.ack = full ? 0 : 1;
   Span out[CCB_MAX_RANKS], in[CCB_MAX_RANKS];
   const size_t es = elem_size(dtype);
-  bool own_direct = true;
+  bool own_direct = true, aligned = true;
   for (int i = 0; i < c->nlocal; ++i) {
     const int r = c->rank0 + i;
     size_t s0 = SIZE_MAX, s1 = 0, r0 = SIZE_MAX, r1 = 0;
     for (int p = 0; p < n; ++p) {
       if (a.cnt[r][p]) {
+        aligned = aligned && span_of(send[i], a.send_off[r][p] * es, 0).lo % 16 == 0;
         s0 = std::min<size_t>(s0, a.send_off[r][p]);
         s1 = std::max<size_t>(s1, a.send_off[r][p] + a.cnt[r][p]);
       }
       if (a.cnt[p][r]) {
+        aligned = aligned && span_of(recv[i], a.recv_off[r][p] * es, 0).lo % 16 == 0;
         r0 = std::min<size_t>(r0, a.recv_off[r][p]);
         r1 = std::max<size_t>(r1, a.recv_off[r][p] + a.cnt[p][r]);
       }
@@ -1362,7 +1365,12 @@ extern "C" int ccb_exchange(ccb_comm* c, const void* const* send, void* const* r
         span_of(send[i], a.send_off[r][r] * es, 0).lo != span_of(recv[i], a.recv_off[r][r] * es, 0).lo)
       own_direct = false;
   }
-  if (!own_direct || !ranks_apart(in, out, c->nlocal)) fn = exchange_fn(dtype, codec, false);
+  own_direct = own_direct && ranks_apart(in, out, c->nlocal);
+  // Between two ranks that move 16-bit values as they are the form for any offset is the faster one
+  // (all-gather of 121,344 values 10.3 us with it and 10.9 with the aligned one; 4 ranks 13.9 and
+  // 13.2, 8 ranks 18.9 and 18.0; fp32 and the codecs gain by the aligned one everywhere).
+  if (n == 2 && codec == CCB_CODEC_NONE && es == 2) aligned = false;
+  if (!own_direct || !aligned) fn = exchange_fn(dtype, codec, own_direct, aligned);
   const int ctas = ctas_for(c, fn, maxcnt, &a.tile_warps);
   return launch(c, fn, ctas, &a, static_cast<cudaStream_t>(stream_));
 }
