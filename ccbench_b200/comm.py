@@ -1,9 +1,9 @@
 """Communicator: the Python face of libccb.so.
 
 One `Communicator` per process and GPU (`Communicator.from_torch_distributed`) or one
-that plays all ranks on a single GPU inside one cooperative launch
-(`Communicator.local`, for boxes with fewer GPUs than ranks). Every method is one
-fused kernel launch on the current torch CUDA stream.
+that plays all ranks on a single GPU inside one launch (`Communicator.local`, for boxes
+with fewer GPUs than ranks). Every method is one fused kernel launch on the current torch
+CUDA stream.
 
 The reference exposes these collectives only as interposed `nccl*` symbols
 (userconfig/wrapper_code_examples/communication/plain_nccl_compress/
@@ -61,7 +61,10 @@ class Communicator:
     # ------------------------------------------------------------ creation --
     @classmethod
     def local(cls, nranks: int, arena_bytes: int = 0, device: Optional[torch.device] = None) -> "Communicator":
-        """All `nranks` ranks on one GPU; every call takes one tensor per rank."""
+        """All `nranks` ranks on one GPU; every call takes one tensor per rank. Their calls give the
+        bits that ranks on several GPUs get, but pass no data through the arena; set_trace(True),
+        set_max_ctas(), set_waves() and set_pipeline() other than mode 1 make them take the kernels
+        of ranks on several GPUs (for traces and tests), as do buffers of the ranks that overlap."""
         device = device or torch.device("cuda", torch.cuda.current_device())
         with torch.cuda.device(device):
             h = ctypes.c_void_p()

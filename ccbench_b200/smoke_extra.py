@@ -38,32 +38,37 @@ def run() -> None:
         routes = [moe.plan_route(*(t.to(dev) for t in moe_routing(T, n, 2, seed=r, device="cpu")), n) for r in range(n)]
         cm = [rt.send_counts.tolist() for rt in routes]
         rows = [max(sum(cm[s][d] for s in range(n)), 1) for d in range(n)]
-        got = [torch.zeros(rows[d], H, dtype=dt, device=dev) for d in range(n)]
-        moe.dispatch(comm, tok, got, routes, cm, codec="fp8")
-        out = [torch.zeros(T, H, dtype=dt, device=dev) for _ in range(n)]
-        moe.combine(comm, got, out, routes, cm, codec="fp8")
-        torch.cuda.synchronize()
-        rel = ((out[0].float() - tok[0].float()).norm() / tok[0].float().norm()).item()
-        assert rel < 0.15, rel
+        for arena in (False, True):   # in registers, and by the kernels of ranks on several GPUs
+            comm.set_trace(arena)
+            got = [torch.zeros(rows[d], H, dtype=dt, device=dev) for d in range(n)]
+            moe.dispatch(comm, tok, got, routes, cm, codec="fp8")
+            out = [torch.zeros(T, H, dtype=dt, device=dev) for _ in range(n)]
+            moe.combine(comm, got, out, routes, cm, codec="fp8")
+            torch.cuda.synchronize()
+            rel = ((out[0].float() - tok[0].float()).norm() / tok[0].float().norm()).item()
+            assert rel < 0.15, rel
 
         # exchange family: all-gather with fp8 lanes, all-to-all verbatim
         per = 4096 + 3
         xs = [torch.randn(per * n, generator=torch.Generator().manual_seed(r)) for r in range(n)]
         xg = [x.to(dev) for x in xs]
-        ag = [torch.empty(per * n * n, device=dev) for _ in range(n)]
-        comm.all_gather(xg, ag, codec="fp8")
-        a2a = [torch.empty(per * n, device=dev) for _ in range(n)]
-        comm.all_to_all(xg, a2a, codec="none")
-        torch.cuda.synchronize()
-        assert torch.equal(ag[1].cpu(), torch.cat([C.roundtrip(x, "fp8") for x in xs]))
-        assert torch.equal(a2a[2].cpu(), torch.cat([x[2 * per:3 * per] for x in xs]))
+        for arena in (False, True):
+            comm.set_trace(arena)
+            ag = [torch.empty(per * n * n, device=dev) for _ in range(n)]
+            comm.all_gather(xg, ag, codec="fp8")
+            a2a = [torch.empty(per * n, device=dev) for _ in range(n)]
+            comm.all_to_all(xg, a2a, codec="none")
+            torch.cuda.synchronize()
+            assert torch.equal(ag[1].cpu(), torch.cat([C.roundtrip(x, "fp8") for x in xs]))
+            assert torch.equal(a2a[2].cpu(), torch.cat([x[2 * per:3 * per] for x in xs]))
 
-        # reduce-scatter with int8 lanes
-        rs = [torch.empty(per, device=dev) for _ in range(n)]
-        comm.reduce_scatter(xg, rs, codec="int8")
-        torch.cuda.synchronize()
-        exact = sum(x[per:2 * per].double() for x in xs).float()
-        assert ((rs[1].cpu() - exact).norm() / exact.norm()).item() < 0.03
+            # reduce-scatter with int8 lanes
+            rs = [torch.empty(per, device=dev) for _ in range(n)]
+            comm.reduce_scatter(xg, rs, codec="int8")
+            torch.cuda.synchronize()
+            exact = sum(x[per:2 * per].double() for x in xs).float()
+            assert ((rs[1].cpu() - exact).norm() / exact.norm()).item() < 0.03
+        comm.set_trace(False)
 
         # the warp-specialised pipelined two-shot kernel, forced on for a small message
         comm.set_pipeline(2)

@@ -182,16 +182,107 @@ __global__ void __launch_bounds__(kThreads, 2) moe_kernel(const __grid_constant_
   }
 }
 
-template <bool kCombine>
-static const void* moe_fn(int dtype, int codec) {
-#define CCB_MOE_CODEC(T)                                                                              \
-  switch (codec) {                                                                                    \
-    case CCB_CODEC_NONE: return reinterpret_cast<const void*>(&moe_kernel<T, CodecNone<T>, kCombine>);          \
-    case CCB_CODEC_INT8: return reinterpret_cast<const void*>(&moe_kernel<T, CodecInt8<128>, kCombine>);        \
-    case CCB_CODEC_INT8_G256: return reinterpret_cast<const void*>(&moe_kernel<T, CodecInt8<256>, kCombine>);   \
-    case CCB_CODEC_FP8: return reinterpret_cast<const void*>(&moe_kernel<T, CodecFp8, kCombine>);               \
-    case CCB_CODEC_INT4: return reinterpret_cast<const void*>(&moe_kernel<T, CodecInt4, kCombine>);             \
-    default: return nullptr;                                                                          \
+// Ranks that share one GPU (see ccb_local.cuh): rows go from the senders' tensors to the receivers'
+// through the codec in registers, without staging and flags.
+struct MoeLocalArgs {
+  const void* src[CCB_MAX_RANKS];
+  void* dst[CCB_MAX_RANKS];
+  const int32_t* perm[CCB_MAX_RANKS];
+  const int32_t* dest_rank[CCB_MAX_RANKS];
+  const int32_t* pos[CCB_MAX_RANKS];
+  const float* gate[CCB_MAX_RANKS];
+  uint32_t cnt[CCB_MAX_RANKS][CCB_MAX_RANKS];      // rows [src][dst]
+  uint32_t first_in[CCB_MAX_RANKS][CCB_MAX_RANKS];   // [holder][origin]: first row of that origin in the holder's buffer
+  uint32_t first_out[CCB_MAX_RANKS][CCB_MAX_RANKS];  // [src][dst]: first entry of that block in perm
+  uint64_t hidden;
+  uint32_t tokens, row_units, chunk_rows, chunks;
+  int topk, n;
+};
+constexpr int kMoeLocalThreads = 256;
+
+// Dispatch. The rows of a rank are sorted by destination, and within one by token. A CTA takes
+// `chunk_rows` rows of one block; the blocks of a rank take turns chunk by chunk, so that the topk
+// copies of a token, which lie at about the same depth of their blocks, are read from memory once
+// and from L2 after that.
+template <class T, class C>
+__global__ void __launch_bounds__(kMoeLocalThreads, sizeof(T) == 4 ? 3 : 4) moe_local_dispatch_kernel(const __grid_constant__ MoeLocalArgs a) {
+  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+  const uint32_t n = (uint32_t)a.n, upr = a.row_units;
+  const uint32_t p = blockIdx.x % n, c = blockIdx.x / n % a.chunks, r = blockIdx.x / n / a.chunks;
+  const uint32_t j0 = c * a.chunk_rows, rows = a.cnt[r][p];
+  if (j0 >= rows) return;
+  const uint32_t units = min(a.chunk_rows, rows - j0) * upr;
+  const T* src = static_cast<const T*>(a.src[r]);
+  const int32_t* perm = a.perm[r] + a.first_out[r][p] + j0;
+  T* dst = static_cast<T*>(a.dst[p]) + (size_t)(a.first_in[p][r] + j0) * a.hidden;   // unit u of whole rows starts at element 512 u
+  Wide16<T> raw;
+  auto request = [&](uint32_t u) {
+    const uint32_t j = u / upr;
+    load16_wide<T>(src + (size_t)perm[j] * a.hidden, (size_t)(u - j * upr) * kWarpElems + lane * kLaneElems, a.hidden, raw);
+  };
+  uint32_t u = warp;
+  if (u < units) request(u);
+  while (u < units) {
+    float v[16];
+    wide16_to_f<T>(raw, v);
+    const size_t at = (size_t)u * kWarpElems + lane * kLaneElems;
+    u += warps;
+    if (u < units) request(u);
+    typename C::Packet pk;
+    C::encode(v, pk);
+    C::decode(pk, v);
+    store16_wide<T>(dst, at, at + 16, v);
+  }
+}
+
+// Combine: a warp takes 512 elements of one token and fetches them from the topk rows that hold it.
+// An index outside its block (the entry of a dropped pair) contributes nothing.
+template <class T, class C>
+__global__ void __launch_bounds__(kMoeLocalThreads, sizeof(T) == 4 ? 3 : 4) moe_local_combine_kernel(const __grid_constant__ MoeLocalArgs a) {
+  const uint32_t lane = threadIdx.x & 31, upr = a.row_units;
+  const uint32_t step = (gridDim.x * blockDim.x) >> 5, per_rank = a.tokens * upr;
+  for (uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < per_rank * (uint32_t)a.n; w += step) {
+    const uint32_t r = w / per_rank, u = w - r * per_rank, tok = u / upr;
+    const size_t col = (size_t)(u - tok * upr) * kWarpElems + lane * kLaneElems;
+    const size_t pair0 = (size_t)tok * a.topk;
+    Wide16<T> next;
+    bool have = false;
+    auto request = [&](int k) {
+      const uint32_t q = (uint32_t)a.dest_rank[r][pair0 + k], j = (uint32_t)a.pos[r][pair0 + k];
+      have = q < (uint32_t)a.n && j < a.cnt[r][q];
+      if (have) load16_wide<T>(static_cast<const T*>(a.src[q]) + (size_t)(a.first_in[q][r] + j) * a.hidden, col, a.hidden, next);
+    };
+    float acc[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) acc[i] = 0.f;
+    if (a.topk > 0) request(0);
+    for (int k = 0; k < a.topk; ++k) {
+      const bool now = have;
+      float d[16];
+      wide16_to_f<T>(next, d);
+      const float g = a.gate[r][pair0 + k];
+      if (k + 1 < a.topk) request(k + 1);
+      if (!now) continue;
+      typename C::Packet pk;
+      C::encode(d, pk);
+      C::decode(pk, d);
+#pragma unroll
+      for (int i = 0; i < 16; ++i) acc[i] += g * d[i];
+    }
+    store16_wide<T>(static_cast<T*>(a.dst[r]) + (size_t)tok * a.hidden, col, a.hidden, acc);
+  }
+}
+
+template <template <class, class> class K>
+static const void* moe_by_type(int dtype, int codec) {
+#define CCB_MOE_CODEC(T)                                                  \
+  switch (codec) {                                                        \
+    case CCB_CODEC_NONE: return K<T, CodecNone<T>>::fn();                 \
+    case CCB_CODEC_INT8: return K<T, CodecInt8<128>>::fn();               \
+    case CCB_CODEC_INT8_G256: return K<T, CodecInt8<256>>::fn();          \
+    case CCB_CODEC_FP8: return K<T, CodecFp8>::fn();                      \
+    case CCB_CODEC_INT4: return K<T, CodecInt4>::fn();                    \
+    default: return nullptr;                                              \
   }
   switch (dtype) {
     case CCB_F32: CCB_MOE_CODEC(float)
@@ -201,8 +292,63 @@ static const void* moe_fn(int dtype, int codec) {
 #undef CCB_MOE_CODEC
   return nullptr;
 }
+template <class T, class C> struct MoeDispatch { static const void* fn() { return reinterpret_cast<const void*>(&moe_kernel<T, C, false>); } };
+template <class T, class C> struct MoeCombine { static const void* fn() { return reinterpret_cast<const void*>(&moe_kernel<T, C, true>); } };
+template <class T, class C> struct MoeLocalDispatch { static const void* fn() { return reinterpret_cast<const void*>(&moe_local_dispatch_kernel<T, C>); } };
+template <class T, class C> struct MoeLocalCombine { static const void* fn() { return reinterpret_cast<const void*>(&moe_local_combine_kernel<T, C>); } };
 
-static int moe_launch(ccb_comm* c, const void* fn, MoeArgs& a, int dtype, int codec, uint64_t max_rows, uint64_t work_rows, cudaStream_t stream) {
+static int moe_local_launch(ccb_comm* c, const MoeArgs& m, bool combine, int dtype, int codec, uint64_t max_rows, cudaStream_t stream) {
+  MoeLocalArgs a;
+  memset(&a, 0, sizeof(a));
+  a.n = ccb_comm_nranks(c);
+  for (int i = 0; i < a.n; ++i) {
+    a.src[i] = m.src[i];
+    a.dst[i] = m.dst[i];
+    a.perm[i] = m.perm[i];
+    a.dest_rank[i] = m.dest_rank[i];
+    a.pos[i] = m.pos[i];
+    a.gate[i] = m.gate[i];
+    for (int k = 0; k < a.n; ++k) {
+      a.cnt[i][k] = (uint32_t)m.cnt[i][k];
+      for (int s = 0; s < k; ++s) {
+        a.first_in[i][k] += (uint32_t)m.cnt[s][i];
+        a.first_out[i][k] += (uint32_t)m.cnt[i][s];
+      }
+    }
+  }
+  a.hidden = m.hidden;
+  a.row_units = (uint32_t)(m.hidden / kWarpElems);
+  a.tokens = (uint32_t)m.tokens;
+  a.topk = m.topk;
+  const uint64_t sms = (uint64_t)comm_sms(c);
+  uint64_t ctas, warps = kMoeLocalThreads / 32;
+  if (combine) {
+    const uint64_t units = (uint64_t)a.n * m.tokens * a.row_units;
+    while (warps > 1 && units / warps < sms) warps >>= 1;
+    ctas = (units + warps - 1) / warps;
+    if (ctas > (1u << 20)) ctas = 1u << 20;
+  } else {
+    // Chunks of up to 64 units (eight for each warp), smaller where the blocks would not fill the chip twice.
+    uint64_t rows = 64 / a.row_units;
+    if (rows < 1) rows = 1;
+    while (rows > 1 && (uint64_t)a.n * a.n * ((max_rows + rows - 1) / rows) < 8 * sms) rows >>= 1;
+    a.chunk_rows = (uint32_t)rows;
+    a.chunks = (uint32_t)((max_rows + rows - 1) / rows);
+    ctas = (uint64_t)a.n * a.n * a.chunks;
+  }
+  if (ctas == 0) return CCB_OK;
+  const void* fn = combine ? moe_by_type<MoeLocalCombine>(dtype, codec) : moe_by_type<MoeLocalDispatch>(dtype, codec);
+  void* params[] = {&a};
+  const cudaError_t e = cudaLaunchKernel(fn, dim3((unsigned)ctas), dim3((unsigned)(32 * warps)), params, 0, stream);
+  if (e != cudaSuccess) {
+    set_error("kernel launch failed: %s", cudaGetErrorString(e));
+    return CCB_ERR_CUDA;
+  }
+  count_launch();
+  return CCB_OK;
+}
+
+static int moe_launch(ccb_comm* c, const void* fn, MoeArgs& a, bool combine, int dtype, int codec, uint64_t max_rows, uint64_t work_rows, cudaStream_t stream) {
   if (!fn) {
     set_error("unsupported dtype %d / codec %d", dtype, codec);
     return CCB_ERR_UNSUPPORTED;
@@ -220,14 +366,31 @@ static int moe_launch(ccb_comm* c, const void* fn, MoeArgs& a, int dtype, int co
               (unsigned long long)((uint64_t)n * a.slot_bytes * 2));
     return CCB_ERR_CAPACITY;
   }
-  a.c = comm_dev(c, next_epoch(c));
-  a.rank0 = ccb_comm_rank(c);
-  a.nlocal = ccb_comm_nlocal(c);
   const size_t units = (size_t)work_rows * (a.hidden / kWarpElems);
   if (units >> 32 || ((uint64_t)max_rows * (a.hidden / kWarpElems)) >> 32) {  // the kernel indexes units with 32 bits
     set_error("MoE block too large: %llu rows of %llu elements", (unsigned long long)work_rows, (unsigned long long)a.hidden);
     return CCB_ERR_CAPACITY;
   }
+  // The kernels above index all ranks' units, and the rows of a buffer, with 32 bits. A combine over
+  // the arena has read all rows before it writes a token, so there its results may lie on the rows.
+  // (A dispatch has not, there or here: its results may not lie on what the ranks send.)
+  uint64_t all_rows = 0;
+  bool apart = true;
+  for (int s = 0; s < n; ++s) {
+    uint64_t rows = 0;
+    for (int d = 0; d < n; ++d) rows += a.cnt[d][s];
+    all_rows += rows;
+    const uint64_t row_bytes = a.hidden * elem_size(dtype);
+    for (int d = 0; combine && d < n; ++d) {
+      const uintptr_t y = reinterpret_cast<uintptr_t>(a.src[s]), out = reinterpret_cast<uintptr_t>(a.dst[d]);
+      apart = apart && !(y < out + a.tokens * row_bytes && out < y + rows * row_bytes);
+    }
+  }
+  if (ranks_in_registers(c) && apart && !(((all_rows + (uint64_t)n * a.tokens) * (a.hidden / kWarpElems)) >> 31))
+    return moe_local_launch(c, a, combine, dtype, codec, max_rows, stream);
+  a.c = comm_dev(c, next_epoch(c));
+  a.rank0 = ccb_comm_rank(c);
+  a.nlocal = ccb_comm_nlocal(c);
   size_t tiles = (units + kWarps - 1) / kWarps;
   int cap = grid_cap(c, fn);
   if (tiles < 1) tiles = 1;
@@ -257,7 +420,7 @@ extern "C" int ccb_moe_dispatch(ccb_comm* c, const void* const* x, void* const* 
     a.perm[i] = perm[i];
   }
   a.hidden = hidden;
-  return moe_launch(c, moe_fn<false>(dtype, codec), a, dtype, codec, mx, mx, static_cast<cudaStream_t>(stream));
+  return moe_launch(c, moe_by_type<MoeDispatch>(dtype, codec), a, false, dtype, codec, mx, mx, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int ccb_moe_combine(ccb_comm* c, const void* const* y, void* const* out, const int32_t* const* dest_rank,
@@ -284,5 +447,5 @@ extern "C" int ccb_moe_combine(ccb_comm* c, const void* const* y, void* const* o
   a.hidden = hidden;
   a.tokens = tokens;
   a.topk = topk;
-  return moe_launch(c, moe_fn<true>(dtype, codec), a, dtype, codec, mx, tokens > mx ? tokens : mx, static_cast<cudaStream_t>(stream));
+  return moe_launch(c, moe_by_type<MoeCombine>(dtype, codec), a, true, dtype, codec, mx, tokens > mx ? tokens : mx, static_cast<cudaStream_t>(stream));
 }

@@ -25,6 +25,7 @@
 #include "../kernels/ccb_nvls.cuh"
 #include "../kernels/ccb_p2p.cuh"
 #include "../kernels/ccb_linkprobe.cuh"
+#include "../kernels/ccb_local.cuh"
 #include "../kernels/ccb_reduce.cuh"
 #include "../kernels/ccb_ring.cuh"
 #include "ccb/ccb.h"
@@ -960,6 +961,31 @@ static bool ranks_apart(const Span* send, const Span* recv, int nlocal) {
   return true;
 }
 
+// All ranks of the communicator are played by this process on one GPU: their calls need no arena
+// (csrc/kernels/ccb_local.cuh). What a communicator has been told about the kernels that talk over
+// peer memory (a phase trace, a grid cap, waves, the pipelined kernel's mode or smallest size) asks
+// for those kernels, so that they can be traced and tested on one GPU.
+bool ranks_in_registers(const ccb_comm* c) {
+  return c->nlocal == c->nranks && !c->trace && c->max_ctas <= 0 && c->waves <= 0 && c->pipe_mode == 1 && !c->pipe_min_given;
+}
+int comm_sms(const ccb_comm* c) { return c->num_sms; }
+
+// A warp reads an element from every rank that contributes to it and then writes every result of
+// it, so a rank's result may lie exactly on the elements it comes from; any other meeting of what
+// is read and what is written wants the order that the flags of the other kernels give.
+static bool reduces_in_registers(const ccb_comm* c, const ReduceArgs& a, size_t es) {
+  if (!ranks_in_registers(c)) return false;
+  Span in[CCB_MAX_RANKS], out[CCB_MAX_RANKS];
+  for (int i = 0; i < c->nlocal; ++i) {
+    const bool scatter = a.mode == CCB_MODE_REDUCESCATTER, gets = a.mode != CCB_MODE_REDUCE || i == a.root;
+    in[i] = span_of(a.send[i], 0, a.count * es);
+    out[i] = gets ? span_of(a.recv[i], 0, (scatter ? a.shard_elems : a.count) * es) : Span{0, 0};
+    const bool meets = in[i].lo < out[i].hi && out[i].lo < in[i].hi;
+    if (meets && out[i].lo != in[i].lo + (scatter ? (size_t)i * a.shard_elems * es : 0)) return false;
+  }
+  return ranks_apart(in, out, c->nlocal);
+}
+
 // One launch of the reduce family on `count` elements starting at element `base`
 // of every buffer (base is a multiple of 512, so vector alignment is preserved).
 static int reduce_launch(ccb_comm* c, const void* const* send, void* const* recv, float* const* ef, size_t base,
@@ -972,6 +998,24 @@ static int reduce_launch(ccb_comm* c, const void* const* send, void* const* recv
     set_error("unsupported dtype %d / codec %d", dtype, codec);
     return CCB_ERR_UNSUPPORTED;
   }
+  const size_t es = elem_size(dtype);
+  ReduceArgs a;
+  memset(&a, 0, sizeof(a));
+  a.c.nranks = c->nranks;
+  for (int i = 0; i < c->nlocal; ++i) {
+    a.send[i] = static_cast<const char*>(send[i]) + base * es;
+    a.recv[i] = static_cast<char*>(recv[i]) + recv_base * es;
+    a.ef[i] = (ef && ef[i]) ? ef[i] + base : nullptr;
+  }
+  a.count = count;
+  a.shard_elems = shard_elems;
+  a.rank0 = c->rank0;
+  a.nlocal = c->nlocal;
+  a.op = op;
+  a.root = root;
+  a.mode = mode;
+  if (reduces_in_registers(c, a, es))
+    return local_reduce(c, a, mode != CCB_MODE_ALLREDUCE ? kLocalScatter : shape == kOneShot ? kLocalOneShot : kLocalTwoShot, dtype, codec, stream);
   // Large two-shot AllReduce / ReduceScatter calls go to the warp-specialised pipelined
   // kernel: it needs a few chunks (8 units of 512 elements) per CTA and wave to pay.
   int pipe_waves = 0, pipe_ctas = 0;
@@ -982,16 +1026,16 @@ static int reduce_launch(ccb_comm* c, const void* const* send, void* const* recv
     const size_t chunks = (per + kPipeChunkElems - 1) / kPipeChunkElems;
     const size_t ctas = chunks < (size_t)cap ? chunks : (size_t)cap;
     const size_t per_cta = ctas ? chunks / ctas : 0;
-    // Several ranks on one GPU have no link whose stores could overlap with the decode, and every
+    // Several ranks on one GPU (they come here for a trace, a schedule that was asked for, or buffers
+    // that overlap) have no link whose stores could overlap with the decode, and every
     // wave still costs its fences and flags. Measured there with 2 to 8 ranks, int8, fp8, int4 and
     // no codec, bf16 and fp32, 2 to 192 chunks a CTA: from 7 chunks the plain kernel is the faster
     // one everywhere, by most around 24 (4 ranks, bf16 in int8: 8 chunks 48 against 55 us, 24: 97
     // and 134, 48: 173 and 198, 192: 624 and 679), in reduce-scatters from 4. At 4 to 6 chunks the
     // pipelined one gains where a residual adds to a 16-bit message (8 ranks: 86 against 78 us at
     // 4 chunks, 115 against 111 at 6). From 24 chunks it is kept all the same, though it is the
-    // slower one: such a communicator stands in for one over several GPUs, and large messages
-    // (those that a small arena cuts into slices of this size among them) are to take the kernel that
-    // they take there. A smallest size that the environment gives holds as it is given.
+    // slower one: what is traced and tested on one GPU is to be the kernel that large messages
+    // (those that a small arena cuts into slices of this size among them) take on several. A smallest size that the environment gives holds as it is given.
     bool pays = per_cta >= (size_t)c->pipe_min_chunks;
     if (c->nlocal > 1 && !c->pipe_min_given) {
       const bool small_ef = per_cta <= 6 && any_ef && mode == CCB_MODE_ALLREDUCE && elem_size(dtype) == 2;
@@ -1013,15 +1057,7 @@ static int reduce_launch(ccb_comm* c, const void* const* send, void* const* recv
       fn = pfn;
     }
   }
-  ReduceArgs a;
-  memset(&a, 0, sizeof(a));
   a.c = comm_dev(c, next_epoch(c));
-  const size_t es = elem_size(dtype);
-  for (int i = 0; i < c->nlocal; ++i) {
-    a.send[i] = static_cast<const char*>(send[i]) + base * es;
-    a.recv[i] = static_cast<char*>(recv[i]) + recv_base * es;
-    a.ef[i] = (ef && ef[i]) ? ef[i] + base : nullptr;
-  }
   // Below 8 MiB over the ranks played the arena's copy of a rank's own values comes from L2 sooner
   // than the values themselves (8 ranks of 65,536 fp32 values: 23.2 us through it, 24.6 from
   // send; 8 ranks of 1 Mi bf16 values, 16 MiB: 69.4 and 65.0).
@@ -1036,15 +1072,8 @@ static int reduce_launch(ccb_comm* c, const void* const* send, void* const* recv
            : dtype == CCB_BF16 ? reinterpret_cast<const void*>(&reduce_kernel<__nv_bfloat16, CodecNone<__nv_bfloat16>, kOneShotOwn>)
                                : reinterpret_cast<const void*>(&reduce_kernel<__half, CodecNone<__half>, kOneShotOwn>);
   }
-  a.count = count;
-  a.shard_elems = shard_elems;
   a.shard_pad = round_up(shard_elems, kWarpElems);
   a.slot_bytes = codec_slot_bytes(codec, dtype, a.shard_pad);
-  a.rank0 = c->rank0;
-  a.nlocal = c->nlocal;
-  a.op = op;
-  a.root = root;
-  a.mode = mode;
   if (pipe_waves) {
     a.waves = pipe_waves;
     a.tile_warps = kWarps;
@@ -1210,7 +1239,7 @@ extern "C" int ccb_all_reduce(ccb_comm* c, const void* const* send, void* const*
       if (slice > left) slice = left;
       ReduceArgs a;
       memset(&a, 0, sizeof(a));
-      a.c = comm_dev(c, next_epoch(c));
+      a.c.nranks = n;
       for (int i = 0; i < c->nlocal; ++i) {
         a.send[i] = static_cast<const char*>(send[i]) + done * es;
         a.recv[i] = static_cast<char*>(recv[i]) + done * es;
@@ -1228,8 +1257,13 @@ extern "C" int ccb_all_reduce(ccb_comm* c, const void* const* send, void* const*
       a.nlocal = c->nlocal;
       a.op = op;
       a.mode = CCB_MODE_ALLREDUCE;
-      const int ctas = ctas_for(c, fn, a.shard_elems < slice ? a.shard_elems : slice, &a.tile_warps);
-      rc = launch(c, fn, ctas, &a, stream);
+      if (reduces_in_registers(c, a, es)) {
+        rc = local_reduce(c, a, algo == CCB_ALGO_RING ? kLocalRing : kLocalTree, dtype, codec, stream);
+      } else {
+        a.c = comm_dev(c, next_epoch(c));
+        const int ctas = ctas_for(c, fn, a.shard_elems < slice ? a.shard_elems : slice, &a.tile_warps);
+        rc = launch(c, fn, ctas, &a, stream);
+      }
       if (rc) return rc;
       done += slice;
     }
@@ -1332,7 +1366,6 @@ extern "C" int ccb_exchange(ccb_comm* c, const void* const* send, void* const* r
               (unsigned long long)((size_t)n * a.slot_bytes));
     return CCB_ERR_CAPACITY;
   }
-  a.c = comm_dev(c, next_epoch(c));
   for (int i = 0; i < c->nlocal; ++i) {
     a.send[i] = send[i];
     a.recv[i] = recv[i];
@@ -1342,7 +1375,7 @@ extern "C" int ccb_exchange(ccb_comm* c, const void* const* send, void* const* r
   a.ack = full ? 0 : 1;
   Span out[CCB_MAX_RANKS], in[CCB_MAX_RANKS];
   const size_t es = elem_size(dtype);
-  bool own_direct = true, aligned = true;
+  bool own_direct = true, aligned = true, in_registers = ranks_in_registers(c);
   for (int i = 0; i < c->nlocal; ++i) {
     const int r = c->rank0 + i;
     size_t s0 = SIZE_MAX, s1 = 0, r0 = SIZE_MAX, r1 = 0;
@@ -1361,11 +1394,20 @@ extern "C" int ccb_exchange(ccb_comm* c, const void* const* send, void* const* r
     in[i] = s1 ? span_of(send[i], s0 * es, s1 * es) : Span{0, 0};
     out[i] = r1 ? span_of(recv[i], r0 * es, r1 * es) : Span{0, 0};
     // a rank's own buffers may meet too, if its own block stays where it is (the calls in place)
-    if (a.cnt[r][r] && in[i].lo < out[i].hi && out[i].lo < in[i].hi &&
-        span_of(send[i], a.send_off[r][r] * es, 0).lo != span_of(recv[i], a.recv_off[r][r] * es, 0).lo)
-      own_direct = false;
+    const bool meet = in[i].lo < out[i].hi && out[i].lo < in[i].hi;
+    const Span mine = span_of(send[i], a.send_off[r][r] * es, (a.send_off[r][r] + a.cnt[r][r]) * es);
+    const bool in_place = a.cnt[r][r] && mine.lo == span_of(recv[i], a.recv_off[r][r] * es, 0).lo;
+    if (a.cnt[r][r] && meet && !in_place) own_direct = false;
+    // without an arena all that this rank sends has to be its own block (an all-gather in place)
+    if (meet && !(in_place && in[i].lo == mine.lo && in[i].hi == mine.hi)) in_registers = false;
   }
-  own_direct = own_direct && ranks_apart(in, out, c->nlocal);
+  const bool apart = ranks_apart(in, out, c->nlocal);
+  own_direct = own_direct && apart;
+  if (in_registers && apart) {
+    a.c.nranks = n;
+    return local_exchange(c, a, aligned, dtype, codec, static_cast<cudaStream_t>(stream_));
+  }
+  a.c = comm_dev(c, next_epoch(c));
   // Between two ranks that move 16-bit values as they are the form for any offset is the faster one
   // (all-gather of 121,344 values 10.3 us with it and 10.9 with the aligned one; 4 ranks 13.9 and
   // 13.2, 8 ranks 18.9 and 18.0; fp32 and the codecs gain by the aligned one everywhere).

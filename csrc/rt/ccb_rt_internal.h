@@ -21,6 +21,12 @@ size_t codec_slot_bytes(int codec, int dtype, size_t pad);
 constexpr int kPipeChunkElems = 4096;
 const void* pipe_kernel_fn(int dtype, int codec);
 int pipe_kernel_threads();
+// Ranks that share one GPU (csrc/kernels/ccb_local.cu). ranks_in_registers(): all ranks of the
+// communicator are this process's and nothing asks for the schedule of ranks on several GPUs.
+bool ranks_in_registers(const ccb_comm* c);
+int comm_sms(const ccb_comm* c);
+int local_reduce(ccb_comm* c, const ReduceArgs& r, int algo, int dtype, int codec, cudaStream_t stream);
+int local_exchange(ccb_comm* c, const ExchangeArgs& x, bool aligned, int dtype, int codec, cudaStream_t stream);
 int nvls_all_reduce(ccb_comm* c, const void* const* send, void* const* recv, uint64_t count, int dtype, int op,
                     cudaStream_t stream);
 }  // namespace ccb

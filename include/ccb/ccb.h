@@ -8,7 +8,7 @@
  *
  * `send`, `recv` and `ef` are arrays with one pointer per LOCAL rank: one entry in
  * the normal one-process-per-GPU case, `nranks` entries for a communicator made by
- * ccb_comm_create_local(), which plays all ranks inside a single cooperative launch
+ * ccb_comm_create_local(), which plays all ranks inside a single launch
  * on one GPU (used for tests on boxes with fewer GPUs than ranks).
  *
  * Calls on one communicator must be issued in the same order on every rank and are
