@@ -8,6 +8,10 @@
 // ones for ranks on several GPUs, and a local communicator takes them where their schedule is
 // asked for (a phase trace, a grid cap, waves, a pipeline mode) and where the ranks' buffers
 // overlap: see ranks_in_registers() and its callers in the runtime.
+//
+// All of them are bound by memory, or by the instructions of the codec where many ranks contribute.
+// A warp does one unit and ends: nothing is carried, registers stay few, and the hardware hands out
+// CTAs in the order of the addresses.
 #pragma once
 #include "ccb_codec.cuh"
 
@@ -25,52 +29,78 @@ struct LocalReduceArgs {
   uint64_t shard_elems;        // distance of the shards in the send buffers
   uint32_t units;              // warps' units of 512 elements in the whole call
   uint32_t shard_units;        // units of one shard
-  int wide;                    // every buffer starts on 32 bytes (or kAnyOffset)
   int n, op, root;             // root: kLocalScatter delivers to this rank alone (>= 0), or shard s to rank s (< 0)
 };
 
 // Ranks whose values are requested before the first is used, and CTAs of 256 threads on an SM: what
-// was fastest of one to four ranks at 64, 80 and 128 registers a thread. (B200; 4 ranks of 64 MiB
-// of bf16, ring, fp8: two ranks at 64 registers 83 us, four at 80 registers 98, one 92. 8 ranks of
-// 25 MiB to their owners in int8: 51, 70, 57. Shards at odd places, one rank at a time 70 us, two
-// 76. 2 ranks of 5,000,011 fp32 values: two at 128 registers 12.6, at 64 17.3. 4 ranks of 25 MiB
-// with residuals: one at 128 registers 102, two 112, one at 80 114: those spill.)
+// was fastest of one, two and four ranks at 40 to 128 registers a thread, where nothing spills.
+// (B200. 4 ranks of 64 MiB of bf16, two-shot int8: two ranks at 64 registers 82.4 us, at 48, which
+// spill, 105, four at 80 123. 8 ranks of 25 MiB to their owners: 43.3; one rank at 48 53. Shards at
+// odd places: one at 64 registers 66, two 70. 2 ranks of 5,000,011 fp32 values: one at 64 10.5, two
+// at 128 12.6. 4 ranks of 25 MiB of bf16 with residuals: two at 128 registers 96.7, one 100.6.)
 template <class T, int ALGO, bool kEf, bool kAnyOffset> struct LocalShape {
-  static constexpr int kBatch = kEf || kAnyOffset ? 1 : 2;
-  static constexpr int kCtas = kEf || sizeof(T) == 4 ? 2 : ALGO == kLocalTree ? 3 : 4;
+  static constexpr int kBatch = sizeof(T) == 4 || kAnyOffset ? 1 : 2;
+  static constexpr int kCtas = kEf ? 2 : (ALGO == kLocalTree ? 3 : 4) - (sizeof(T) == 4 && (kAnyOffset || ALGO == kLocalTree) ? 1 : 0);
 };
 
-// kInside: the unit lies inside the message, and (but for kAnyOffset) on 32 bytes. One access a
-// lane and 32 bytes then, without the branches and the element loop of the general form.
-template <class T, bool kInside, bool kAnyOffset = false>
-__device__ __forceinline__ void local_load(const T* base, size_t idx, size_t limit, Wide16<T>& raw) {
-  constexpr int W = 4 * (int)sizeof(T);
-  if constexpr (!kInside) {
-    load16_wide<T, kAnyOffset>(base, idx, limit, raw);
+template <class T>
+__device__ __forceinline__ void store_elem(T* p, uint32_t word, int half) {
+  if constexpr (sizeof(T) == 4) *reinterpret_cast<uint32_t*>(p) = word;
+  else *reinterpret_cast<unsigned short*>(p) = (unsigned short)(word >> (16 * half));
+}
+
+// Every buffer starts on 32 bytes (kAnyOffset: anywhere). `inside`: the unit lies inside the message,
+// the same in all lanes. At the ragged end a lane reads the 32-byte sectors that hold any of its
+// elements (which stay inside their allocation) and clears the rest; 16 loads one by one took as
+// long as a call of a few thousand units. The callers have a body for each: with the two in one the
+// reduce-scatter of 8 x 25 MiB took 58 us instead of 49.
+template <class T, bool kAnyOffset = false>
+__device__ __forceinline__ void local_load(const T* base, size_t idx, size_t limit, bool inside, Wide16<T>& raw) {
+  constexpr int W = 4 * (int)sizeof(T), kPer = 4 / (int)sizeof(T);
+  const char* p = reinterpret_cast<const char*>(base + idx);
+  const uint32_t off = kAnyOffset ? (uint32_t)(reinterpret_cast<uintptr_t>(p) & 31) : 0u;
+  constexpr int kWords = kAnyOffset ? W + 8 : W;
+  uint32_t w[kWords];
+  if (inside) {
+#pragma unroll
+    for (int k = 0; k < W; k += 8) ldg_stream32(p - off + 4 * k, w + k);
+    if (kAnyOffset && off) ldg_stream32(p - off + 4 * W, w + kWords - 8);
   } else {
-    const char* p = reinterpret_cast<const char*>(base + idx);
-    if constexpr (kAnyOffset) {
-      const uint32_t off = (uint32_t)(reinterpret_cast<uintptr_t>(p) & 31);
-      uint32_t w[W + 8];
+    const uint32_t bytes = idx < limit ? (uint32_t)min((size_t)16, limit - idx) * (uint32_t)sizeof(T) : 0u;
 #pragma unroll
-      for (int k = 0; k < W; k += 8) ldg_stream32(p - off + 4 * k, w + k);
-      if (off) ldg_stream32(p - off + 4 * W, w + W);
-      shift_down<T>(w, off / (uint32_t)sizeof(T));
+    for (int k = 0; k < kWords; k += 8) {
+      if (bytes && 4u * k < off + bytes) {
+        ldg_stream32(p - off + 4 * k, w + k);
+      } else {
 #pragma unroll
-      for (int k = 0; k < W; ++k) raw.w[k] = w[k];
-    } else {
+        for (int i = 0; i < 8; ++i) w[k + i] = 0u;
+      }
+    }
+  }
+  if constexpr (kAnyOffset) shift_down<T>(w, off / (uint32_t)sizeof(T));
 #pragma unroll
-      for (int k = 0; k < W; k += 8) ldg_stream32(p + 4 * k, raw.w + k);
+  for (int k = 0; k < W; ++k) raw.w[k] = w[k];
+  if (!inside) {
+    const uint32_t n = idx < limit ? (uint32_t)min((size_t)16, limit - idx) : 0u;
+#pragma unroll
+    for (int k = 0; k < W; ++k) {
+      if ((uint32_t)(kPer * k) >= n) raw.w[k] = 0u;
+      else if (kPer == 2 && (uint32_t)(2 * k + 1) >= n) raw.w[k] &= 0xffffu;
     }
   }
 }
-template <class T, bool kInside, bool kAnyOffset = false>
-__device__ __forceinline__ void local_store(T* base, size_t idx, size_t limit, const Wide16<T>& raw) {
-  if constexpr (kInside && !kAnyOffset) {
+template <class T, bool kAnyOffset = false>
+__device__ __forceinline__ void local_store(T* base, size_t idx, size_t limit, bool inside, const Wide16<T>& raw) {
+  constexpr int W = 4 * (int)sizeof(T), kPer = 4 / (int)sizeof(T);
+  if (inside && kAnyOffset) {
+    store16_wide<T, true>(base, idx, limit, raw);
+  } else if (!kAnyOffset && (inside || idx + 16 <= limit)) {
 #pragma unroll
-    for (int k = 0; k < 4 * (int)sizeof(T); k += 8) stg_stream32(reinterpret_cast<char*>(base + idx) + 4 * k, raw.w + k);
+    for (int k = 0; k < W; k += 8) stg_stream32(reinterpret_cast<char*>(base + idx) + 4 * k, raw.w + k);
   } else {
-    store16_wide<T, kAnyOffset>(base, idx, limit, raw);
+#pragma unroll
+    for (int i = 0; i < 16; ++i)
+      if (idx + i < limit) store_elem<T>(base + idx + i, raw.w[i / kPer], i % kPer);
   }
 }
 
@@ -83,11 +113,6 @@ __device__ __forceinline__ void pack16(const float (&v)[16], Wide16<T>& o) {
 #pragma unroll
     for (int i = 0; i < 8; ++i) o.w[i] = pack2<T>(v[2 * i], v[2 * i + 1]);
   }
-}
-template <class T>
-__device__ __forceinline__ void store_elem(T* p, uint32_t word, int half) {
-  if constexpr (sizeof(T) == 4) *reinterpret_cast<uint32_t*>(p) = word;
-  else *reinterpret_cast<unsigned short*>(p) = (unsigned short)(word >> (16 * half));
 }
 
 // Lossy codecs add and do nothing else (the entry points refuse the rest).
@@ -104,35 +129,39 @@ __device__ __forceinline__ void combine16(int op, float (&a)[16], const float (&
 
 // v becomes what a receiver of the packet decodes; with a residual, v - that is kept for the next call.
 // kSentOnly: the kernels over peer memory decode this packet for the residual alone (see CodecInt4::residual).
-template <class C, bool kEf, bool kInside, bool kSentOnly = false>
-__device__ __forceinline__ void through_codec(float (&v)[16], float* ef, size_t idx, size_t limit) {
-  typename C::Packet pk;
-  C::encode(v, pk);
-  float d[16];
-  C::decode(pk, d);
-  if constexpr (kEf) {
-    if (ef) {
-      float r[16];
-      if constexpr (kSentOnly && C::kId == CCB_CODEC_INT4) {
-        C::residual(pk, v, r);
-      } else {
+template <class C, bool kEf, bool kAnyOffset = false, bool kSentOnly = false>
+__device__ __forceinline__ void through_codec(float (&v)[16], float* ef, size_t idx, size_t limit, bool inside) {
+  if constexpr (!kEf) {
+    C::round_trip(v);
+  } else {
+    float d[16], r[16];
+    if constexpr (kSentOnly && C::kId == CCB_CODEC_INT4) {
+      typename C::Packet pk;
+      C::encode(v, pk);
+      C::decode(pk, d);
+      C::residual(pk, v, r);
+    } else {
 #pragma unroll
-        for (int i = 0; i < 16; ++i) r[i] = __fsub_rn(v[i], d[i]);
-      }
+      for (int i = 0; i < 16; ++i) d[i] = v[i];
+      C::round_trip(d);
+#pragma unroll
+      for (int i = 0; i < 16; ++i) r[i] = __fsub_rn(v[i], d[i]);
+    }
+    if (ef) {
       Wide16<float> e;
       pack16<float>(r, e);
-      local_store<float, kInside>(ef, idx, limit, e);
+      local_store<float, kAnyOffset>(ef, idx, limit, inside, e);
     }
-  }
 #pragma unroll
-  for (int i = 0; i < 16; ++i) v[i] = d[i];
+    for (int i = 0; i < 16; ++i) v[i] = d[i];
+  }
 }
-template <bool kEf, bool kInside>
-__device__ __forceinline__ void add_residual(float (&v)[16], const float* ef, size_t idx, size_t limit) {
+template <bool kEf, bool kAnyOffset = false>
+__device__ __forceinline__ void add_residual(float (&v)[16], const float* ef, size_t idx, size_t limit, bool inside) {
   if constexpr (kEf) {
     if (ef) {
       Wide16<float> e;
-      local_load<float, kInside>(ef, idx, limit, e);
+      local_load<float, kAnyOffset>(ef, idx, limit, inside, e);
 #pragma unroll
       for (int i = 0; i < 16; ++i) v[i] += __uint_as_float(e.w[i]);
     }
@@ -140,17 +169,17 @@ __device__ __forceinline__ void add_residual(float (&v)[16], const float* ef, si
 }
 
 // The binomial tree below rank r with kRounds rounds: v = what r's parent decodes.
-template <class T, class C, bool kEf, bool kInside, int kRounds>
-__device__ __forceinline__ void local_subtree(const LocalReduceArgs& a, int r, size_t idx, float (&v)[16]) {
+template <class T, class C, bool kEf, bool kAnyOffset, int kRounds>
+__device__ __forceinline__ void local_subtree(const LocalReduceArgs& a, int r, size_t idx, bool inside, float (&v)[16]) {
   Wide16<T> raw;
-  local_load<T, kInside>(static_cast<const T*>(a.send[r]), idx, a.count, raw);
+  local_load<T, kAnyOffset>(static_cast<const T*>(a.send[r]), idx, a.count, inside, raw);
   wide16_to_f<T>(raw, v);
   auto child = [&](auto round) {
     constexpr int k = decltype(round)::value;
     if constexpr (k < kRounds) {
       if (r + (1 << k) < a.n) {
         float d[16];
-        local_subtree<T, C, kEf, kInside, k>(a, r + (1 << k), idx, d);
+        local_subtree<T, C, kEf, kAnyOffset, k>(a, r + (1 << k), idx, inside, d);
         combine16<C>(a.op, v, d);
       }
     }
@@ -158,21 +187,20 @@ __device__ __forceinline__ void local_subtree(const LocalReduceArgs& a, int r, s
   child(Int<0>{});
   child(Int<1>{});
   child(Int<2>{});
-  add_residual<kEf, kInside>(v, a.ef[r], idx, a.count);
-  through_codec<C, kEf, kInside>(v, a.ef[r], idx, a.count);
+  add_residual<kEf, kAnyOffset>(v, a.ef[r], idx, a.count, inside);
+  through_codec<C, kEf, kAnyOffset>(v, a.ef[r], idx, a.count, inside);
 }
 
-// One unit: element idx of the message (kLocalScatter: of shard s) and the 15 after it.
-template <class T, class C, int ALGO, bool kEf, bool kAnyOffset, bool kInside>
+// One unit of 512 elements: element idx (of the message; kLocalScatter: of shard s) and the 15 after it.
+template <class T, class C, int ALGO, bool kEf, bool kAnyOffset, bool inside>
 __device__ __forceinline__ void local_reduce_unit(const LocalReduceArgs& a, uint32_t s, size_t idx) {
   const int n = a.n;
   const int owner = ALGO == kLocalScatter && a.root >= 0 ? a.root : (int)s;
   float acc[16];
   if constexpr (ALGO == kLocalTree) {
     static_assert(CCB_MAX_RANKS <= 8, "three rounds");
-    local_subtree<T, C, kEf, kInside, 3>(a, 0, idx, acc);
+    local_subtree<T, C, kEf, kAnyOffset, 3>(a, 0, idx, inside, acc);
   } else {
-    constexpr int kBatch = kInside ? LocalShape<T, ALGO, kEf, kAnyOffset>::kBatch : 1;
     const size_t at = ALGO == kLocalScatter ? (size_t)s * a.shard_elems : 0;
     // the order in which contributions enter the sum: the owner, then ascending ranks (two-shot,
     // reduce-scatter); ascending ranks (one-shot); once round from the shard's number (ring)
@@ -181,80 +209,107 @@ __device__ __forceinline__ void local_reduce_unit(const LocalReduceArgs& a, uint
       if (ALGO == kLocalRing) return (int)s + j < n ? (int)s + j : (int)s + j - n;
       return j == 0 ? owner : j - (j <= owner ? 1 : 0);
     };
-#pragma unroll 1
-    for (int j0 = 0; j0 < n; j0 += kBatch) {
-      Wide16<T> raw[kBatch];
-      Wide16<float> e[kEf ? kBatch : 1];
+    auto take = [&](auto batch, int j0) {   // ranks rank_of(j0), ... into the sum
+      constexpr int kN = decltype(batch)::value;
+      Wide16<T> raw[kN];
+      [[maybe_unused]] Wide16<float> e[kEf ? kN : 1];
 #pragma unroll
-      for (int i = 0; i < kBatch; ++i) {
-        if (j0 + i < n) {
-          const int q = rank_of(j0 + i);
-          local_load<T, kInside, kAnyOffset>(static_cast<const T*>(a.send[q]) + at, idx, a.count, raw[i]);
-          if constexpr (kEf)
-            if (a.ef[q]) local_load<float, kInside && !kAnyOffset, kAnyOffset>(a.ef[q] + at, idx, a.count, e[i]);
-        }
+      for (int i = 0; i < kN; ++i) {
+        const int q = rank_of(j0 + i);
+        local_load<T, kAnyOffset>(static_cast<const T*>(a.send[q]) + at, idx, a.count, inside, raw[i]);
+        if constexpr (kEf)
+          if (a.ef[q]) local_load<float, kAnyOffset>(a.ef[q] + at, idx, a.count, inside, e[i]);
       }
 #pragma unroll
-      for (int i = 0; i < kBatch; ++i) {
+      for (int i = 0; i < kN; ++i) {
         const int j = j0 + i;
-        if (j < n) {
-          float v[16];
-          wide16_to_f<T>(raw[i], v);
-          if ((ALGO == kLocalTwoShot || ALGO == kLocalScatter) && j == 0) {   // the owner's own values: not compressed
+        float v[16];
+        wide16_to_f<T>(raw[i], v);
+        if ((ALGO == kLocalTwoShot || ALGO == kLocalScatter) && j == 0) {   // the owner's own values: not compressed
 #pragma unroll
-            for (int k = 0; k < 16; ++k) acc[k] = v[k];
-            continue;
-          }
-          const int q = rank_of(j);
-          if (ALGO == kLocalRing && j > 0) combine16<C>(a.op, v, acc);
-          if constexpr (kEf) {
-            if (a.ef[q]) {
+          for (int k = 0; k < 16; ++k) acc[k] = v[k];
+          continue;
+        }
+        const int q = rank_of(j);
+        if (ALGO == kLocalRing && j > 0) combine16<C>(a.op, v, acc);
+        if constexpr (kEf) {
+          if (a.ef[q]) {
 #pragma unroll
-              for (int k = 0; k < 16; ++k) v[k] += __uint_as_float(e[i].w[k]);
-            }
-          }
-          through_codec<C, kEf, kInside && !kAnyOffset, ALGO != kLocalRing>(v, kEf && a.ef[q] ? a.ef[q] + at : nullptr, idx, a.count);
-          if (ALGO == kLocalRing || (ALGO == kLocalOneShot && j == 0)) {
-#pragma unroll
-            for (int k = 0; k < 16; ++k) acc[k] = v[k];
-          } else {
-            combine16<C>(a.op, acc, v);
+            for (int k = 0; k < 16; ++k) v[k] += __uint_as_float(e[i].w[k]);
           }
         }
+        through_codec<C, kEf, kAnyOffset, ALGO != kLocalRing>(v, kEf && a.ef[q] ? a.ef[q] + at : nullptr, idx, a.count, inside);
+        if (ALGO == kLocalRing || (ALGO == kLocalOneShot && j == 0)) {
+#pragma unroll
+          for (int k = 0; k < 16; ++k) acc[k] = v[k];
+        } else {
+          combine16<C>(a.op, acc, v);
+        }
       }
+    };
+    // whole batches without a test for each rank (reduce-scatter of 8 x 25 MiB: 43 us, 49 with one)
+    constexpr int kBatch = inside ? LocalShape<T, ALGO, kEf, kAnyOffset>::kBatch : 1;
+    int j0 = 0;
+#pragma unroll 1
+    for (; j0 + kBatch <= n; j0 += kBatch) take(Int<kBatch>{}, j0);
+    if constexpr (kBatch > 1) {
+#pragma unroll 1
+      for (; j0 < n; ++j0) take(Int<1>{}, j0);
     }
     if constexpr (ALGO == kLocalTwoShot) {   // the owner compresses the sum once more; everybody decodes that
-      add_residual<kEf, kInside>(acc, a.ef[owner], idx, a.count);
-      through_codec<C, kEf, kInside>(acc, a.ef[owner], idx, a.count);
+      add_residual<kEf, kAnyOffset>(acc, a.ef[owner], idx, a.count, inside);
+      through_codec<C, kEf, kAnyOffset>(acc, a.ef[owner], idx, a.count, inside);
     }
   }
   Wide16<T> o;
   pack16<T>(acc, o);
   if constexpr (ALGO == kLocalScatter) {
-    local_store<T, kInside, kAnyOffset>(static_cast<T*>(a.recv[owner]), idx, a.count, o);
+    local_store<T, kAnyOffset>(static_cast<T*>(a.recv[owner]), idx, a.count, inside, o);
   } else {
 #pragma unroll 1
-    for (int p = 0; p < n; ++p) local_store<T, kInside>(static_cast<T*>(a.recv[p]), idx, a.count, o);
+    for (int p = 0; p < n; ++p) local_store<T, kAnyOffset>(static_cast<T*>(a.recv[p]), idx, a.count, inside, o);
   }
-}
-
-// The ragged end of a message, and buffers off the 32-byte boundaries: out of line, because its
-// branches and element loops cost the common unit registers.
-template <class T, class C, int ALGO, bool kEf, bool kAnyOffset>
-__device__ __noinline__ void local_reduce_ragged(const LocalReduceArgs& a, uint32_t s, size_t idx) {
-  local_reduce_unit<T, C, ALGO, kEf, kAnyOffset, false>(a, s, idx);
 }
 
 template <class T, class C, int ALGO, bool kEf, bool kAnyOffset>
 __global__ void __launch_bounds__(kLocalThreads, LocalShape<T, ALGO, kEf, kAnyOffset>::kCtas) local_reduce_kernel(const __grid_constant__ LocalReduceArgs a) {
-  const int lane = threadIdx.x & 31;
-  const uint32_t step = (gridDim.x * blockDim.x) >> 5;
-  for (uint32_t u = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; u < a.units; u += step) {
-    const uint32_t s = ALGO == kLocalTwoShot || ALGO == kLocalRing || ALGO == kLocalScatter ? u / a.shard_units : 0u;
-    const size_t e0 = (size_t)(ALGO == kLocalScatter ? u - s * a.shard_units : u) * kWarpElems;
-    if (a.wide && e0 + kWarpElems <= a.count) local_reduce_unit<T, C, ALGO, kEf, kAnyOffset, true>(a, s, e0 + lane * kLaneElems);
-    else local_reduce_ragged<T, C, ALGO, kEf, kAnyOffset>(a, s, e0 + lane * kLaneElems);
+  const uint32_t u = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (u >= a.units) return;
+  const uint32_t s = ALGO == kLocalTwoShot || ALGO == kLocalRing || ALGO == kLocalScatter ? u / a.shard_units : 0u;
+  const size_t e0 = (size_t)(ALGO == kLocalScatter ? u - s * a.shard_units : u) * kWarpElems, idx = e0 + (threadIdx.x & 31) * kLaneElems;
+  if (e0 + kWarpElems <= a.count) local_reduce_unit<T, C, ALGO, kEf, kAnyOffset, true>(a, s, idx);
+  else local_reduce_unit<T, C, ALGO, kEf, kAnyOffset, false>(a, s, idx);
+}
+
+// ----------------------------------------------------------------------- one rank --
+// An all-reduce of one rank: a round trip through the codec, one unit a warp. With nothing carried
+// from unit to unit a thread has 32 registers (16-bit types) and an SM all of its 64 warps, each
+// waits once, and CTAs are handed out in the order of the addresses, which is what the memory likes
+// best: 256 MiB of bf16 in int8 81 us, 6.6 TB/s, the rate of a plain copy, where resident CTAs that
+// looped over the message with a unit requested ahead took 100 (and 88 at 46 registers a thread). B200.
+template <class T, class C, bool kEf, bool kAnyOffset, bool inside>
+__device__ __forceinline__ void local_solo_unit(const LocalReduceArgs& a, size_t idx) {
+  Wide16<T> raw;
+  local_load<T, kAnyOffset>(static_cast<const T*>(a.send[0]), idx, a.count, inside, raw);
+  [[maybe_unused]] Wide16<float> e;
+  if constexpr (kEf) local_load<float, kAnyOffset>(a.ef[0], idx, a.count, inside, e);
+  float v[16];
+  wide16_to_f<T>(raw, v);
+  if constexpr (kEf) {
+#pragma unroll
+    for (int i = 0; i < 16; ++i) v[i] += __uint_as_float(e.w[i]);
   }
+  through_codec<C, kEf, kAnyOffset>(v, kEf ? a.ef[0] : nullptr, idx, a.count, inside);
+  Wide16<T> o;
+  pack16<T>(v, o);
+  local_store<T, kAnyOffset>(static_cast<T*>(a.recv[0]), idx, a.count, inside, o);
+}
+template <class T, class C, bool kEf, bool kAnyOffset>
+__global__ void __launch_bounds__(kLocalThreads, kEf ? 4 : sizeof(T) == 4 ? (kAnyOffset ? 4 : 6) : kAnyOffset ? 6 : 8) local_solo_kernel(const __grid_constant__ LocalReduceArgs a) {
+  const size_t e0 = (((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * kWarpElems, idx = e0 + (threadIdx.x & 31) * kLaneElems;
+  if (e0 >= a.count) return;
+  if (e0 + kWarpElems <= a.count) local_solo_unit<T, C, kEf, kAnyOffset, true>(a, idx);
+  else local_solo_unit<T, C, kEf, kAnyOffset, false>(a, idx);
 }
 
 // ------------------------------------------------------------------------- exchange --
@@ -274,85 +329,91 @@ struct LocalExchangeArgs {
 // kAnyOffset: blocks may start anywhere. Where the destinations of a block lie alike on their
 // 32-byte sectors the warp rotates a unit once for all of them, and the first sector of a unit is
 // completed with what the unit before left over, so that only the ends of a run are written
-// element by element.
+// element by element. (Without kAnyOffset a run is one unit.)
 template <class T, class C, bool kAnyOffset>
-__global__ void __launch_bounds__(kLocalThreads, kAnyOffset || sizeof(T) == 4 ? 3 : 4) local_exchange_kernel(const __grid_constant__ LocalExchangeArgs a) {
+__global__ void __launch_bounds__(kLocalThreads, kAnyOffset ? (sizeof(T) == 4 ? 2 : 3) : 6) local_exchange_kernel(const __grid_constant__ LocalExchangeArgs a) {
   constexpr int W = 4 * (int)sizeof(T), kPer = 4 / (int)sizeof(T);   // words of a lane, elements of a word
   const int lane = threadIdx.x & 31;
-  const uint32_t step = (gridDim.x * blockDim.x) >> 5, runs = a.first_run[a.nblocks];
+  const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (w >= a.first_run[a.nblocks]) return;
   int b = 0;
-  for (uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < runs; w += step) {
-    while (w >= a.first_run[b + 1]) ++b;
-    const T* src = static_cast<const T*>(a.src[b]);
-    const size_t cnt = a.cnt[b];
-    const int d0 = a.first_dst[b], d1 = a.first_dst[b + 1];
-    const size_t u0 = (size_t)(w - a.first_run[b]) * a.run;
-    size_t u1 = u0 + a.run;
-    const size_t all = (cnt + kWarpElems - 1) / kWarpElems;
-    if (u1 > all) u1 = all;
-    uint32_t mis = 0;
-    Wide16<T> left;   // lane 0: the last `mis` elements of the unit before
-    if constexpr (kAnyOffset) {
-      const uint32_t off = (uint32_t)(reinterpret_cast<uintptr_t>(a.dst[d0]) & 31);   // a unit is a whole number of sectors
-      if (off & 15) {
-        mis = off / (uint32_t)sizeof(T);
-        for (int d = d0 + 1; d < d1; ++d)
-          if ((uint32_t)(reinterpret_cast<uintptr_t>(a.dst[d]) & 31) != off) mis = 0;
-      }
-    }
-    Wide16<T> next;
-    load16_wide<T, kAnyOffset>(src, u0 * kWarpElems + lane * kLaneElems, cnt, next);
-    bool carried = false;
-    for (size_t u = u0; u < u1; ++u) {
-      const size_t idx = u * kWarpElems + lane * kLaneElems;
-      float v[16];
-      wide16_to_f<T>(next, v);
-      if (u + 1 < u1) load16_wide<T, kAnyOffset>(src, idx + kWarpElems, cnt, next);
-      through_codec<C, false, true>(v, nullptr, 0, 0);
-      Wide16<T> o;
-      pack16<T>(v, o);
-      if constexpr (kAnyOffset) {
-        const bool whole = mis && (u + 1) * kWarpElems <= cnt;   // the same in all lanes
-        if (whole) {
-          rotate_up<T>(o.w, mis, lane);
-          const Wide16<T> mine = o;   // lane 0: this unit's last `mis` elements, then its first 16 - mis
-          if (lane == 0 && carried) {
+  while (w >= a.first_run[b + 1]) ++b;
+  const T* src = static_cast<const T*>(a.src[b]);
+  const size_t cnt = a.cnt[b];
+  const int d0 = a.first_dst[b], d1 = a.first_dst[b + 1];
+  auto plain = [&](size_t e0, auto whole) {   // a unit by itself
+    constexpr bool inside = decltype(whole)::value != 0;
+    const size_t idx = e0 + lane * kLaneElems;
+    Wide16<T> o;
+    local_load<T, kAnyOffset>(src, idx, cnt, inside, o);
+    float v[16];
+    wide16_to_f<T>(o, v);
+    C::round_trip(v);
+    pack16<T>(v, o);
+#pragma unroll 1
+    for (int d = d0; d < d1; ++d) local_store<T, kAnyOffset>(static_cast<T*>(a.dst[d]), idx, cnt, inside, o);
+  };
+  if constexpr (!kAnyOffset) {
+    const size_t e0 = (size_t)(w - a.first_run[b]) * kWarpElems;
+    if (e0 + kWarpElems <= cnt) plain(e0, Int<1>{});
+    else plain(e0, Int<0>{});
+  } else {
+    const size_t u0 = (size_t)(w - a.first_run[b]) * a.run, whole = cnt / kWarpElems;
+    const size_t u1 = u0 + a.run < whole ? u0 + a.run : whole;   // the run's whole units; a ragged one may follow
+    const uint32_t off = (uint32_t)(reinterpret_cast<uintptr_t>(a.dst[d0]) & 31);   // a unit is a whole number of sectors
+    const uint32_t mis = off / (uint32_t)sizeof(T);
+    bool alike = true;
+    for (int d = d0 + 1; d < d1; ++d) alike = alike && (uint32_t)(reinterpret_cast<uintptr_t>(a.dst[d]) & 31) == off;
+    if (!alike) {
+#pragma unroll 1
+      for (size_t u = u0; u < u1; ++u) plain(u * kWarpElems, Int<1>{});
+    } else if (u0 < u1) {
+      Wide16<T> next, left;   // left, in lane 0: the last `mis` elements of the unit before
+      local_load<T, true>(src, u0 * kWarpElems + lane * kLaneElems, cnt, true, next);
+#pragma unroll 1
+      for (size_t u = u0; u < u1; ++u) {
+        const size_t idx = u * kWarpElems + lane * kLaneElems;
+        float v[16];
+        wide16_to_f<T>(next, v);
+        if (u + 1 < u1) local_load<T, true>(src, idx + kWarpElems, cnt, true, next);
+        C::round_trip(v);
+        Wide16<T> o;
+        pack16<T>(v, o);
+        rotate_up<T>(o.w, mis, lane);
+        const Wide16<T> mine = o;   // lane 0: this unit's last `mis` elements, then its first 16 - mis
+        if (lane == 0 && u > u0) {
 #pragma unroll
-            for (int k = 0; k < W; ++k) {
-              if ((uint32_t)(kPer * k + kPer - 1) < mis) o.w[k] = left.w[k];
-              else if (kPer == 2 && (uint32_t)(2 * k) < mis) o.w[k] = __byte_perm(left.w[k], o.w[k], 0x7610);
-            }
+          for (int k = 0; k < W; ++k) {
+            if ((uint32_t)(kPer * k + kPer - 1) < mis) o.w[k] = left.w[k];
+            else if (kPer == 2 && (uint32_t)(2 * k) < mis) o.w[k] = __byte_perm(left.w[k], o.w[k], 0x7610);
           }
-          const bool sector = lane != 0 || carried;
-          for (int d = d0; d < d1; ++d) {
-            T* p = static_cast<T*>(a.dst[d]) + idx - mis;
-            if (sector) {
-#pragma unroll
-              for (int k = 0; k < W; k += 8) stg_stream32(reinterpret_cast<char*>(p) + 4 * k, o.w + k);
-            } else {
-#pragma unroll
-              for (int i = 0; i < 16; ++i)
-                if ((uint32_t)i >= mis) store_elem<T>(p + i, o.w[(i / kPer) & (W - 1)], i % kPer);
-            }
-          }
-          left = mine;
-          carried = true;
-          continue;
         }
-      }
-      for (int d = d0; d < d1; ++d) store16_wide<T, kAnyOffset>(static_cast<T*>(a.dst[d]), idx, cnt, o);
-    }
-    if constexpr (kAnyOffset) {
-      if (carried && lane == 0) {   // behind the last whole unit of the run
-        const size_t end = (u1 * kWarpElems <= cnt ? u1 : u1 - 1) * kWarpElems;
+        const bool sector = lane != 0 || u > u0 || mis == 0;
+#pragma unroll 1
         for (int d = d0; d < d1; ++d) {
-          T* p = static_cast<T*>(a.dst[d]) + end - mis;
+          T* p = static_cast<T*>(a.dst[d]) + idx - mis;
+          if (sector) {
+#pragma unroll
+            for (int k = 0; k < W; k += 8) stg_stream32(reinterpret_cast<char*>(p) + 4 * k, o.w + k);
+          } else {
+#pragma unroll
+            for (int i = 0; i < 16; ++i)
+              if ((uint32_t)i >= mis) store_elem<T>(p + i, o.w[(i / kPer) & (W - 1)], i % kPer);
+          }
+        }
+        left = mine;
+      }
+      if (lane == 0) {   // behind the last whole unit of the run
+#pragma unroll 1
+        for (int d = d0; d < d1; ++d) {
+          T* p = static_cast<T*>(a.dst[d]) + u1 * kWarpElems - mis;
 #pragma unroll
           for (int i = 0; i < 16; ++i)
             if ((uint32_t)i < mis) store_elem<T>(p + i, left.w[(i / kPer) & (W - 1)], i % kPer);
         }
       }
     }
+    if (u1 == whole && u0 + a.run > whole && whole * kWarpElems < cnt) plain(whole * kWarpElems, Int<0>{});
   }
 }
 

@@ -11,6 +11,7 @@
 
 #include "../rt/ccb_rt_internal.h"
 #include "ccb/ccb_moe.h"
+#include "ccb_local.cuh"
 #include "ccb_reduce.cuh"
 
 namespace ccb {
@@ -195,82 +196,84 @@ struct MoeLocalArgs {
   uint32_t first_in[CCB_MAX_RANKS][CCB_MAX_RANKS];   // [holder][origin]: first row of that origin in the holder's buffer
   uint32_t first_out[CCB_MAX_RANKS][CCB_MAX_RANKS];  // [src][dst]: first entry of that block in perm
   uint64_t hidden;
-  uint32_t tokens, row_units, chunk_rows, chunks;
+  uint32_t tokens, row_units, chunk_rows, chunks;   // a chunk of a block: its rows for one CTA
   int topk, n;
 };
 constexpr int kMoeLocalThreads = 256;
 
 // Dispatch. The rows of a rank are sorted by destination, and within one by token. A CTA takes
-// `chunk_rows` rows of one block; the blocks of a rank take turns chunk by chunk, so that the topk
-// copies of a token, which lie at about the same depth of their blocks, are read from memory once
-// and from L2 after that.
+// `chunk_rows` rows of one block, a warp one unit at a time; the blocks of a rank take turns chunk by
+// chunk, so that the topk copies of a token, which lie at about the same depth of their blocks, are
+// read from memory once and from L2 after that.
 template <class T, class C>
-__global__ void __launch_bounds__(kMoeLocalThreads, sizeof(T) == 4 ? 3 : 4) moe_local_dispatch_kernel(const __grid_constant__ MoeLocalArgs a) {
-  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
-  const uint32_t n = (uint32_t)a.n, upr = a.row_units;
-  const uint32_t p = blockIdx.x % n, c = blockIdx.x / n % a.chunks, r = blockIdx.x / n / a.chunks;
+__global__ void __launch_bounds__(kMoeLocalThreads, 6) moe_local_dispatch_kernel(const __grid_constant__ MoeLocalArgs a) {
+  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, upr = a.row_units;
+  const uint32_t n = (uint32_t)a.n, p = blockIdx.x % n, c = blockIdx.x / n % a.chunks, r = blockIdx.x / n / a.chunks;
   const uint32_t j0 = c * a.chunk_rows, rows = a.cnt[r][p];
   if (j0 >= rows) return;
   const uint32_t units = min(a.chunk_rows, rows - j0) * upr;
   const T* src = static_cast<const T*>(a.src[r]);
   const int32_t* perm = a.perm[r] + a.first_out[r][p] + j0;
   T* dst = static_cast<T*>(a.dst[p]) + (size_t)(a.first_in[p][r] + j0) * a.hidden;   // unit u of whole rows starts at element 512 u
-  Wide16<T> raw;
-  auto request = [&](uint32_t u) {
+#pragma unroll 1
+  for (uint32_t u = warp; u < units; u += kMoeLocalThreads / 32) {
     const uint32_t j = u / upr;
-    load16_wide<T>(src + (size_t)perm[j] * a.hidden, (size_t)(u - j * upr) * kWarpElems + lane * kLaneElems, a.hidden, raw);
-  };
-  uint32_t u = warp;
-  if (u < units) request(u);
-  while (u < units) {
+    Wide16<T> raw;
+    local_load<T>(src + (size_t)perm[j] * a.hidden, (size_t)(u - j * upr) * kWarpElems + lane * kLaneElems, 0, true, raw);
     float v[16];
     wide16_to_f<T>(raw, v);
-    const size_t at = (size_t)u * kWarpElems + lane * kLaneElems;
-    u += warps;
-    if (u < units) request(u);
-    typename C::Packet pk;
-    C::encode(v, pk);
-    C::decode(pk, v);
-    store16_wide<T>(dst, at, at + 16, v);
+    C::round_trip(v);
+    pack16<T>(v, raw);
+    local_store<T>(dst, (size_t)u * kWarpElems + lane * kLaneElems, 0, true, raw);
   }
 }
 
-// Combine: a warp takes 512 elements of one token and fetches them from the topk rows that hold it.
-// An index outside its block (the entry of a dropped pair) contributes nothing.
+// Combine: a warp takes 512 elements of one token and fetches them from the topk rows that hold it,
+// two at a time. An index outside its block (the entry of a dropped pair) contributes nothing.
 template <class T, class C>
 __global__ void __launch_bounds__(kMoeLocalThreads, sizeof(T) == 4 ? 3 : 4) moe_local_combine_kernel(const __grid_constant__ MoeLocalArgs a) {
-  const uint32_t lane = threadIdx.x & 31, upr = a.row_units;
-  const uint32_t step = (gridDim.x * blockDim.x) >> 5, per_rank = a.tokens * upr;
-  for (uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < per_rank * (uint32_t)a.n; w += step) {
-    const uint32_t r = w / per_rank, u = w - r * per_rank, tok = u / upr;
-    const size_t col = (size_t)(u - tok * upr) * kWarpElems + lane * kLaneElems;
-    const size_t pair0 = (size_t)tok * a.topk;
-    Wide16<T> next;
-    bool have = false;
-    auto request = [&](int k) {
-      const uint32_t q = (uint32_t)a.dest_rank[r][pair0 + k], j = (uint32_t)a.pos[r][pair0 + k];
-      have = q < (uint32_t)a.n && j < a.cnt[r][q];
-      if (have) load16_wide<T>(static_cast<const T*>(a.src[q]) + (size_t)(a.first_in[q][r] + j) * a.hidden, col, a.hidden, next);
-    };
-    float acc[16];
+  const uint32_t lane = threadIdx.x & 31, upr = a.row_units, per_rank = a.tokens * upr;
+  const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (w >= per_rank * (uint32_t)a.n) return;
+  const uint32_t r = w / per_rank, u = w - r * per_rank, tok = u / upr;
+  const size_t col = (size_t)(u - tok * upr) * kWarpElems + lane * kLaneElems, pair0 = (size_t)tok * a.topk;
+  float acc[16];
 #pragma unroll
-    for (int i = 0; i < 16; ++i) acc[i] = 0.f;
-    if (a.topk > 0) request(0);
-    for (int k = 0; k < a.topk; ++k) {
-      const bool now = have;
-      float d[16];
-      wide16_to_f<T>(next, d);
-      const float g = a.gate[r][pair0 + k];
-      if (k + 1 < a.topk) request(k + 1);
-      if (!now) continue;
-      typename C::Packet pk;
-      C::encode(d, pk);
-      C::decode(pk, d);
+  for (int i = 0; i < 16; ++i) acc[i] = 0.f;
+  auto take = [&](auto batch, int k0) {
+    constexpr int kN = decltype(batch)::value;
+    Wide16<T> raw[kN];
+    uint32_t q[kN], j[kN];
+    float g[kN];
+    bool held[kN];
 #pragma unroll
-      for (int i = 0; i < 16; ++i) acc[i] += g * d[i];
+    for (int i = 0; i < kN; ++i) {
+      q[i] = (uint32_t)a.dest_rank[r][pair0 + k0 + i];
+      j[i] = (uint32_t)a.pos[r][pair0 + k0 + i];
+      g[i] = a.gate[r][pair0 + k0 + i];
     }
-    store16_wide<T>(static_cast<T*>(a.dst[r]) + (size_t)tok * a.hidden, col, a.hidden, acc);
-  }
+#pragma unroll
+    for (int i = 0; i < kN; ++i) {
+      held[i] = q[i] < (uint32_t)a.n && j[i] < a.cnt[r][q[i] & (CCB_MAX_RANKS - 1)];
+      if (held[i]) local_load<T>(static_cast<const T*>(a.src[q[i]]) + (size_t)(a.first_in[q[i]][r] + j[i]) * a.hidden, col, 0, true, raw[i]);
+    }
+#pragma unroll
+    for (int i = 0; i < kN; ++i) {
+      if (!held[i]) continue;
+      float d[16];
+      wide16_to_f<T>(raw[i], d);
+      C::round_trip(d);
+#pragma unroll
+      for (int e = 0; e < 16; ++e) acc[e] += g[i] * d[e];
+    }
+  };
+  int k = 0;
+#pragma unroll 1
+  for (; k + 2 <= a.topk; k += 2) take(Int<2>{}, k);
+  if (k < a.topk) take(Int<1>{}, k);
+  Wide16<T> o;
+  pack16<T>(acc, o);
+  local_store<T>(static_cast<T*>(a.dst[r]) + (size_t)tok * a.hidden, col, 0, true, o);
 }
 
 template <template <class, class> class K>
@@ -320,18 +323,13 @@ static int moe_local_launch(ccb_comm* c, const MoeArgs& m, bool combine, int dty
   a.row_units = (uint32_t)(m.hidden / kWarpElems);
   a.tokens = (uint32_t)m.tokens;
   a.topk = m.topk;
-  const uint64_t sms = (uint64_t)comm_sms(c);
   uint64_t ctas, warps = kMoeLocalThreads / 32;
   if (combine) {
-    const uint64_t units = (uint64_t)a.n * m.tokens * a.row_units;
+    const uint64_t units = (uint64_t)a.n * m.tokens * a.row_units, sms = (uint64_t)comm_sms(c);
     while (warps > 1 && units / warps < sms) warps >>= 1;
     ctas = (units + warps - 1) / warps;
-    if (ctas > (1u << 20)) ctas = 1u << 20;
   } else {
-    // Chunks of up to 64 units (eight for each warp), smaller where the blocks would not fill the chip twice.
-    uint64_t rows = 64 / a.row_units;
-    if (rows < 1) rows = 1;
-    while (rows > 1 && (uint64_t)a.n * a.n * ((max_rows + rows - 1) / rows) < 8 * sms) rows >>= 1;
+    const uint64_t rows = warps > a.row_units ? warps / a.row_units : 1;   // about a unit a warp
     a.chunk_rows = (uint32_t)rows;
     a.chunks = (uint32_t)((max_rows + rows - 1) / rows);
     ctas = (uint64_t)a.n * a.n * a.chunks;
@@ -375,8 +373,9 @@ static int moe_launch(ccb_comm* c, const void* fn, MoeArgs& a, bool combine, int
   // the arena has read all rows before it writes a token, so there its results may lie on the rows.
   // (A dispatch has not, there or here: its results may not lie on what the ranks send.)
   uint64_t all_rows = 0;
-  bool apart = true;
+  bool apart = true, aligned = true;
   for (int s = 0; s < n; ++s) {
+    aligned = aligned && ((reinterpret_cast<uintptr_t>(a.src[s]) | reinterpret_cast<uintptr_t>(a.dst[s])) & 31) == 0;
     uint64_t rows = 0;
     for (int d = 0; d < n; ++d) rows += a.cnt[d][s];
     all_rows += rows;
@@ -386,7 +385,7 @@ static int moe_launch(ccb_comm* c, const void* fn, MoeArgs& a, bool combine, int
       apart = apart && !(y < out + a.tokens * row_bytes && out < y + rows * row_bytes);
     }
   }
-  if (ranks_in_registers(c) && apart && !(((all_rows + (uint64_t)n * a.tokens) * (a.hidden / kWarpElems)) >> 31))
+  if (ranks_in_registers(c) && apart && aligned && !(((all_rows + (uint64_t)n * a.tokens) * (a.hidden / kWarpElems)) >> 31))
     return moe_local_launch(c, a, combine, dtype, codec, max_rows, stream);
   a.c = comm_dev(c, next_epoch(c));
   a.rank0 = ccb_comm_rank(c);

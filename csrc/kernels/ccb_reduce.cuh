@@ -340,12 +340,11 @@ __global__ void __launch_bounds__(kThreads, 2) reduce_kernel(const __grid_consta
   }
 }
 
-// A communicator of one rank: an all-reduce is one round trip through the codec (with error
-// feedback, its residual), whatever the algorithm. No peers, so no flags, no arena and no
-// cooperative launch, and a body small enough for 1280 threads an SM with a unit ahead each: the
-// pass is bound by memory. The next unit is requested before the one in hand is encoded.
-// (256 MiB of bf16 in int8: 113 us in the two-shot kernel, 32 warps an SM that each waited for
-// one unit at a time in 16-byte accesses; 100.5 us here, 5.3 TB/s, B200.)
+// A communicator of one rank whose grid is capped or whose phases are traced: an all-reduce is one
+// round trip through the codec (with error feedback, its residual), whatever the algorithm. No
+// peers, so no flags, no arena and no cooperative launch. The next unit is requested before the one
+// in hand is encoded. (256 MiB of bf16 in int8: 113 us in the two-shot kernel, 100.5 us here; 81
+// in local_solo_kernel, which takes the calls without a cap. B200.)
 // kAny is the form with the phase marks and for other CTA sizes (a capped grid, see the host): in
 // the usual form they take up to eight registers, and 256 MiB of bf16 in fp8 went from 92.0 to
 // 93.5 us. Its launch bounds give the same registers a thread for larger CTAs.

@@ -973,8 +973,9 @@ int comm_sms(const ccb_comm* c) { return c->num_sms; }
 // A warp reads an element from every rank that contributes to it and then writes every result of
 // it, so a rank's result may lie exactly on the elements it comes from; any other meeting of what
 // is read and what is written wants the order that the flags of the other kernels give.
-static bool reduces_in_registers(const ccb_comm* c, const ReduceArgs& a, size_t es) {
-  if (!ranks_in_registers(c)) return false;
+static bool reduces_in_registers(const ccb_comm* c, const ReduceArgs& a, int dtype) {
+  if (!ranks_in_registers(c) || !local_reduce_takes(a, dtype)) return false;
+  const size_t es = elem_size(dtype);
   Span in[CCB_MAX_RANKS], out[CCB_MAX_RANKS];
   for (int i = 0; i < c->nlocal; ++i) {
     const bool scatter = a.mode == CCB_MODE_REDUCESCATTER, gets = a.mode != CCB_MODE_REDUCE || i == a.root;
@@ -1014,7 +1015,7 @@ static int reduce_launch(ccb_comm* c, const void* const* send, void* const* recv
   a.op = op;
   a.root = root;
   a.mode = mode;
-  if (reduces_in_registers(c, a, es))
+  if (reduces_in_registers(c, a, dtype))
     return local_reduce(c, a, mode != CCB_MODE_ALLREDUCE ? kLocalScatter : shape == kOneShot ? kLocalOneShot : kLocalTwoShot, dtype, codec, stream);
   // Large two-shot AllReduce / ReduceScatter calls go to the warp-specialised pipelined
   // kernel: it needs a few chunks (8 units of 512 elements) per CTA and wave to pay.
@@ -1092,9 +1093,13 @@ static int reduce_launch(ccb_comm* c, const void* const* send, void* const* recv
   return launch(c, fn, ctas, &a, stream);
 }
 
-// An all-reduce of one rank (see solo_kernel): as many CTAs as are resident at once.
+// An all-reduce of one rank: one unit a warp (local_solo_kernel), or under a grid cap, for a phase
+// trace and with a residual off the 32-byte boundaries as many CTAs as are resident at once
+// (solo_kernel).
 static int solo_launch(ccb_comm* c, const void* const* send, void* const* recv, float* const* ef, uint64_t count, int dtype, int codec,
                        cudaStream_t stream) {
+  if (!c->trace && c->max_ctas <= 0 && local_solo_takes(send[0], recv[0], ef ? ef[0] : nullptr))
+    return local_solo(c, send[0], recv[0], ef ? ef[0] : nullptr, count, dtype, codec, stream);
   // A grid capped at a CTA an SM or less gets CTAs of 512 threads, the size that the other kernels
   // have: 128 Mi bf16 values in fp8 under a cap of 148 took 145 us in the two-shot kernel, 152 in
   // CTAs of 256 threads and 102 so (cap 16: 1085, 1077, 577). From two a SM the small ones are
@@ -1257,7 +1262,7 @@ extern "C" int ccb_all_reduce(ccb_comm* c, const void* const* send, void* const*
       a.nlocal = c->nlocal;
       a.op = op;
       a.mode = CCB_MODE_ALLREDUCE;
-      if (reduces_in_registers(c, a, es)) {
+      if (reduces_in_registers(c, a, dtype)) {
         rc = local_reduce(c, a, algo == CCB_ALGO_RING ? kLocalRing : kLocalTree, dtype, codec, stream);
       } else {
         a.c = comm_dev(c, next_epoch(c));
@@ -1405,7 +1410,7 @@ extern "C" int ccb_exchange(ccb_comm* c, const void* const* send, void* const* r
   own_direct = own_direct && apart;
   if (in_registers && apart) {
     a.c.nranks = n;
-    return local_exchange(c, a, aligned, dtype, codec, static_cast<cudaStream_t>(stream_));
+    return local_exchange(c, a, dtype, codec, static_cast<cudaStream_t>(stream_));
   }
   a.c = comm_dev(c, next_epoch(c));
   // Between two ranks that move 16-bit values as they are the form for any offset is the faster one

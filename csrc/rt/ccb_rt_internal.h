@@ -25,8 +25,11 @@ int pipe_kernel_threads();
 // communicator are this process's and nothing asks for the schedule of ranks on several GPUs.
 bool ranks_in_registers(const ccb_comm* c);
 int comm_sms(const ccb_comm* c);
+bool local_reduce_takes(const ReduceArgs& r, int dtype);   // residuals want buffers on 32 bytes
+bool local_solo_takes(const void* send, const void* recv, const float* ef);
 int local_reduce(ccb_comm* c, const ReduceArgs& r, int algo, int dtype, int codec, cudaStream_t stream);
-int local_exchange(ccb_comm* c, const ExchangeArgs& x, bool aligned, int dtype, int codec, cudaStream_t stream);
+int local_solo(ccb_comm* c, const void* send, void* recv, float* ef, uint64_t count, int dtype, int codec, cudaStream_t stream);
+int local_exchange(ccb_comm* c, const ExchangeArgs& x, int dtype, int codec, cudaStream_t stream);
 int nvls_all_reduce(ccb_comm* c, const void* const* send, void* const* recv, uint64_t count, int dtype, int op,
                     cudaStream_t stream);
 }  // namespace ccb
