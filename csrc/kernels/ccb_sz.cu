@@ -63,7 +63,6 @@ constexpr int kRows = kTY * kTZ;                  // 64
 constexpr int kSzThreads = 256;                   // warp = z plane, lane = x
 constexpr int kClusterSize = 8;
 constexpr int kTileCap = kRows + kTileVals * 4;   // 8256 bytes, worst case (w = 32 everywhere)
-constexpr uint32_t kLostTile = 1u << 24;          // size word of the tiles of a group that could not be packed: more than a group can hold
 constexpr int kGroupHeader = 32;
 constexpr int kGroupStride = kGroupHeader + kClusterSize * kTileCap + 32;  // 66112, multiple of 16
 static_assert(kGroupStride % 16 == 0, "slots must keep 16-byte alignment");
@@ -79,14 +78,12 @@ struct SzArgs {
   CUtensorMap tmap[CCB_MAX_RANKS];   // one per local rank, over `in`
   SzField f[CCB_MAX_RANKS];          // per local rank
   unsigned long long* used_bytes;    // per local rank: compressed bytes produced (atomicAdd), or 0
-  char* local_out;                   // compress-only: destination buffer (rank-less)
-  const char* local_in;              // decompress-only: source buffer
   int nx, ny, nz;
   int tiles_x, tiles_y, tiles_z;
   unsigned int ngroups;
   float eb, two_eb, inv_two_eb;
   int use_tma;
-  int mode;                          // 0 compress to local_out, 1 decompress from local_in, 2 all-gather, 3 broadcast
+  int mode;                          // 2 all-gather, 3 broadcast
   int root;
   int rank0, nlocal;
   unsigned int bcast_waves;          // progress steps a broadcast root publishes (1..kMaxBcastWaves)
@@ -125,32 +122,9 @@ __device__ __forceinline__ void tma_load_3d(void* smem_dst, const CUtensorMap* m
       ::"r"(smem_u32(smem_dst)), "l"(map), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar)) : "memory");
 }
 
-// One word into the shared memory of CTA `rank` of the cluster, at the place that `dst` has in
-// this CTA's; its arrival counts 4 bytes on that CTA's mbarrier.
-__device__ __forceinline__ void st_async_u32(uint32_t* dst, uint64_t* bar, uint32_t rank, uint32_t v) {
-  asm volatile(
-      "{\n.reg .b32 a, b;\n"
-      "mapa.shared::cluster.u32 a, %0, %2;\n"
-      "mapa.shared::cluster.u32 b, %1, %2;\n"
-      "st.async.shared::cluster.mbarrier::complete_tx::bytes.u32 [a], %3, [b];\n}\n"
-      ::"r"(smem_u32(dst)), "r"(smem_u32(bar)), "r"(rank), "r"(v) : "memory");
-}
-// mbar_wait for words that other CTAs of the cluster wrote.
-__device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity) {
-  for (uint32_t spin = 0; spin < (1u << 26); ++spin) {
-    uint32_t done;
-    asm volatile(
-        "{\n.reg .pred p;\n"
-        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
-        "selp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(done) : "r"(smem_u32(bar)), "r"(parity) : "memory");
-    if (done) return true;
-  }
-  return false;
-}
-
 struct TileCoord { int x0, y0, z0; };
-__device__ __forceinline__ TileCoord tile_coord(const SzArgs& a, unsigned int tile) {
+template <class Args>
+__device__ __forceinline__ TileCoord tile_coord(const Args& a, unsigned int tile) {
   TileCoord t;
   unsigned int tx, ty, tz;
   if (a.magic_x) {
@@ -495,15 +469,12 @@ __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.w
 constexpr int kStage = kTileCap + 16;
 constexpr unsigned int kMaxBcastWaves = 8;   // most progress steps of a broadcast (flag slots 0..7)   // one packed tile, 16-byte granular
 
-// kKind: 0 compress into a local buffer, 1 decompress from one, 2 the collectives (mode 2
-// all-gather, 3 broadcast). One body, three instantiations, so that each direction gets its
-// own register allocation and occupancy.
+// The collectives: mode 2 all-gather, 3 broadcast.
 // The cluster shape belongs to the kernel, not to the launch: as a launch attribute it was lost where
 // a profiler took over the collectives' cooperative launch, every CTA took itself for tile 0 of
 // its group, and seven tiles of eight were never written.
-template <int kKind>
-__global__ void __cluster_dims__(kClusterSize, 1, 1) __launch_bounds__(kSzThreads, kKind == 1 ? 6 : kKind == 2 ? 5 : 4) sz_kernel(const __grid_constant__ SzArgs a) {
-  const int mode = kKind == 2 ? a.mode : kKind;
+__global__ void __cluster_dims__(kClusterSize, 1, 1) __launch_bounds__(kSzThreads, 5) sz_kernel(const __grid_constant__ SzArgs a) {
+  const int mode = a.mode;
   const unsigned int kBcastWaves = a.bcast_waves;
   // Two 8 KB buffers: compress lands the next tile in one while the other is packed;
   // decompress prefixes one tile in one of them and the next in the other.
@@ -512,8 +483,6 @@ __global__ void __cluster_dims__(kClusterSize, 1, 1) __launch_bounds__(kSzThread
   __shared__ int s_tot[kTZ];
   __shared__ uint32_t s_size[2];         // this CTA's packed size per group parity, read by the cluster
   __shared__ __align__(8) uint64_t mbar[2];
-  __shared__ uint32_t s_sizes[2][kClusterSize];     // compress: the cluster's sizes, sent by their CTAs
-  __shared__ __align__(8) uint64_t size_bar[2];     // counts their arrival, per group parity
   __shared__ CtaSync sync;
 
   cg::cluster_group cluster = cg::this_cluster();
@@ -522,21 +491,15 @@ __global__ void __cluster_dims__(kClusterSize, 1, 1) __launch_bounds__(kSzThread
   const int lr = blockIdx.y, r = a.rank0 + lr, n = a.c.nranks;
   const int b = blockIdx.x;                         // flag column
   const unsigned int ntiles = (unsigned)a.tiles_x * a.tiles_y * a.tiles_z;
-  const bool collective = mode >= 2;
-  const bool i_send = mode == 0 || mode == 2 || (mode == 3 && r == a.root);
+  const bool i_send = mode == 2 || r == a.root;
   const size_t area = CCB_DATA_OFFSET + (size_t)(a.c.epoch & 1u) * a.c.half_bytes;
   if (threadIdx.x == 0) {
     sync.fail = 0;
     mbar_init(&mbar[0], 1);
     mbar_init(&mbar[1], 1);
-    if (kKind == 0) {
-      mbar_init(&size_bar[0], 1);
-      mbar_init(&size_bar[1], 1);
-    }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncthreads();
-  if (kKind == 0) cluster.sync();   // the mbarriers exist before anybody counts on them
   uint32_t phases = 0u;     // bit s: parity the next wait on mbarrier s expects
   auto landed = [&](int slot) {   // bounded wait for the copy into buffer `slot`; reports a copy that never came
     const bool ok = mbar_wait(&mbar[slot], (phases >> slot) & 1u);
@@ -548,9 +511,9 @@ __global__ void __cluster_dims__(kClusterSize, 1, 1) __launch_bounds__(kSzThread
     return ok;
   };
 
-  if (collective) trace_mark(a.c, 0);
+  trace_mark(a.c, 0);
   // ------------------------------------------------------------- compress ----
-  if (i_send && mode != 1) {
+  if (i_send) {
     const float* in = a.f[lr].in;
     unsigned long long produced = 0;
     // one thread starts the copy of this CTA's tile of group g into landing buffer `slot`
@@ -563,11 +526,10 @@ __global__ void __cluster_dims__(kClusterSize, 1, 1) __launch_bounds__(kSzThread
       mbar_expect_tx(&mbar[slot], kTileVals * 4);
       tma_load_3d(vals2[slot], &a.tmap[lr], t.x0, t.y0, t.z0, &mbar[slot]);
     };
-    // copies a packed tile out: to the local buffer, to every peer's arena one by one, or,
-    // where the arenas are bound to an NVLink multicast object, ONCE to the multicast
+    // copies a packed tile out: to every peer's arena one by one, or, where the arenas are bound to an NVLink multicast object, ONCE to the multicast
     // address: the switch replicates it, the sender's link carries the bytes one time.
     // The sender keeps no packed copy of its own field (pack_tile wrote the reconstruction).
-    const bool use_mc = kKind == 2 && a.c.mc_arena != nullptr && a.nlocal == 1;
+    const bool use_mc = a.c.mc_arena != nullptr && a.nlocal == 1;
     auto emit = [&](unsigned int g, uint32_t off, uint32_t size, const unsigned char* pk) {
       const uint4* s4 = reinterpret_cast<const uint4*>(pk);
       auto to = [&](char* slot_base) {
@@ -576,9 +538,7 @@ __global__ void __cluster_dims__(kClusterSize, 1, 1) __launch_bounds__(kSzThread
         char* dst = grp + kGroupHeader + off;
         for (uint32_t i = threadIdx.x; i < size / 16; i += kSzThreads) stg(dst + 16 * i, s4[i]);
       };
-      if (mode == 0) {
-        to(a.local_out);
-      } else if (use_mc) {
+      if (use_mc) {
         char* grp = a.c.mc_arena + area + (size_t)r * a.slot_bytes + (size_t)g * kGroupStride;
         if (threadIdx.x == 0) multimem_st_u32(grp + 4 * k, size);
         char* dst = grp + kGroupHeader + off;
@@ -592,7 +552,7 @@ __global__ void __cluster_dims__(kClusterSize, 1, 1) __launch_bounds__(kSzThread
     const unsigned int my_iters = cl < a.ngroups ? (a.ngroups - cl + ncl - 1) / ncl : 0;
     auto wave_end = [&](unsigned int w) { return (unsigned int)(((unsigned long long)my_iters * (w + 1)) / kBcastWaves); };
     unsigned int wave = 0;
-    float* own_out = kKind == 2 ? a.f[lr].out + (mode == 2 ? (size_t)r * a.nx * a.ny * a.nz : 0) : nullptr;
+    float* own_out = a.f[lr].out + (mode == 2 ? (size_t)r * a.nx * a.ny * a.nz : 0);
     prefetch(cl, 0);
     uint32_t it = 0, pend_size = 0, pend_off = 0;
     unsigned int pend_g = 0;
@@ -616,24 +576,6 @@ __global__ void __cluster_dims__(kClusterSize, 1, 1) __launch_bounds__(kSzThread
         size = pack_tile(cur, pk2[slot], s_tot, a, !ok, own_out, tile_coord(a, tile));
       } else {
         __syncthreads();   // keeps one CTA barrier per iteration between a copy-out and its signal
-      }
-      if constexpr (kKind == 0) {
-        // Compressing into a local buffer the CTAs exchange nothing but their sizes: each sends
-        // its own to the eight and waits for eight words. A cluster barrier's release waited
-        // for the copy-out's global stores as well, a fifth of the stall cycles: packing a 512^3
-        // field took 419 us with it and takes 344 (B200).
-        // The words of this parity are written again two groups on, by a CTA that has this
-        // CTA's size of the next group, sent after all its threads read the words here.
-        if (threadIdx.x == 0) mbar_expect_tx(&size_bar[slot], 4 * kClusterSize);
-        if (threadIdx.x < kClusterSize) st_async_u32(&s_sizes[slot][k], &size_bar[slot], threadIdx.x, size);
-        if (pend) emit(pend_g, pend_off, pend_size, pk2[slot ^ 1]);
-        const bool ok = mbar_wait_cluster(&size_bar[slot], (it >> 1) & 1u);
-        const int ln = threadIdx.x & 31;
-        uint32_t off = __reduce_add_sync(0xffffffffu, ok && ln < k ? s_sizes[slot][ln] : 0u);
-        if (!ok) sync.fail = 1;   // the tile may land in another's place, inside the slot: the whole group is given up below
-        pend = true; pend_g = g; pend_off = off; pend_size = size;
-        produced += size;
-        continue;
       }
       if (threadIdx.x == 0) s_size[slot] = size;
       // One cluster barrier per group, split in two so that the copy-out of the PREVIOUS
@@ -665,24 +607,14 @@ __global__ void __cluster_dims__(kClusterSize, 1, 1) __launch_bounds__(kSzThread
           if (wave_end(wave) > (wave ? wave_end(wave - 1) : 0u)) signal_peers(a.c, ((1u << n) - 1u) & ~(1u << r), (int)wave, r, b);
     }
     cluster.sync();      // nobody leaves while a neighbour may still read its sizes
-    if (kKind == 0 && sync.fail && threadIdx.x == 0) {
-      // A wait above gave up: none of these groups is to be trusted. Their size words say so (a
-      // container is refused, unpacking stays inside the slot), and the top bit of the byte count.
-      for (unsigned int g = cl; g < a.ngroups; g += ncl)
-        for (int j = 0; j < kClusterSize; ++j) reinterpret_cast<uint32_t*>(a.local_out + (size_t)g * kGroupStride)[j] = kLostTile;
-      if (a.used_bytes) atomicOr(a.used_bytes + lr, 1ull << 63);
-    }
     if (a.used_bytes && threadIdx.x == 0 && produced) atomicAdd(a.used_bytes + lr, produced + 0ull);
   }
-  if (mode == 0) return;
 
   // --------------------------------------------------------------- signal ----
-  if (collective) trace_mark(a.c, 1);
-  if (collective) {
-    __syncthreads();
-    if (mode == 2 && threadIdx.x == 0) signal_peers(a.c, ((1u << n) - 1u) & ~(1u << r), 0, r, b);
-    // All-gather waits source by source inside the decode loop; broadcast wave by wave.
-  }
+  trace_mark(a.c, 1);
+  __syncthreads();
+  if (mode == 2 && threadIdx.x == 0) signal_peers(a.c, ((1u << n) - 1u) & ~(1u << r), 0, r, b);
+  // All-gather waits source by source inside the decode loop; broadcast wave by wave.
 
   // ------------------------------------------------------------ decompress ---
   // Work items (source, group) of this cluster, flattened; the size words of the next
@@ -693,20 +625,20 @@ __global__ void __cluster_dims__(kClusterSize, 1, 1) __launch_bounds__(kSzThread
   const int ln = threadIdx.x & 31;
   auto group_of = [&](unsigned int f) -> const char* {
     const int q = mode == 2 ? (r + 1 + (int)(f / per_src)) % n : a.root;
-    const char* slot = mode == 1 ? a.local_in : a.c.arena[r] + area + (size_t)q * a.slot_bytes;
+    const char* slot = a.c.arena[r] + area + (size_t)q * a.slot_bytes;
     return slot + (size_t)(cl + (f % per_src) * ncl) * kGroupStride;
   };
   auto valid = [&](unsigned int f) { return f < nitems && (cl + (f % per_src) * ncl) * kClusterSize + k < ntiles; };
   auto sizes_of = [&](unsigned int f) -> uint32_t {   // lane j < k gets the size of tile j of the group
     return (valid(f) && ln < k) ? ldg_cg_u32(group_of(f) + 4 * ln) : 0u;
   };
-  if (collective) trace_mark(a.c, 2);
+  trace_mark(a.c, 2);
   auto dwave_end = [&](unsigned int w) { return (unsigned int)(((unsigned long long)per_src * (w + 1)) / kBcastWaves); };
   unsigned int dwave = 0;
   int scratch = 0;
-  uint32_t sz_next = (mode == 1) ? sizes_of(0) : 0u;
+  uint32_t sz_next = 0u;
   for (unsigned int f = 0; f < nitems; ++f) {
-    if (collective && per_src && f == per_src) trace_mark(a.c, 3);   // first received field decoded
+    if (per_src && f == per_src) trace_mark(a.c, 3);   // first received field decoded
     if (mode == 2 && f % per_src == 0) {   // first item of the next source: its CTA of the same index must be done
       const int src = (r + 1 + (int)(f / per_src)) % n;
       if (!cta_wait_sources(sync, a.c, a.c.arena[r], 0, r, 1u << src, 0xA0)) return;
@@ -739,8 +671,412 @@ __global__ void __cluster_dims__(kClusterSize, 1, 1) __launch_bounds__(kSzThread
     unpack_tile(reinterpret_cast<const unsigned char*>(group_of(f)) + kGroupHeader + off, reinterpret_cast<int*>(vals2[0]), scratch, a,
                 out, tile_coord(a, (cl + (f % per_src) * ncl) * kClusterSize + k));
   }
-  if (collective) trace_mark(a.c, 4);
+  trace_mark(a.c, 4);
   if (mode == 3) end_handshake(sync, a.c, r);
+}
+
+// ------------------------------------------------------- local buffers, a warp a tile --
+// Compression into and decompression from a buffer of this GPU. A warp owns a tile and walks its
+// eight planes: a lane holds eight consecutive x of line y = lane / 4 (the mapping above), the plane
+// before stays in its registers, y and x neighbours come by shuffles, and the words of a plane go
+// behind those of the plane before. So nothing of a tile is exchanged between warps, there is one
+// barrier a GROUP (a CTA of eight warps), for the tiles' sizes, and no cluster. Both directions are
+// bound by instruction issue, not far above the memory's rate. (512^3 field, bound 1e-4 of its range,
+// B200: with a CTA a tile, its planes on eight warps, three barriers a tile and the sizes sent round a
+// cluster, packing took 345 us and unpacking 275, 458 and 389 warp instructions for 256 values.)
+struct SzLocalArgs {
+  const float* in;
+  float* out;
+  char* slots;
+  unsigned long long* used_bytes;
+  int nx, ny, nz, tiles_x, tiles_y, tiles_z;
+  unsigned int ngroups;
+  float eb, two_eb, inv_two_eb;
+  unsigned long long magic_x, magic_xy;
+};
+constexpr int kWarpStage = 4096;   // bytes of a packed tile that a warp stages; what is larger is packed a second time, to its place
+
+// How a lane's eight values lie in memory: every line on 32 bytes (kVec 8), on 16 (4), or anywhere
+// (1: a plane goes through shared memory, so that the accesses of a warp lie side by side).
+template <int kVec>
+struct PlaneIO {
+  const SzLocalArgs& a;
+  TileCoord t;
+  float* sh;   // kVec 1: 256 floats of this warp
+  int lane;
+  __device__ __forceinline__ void load(int z, float (&v)[8]) const {   // raw: kVec 1 holds column `lane` of the eight lines
+    const int gz = t.z0 + z;
+    if constexpr (kVec == 1) {
+      const int gx = t.x0 + lane;
+      const float* p = a.in + ((size_t)gz * a.ny + t.y0) * a.nx + gx;
+#pragma unroll
+      for (int y = 0; y < kTY; ++y) v[y] = gx < a.nx && t.y0 + y < a.ny && gz < a.nz ? __ldcs(p + (size_t)y * a.nx) : 0.f;
+    } else {
+      const int gx = t.x0 + 8 * (lane & 3), gy = t.y0 + (lane >> 2);
+      const float* p = a.in + ((size_t)gz * a.ny + gy) * a.nx + gx;
+      const bool in = gx < a.nx && gy < a.ny && gz < a.nz;
+      uint32_t w[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
+      if constexpr (kVec == 8) {
+        if (in) ldg_stream32(p, w);
+      } else {
+        if (in) { const uint4 u = ldg_stream(p); w[0] = u.x; w[1] = u.y; w[2] = u.z; w[3] = u.w; }
+        if (in && gx + 4 < a.nx) { const uint4 u = ldg_stream(p + 4); w[4] = u.x; w[5] = u.y; w[6] = u.z; w[7] = u.w; }
+      }
+#pragma unroll
+      for (int e = 0; e < 8; ++e) v[e] = __uint_as_float(w[e]);
+    }
+  }
+  __device__ __forceinline__ void settle(float (&v)[8]) const {   // raw -> the lane's eight consecutive x
+    if constexpr (kVec == 1) {
+#pragma unroll
+      for (int y = 0; y < kTY; ++y) sh[kTX * y + lane] = v[y];
+      __syncwarp();
+      const float4 p = reinterpret_cast<const float4*>(sh)[2 * lane], q = reinterpret_cast<const float4*>(sh)[2 * lane + 1];
+      v[0] = p.x; v[1] = p.y; v[2] = p.z; v[3] = p.w; v[4] = q.x; v[5] = q.y; v[6] = q.z; v[7] = q.w;
+      __syncwarp();
+    }
+  }
+  __device__ __forceinline__ void store(int z, const float (&v)[8]) const {
+    const int gz = t.z0 + z;
+    if constexpr (kVec == 1) {
+      reinterpret_cast<float4*>(sh)[2 * lane] = make_float4(v[0], v[1], v[2], v[3]);
+      reinterpret_cast<float4*>(sh)[2 * lane + 1] = make_float4(v[4], v[5], v[6], v[7]);
+      __syncwarp();
+      const int gx = t.x0 + lane;
+      float* p = a.out + ((size_t)gz * a.ny + t.y0) * a.nx + gx;
+#pragma unroll
+      for (int y = 0; y < kTY; ++y)
+        if (gx < a.nx && t.y0 + y < a.ny && gz < a.nz) p[(size_t)y * a.nx] = sh[kTX * y + lane];
+      __syncwarp();
+    } else {
+      const int gx = t.x0 + 8 * (lane & 3), gy = t.y0 + (lane >> 2);
+      float* p = a.out + ((size_t)gz * a.ny + gy) * a.nx + gx;
+      if (gx >= a.nx || gy >= a.ny || gz >= a.nz) return;
+      uint32_t w[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) w[e] = __float_as_uint(v[e]);
+      if constexpr (kVec == 8) {
+        stg_stream32(p, w);
+      } else {
+        stg_stream(p, make_uint4(w[0], w[1], w[2], w[3]));
+        if (gx + 4 < a.nx) stg_stream(p + 4, make_uint4(w[4], w[5], w[6], w[7]));
+      }
+    }
+  }
+};
+
+// Codes of one plane; see pack_tile for the arithmetic, which is the same.
+__device__ __forceinline__ void plane_codes(const float (&x)[8], const SzLocalArgs& a, int (&q)[8], bool& bad) {
+  const float half = 0.5f * a.two_eb;
+  float s[8], r[8], smax = 0.f;
+  bool far = false;
+#pragma unroll
+  for (int e = 0; e < 8; ++e) s[e] = x[e];
+#pragma unroll
+  for (int e = 0; e < 8; e += 2) mul2(s[e], s[e + 1], a.inv_two_eb);
+#pragma unroll
+  for (int e = 0; e < 8; ++e) {
+    smax = fmaxf(smax, fabsf(s[e]));
+    r[e] = __fadd_rn(s[e], kRoundMagic);
+    q[e] = __float_as_int(r[e]) - __float_as_int(kRoundMagic);
+  }
+#pragma unroll
+  for (int e = 0; e < 8; e += 2) {
+    add2(r[e], r[e + 1], -kRoundMagic);
+    mul2(r[e], r[e + 1], a.two_eb);
+  }
+#pragma unroll
+  for (int e = 0; e < 8; ++e) far |= !(fabsf(__fsub_rn(x[e], r[e])) <= half);
+  bad |= !(smax < kQMax);
+  if (__any_sync(0xffffffffu, far)) {
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      const float se = __fmul_rn(x[e], a.inv_two_eb);
+      bad |= !(fabsf(se) < kQMax);
+      float rf = __fadd_rn(__fadd_rn(se, kRoundMagic), -kRoundMagic);
+      const float diff = __fsub_rn(x[e], __fmul_rn(rf, a.two_eb));
+      rf += diff > half ? 1.f : 0.f;
+      rf -= -diff > half ? 1.f : 0.f;
+      bad |= fabsf(__fsub_rn(x[e], __fmul_rn(rf, a.two_eb))) > a.eb;
+      q[e] = (int)rf;
+    }
+  }
+}
+
+// Packs the warp's tile to `pk` (64 width bytes, then the planes). Returns its words and whether it
+// has to be stored raw. Words beyond `room` are counted and not written.
+template <int kVec>
+__device__ __forceinline__ uint32_t pack_planes(const PlaneIO<kVec>& io, unsigned char* pk, uint32_t room, bool& bad) {
+  const int lane = io.lane;
+  uint32_t* words = reinterpret_cast<uint32_t*>(pk + kRows);
+  int before[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+  uint32_t run = 0;
+  float ahead[8];
+  io.load(0, ahead);
+#pragma unroll 1
+  for (int z = 0; z < kTZ; ++z) {
+    float x[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) x[e] = ahead[e];
+    if (z + 1 < kTZ) io.load(z + 1, ahead);   // the next plane is on its way while this one is packed
+    io.settle(x);
+    int q[8], d[8];
+    plane_codes(x, io.a, q, bad);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      d[e] = q[e] - before[e];
+      before[e] = q[e];
+    }
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      const int up = __shfl_up_sync(0xffffffffu, d[e], 4);
+      if (lane >= 4) d[e] -= up;
+    }
+    const int left = __shfl_up_sync(0xffffffffu, d[7], 1);
+#pragma unroll
+    for (int e = 7; e >= 1; --e) d[e] -= d[e - 1];
+    if (lane & 3) d[0] -= left;
+    // Residuals of eight bits or less, nearly always: as bytes d + 128, four to a word. The zig-zag of
+    // four bytes is five operations; rows, planes and widths as in pack_tile.
+    uint32_t t[8], high = 0u;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      t[e] = (uint32_t)(d[e] + 128);
+      high |= t[e];
+    }
+    uint32_t W0 = 0u, W1 = 0u, u[8], tot_lo, tot;
+    const bool narrow = !__any_sync(0xffffffffu, high > 0xffu);
+    if (narrow) {
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        const uint32_t b = __byte_perm(__byte_perm(t[4 * k], t[4 * k + 1], 0x0040), __byte_perm(t[4 * k + 2], t[4 * k + 3], 0x0040), 0x5410);
+        const uint32_t minus = ((b >> 7) & 0x01010101u) ^ 0x01010101u;
+        u[k] = transpose32(((b << 1) & 0xfefefefeu) ^ (minus * 0xffu), lane);
+      }
+      W0 = __ballot_sync(0xffffffffu, u[0] != 0u);
+      W1 = __ballot_sync(0xffffffffu, u[1] != 0u);
+      W0 |= (W0 >> 1) & 0x7f7f7f7fu;
+      W1 |= (W1 >> 1) & 0x7f7f7f7fu;
+      W0 |= (W0 >> 2) & 0x3f3f3f3fu;
+      W1 |= (W1 >> 2) & 0x3f3f3f3fu;
+      W0 |= (W0 >> 4) & 0x0f0f0f0fu;
+      W1 |= (W1 >> 4) & 0x0f0f0f0fu;
+      if (lane < 8) pk[8 * z + lane] = (unsigned char)__popc(((lane < 4 ? W0 : W1) >> (8 * (lane & 3))) & 0xffu);
+      tot_lo = __popc(W0);
+      tot = tot_lo + __popc(W1);
+      if (run + tot <= room) {
+        const uint32_t below = (1u << lane) - 1u;
+        if ((W0 >> lane) & 1u) words[run + __popc(W0 & below)] = u[0];
+        if ((W1 >> lane) & 1u) words[run + tot_lo + __popc(W1 & below)] = u[1];
+      }
+    } else {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) u[e] = ((uint32_t)d[e] << 1) ^ (uint32_t)(d[e] >> 31);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const uint32_t w = 32 - __clz((int)__reduce_or_sync(0xffffffffu, u[e]));
+        if (e < 4) W0 |= w << (8 * e);
+        else W1 |= w << (8 * (e - 4));
+      }
+      tot_lo = bytesum(W0);
+      tot = tot_lo + bytesum(W1);
+      if (lane == 0) reinterpret_cast<uint2*>(pk)[z] = make_uint2(W0, W1);
+      if (run + tot <= room) {
+        uint32_t ua[4] = {u[0], u[1], u[2], u[3]}, ub[4] = {u[4], u[5], u[6], u[7]};
+        wide_planes4<true>(ua, W0, run, words, lane);
+        wide_planes4<true>(ub, W1, run + tot_lo, words, lane);
+      }
+    }
+    run += tot;
+  }
+  const uint32_t pad = (0u - run) & 3u;   // the tile ends on 16 bytes (64 width bytes before the words)
+  if ((uint32_t)lane < pad && run + pad <= room) words[run + lane] = 0u;
+  return run;
+}
+
+template <int kVec>
+__global__ void __launch_bounds__(kSzThreads, 4) sz_pack_kernel(const __grid_constant__ SzLocalArgs a) {
+  __shared__ __align__(16) unsigned char stage[kClusterSize][kWarpStage];
+  __shared__ __align__(16) float plane[kVec == 1 ? kClusterSize : 1][kVec == 1 ? kTX * kTY : 4];
+  __shared__ uint32_t s_size[kClusterSize];
+  const int lane = threadIdx.x & 31, k = threadIdx.x >> 5;
+  const unsigned int tile = blockIdx.x * kClusterSize + k;
+  char* group = a.slots + (size_t)blockIdx.x * kGroupStride;
+  const PlaneIO<kVec> io = {a, tile_coord(a, tile), plane[kVec == 1 ? k : 0], lane};
+  uint32_t size = 0;
+  bool raw = false;
+  if (tile < (unsigned)a.tiles_x * a.tiles_y * a.tiles_z) {
+    bool bad = false;
+    const uint32_t words = pack_planes<kVec>(io, stage[k], (kWarpStage - kRows) / 4, bad);
+    raw = __any_sync(0xffffffffu, bad);
+    size = raw ? kRows + kTileVals * 4u : (kRows + 4u * words + 15u) & ~15u;
+  }
+  if (lane == 0) s_size[k] = size;
+  __syncthreads();
+  const uint32_t of = lane < kClusterSize ? s_size[lane] : 0u;
+  const uint32_t off = __reduce_add_sync(0xffffffffu, lane < k ? of : 0u);
+  if (k == 0) {
+    const uint32_t all = __reduce_add_sync(0xffffffffu, of);
+    if (lane < kClusterSize) reinterpret_cast<uint32_t*>(group)[lane] = of;
+    if (lane == 0 && a.used_bytes) atomicAdd(a.used_bytes, (unsigned long long)all);
+  }
+  if (size == 0) return;
+  char* dst = group + kGroupHeader + off;
+  if (raw) {   // marker and the fp32 values
+    reinterpret_cast<uint16_t*>(dst)[lane] = lane == 0 ? 255 : 0;
+#pragma unroll 1
+    for (int z = 0; z < kTZ; ++z) {
+      float x[8];
+      io.load(z, x);
+      io.settle(x);
+      float4* to = reinterpret_cast<float4*>(dst + kRows) + 2 * (32 * z + lane);
+      to[0] = make_float4(x[0], x[1], x[2], x[3]);
+      to[1] = make_float4(x[4], x[5], x[6], x[7]);
+    }
+  } else if (size <= (uint32_t)kWarpStage) {
+    __syncwarp();
+    for (uint32_t i = lane; i < size / 16; i += 32) stg(dst + 16 * i, reinterpret_cast<const uint4*>(stage[k])[i]);
+  } else {
+    bool bad = false;
+    pack_planes<kVec>(io, reinterpret_cast<unsigned char*>(dst), (uint32_t)kTileVals, bad);
+  }
+}
+
+template <int kVec>
+__global__ void __launch_bounds__(kSzThreads, 4) sz_unpack_kernel(const __grid_constant__ SzLocalArgs a) {
+  __shared__ __align__(16) float plane[kVec == 1 ? kClusterSize : 1][kVec == 1 ? kTX * kTY : 4];
+  const int lane = threadIdx.x & 31, k = threadIdx.x >> 5;
+  const unsigned int tile = blockIdx.x * kClusterSize + k;
+  if (tile >= (unsigned)a.tiles_x * a.tiles_y * a.tiles_z) return;
+  const char* group = a.slots + (size_t)blockIdx.x * kGroupStride;
+  const PlaneIO<kVec> io = {a, tile_coord(a, tile), plane[kVec == 1 ? k : 0], lane};
+  uint32_t off = __reduce_add_sync(0xffffffffu, lane < k ? ldg_cg_u32(group + 4 * lane) : 0u);
+  if (off > (uint32_t)(kClusterSize * kTileCap)) off = 0;   // damaged size words: stay inside the slot
+  const unsigned char* src = reinterpret_cast<const unsigned char*>(group) + kGroupHeader + off;
+  const uint32_t hw = lane < 16 ? ldg_cg_u32(src + 4 * lane) : 0u;   // the row widths, four a word
+  if ((__shfl_sync(0xffffffffu, hw, 0) & 0xffu) == 255u) {
+    const float4* raw = reinterpret_cast<const float4*>(src + kRows);
+#pragma unroll 1
+    for (int z = 0; z < kTZ; ++z) {
+      const uint4 p = ldg_cg(raw + 2 * (32 * z + lane)), q = ldg_cg(raw + 2 * (32 * z + lane) + 1);
+      const float v[8] = {__uint_as_float(p.x), __uint_as_float(p.y), __uint_as_float(p.z), __uint_as_float(p.w),
+                          __uint_as_float(q.x), __uint_as_float(q.y), __uint_as_float(q.z), __uint_as_float(q.w)};
+      io.store(z, v);
+    }
+    return;
+  }
+  uint32_t* words = reinterpret_cast<uint32_t*>(const_cast<unsigned char*>(src) + kRows);
+  // the words of a plane with widths of eight bits or less: lane 8 r + j fetches plane j of row r
+  struct Ahead { uint32_t W0, W1, X0, X1; bool narrow; };
+  uint32_t run = 0, next_run = 0;
+  auto fetch = [&](int z) -> Ahead {
+    Ahead h;
+    h.W0 = __shfl_sync(0xffffffffu, hw, 2 * z);
+    h.W1 = __shfl_sync(0xffffffffu, hw, 2 * z + 1);
+    h.narrow = bytes_le8(h.W0) && bytes_le8(h.W1);
+    h.X0 = h.X1 = 0u;
+    const uint32_t lo = bytesum(h.W0);
+    if (h.narrow) {
+      const int sh = lane & 24, j = lane & 7;
+      const uint32_t below = (1u << sh) - 1u;
+      if ((uint32_t)j < ((h.W0 >> sh) & 0xffu)) h.X0 = ldg_cg_u32(words + next_run + bytesum(h.W0 & below) + j);
+      if ((uint32_t)j < ((h.W1 >> sh) & 0xffu)) h.X1 = ldg_cg_u32(words + next_run + lo + bytesum(h.W1 & below) + j);
+    }
+    next_run += lo + bytesum(h.W1);
+    return h;
+  };
+  int acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};   // the plane before, then this one
+  // A narrow plane's residuals are summed along x and y as bytes d + 128 in halves of a word: 256 of
+  // them fit 16 bits, and what the 128s come to at (x, y) is known.
+  const int bias0 = 128 * (8 * (lane & 3) + 1) * ((lane >> 2) + 1), bias_step = 128 * ((lane >> 2) + 1);
+  Ahead ahead = fetch(0);
+#pragma unroll 1
+  for (int z = 0; z < kTZ; ++z) {
+    const Ahead h = ahead;
+    const uint32_t at = run;
+    run = next_run;
+    if (z + 1 < kTZ) ahead = fetch(z + 1);
+    if (h.narrow) {
+      uint32_t A[2], B[2];   // elements (0, 2) and (1, 3) of each four
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const uint32_t U = transpose32(i ? h.X1 : h.X0, lane);
+        const uint32_t b = ((U >> 1) & 0x7f7f7f7fu) ^ (0x80808080u - (U & 0x01010101u));   // zig-zag undone, plus 128
+        A[i] = b & 0x00ff00ffu;
+        B[i] = ((b >> 8) & 0x00ff00ffu) + A[i];
+        const uint32_t lower = B[i] << 16;
+        A[i] += lower;
+        B[i] += lower;
+      }
+      uint32_t c = (B[0] >> 16) * 0x00010001u;
+      A[1] += c;
+      B[1] += c;
+      const uint32_t line = B[1] >> 16;   // then across the four threads of the line
+      uint32_t sum = line, v = __shfl_up_sync(0xffffffffu, sum, 1);
+      if ((lane & 3) >= 1) sum += v;
+      v = __shfl_up_sync(0xffffffffu, sum, 2);
+      if ((lane & 3) >= 2) sum += v;
+      c = (sum - line) * 0x00010001u;
+      uint32_t p[4] = {A[0] + c, B[0] + c, A[1] + c, B[1] + c};
+#pragma unroll
+      for (int s = 4; s < 32; s <<= 1) {   // and down the eight lines
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const uint32_t w = __shfl_up_sync(0xffffffffu, p[i], s);
+          if (lane >= s) p[i] += w;
+        }
+      }
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const uint32_t w = p[(e >> 2) * 2 + (e & 1)];
+        acc[e] += (int)(e & 2 ? w >> 16 : w & 0xffffu) - (bias0 + e * bias_step);
+      }
+    } else {
+      uint32_t u[8];
+      auto four = [&](int first, uint32_t W, uint32_t from) {
+        uint32_t f[4];
+        if (bytes_le8(W)) {
+          const int sh = lane & 24, j = lane & 7;
+          const uint32_t U = transpose32((uint32_t)j < ((W >> sh) & 0xffu) ? ldg_cg_u32(words + from + bytesum(W & ((1u << sh) - 1u)) + j) : 0u, lane);
+#pragma unroll
+          for (int r = 0; r < 4; ++r) f[r] = (U >> (8 * r)) & 0xffu;
+        } else {
+          wide_planes4<false>(f, W, from, words, lane);
+        }
+#pragma unroll
+        for (int r = 0; r < 4; ++r) u[first + r] = f[r];
+      };
+      four(0, h.W0, at);
+      four(4, h.W1, at + bytesum(h.W0));
+      int p[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const int d = (int)(u[e] >> 1) ^ -(int)(u[e] & 1u);
+        p[e] = e ? p[e - 1] + d : d;
+      }
+      int sum = p[7], v = __shfl_up_sync(0xffffffffu, sum, 1);
+      if ((lane & 3) >= 1) sum += v;
+      v = __shfl_up_sync(0xffffffffu, sum, 2);
+      if ((lane & 3) >= 2) sum += v;
+      const int before = sum - p[7];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) p[e] += before;
+#pragma unroll
+      for (int s = 4; s < 32; s <<= 1) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+          const int w = __shfl_up_sync(0xffffffffu, p[e], s);
+          if (lane >= s) p[e] += w;
+        }
+      }
+#pragma unroll
+      for (int e = 0; e < 8; ++e) acc[e] += p[e];
+    }
+    float f[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) f[e] = __fmul_rn((float)acc[e], a.two_eb);
+    io.store(z, f);
+  }
 }
 
 // ----------------------------------------------------------------- container ----
@@ -895,7 +1231,8 @@ static bool make_tmap(CUtensorMap* m, const float* base, int nx, int ny, int nz)
              CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-static void fill_geometry(SzArgs& a, int nx, int ny, int nz, float eb) {
+template <class Args>
+static void fill_geometry(Args& a, int nx, int ny, int nz, float eb) {
   a.nx = nx; a.ny = ny; a.nz = nz;
   a.tiles_x = (nx + kTX - 1) / kTX;
   a.tiles_y = (ny + kTY - 1) / kTY;
@@ -934,9 +1271,9 @@ static int resident_clusters(void (*kernel)(const SzArgs), const cudaLaunchConfi
   return clusters;
 }
 
-// Launch of clusters of 8 CTAs (__cluster_dims__); cooperative when the kernel waits on peers.
-static int sz_launch(SzArgs& a, int nlocal, int num_sms, bool waits, cudaStream_t stream) {
-  void (*kernel)(const SzArgs) = a.mode == 0 ? sz_kernel<0> : a.mode == 1 ? sz_kernel<1> : sz_kernel<2>;
+// Launch of clusters of 8 CTAs (__cluster_dims__), cooperative: the kernel waits on peers.
+static int sz_launch(SzArgs& a, int nlocal, int num_sms, cudaStream_t stream) {
+  void (*kernel)(const SzArgs) = sz_kernel;
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof(cfg));
   cudaLaunchAttribute attr;
@@ -951,15 +1288,13 @@ static int sz_launch(SzArgs& a, int nlocal, int num_sms, bool waits, cudaStream_
   if (clusters > cap) clusters = cap;
   if (clusters * kClusterSize > CCB_MAX_CTAS) clusters = CCB_MAX_CTAS / kClusterSize;
   cfg.gridDim = dim3(clusters * kClusterSize, (unsigned)nlocal, 1);
-  if (waits) {
-    attr.id = cudaLaunchAttributeCooperative;
-    attr.val.cooperative = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-  }
+  attr.id = cudaLaunchAttributeCooperative;
+  attr.val.cooperative = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
   cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, a);
-  if (waits) g_sz_launch_path = 1;
-  if (e != cudaSuccess && waits) {  // some drivers refuse cluster + cooperative: the bounded grid still fits
+  g_sz_launch_path = 1;
+  if (e != cudaSuccess) {  // some drivers refuse cluster + cooperative: the bounded grid still fits
     (void)cudaGetLastError();
     cfg.numAttrs = 0;
     g_sz_launch_path = 2;
@@ -985,7 +1320,12 @@ static unsigned int container_grid(uint64_t ngroups) {
   const uint64_t most = (uint64_t)device_sms() * 8;
   return (unsigned int)(ngroups < most ? ngroups : most);
 }
-static int container_done(const char* what) {
+// See PlaneIO.
+static int line_width(const void* field, int nx) {
+  const uintptr_t at = reinterpret_cast<uintptr_t>(field);
+  return nx % 8 == 0 && at % 32 == 0 ? 8 : nx % 4 == 0 && at % 16 == 0 ? 4 : 1;
+}
+static int launched(const char* what) {
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {
     set_error("%s: %s", what, cudaGetErrorString(e));
@@ -1014,18 +1354,20 @@ extern "C" int ccb_sz_compress(const float* in, int nx, int ny, int nz, float eb
     set_error("ccb_sz_compress: bad arguments");
     return CCB_ERR_ARG;
   }
-  SzArgs a;
+  SzLocalArgs a;
   memset(&a, 0, sizeof(a));
   fill_geometry(a, nx, ny, nz, eb);
-  a.c.nranks = 1;
-  a.f[0].in = in;
-  a.local_out = static_cast<char*>(out);
+  a.in = in;
+  a.slots = static_cast<char*>(out);
   a.used_bytes = d_used;
-  a.use_tma = make_tmap(&a.tmap[0], in, nx, ny, nz) ? 1 : 0;
-  a.mode = 0;
-  a.nlocal = 1;
-  if (d_used) cudaMemsetAsync(d_used, 0, sizeof(unsigned long long), static_cast<cudaStream_t>(stream));
-  return sz_launch(a, 1, device_sms(), false, static_cast<cudaStream_t>(stream));
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  if (d_used) cudaMemsetAsync(d_used, 0, sizeof(unsigned long long), s);
+  switch (line_width(in, nx)) {
+    case 8: sz_pack_kernel<8><<<a.ngroups, kSzThreads, 0, s>>>(a); break;
+    case 4: sz_pack_kernel<4><<<a.ngroups, kSzThreads, 0, s>>>(a); break;
+    default: sz_pack_kernel<1><<<a.ngroups, kSzThreads, 0, s>>>(a);
+  }
+  return launched("ccb_sz_compress");
 }
 
 extern "C" int ccb_sz_decompress(const void* in, int nx, int ny, int nz, float eb, float* out, ccb_stream_t stream) {
@@ -1033,15 +1375,18 @@ extern "C" int ccb_sz_decompress(const void* in, int nx, int ny, int nz, float e
     set_error("ccb_sz_decompress: bad arguments");
     return CCB_ERR_ARG;
   }
-  SzArgs a;
+  SzLocalArgs a;
   memset(&a, 0, sizeof(a));
   fill_geometry(a, nx, ny, nz, eb);
-  a.c.nranks = 1;
-  a.f[0].out = out;
-  a.local_in = static_cast<const char*>(in);
-  a.mode = 1;
-  a.nlocal = 1;
-  return sz_launch(a, 1, device_sms(), false, static_cast<cudaStream_t>(stream));
+  a.out = out;
+  a.slots = const_cast<char*>(static_cast<const char*>(in));
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  switch (line_width(out, nx)) {
+    case 8: sz_unpack_kernel<8><<<a.ngroups, kSzThreads, 0, s>>>(a); break;
+    case 4: sz_unpack_kernel<4><<<a.ngroups, kSzThreads, 0, s>>>(a); break;
+    default: sz_unpack_kernel<1><<<a.ngroups, kSzThreads, 0, s>>>(a);
+  }
+  return launched("ccb_sz_decompress");
 }
 
 // offsets: ngroups + 2 words of 64 bits (see container_scan_kernel). Exactly one of slots and
@@ -1053,7 +1398,7 @@ extern "C" int ccb_sz_container_scan(const void* slots, const uint32_t* sizes, u
     return CCB_ERR_ARG;
   }
   container_scan_kernel<<<1, kScanThreads, 0, static_cast<cudaStream_t>(stream)>>>(static_cast<const char*>(slots), sizes, (unsigned int)ngroups, offsets);
-  return container_done("ccb_sz_container_scan");
+  return launched("ccb_sz_container_scan");
 }
 
 // out: 40 + 4 * ngroups + offsets[ngroups] bytes, 4-byte aligned.
@@ -1065,7 +1410,7 @@ extern "C" int ccb_sz_container_pack(const void* slots, const unsigned long long
   }
   const ContainerHead head = {kContainerMagic, kContainerVersion, nx, ny, nz, eb, 2.f * eb * (1.f - 0.0009765625f), (uint32_t)ngroups, 0};
   container_pack_kernel<<<container_grid(ngroups), 256, 0, static_cast<cudaStream_t>(stream)>>>(static_cast<const char*>(slots), offsets, head, static_cast<char*>(out));
-  return container_done("ccb_sz_container_pack");
+  return launched("ccb_sz_container_pack");
 }
 
 // payload: offsets[ngroups] bytes; slots: ngroups * kGroupStride bytes, 16-byte aligned.
@@ -1076,7 +1421,7 @@ extern "C" int ccb_sz_container_unpack(const void* payload, const unsigned long 
   }
   container_unpack_kernel<<<container_grid(ngroups), 256, 0, static_cast<cudaStream_t>(stream)>>>(static_cast<const char*>(payload), offsets,
                                                                                                    (unsigned int)ngroups, static_cast<char*>(slots));
-  return container_done("ccb_sz_container_unpack");
+  return launched("ccb_sz_container_unpack");
 }
 
 // Error-bounded AllGather (root < 0) or Broadcast (root >= 0) of one nx*ny*nz field per
@@ -1129,5 +1474,5 @@ extern "C" int ccb_sz_collective(ccb_comm* c, const float* const* send, float* c
     a.bcast_waves = (unsigned int)waves;
   }
   if (d_used) cudaMemsetAsync(d_used, 0, sizeof(unsigned long long) * nlocal, stream);
-  return sz_launch(a, nlocal, device_sms(), true, stream);
+  return sz_launch(a, nlocal, device_sms(), stream);
 }
