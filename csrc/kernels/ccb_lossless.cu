@@ -10,8 +10,8 @@
 // exponents of neighbouring values within a few octaves, so 3 to 5 planes replace 8 bits.
 //
 // Work decomposition: a warp owns a block of 512 values (16 per lane, like the other
-// codecs); the bit planes are built with warp ballots, one 32-bit word per (plane,
-// element-of-lane), and read back with warp-uniform loads. A CTA of 8 warps owns a TILE of
+// codecs); the bit planes are built, and read back, by bit-matrix transposes across the warp, one
+// 32-bit word per (plane, element-of-lane). A CTA of 8 warps owns a TILE of
 // 8 blocks = 4096 values and packs the variable-length exponent planes of its blocks
 // back to back inside the tile's fixed-capacity slot:
 //
@@ -41,6 +41,7 @@ constexpr int kLlBlocksPerTile = kLlThreads / 32;          // 8
 constexpr int kLlTileElems = kLlBlocksPerTile * kWarpElems;  // 4096
 constexpr uint32_t kLlMagic = 0x4C424343u;                 // "CCBL"
 constexpr int kLlHeader = 32;
+constexpr int kLlCtas = 4;   // resident on an SM, and launched: each takes its tiles in turn
 
 template <class T> struct LlTraits;
 template <> struct LlTraits<float> {
@@ -61,26 +62,62 @@ __device__ __forceinline__ uint32_t bytes_of(uint32_t a, uint32_t b, uint32_t c,
   return __byte_perm(__byte_perm(a, b, pair), __byte_perm(c, d, pair), 0x5410);
 }
 
+// Four words as a 4 x 4 matrix of bytes, transposed: its own inverse.
+__device__ __forceinline__ void transpose_bytes(uint32_t (&w)[4]) {
+  const uint32_t a = __byte_perm(w[0], w[1], 0x5140), b = __byte_perm(w[2], w[3], 0x5140);   // bytes 0 and 1 of each
+  const uint32_t c = __byte_perm(w[0], w[1], 0x7362), d = __byte_perm(w[2], w[3], 0x7362);   // 2 and 3
+  w[0] = __byte_perm(a, b, 0x5410);
+  w[1] = __byte_perm(a, b, 0x7632);
+  w[2] = __byte_perm(c, d, 0x5410);
+  w[3] = __byte_perm(c, d, 0x7632);
+}
+
 // Bit planes of the 16 small values (8 bits at most) of each lane of a warp. The values 4 r + g
 // (r = 0..3) of a lane share the word u[g], value 4 r + g in byte r; a 32 x 32 bit-matrix
 // transpose of u[g] across the warp leaves plane p of value 4 r + g in lane 8 r + p. The four
 // words of a lane are then the words 16 p + 4 r .. + 3 of the plane section: ONE 16-byte store
-// by the lanes whose plane exists. Four transposes of five shuffles replace 16 ballots and 16
-// selects of the storing lane per plane; the encoder issued about 700 instructions per block of
-// 512 bf16 values for four planes and issues 272 now (ncu).
+// by the lanes whose plane exists. Where four planes are enough, nearly always, two values share a
+// byte and two transposes do: plane p of the values 2 s, 2 s + 1 comes to lane 4 s + p.
 __device__ __forceinline__ void store_planes(uint32_t* section, uint32_t (&u)[4], int planes, int lane) {
+  if (planes <= 4) {
+    const uint32_t a = transpose32(u[0] + 16u * u[2], lane), b = transpose32(u[1] + 16u * u[3], lane);
+    const int s = lane >> 2, p = lane & 3;
+    if (p < planes) *reinterpret_cast<uint2*>(section + 16 * p + 2 * s) = make_uint2(a, b);
+    return;
+  }
 #pragma unroll
   for (int g = 0; g < 4; ++g) u[g] = transpose32(u[g], lane);
   const int r = lane >> 3, p = lane & 7;
   if (p < planes) *reinterpret_cast<uint4*>(section + 16 * p + 4 * r) = make_uint4(u[0], u[1], u[2], u[3]);
 }
-__device__ __forceinline__ void load_planes(const uint32_t* section, uint32_t (&u)[4], int planes, int lane) {
-  const int r = lane >> 3, p = lane & 7;
-  const uint4 q = p < planes ? *reinterpret_cast<const uint4*>(section + 16 * p + 4 * r) : make_uint4(0u, 0u, 0u, 0u);
+// The words of a lane, as they lie in memory (two of them where four planes are enough), and the values from them.
+__device__ __forceinline__ uint4 fetch_planes(const uint32_t* section, int planes, int lane) {
+  uint4 q = make_uint4(0u, 0u, 0u, 0u);
+  if (planes <= 4) {
+    const int s = lane >> 2, p = lane & 3;
+    if (p < planes) {
+      const uint2 h = *reinterpret_cast<const uint2*>(section + 16 * p + 2 * s);
+      q.x = h.x;
+      q.y = h.y;
+    }
+  } else {
+    const int r = lane >> 3, p = lane & 7;
+    if (p < planes) q = *reinterpret_cast<const uint4*>(section + 16 * p + 4 * r);
+  }
+  return q;
+}
+__device__ __forceinline__ void values_of_planes(const uint4& q, uint32_t (&u)[4], int planes, int lane) {
   u[0] = transpose32(q.x, lane);
   u[1] = transpose32(q.y, lane);
-  u[2] = transpose32(q.z, lane);
-  u[3] = transpose32(q.w, lane);
+  if (planes <= 4) {
+    u[2] = (u[0] >> 4) & 0x0f0f0f0fu;
+    u[3] = (u[1] >> 4) & 0x0f0f0f0fu;
+    u[0] &= 0x0f0f0f0fu;
+    u[1] &= 0x0f0f0f0fu;
+  } else {
+    u[2] = transpose32(q.z, lane);
+    u[3] = transpose32(q.w, lane);
+  }
 }
 // The words u[] of values held in pairs (value 2 k in the low half of w[k], byte `at` of each half), and back.
 __device__ __forceinline__ void planes_of_pairs(const uint32_t (&w)[8], int at, uint32_t (&u)[4]) {
@@ -97,13 +134,16 @@ __device__ __forceinline__ void pairs_of_planes(const uint32_t (&u)[4], uint32_t
   }
 }
 
-// The encoder is bound by instruction issue still (ncu: SM 73 %, DRAM 34 %, most stalls for a
-// slot or the math pipe), so memory is kept out of its way: a tile's values are
-// requested while the tile before is packed, and one barrier per tile passes the widths round.
-// 32 Mi bf16 gradients through encode and decode: 177 us with ballots, 60 us so (B200; 235 MB
-// have to move, 36 us at 6.55 TB/s).
+// Both directions were bound by the pipe of the logical and byte operations (encoding 85 % busy, ncu),
+// and work on four values at a time as far as they can: the exponents and the bytes of sign and
+// mantissa of four values are one word each. A tile's values are requested while the tile before is
+// packed, and one barrier per tile passes the widths round. The decoder has the planes of the next
+// tile and the head of the one after on their way. 32 Mi bf16 values, encoding and decoding: 29.2 and
+// 27.5 us with two values at a time and four transposes a block, 24.9 and 24.7 so; 16 Mi fp32 values
+// 22.0 and 20.7. (B200; the memory needs 18 and 19 us at 6.55 TB/s. Five or six resident CTAs, with
+// the fewer registers that leaves them, are slower: fp32 24 and 28 us, 33 and 33.)
 template <class T>
-__global__ void __launch_bounds__(kLlThreads) lossless_encode_kernel(const T* __restrict__ in, size_t count, char* out, size_t ntiles) {
+__global__ void __launch_bounds__(kLlThreads, kLlCtas) lossless_encode_kernel(const T* __restrict__ in, size_t count, char* out, size_t ntiles) {
   using Tr = LlTraits<T>;
   __shared__ uint2 info[2][kLlBlocksPerTile];   // (width, minimum) of each block, by parity of the tile
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -119,24 +159,44 @@ __global__ void __launch_bounds__(kLlThreads) lossless_encode_kernel(const T* __
     char* restp = slot + 32 + warp * kWarpElems + lane * 16;
     uint32_t u[4], kmin, kmax;
     // sign and mantissa: raw byte planes (and for f16 three bit planes); then the exponents
-    if constexpr (sizeof(T) == 4) {
-      uint32_t key[16], rest[16];
-      kmin = 0xffu, kmax = 0u;
+    if constexpr (Tr::kExpBits == 8) {
+      // high = sign and the exponent's upper seven bits, low = its last bit and seven of the mantissa
+      uint32_t high[4], low[4], rest[4];
+      [[maybe_unused]] uint32_t b0[4], b1[4];   // fp32: the two bytes below
 #pragma unroll
-      for (int j = 0; j < 16; ++j) {
-        key[j] = (raw.w[j] >> 23) & 0xffu;
-        rest[j] = (raw.w[j] & 0x7fffffu) | ((raw.w[j] >> 8) & 0x800000u);
-        kmin = min(kmin, key[j]);
-        kmax = max(kmax, key[j]);
+      for (int r = 0; r < 4; ++r) {
+        if constexpr (sizeof(T) == 4) {
+          uint32_t w[4] = {raw.w[4 * r], raw.w[4 * r + 1], raw.w[4 * r + 2], raw.w[4 * r + 3]};
+          transpose_bytes(w);
+          b0[r] = w[0];
+          b1[r] = w[1];
+          low[r] = w[2];
+          high[r] = w[3];
+        } else {
+          low[r] = __byte_perm(raw.w[2 * r], raw.w[2 * r + 1], 0x6420);
+          high[r] = __byte_perm(raw.w[2 * r], raw.w[2 * r + 1], 0x7531);
+        }
+        rest[r] = (high[r] & 0x80808080u) | (low[r] & 0x7f7f7f7fu);
+        u[r] = ((high[r] * 2u) & 0xfefefefeu) | ((low[r] >> 7) & 0x01010101u);
       }
+      if constexpr (sizeof(T) == 4) {
+        stg(restp, make_uint4(b0[0], b0[1], b0[2], b0[3]));
+        stg(restp + kLlTileElems, make_uint4(b1[0], b1[1], b1[2], b1[3]));
+      }
+      stg(restp + (sizeof(T) == 4 ? 2 * kLlTileElems : 0), make_uint4(rest[0], rest[1], rest[2], rest[3]));
+      // extremes of the bytes two at a time: odd bytes decide a halfword by themselves, even ones once shifted up
+      uint32_t lo = 0xffffffffu, hi = 0u;
 #pragma unroll
-      for (int p = 0; p < 3; ++p)
-        stg(restp + (size_t)p * kLlTileElems, make_uint4(bytes_of(rest[0], rest[1], rest[2], rest[3], p), bytes_of(rest[4], rest[5], rest[6], rest[7], p),
-                                                         bytes_of(rest[8], rest[9], rest[10], rest[11], p), bytes_of(rest[12], rest[13], rest[14], rest[15], p)));
-      kmin = __reduce_min_sync(0xffffffffu, kmin);
-      kmax = __reduce_max_sync(0xffffffffu, kmax);
+      for (int r = 0; r < 4; ++r) {
+        const uint32_t even = u[r] * 256u;
+        lo = __vminu2(__vminu2(lo, u[r]), even);
+        hi = __vmaxu2(__vmaxu2(hi, u[r]), even);
+      }
+      kmin = __reduce_min_sync(0xffffffffu, min(lo & 0xffffu, lo >> 16)) >> 8;
+      kmax = __reduce_max_sync(0xffffffffu, max(hi & 0xffffu, hi >> 16)) >> 8;
 #pragma unroll
-      for (int g = 0; g < 4; ++g) u[g] = bytes_of(key[g] - kmin, key[4 + g] - kmin, key[8 + g] - kmin, key[12 + g] - kmin, 0);
+      for (int r = 0; r < 4; ++r) u[r] -= kmin * 0x01010101u;
+      transpose_bytes(u);
     } else {
       constexpr uint32_t kKey = ((1u << Tr::kExpBits) - 1u) * 0x00010001u;
       constexpr uint32_t kMan = ((1u << Tr::kExpShift) - 1u) * 0x00010001u;
@@ -197,53 +257,80 @@ __global__ void __launch_bounds__(kLlThreads) lossless_encode_kernel(const T* __
 
 // MODE 0: out = decoded values; MODE 1: out += decoded values (in T, one rounding)
 template <class T, int MODE>
-__global__ void __launch_bounds__(kLlThreads) lossless_decode_kernel(const char* __restrict__ in, size_t count, T* out, size_t ntiles) {
+__global__ void __launch_bounds__(kLlThreads, kLlCtas) lossless_decode_kernel(const char* __restrict__ in, size_t count, T* out, size_t ntiles) {
   using Tr = LlTraits<T>;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (size_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
-    const char* slot = in + kLlHeader + t * ll_slot_bytes<T>();
+  constexpr int kRest = sizeof(T) == 4 ? 3 : 1;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, sh = 8 * (warp & 3);
+  struct Head { uint4 h; uint32_t high_min; };   // used, widths 0-3, widths 4-7, minima 0-3; minima 4-7
+  struct Body { uint4 rest[kRest], planes, high; uint32_t kmin; int w; };
+  auto slot_of = [&](size_t t) { return in + kLlHeader + t * ll_slot_bytes<T>(); };
+  auto mine = [&](size_t t) { return t < ntiles && t * kLlTileElems + (size_t)warp * kWarpElems < count; };
+  auto head_of = [&](size_t t) -> Head {
+    return Head{*reinterpret_cast<const uint4*>(slot_of(t)), *reinterpret_cast<const uint32_t*>(slot_of(t) + 16)};
+  };
+  auto body_of = [&](size_t t, const Head& d) -> Body {
+    Body b;
+    const char* slot = slot_of(t);
+    const uint32_t wsel = warp < 4 ? d.h.y : d.h.z;
+    b.w = (int)((wsel >> sh) & 0xffu);
+    b.kmin = ((warp < 4 ? d.h.w : d.high_min) >> sh) & 0xffu;
+    const uint32_t off = __dp4a(wsel & ((1u << sh) - 1u), 0x01010101u, warp < 4 ? 0u : __dp4a(d.h.y, 0x01010101u, 0u));
+    b.planes = fetch_planes(reinterpret_cast<const uint32_t*>(slot + 32 + Tr::kRestBytesPerTile) + off * 16, b.w, lane);
+#pragma unroll
+    for (int p = 0; p < kRest; ++p) b.rest[p] = *reinterpret_cast<const uint4*>(slot + 32 + warp * kWarpElems + lane * 16 + (size_t)p * kLlTileElems);
+    if constexpr (Tr::kExpBits == 5) b.high = fetch_planes(reinterpret_cast<const uint32_t*>(slot + 32 + kLlTileElems) + warp * 48, 3, lane);
+    return b;
+  };
+  size_t t = blockIdx.x;
+  if (!mine(t)) return;   // only the last tile has blocks that hold nothing
+  Head head = head_of(t);
+  Body next = body_of(t, head);
+  if (mine(t + gridDim.x)) head = head_of(t + gridDim.x);
+  for (;;) {
+    const Body b = next;
     const size_t idx = t * kLlTileElems + (size_t)warp * kWarpElems + (size_t)lane * kLaneElems;
-    if (t * kLlTileElems + (size_t)warp * kWarpElems >= count) continue;
-    const uint4 head = *reinterpret_cast<const uint4*>(slot);       // used, widths 0-3, widths 4-7, minima 0-3
-    const uint32_t high_min = *reinterpret_cast<const uint32_t*>(slot + 16);
-    const char* restp = slot + 32 + warp * kWarpElems + lane * 16;
-    uint4 rq[sizeof(T) == 4 ? 3 : 1];
-#pragma unroll
-    for (int p = 0; p < (sizeof(T) == 4 ? 3 : 1); ++p) rq[p] = *reinterpret_cast<const uint4*>(restp + (size_t)p * kLlTileElems);
-    const uint32_t wsel = warp < 4 ? head.y : head.z, sh = 8 * (warp & 3);
-    const int w = (int)((wsel >> sh) & 0xffu);
-    const uint32_t kmin = ((warp < 4 ? head.w : high_min) >> sh) & 0xffu;
-    const uint32_t off = __dp4a(wsel & ((1u << sh) - 1u), 0x01010101u, warp < 4 ? 0u : __dp4a(head.y, 0x01010101u, 0u));
+    t += gridDim.x;
+    const bool more = mine(t);
+    if (more) {
+      next = body_of(t, head);
+      if (mine(t + gridDim.x)) head = head_of(t + gridDim.x);
+    }
     uint32_t u[4];
-    load_planes(reinterpret_cast<const uint32_t*>(slot + 32 + Tr::kRestBytesPerTile) + off * 16, u, w, lane);
+    values_of_planes(b.planes, u, b.w, lane);
     Wide16<T> raw;
-    if constexpr (sizeof(T) == 4) {
-      const uint32_t p0[4] = {rq[0].x, rq[0].y, rq[0].z, rq[0].w}, p1[4] = {rq[1].x, rq[1].y, rq[1].z, rq[1].w},
-                     p2[4] = {rq[2].x, rq[2].y, rq[2].z, rq[2].w};
+    if constexpr (Tr::kExpBits == 8) {
+      transpose_bytes(u);   // values 4 r .. + 3 in word r, as the bytes of sign and mantissa lie
+      const uint4 top = b.rest[kRest - 1];
+      const uint32_t rest[4] = {top.x, top.y, top.z, top.w};
+      [[maybe_unused]] const uint32_t b0[4] = {b.rest[0].x, b.rest[0].y, b.rest[0].z, b.rest[0].w};
+      [[maybe_unused]] const uint32_t b1[4] = {b.rest[kRest > 1 ? 1 : 0].x, b.rest[kRest > 1 ? 1 : 0].y, b.rest[kRest > 1 ? 1 : 0].z, b.rest[kRest > 1 ? 1 : 0].w};
 #pragma unroll
-      for (int j = 0; j < 16; ++j) {
-        const uint32_t r = j & 3, low = __byte_perm(p0[j >> 2], p1[j >> 2], r | ((r + 4) << 4));    // bytes 0, 1
-        const uint32_t rest = __byte_perm(low, p2[j >> 2], 0x10u | ((r + 4) << 8)) & 0xffffffu;
-        const uint32_t key = ((u[j & 3] >> (8 * (j >> 2))) & 0xffu) + kmin;
-        raw.w[j] = ((rest << 8) & 0x80000000u) | (key << 23) | (rest & 0x7fffffu);
+      for (int r = 0; r < 4; ++r) {
+        const uint32_t key = u[r] + b.kmin * 0x01010101u;
+        const uint32_t high = (rest[r] & 0x80808080u) | ((key >> 1) & 0x7f7f7f7fu);
+        const uint32_t low = (rest[r] & 0x7f7f7f7fu) | ((key * 128u) & 0x80808080u);
+        if constexpr (sizeof(T) == 4) {
+          uint32_t w[4] = {b0[r], b1[r], low, high};
+          transpose_bytes(w);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) raw.w[4 * r + j] = w[j];
+        } else {
+          raw.w[2 * r] = __byte_perm(low, high, 0x5140);
+          raw.w[2 * r + 1] = __byte_perm(low, high, 0x7362);
+        }
       }
     } else {
-      uint32_t key[8], rest[8];
+      uint32_t key[8], rest[8], high[4], hp[8];
       pairs_of_planes(u, key);
-      const uint32_t q[4] = {rq[0].x, rq[0].y, rq[0].z, rq[0].w};
-#pragma unroll
-      for (int k = 0; k < 8; ++k) rest[k] = __byte_perm(q[k >> 1], 0u, k & 1 ? 0x4342 : 0x4140);
-      if constexpr (Tr::kExpBits == 5) {
-        uint32_t high[4], hp[8];
-        load_planes(reinterpret_cast<const uint32_t*>(slot + 32 + kLlTileElems) + warp * 48, high, 3, lane);
-        pairs_of_planes(high, hp);
-#pragma unroll
-        for (int k = 0; k < 8; ++k) rest[k] |= hp[k] << 8;
-      }
+      const uint32_t q[4] = {b.rest[0].x, b.rest[0].y, b.rest[0].z, b.rest[0].w};
+      values_of_planes(b.high, high, 3, lane);
+      pairs_of_planes(high, hp);
       constexpr uint32_t kMan = ((1u << Tr::kExpShift) - 1u) * 0x00010001u;
 #pragma unroll
-      for (int k = 0; k < 8; ++k)
-        raw.w[k] = (((rest[k] << (15 - Tr::kExpShift)) & 0x80008000u) | (rest[k] & kMan)) | ((key[k] + kmin * 0x00010001u) << Tr::kExpShift);
+      for (int k = 0; k < 8; ++k) {
+        rest[k] = __byte_perm(q[k >> 1], 0u, k & 1 ? 0x4342 : 0x4140) | (hp[k] << 8);
+        raw.w[k] = (((rest[k] << (15 - Tr::kExpShift)) & 0x80008000u) | (rest[k] & kMan)) | ((key[k] + b.kmin * 0x00010001u) << Tr::kExpShift);
+      }
     }
     if constexpr (MODE == 1) {
       Wide16<T> have;
@@ -257,6 +344,7 @@ __global__ void __launch_bounds__(kLlThreads) lossless_decode_kernel(const char*
     } else {
       store16_wide<T>(out, idx, count, raw);
     }
+    if (!more) return;
   }
 }
 
@@ -266,7 +354,7 @@ static int ll_grid(size_t ntiles) {
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const size_t cap = (size_t)sms * 8;
+  const size_t cap = (size_t)sms * kLlCtas;
   return (int)(ntiles < cap ? (ntiles ? ntiles : 1) : cap);
 }
 
