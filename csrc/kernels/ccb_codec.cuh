@@ -23,14 +23,25 @@
 
 namespace ccb {
 
-// Two fp32 operations in one instruction. A sum of these and a product of these that follow one
-// another may come out fused, .rn or not: the round trips below multiply packed where plain
-// additions come before or after, and add packed where a product follows.
-__device__ __forceinline__ void mul2(float& a, float& b, float s) {
-  asm("{\n.reg .b64 x, y;\nmov.b64 x, {%0, %1};\nmov.b64 y, {%2, %2};\nmul.rn.f32x2 x, x, y;\nmov.b64 {%0, %1}, x;\n}" : "+f"(a), "+f"(b) : "f"(s));
+// Two fp32 operations in one instruction, on pairs held as 64-bit values. A sum of these and a
+// product of these that follow one another may come out fused, .rn or not: the round trips below
+// multiply packed where plain additions come before or after, and add packed where a product follows.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pair2(float a, float b) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
 }
-__device__ __forceinline__ void add2(float& a, float& b, float s) {
-  asm("{\n.reg .b64 x, y;\nmov.b64 x, {%0, %1};\nmov.b64 y, {%2, %2};\nadd.rn.f32x2 x, x, y;\nmov.b64 {%0, %1}, x;\n}" : "+f"(a), "+f"(b) : "f"(s));
+__device__ __forceinline__ void split2(f32x2 v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
 }
 
 // Every codec has `round_trip`: v becomes decode(encode(v)), bit for bit, special values too.
@@ -155,14 +166,14 @@ struct CodecInt8 {
 #pragma unroll
     for (int d = 1; d < kLanes; d <<= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, d));
     const float inv = m > 0.f ? 127.f / m : 0.f, scale = m / 127.f;
+    const f32x2 inv2 = pair2(inv, inv), scale2 = pair2(scale, scale), bias2 = pair2(-12583040.f, -12583040.f);
 #pragma unroll
     for (int i = 0; i < 16; i += 2) {
-      mul2(v[i], v[i + 1], inv);
-#pragma unroll
-      for (int k = 0; k < 2; ++k)
-        v[i + k] = __uint_as_float((__float_as_uint(__fadd_rn(v[i + k], 12582912.f)) & 0xffu) ^ 0x4B400080u);
-      add2(v[i], v[i + 1], -12583040.f);
-      mul2(v[i], v[i + 1], scale);
+      float a, b;
+      split2(mul2(pair2(v[i], v[i + 1]), inv2), a, b);
+      a = __uint_as_float((__float_as_uint(__fadd_rn(a, 12582912.f)) & 0xffu) ^ 0x4B400080u);
+      b = __uint_as_float((__float_as_uint(__fadd_rn(b, 12582912.f)) & 0xffu) ^ 0x4B400080u);
+      split2(mul2(add2(pair2(a, b), bias2), scale2), v[i], v[i + 1]);
     }
   }
   static __device__ __forceinline__ void store(char* slot, size_t pad, size_t idx, const Packet& pk) {
@@ -273,14 +284,14 @@ struct CodecFp8 {
     m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 1));
     const uint32_t e = scale_byte(m);
     const float inv = __uint_as_float((254u - e) << 23), s = __uint_as_float(e << 23);
+    const f32x2 inv2 = pair2(inv, inv), s2 = pair2(s, s);
 #pragma unroll
     for (int i = 0; i < 16; i += 2) {
-      mul2(v[i], v[i + 1], inv);
-      const __half2_raw h = __nv_cvt_fp8x2_to_halfraw2(__nv_cvt_float2_to_fp8x2(make_float2(v[i], v[i + 1]), __NV_SATFINITE, __NV_E4M3), __NV_E4M3);
-      const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&h));
-      v[i] = f.x;
-      v[i + 1] = f.y;
-      mul2(v[i], v[i + 1], s);
+      float2 f;
+      split2(mul2(pair2(v[i], v[i + 1]), inv2), f.x, f.y);
+      const __half2_raw h = __nv_cvt_fp8x2_to_halfraw2(__nv_cvt_float2_to_fp8x2(f, __NV_SATFINITE, __NV_E4M3), __NV_E4M3);
+      f = __half22float2(*reinterpret_cast<const __half2*>(&h));
+      split2(mul2(pair2(f.x, f.y), s2), v[i], v[i + 1]);
     }
   }
   static __device__ __forceinline__ void store(char* slot, size_t pad, size_t idx, const Packet& pk) {

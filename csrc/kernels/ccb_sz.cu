@@ -681,9 +681,11 @@ __global__ void __cluster_dims__(kClusterSize, 1, 1) __launch_bounds__(kSzThread
 // before stays in its registers, y and x neighbours come by shuffles, and the words of a plane go
 // behind those of the plane before. So nothing of a tile is exchanged between warps, there is one
 // barrier a GROUP (a CTA of eight warps), for the tiles' sizes, and no cluster. Both directions are
-// bound by instruction issue, not far above the memory's rate. (512^3 field, bound 1e-4 of its range,
-// B200: with a CTA a tile, its planes on eight warps, three barriers a tile and the sizes sent round a
-// cluster, packing took 345 us and unpacking 275, 458 and 389 warp instructions for 256 values.)
+// bound by instructions (packing: the pipe of logical operations 69 % busy, 84 % of the issue slots)
+// and the latency of a tile's first loads. (512^3 field, bound 1e-4 of its range, B200: packing 181 us
+// and unpacking 162; with a CTA a tile, its planes on eight warps, three barriers a tile and the sizes
+// sent round a cluster it was 332 and 279. Packing with 64 registers instead of 80 187 us, unpacking
+// with 64 instead of 48 170.)
 struct SzLocalArgs {
   const float* in;
   float* out;
@@ -700,27 +702,35 @@ constexpr int kWarpStage = 4096;   // bytes of a packed tile that a warp stages;
 // (1: a plane goes through shared memory, so that the accesses of a warp lie side by side).
 template <int kVec>
 struct PlaneIO {
-  const SzLocalArgs& a;
-  TileCoord t;
-  float* sh;   // kVec 1: 256 floats of this warp
+  float* at;      // this lane's place in plane 0 of the tile
+  size_t stride;  // of a plane
+  int planes;     // of the tile that this lane has a part in (the others read as 0 and are not written)
+  int width;      // kVec 4: whether the second four are inside; 1: lines of the tile, and
+  int line;       //         their distance
+  float* sh;      // kVec 1: 256 floats of this warp
   int lane;
+  __device__ __forceinline__ PlaneIO(const float* field, const SzLocalArgs& a, TileCoord t, float* shared) {
+    lane = threadIdx.x & 31;
+    sh = shared;
+    line = a.nx;
+    stride = (size_t)a.ny * a.nx;
+    const int gx = kVec == 1 ? t.x0 + lane : t.x0 + 8 * (lane & 3), gy = kVec == 1 ? t.y0 : t.y0 + (lane >> 2);
+    at = const_cast<float*>(field) + ((size_t)t.z0 * a.ny + gy) * a.nx + gx;
+    planes = gx < a.nx && gy < a.ny ? min(kTZ, a.nz - t.z0) : 0;
+    width = kVec == 1 ? a.ny - t.y0 : gx + 4 < a.nx;
+  }
   __device__ __forceinline__ void load(int z, float (&v)[8]) const {   // raw: kVec 1 holds column `lane` of the eight lines
-    const int gz = t.z0 + z;
+    const float* p = at + z * stride;
     if constexpr (kVec == 1) {
-      const int gx = t.x0 + lane;
-      const float* p = a.in + ((size_t)gz * a.ny + t.y0) * a.nx + gx;
 #pragma unroll
-      for (int y = 0; y < kTY; ++y) v[y] = gx < a.nx && t.y0 + y < a.ny && gz < a.nz ? __ldcs(p + (size_t)y * a.nx) : 0.f;
+      for (int y = 0; y < kTY; ++y) v[y] = z < planes && y < width ? __ldcs(p + (size_t)y * line) : 0.f;
     } else {
-      const int gx = t.x0 + 8 * (lane & 3), gy = t.y0 + (lane >> 2);
-      const float* p = a.in + ((size_t)gz * a.ny + gy) * a.nx + gx;
-      const bool in = gx < a.nx && gy < a.ny && gz < a.nz;
       uint32_t w[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
       if constexpr (kVec == 8) {
-        if (in) ldg_stream32(p, w);
+        if (z < planes) ldg_stream32(p, w);
       } else {
-        if (in) { const uint4 u = ldg_stream(p); w[0] = u.x; w[1] = u.y; w[2] = u.z; w[3] = u.w; }
-        if (in && gx + 4 < a.nx) { const uint4 u = ldg_stream(p + 4); w[4] = u.x; w[5] = u.y; w[6] = u.z; w[7] = u.w; }
+        if (z < planes) { const uint4 u = ldg_stream(p); w[0] = u.x; w[1] = u.y; w[2] = u.z; w[3] = u.w; }
+        if (z < planes && width) { const uint4 u = ldg_stream(p + 4); w[4] = u.x; w[5] = u.y; w[6] = u.z; w[7] = u.w; }
       }
 #pragma unroll
       for (int e = 0; e < 8; ++e) v[e] = __uint_as_float(w[e]);
@@ -737,21 +747,17 @@ struct PlaneIO {
     }
   }
   __device__ __forceinline__ void store(int z, const float (&v)[8]) const {
-    const int gz = t.z0 + z;
+    float* p = at + z * stride;
     if constexpr (kVec == 1) {
       reinterpret_cast<float4*>(sh)[2 * lane] = make_float4(v[0], v[1], v[2], v[3]);
       reinterpret_cast<float4*>(sh)[2 * lane + 1] = make_float4(v[4], v[5], v[6], v[7]);
       __syncwarp();
-      const int gx = t.x0 + lane;
-      float* p = a.out + ((size_t)gz * a.ny + t.y0) * a.nx + gx;
 #pragma unroll
       for (int y = 0; y < kTY; ++y)
-        if (gx < a.nx && t.y0 + y < a.ny && gz < a.nz) p[(size_t)y * a.nx] = sh[kTX * y + lane];
+        if (z < planes && y < width) p[(size_t)y * line] = sh[kTX * y + lane];
       __syncwarp();
     } else {
-      const int gx = t.x0 + 8 * (lane & 3), gy = t.y0 + (lane >> 2);
-      float* p = a.out + ((size_t)gz * a.ny + gy) * a.nx + gx;
-      if (gx >= a.nx || gy >= a.ny || gz >= a.nz) return;
+      if (z >= planes) return;
       uint32_t w[8];
 #pragma unroll
       for (int e = 0; e < 8; ++e) w[e] = __float_as_uint(v[e]);
@@ -759,36 +765,33 @@ struct PlaneIO {
         stg_stream32(p, w);
       } else {
         stg_stream(p, make_uint4(w[0], w[1], w[2], w[3]));
-        if (gx + 4 < a.nx) stg_stream(p + 4, make_uint4(w[4], w[5], w[6], w[7]));
+        if (width) stg_stream(p + 4, make_uint4(w[4], w[5], w[6], w[7]));
       }
     }
   }
 };
 
-// Codes of one plane; see pack_tile for the arithmetic, which is the same.
+// Codes of one plane, 2^21 added to each; the arithmetic and its result are pack_tile's. Codes that
+// far from 0 and values that are not finite show in the codes' high bits and take the exact tests.
+constexpr int kCodeBias = 1 << 21;
 __device__ __forceinline__ void plane_codes(const float (&x)[8], const SzLocalArgs& a, int (&q)[8], bool& bad) {
   const float half = 0.5f * a.two_eb;
-  float s[8], r[8], smax = 0.f;
-  bool far = false;
-#pragma unroll
-  for (int e = 0; e < 8; ++e) s[e] = x[e];
-#pragma unroll
-  for (int e = 0; e < 8; e += 2) mul2(s[e], s[e + 1], a.inv_two_eb);
-#pragma unroll
-  for (int e = 0; e < 8; ++e) {
-    smax = fmaxf(smax, fabsf(s[e]));
-    r[e] = __fadd_rn(s[e], kRoundMagic);
-    q[e] = __float_as_int(r[e]) - __float_as_int(kRoundMagic);
-  }
+  const f32x2 inv2 = pair2(a.inv_two_eb, a.inv_two_eb), step2 = pair2(a.two_eb, a.two_eb), magic2 = pair2(-kRoundMagic, -kRoundMagic);
+  float worst = 0.f;
+  uint32_t high = 0u;
 #pragma unroll
   for (int e = 0; e < 8; e += 2) {
-    add2(r[e], r[e + 1], -kRoundMagic);
-    mul2(r[e], r[e + 1], a.two_eb);
+    float s0, s1, p0, p1;
+    split2(mul2(pair2(x[e], x[e + 1]), inv2), s0, s1);
+    const float r0 = __fadd_rn(s0, kRoundMagic), r1 = __fadd_rn(s1, kRoundMagic);
+    q[e] = __float_as_int(r0) - (__float_as_int(kRoundMagic) - kCodeBias);
+    q[e + 1] = __float_as_int(r1) - (__float_as_int(kRoundMagic) - kCodeBias);
+    high |= (uint32_t)q[e] | (uint32_t)q[e + 1];
+    split2(mul2(add2(pair2(r0, r1), magic2), step2), p0, p1);
+    worst = fmaxf(worst, fmaxf(fabsf(__fsub_rn(x[e], p0)), fabsf(__fsub_rn(x[e + 1], p1))));
   }
-#pragma unroll
-  for (int e = 0; e < 8; ++e) far |= !(fabsf(__fsub_rn(x[e], r[e])) <= half);
-  bad |= !(smax < kQMax);
-  if (__any_sync(0xffffffffu, far)) {
+  const bool wild = (high >> 22) != 0u;   // NaN and infinities among them, so `worst` may pass them over
+  if (__any_sync(0xffffffffu, wild || worst > half)) {
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
       const float se = __fmul_rn(x[e], a.inv_two_eb);
@@ -798,7 +801,7 @@ __device__ __forceinline__ void plane_codes(const float (&x)[8], const SzLocalAr
       rf += diff > half ? 1.f : 0.f;
       rf -= -diff > half ? 1.f : 0.f;
       bad |= fabsf(__fsub_rn(x[e], __fmul_rn(rf, a.two_eb))) > a.eb;
-      q[e] = (int)rf;
+      q[e] = (int)rf + kCodeBias;
     }
   }
 }
@@ -806,14 +809,16 @@ __device__ __forceinline__ void plane_codes(const float (&x)[8], const SzLocalAr
 // Packs the warp's tile to `pk` (64 width bytes, then the planes). Returns its words and whether it
 // has to be stored raw. Words beyond `room` are counted and not written.
 template <int kVec>
-__device__ __forceinline__ uint32_t pack_planes(const PlaneIO<kVec>& io, unsigned char* pk, uint32_t room, bool& bad) {
+__device__ __forceinline__ uint32_t pack_planes(const PlaneIO<kVec>& io, const SzLocalArgs& a, unsigned char* pk, uint32_t room, bool& bad) {
   const int lane = io.lane;
   uint32_t* words = reinterpret_cast<uint32_t*>(pk + kRows);
-  int before[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+  int before[8];
+#pragma unroll
+  for (int e = 0; e < 8; ++e) before[e] = kCodeBias;
   uint32_t run = 0;
   float ahead[8];
   io.load(0, ahead);
-#pragma unroll 1
+#pragma unroll 2
   for (int z = 0; z < kTZ; ++z) {
     float x[8];
 #pragma unroll
@@ -821,7 +826,7 @@ __device__ __forceinline__ uint32_t pack_planes(const PlaneIO<kVec>& io, unsigne
     if (z + 1 < kTZ) io.load(z + 1, ahead);   // the next plane is on its way while this one is packed
     io.settle(x);
     int q[8], d[8];
-    plane_codes(x, io.a, q, bad);
+    plane_codes(x, a, q, bad);
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
       d[e] = q[e] - before[e];
@@ -853,14 +858,9 @@ __device__ __forceinline__ uint32_t pack_planes(const PlaneIO<kVec>& io, unsigne
         const uint32_t minus = ((b >> 7) & 0x01010101u) ^ 0x01010101u;
         u[k] = transpose32(((b << 1) & 0xfefefefeu) ^ (minus * 0xffu), lane);
       }
-      W0 = __ballot_sync(0xffffffffu, u[0] != 0u);
-      W1 = __ballot_sync(0xffffffffu, u[1] != 0u);
-      W0 |= (W0 >> 1) & 0x7f7f7f7fu;
-      W1 |= (W1 >> 1) & 0x7f7f7f7fu;
-      W0 |= (W0 >> 2) & 0x3f3f3f3fu;
-      W1 |= (W1 >> 2) & 0x3f3f3f3fu;
-      W0 |= (W0 >> 4) & 0x0f0f0f0fu;
-      W1 |= (W1 >> 4) & 0x0f0f0f0fu;
+      // a lane, plane j of its row, is there if any plane from j up of that row holds a bit
+      W0 = __ballot_sync(0xffffffffu, ((__ballot_sync(0xffffffffu, u[0] != 0u) >> lane) & (0xffu >> (lane & 7))) != 0u);
+      W1 = __ballot_sync(0xffffffffu, ((__ballot_sync(0xffffffffu, u[1] != 0u) >> lane) & (0xffu >> (lane & 7))) != 0u);
       if (lane < 8) pk[8 * z + lane] = (unsigned char)__popc(((lane < 4 ? W0 : W1) >> (8 * (lane & 3))) & 0xffu);
       tot_lo = __popc(W0);
       tot = tot_lo + __popc(W1);
@@ -895,35 +895,47 @@ __device__ __forceinline__ uint32_t pack_planes(const PlaneIO<kVec>& io, unsigne
 }
 
 template <int kVec>
-__global__ void __launch_bounds__(kSzThreads, 4) sz_pack_kernel(const __grid_constant__ SzLocalArgs a) {
+__global__ void __launch_bounds__(kSzThreads, 3) sz_pack_kernel(const __grid_constant__ SzLocalArgs a) {
   __shared__ __align__(16) unsigned char stage[kClusterSize][kWarpStage];
   __shared__ __align__(16) float plane[kVec == 1 ? kClusterSize : 1][kVec == 1 ? kTX * kTY : 4];
   __shared__ uint32_t s_size[kClusterSize];
   const int lane = threadIdx.x & 31, k = threadIdx.x >> 5;
   const unsigned int tile = blockIdx.x * kClusterSize + k;
   char* group = a.slots + (size_t)blockIdx.x * kGroupStride;
-  const PlaneIO<kVec> io = {a, tile_coord(a, tile), plane[kVec == 1 ? k : 0], lane};
-  uint32_t size = 0;
-  bool raw = false;
-  if (tile < (unsigned)a.tiles_x * a.tiles_y * a.tiles_z) {
-    bool bad = false;
-    const uint32_t words = pack_planes<kVec>(io, stage[k], (kWarpStage - kRows) / 4, bad);
-    raw = __any_sync(0xffffffffu, bad);
-    size = raw ? kRows + kTileVals * 4u : (kRows + 4u * words + 15u) & ~15u;
-  }
-  if (lane == 0) s_size[k] = size;
-  __syncthreads();
-  const uint32_t of = lane < kClusterSize ? s_size[lane] : 0u;
-  const uint32_t off = __reduce_add_sync(0xffffffffu, lane < k ? of : 0u);
-  if (k == 0) {
-    const uint32_t all = __reduce_add_sync(0xffffffffu, of);
-    if (lane < kClusterSize) reinterpret_cast<uint32_t*>(group)[lane] = of;
-    if (lane == 0 && a.used_bytes) atomicAdd(a.used_bytes, (unsigned long long)all);
-  }
-  if (size == 0) return;
-  char* dst = group + kGroupHeader + off;
-  if (raw) {   // marker and the fp32 values
-    reinterpret_cast<uint16_t*>(dst)[lane] = lane == 0 ? 255 : 0;
+  const PlaneIO<kVec> io(a.in, a, tile_coord(a, tile), plane[kVec == 1 ? k : 0]);
+  unsigned char* pk = stage[k];
+  uint32_t room = (kWarpStage - kRows) / 4;
+  for (bool first = true;; first = false) {   // a second turn for a tile that was too large for its stage: to its place
+    uint32_t size = 0;
+    bool raw = false;
+    if (tile < (unsigned)a.tiles_x * a.tiles_y * a.tiles_z) {
+      bool bad = false;
+      const uint32_t words = pack_planes<kVec>(io, a, pk, room, bad);
+      raw = __any_sync(0xffffffffu, bad);
+      size = raw ? kRows + kTileVals * 4u : (kRows + 4u * words + 15u) & ~15u;
+    }
+    if (!first) return;
+    if (lane == 0) s_size[k] = size;
+    __syncthreads();
+    const uint32_t of = lane < kClusterSize ? s_size[lane] : 0u;
+    const uint32_t off = __reduce_add_sync(0xffffffffu, lane < k ? of : 0u);
+    if (k == 0) {
+      const uint32_t all = __reduce_add_sync(0xffffffffu, of);
+      if (lane < kClusterSize) reinterpret_cast<uint32_t*>(group)[lane] = of;
+      if (lane == 0 && a.used_bytes) atomicAdd(a.used_bytes, (unsigned long long)all);
+    }
+    if (size == 0) return;
+    char* dst = group + kGroupHeader + off;
+    if (!raw && size > (uint32_t)kWarpStage) {
+      pk = reinterpret_cast<unsigned char*>(dst);
+      room = kTileVals;
+      continue;
+    }
+    if (!raw) {
+      for (uint32_t i = lane; i < size / 16; i += 32) stg(dst + 16 * i, reinterpret_cast<const uint4*>(stage[k])[i]);
+      return;
+    }
+    reinterpret_cast<uint16_t*>(dst)[lane] = lane == 0 ? 255 : 0;   // marker, then the fp32 values
 #pragma unroll 1
     for (int z = 0; z < kTZ; ++z) {
       float x[8];
@@ -933,23 +945,18 @@ __global__ void __launch_bounds__(kSzThreads, 4) sz_pack_kernel(const __grid_con
       to[0] = make_float4(x[0], x[1], x[2], x[3]);
       to[1] = make_float4(x[4], x[5], x[6], x[7]);
     }
-  } else if (size <= (uint32_t)kWarpStage) {
-    __syncwarp();
-    for (uint32_t i = lane; i < size / 16; i += 32) stg(dst + 16 * i, reinterpret_cast<const uint4*>(stage[k])[i]);
-  } else {
-    bool bad = false;
-    pack_planes<kVec>(io, reinterpret_cast<unsigned char*>(dst), (uint32_t)kTileVals, bad);
+    return;
   }
 }
 
 template <int kVec>
-__global__ void __launch_bounds__(kSzThreads, 4) sz_unpack_kernel(const __grid_constant__ SzLocalArgs a) {
+__global__ void __launch_bounds__(kSzThreads, kVec == 1 ? 4 : 5) sz_unpack_kernel(const __grid_constant__ SzLocalArgs a) {
   __shared__ __align__(16) float plane[kVec == 1 ? kClusterSize : 1][kVec == 1 ? kTX * kTY : 4];
   const int lane = threadIdx.x & 31, k = threadIdx.x >> 5;
   const unsigned int tile = blockIdx.x * kClusterSize + k;
   if (tile >= (unsigned)a.tiles_x * a.tiles_y * a.tiles_z) return;
   const char* group = a.slots + (size_t)blockIdx.x * kGroupStride;
-  const PlaneIO<kVec> io = {a, tile_coord(a, tile), plane[kVec == 1 ? k : 0], lane};
+  const PlaneIO<kVec> io(a.out, a, tile_coord(a, tile), plane[kVec == 1 ? k : 0]);
   uint32_t off = __reduce_add_sync(0xffffffffu, lane < k ? ldg_cg_u32(group + 4 * lane) : 0u);
   if (off > (uint32_t)(kClusterSize * kTileCap)) off = 0;   // damaged size words: stay inside the slot
   const unsigned char* src = reinterpret_cast<const unsigned char*>(group) + kGroupHeader + off;
@@ -989,6 +996,7 @@ __global__ void __launch_bounds__(kSzThreads, 4) sz_unpack_kernel(const __grid_c
   // A narrow plane's residuals are summed along x and y as bytes d + 128 in halves of a word: 256 of
   // them fit 16 bits, and what the 128s come to at (x, y) is known.
   const int bias0 = 128 * (8 * (lane & 3) + 1) * ((lane >> 2) + 1), bias_step = 128 * ((lane >> 2) + 1);
+  const f32x2 step2 = pair2(a.two_eb, a.two_eb);
   Ahead ahead = fetch(0);
 #pragma unroll 1
   for (int z = 0; z < kTZ; ++z) {
@@ -1074,7 +1082,7 @@ __global__ void __launch_bounds__(kSzThreads, 4) sz_unpack_kernel(const __grid_c
     }
     float f[8];
 #pragma unroll
-    for (int e = 0; e < 8; ++e) f[e] = __fmul_rn((float)acc[e], a.two_eb);
+    for (int e = 0; e < 8; e += 2) split2(mul2(pair2((float)acc[e], (float)acc[e + 1]), step2), f[e], f[e + 1]);
     io.store(z, f);
   }
 }
