@@ -13,6 +13,7 @@ entry points that this class wraps.
 from __future__ import annotations
 
 import ctypes
+import functools
 import uuid
 from typing import Optional, Sequence, Union
 
@@ -28,6 +29,7 @@ _DTYPES = {torch.float32: K.F32, torch.bfloat16: K.BF16, torch.float16: K.F16}
 
 # Not in every torch: an inner function of the package, and absent from builds without CUDA.
 _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+_device = getattr(torch._C, "_cuda_getDevice", torch.cuda.current_device)   # without the check for a first use of CUDA
 
 
 def current_stream_ptr() -> ctypes.c_void_p:
@@ -36,7 +38,7 @@ def current_stream_ptr() -> ctypes.c_void_p:
     where torch does not have the shorter one."""
     if _raw_stream is None:
         return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
-    return ctypes.c_void_p(_raw_stream(torch.cuda.current_device()))
+    return ctypes.c_void_p(_raw_stream(_device()))
 
 
 class CcbError(RuntimeError):
@@ -57,6 +59,7 @@ class Communicator:
         self.rank = L.ccb_comm_rank(self._h)
         self.nranks = L.ccb_comm_nranks(self._h)
         self.nlocal = L.ccb_comm_nlocal(self._h)
+        self._pointers = ctypes.c_void_p * self.nlocal
 
     # ------------------------------------------------------------ creation --
     @classmethod
@@ -204,11 +207,9 @@ class Communicator:
         ts = [t] if isinstance(t, torch.Tensor) else list(t)
         if len(ts) != self.nlocal:
             raise ValueError(f"{name}: expected {self.nlocal} tensor(s), got {len(ts)}")
-        for x in ts:
-            if not x.is_cuda or not x.is_contiguous():
-                raise ValueError(f"{name}: tensors must be contiguous CUDA tensors")
-        arr = (ctypes.c_void_p * self.nlocal)(*[x.data_ptr() for x in ts])
-        return arr, ts
+        if not all([x.is_cuda and x.is_contiguous() for x in ts]):
+            raise ValueError(f"{name}: tensors must be contiguous CUDA tensors")
+        return self._pointers(*[x.data_ptr() for x in ts]), ts
 
     @staticmethod
     def _stream() -> ctypes.c_void_p:
@@ -397,6 +398,7 @@ def _check(rc: int) -> None:
         raise CcbError(rc, (lib().ccb_last_error() or b"").decode(errors="replace"))
 
 
+@functools.lru_cache(maxsize=1024)   # the same few sizes come again and again
 def wire_bytes(codec, dtype: torch.dtype, count: int) -> int:
     return int(lib().ccb_wire_bytes(_code(codec, K.CODECS), _DTYPES[dtype], count))
 

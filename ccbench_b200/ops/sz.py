@@ -24,6 +24,7 @@ def _decl():
     L.ccb_sz_compress.argtypes = [c_vp, c_int, c_int, c_int, c_f, c_vp, c_vp, c_vp]
     L.ccb_sz_decompress.argtypes = [c_vp, c_int, c_int, c_int, c_f, c_vp, c_vp]
     L.ccb_sz_container_scan.argtypes = [c_vp, c_vp, ctypes.c_uint64, c_vp, c_vp]
+    L.ccb_sz_container_open.argtypes = [c_vp, ctypes.c_uint64, ctypes.c_uint64, c_vp, c_vp, c_vp]
     L.ccb_sz_container_pack.argtypes = [c_vp, c_vp, c_int, c_int, c_int, c_f, ctypes.c_uint64, c_vp, c_vp]
     L.ccb_sz_container_unpack.argtypes = [c_vp, c_vp, ctypes.c_uint64, c_vp, c_vp]
     L.ccb_sz_collective.argtypes = [c_vp, ctypes.POINTER(c_vp), ctypes.POINTER(c_vp), c_int, c_int, c_int, c_f, c_int, c_vp, c_vp]
@@ -44,7 +45,7 @@ def compress(field: torch.Tensor, eb: float):
     assert field.is_cuda and field.dtype == torch.float32 and field.dim() == 3 and field.is_contiguous()
     nz, ny, nx = field.shape
     buf = torch.empty(capacity(field.shape), dtype=torch.uint8, device=field.device)
-    used = torch.zeros(1, dtype=torch.int64, device=field.device)
+    used = torch.empty(1, dtype=torch.int64, device=field.device)   # the call clears it
     _check(_decl().ccb_sz_compress(field.data_ptr(), nx, ny, nz, eb, buf.data_ptr(), used.data_ptr(), _stream()))
     return buf, used
 
@@ -90,6 +91,7 @@ def _collective(comm, send, recv, eb, root, used):
 #   [u64 payload bytes][u32 used bytes of each group (header included)] [the used bytes of every group]
 MAGIC, VERSION = 0x5A534343, 2
 GROUP_STRIDE, GROUP_HEADER, HEADER_BYTES = 66112, 32, 40
+_LEAST_GROUP = 4 + GROUP_HEADER + 64   # its size word, the tiles' size words, the row widths of one tile
 
 
 def _by_kernel(t: torch.Tensor, align: int) -> bool:
@@ -130,7 +132,17 @@ def to_container(buf: torch.Tensor, shape, eb: float) -> torch.Tensor:
 
 def from_container(blob: torch.Tensor):
     """Inverse of to_container: returns (buffer of group slots, shape, eb)."""
-    head = blob[:HEADER_BYTES].cpu()
+    opened = None
+    if _by_kernel(blob, 8) and blob.numel() >= HEADER_BYTES + _LEAST_GROUP:
+        # header, scan of the sizes and its sums in one read-back; no group is smaller than an empty tile's
+        with torch.cuda.device(blob.device):
+            room = (blob.numel() - HEADER_BYTES) // _LEAST_GROUP
+            opened = torch.empty(room + 2 + 7, dtype=torch.int64, device=blob.device)
+            _check(_decl().ccb_sz_container_open(blob.data_ptr(), blob.numel(), room, opened.data_ptr(), opened.data_ptr() + 8 * (room + 2), _stream()))
+            found = opened[room + 2:].cpu()
+            head = found.view(torch.uint8)[:HEADER_BYTES]
+    else:
+        head = blob[:HEADER_BYTES].cpu()
     magic, version, nx, ny, nz = head[0:20].view(torch.int32).tolist()
     if magic != MAGIC or version != VERSION:
         raise ValueError(f"not a ccb-sz v{VERSION} container (magic {magic:#x}, version {version})")
@@ -140,13 +152,19 @@ def from_container(blob: torch.Tensor):
     if ngroups * GROUP_STRIDE != capacity((nz, ny, nx)):
         raise ValueError("container header does not match its dimensions")
     if _by_kernel(blob, 4) and ngroups and blob.numel() >= HEADER_BYTES + 4 * ngroups:
+        if opened is not None and ngroups > room:
+            opened = None
         if blob.numel() - HEADER_BYTES - 4 * ngroups != nbytes:
             raise ValueError("container payload is damaged")
         with torch.cuda.device(blob.device):
             L = _decl()
-            offsets = torch.empty(ngroups + 2, dtype=torch.int64, device=blob.device)
-            _check(L.ccb_sz_container_scan(None, blob.data_ptr() + HEADER_BYTES, ngroups, offsets.data_ptr(), _stream()))
-            total, largest = offsets[ngroups:].tolist()
+            if opened is not None:
+                offsets = opened
+                total, largest = found[5:].tolist()
+            else:
+                offsets = torch.empty(ngroups + 2, dtype=torch.int64, device=blob.device)
+                _check(L.ccb_sz_container_scan(None, blob.data_ptr() + HEADER_BYTES, ngroups, offsets.data_ptr(), _stream()))
+                total, largest = offsets[ngroups:].tolist()
             if total != nbytes or largest > GROUP_STRIDE:
                 raise ValueError("container payload is damaged")
             buf = torch.empty(ngroups * GROUP_STRIDE, dtype=torch.uint8, device=blob.device)

@@ -351,9 +351,7 @@ __global__ void __launch_bounds__(kLlThreads, kLlCtas) lossless_decode_kernel(co
 static size_t ll_tiles(size_t count) { return (count + kLlTileElems - 1) / kLlTileElems; }
 static size_t ll_slot(int dtype) { return dtype == CCB_F32 ? ll_slot_bytes<float>() : ll_slot_bytes<__half>(); }
 static int ll_grid(size_t ntiles) {
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int sms = sm_count();
   const size_t cap = (size_t)sms * kLlCtas;
   return (int)(ntiles < cap ? (ntiles ? ntiles : 1) : cap);
 }

@@ -168,9 +168,7 @@ __global__ void __launch_bounds__(kSaThreads) fold_kernel(const T* __restrict__ 
 }
 
 static int sa_grid(size_t units) {
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int sms = sm_count();
   size_t blocks = (units + (kSaThreads / 32) - 1) / (kSaThreads / 32);
   size_t cap = (size_t)sms * 8;
   if (blocks < 1) blocks = 1;

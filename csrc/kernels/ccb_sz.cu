@@ -818,7 +818,8 @@ __device__ __forceinline__ uint32_t pack_planes(const PlaneIO<kVec>& io, const S
   uint32_t run = 0;
   float ahead[8];
   io.load(0, ahead);
-#pragma unroll 2
+  constexpr int kTurns = kVec == 1 ? 1 : 2;   // with two the form for any line spills (511 x 512 x 512: 282 us, 250 with one)
+#pragma unroll kTurns
   for (int z = 0; z < kTZ; ++z) {
     float x[8];
 #pragma unroll
@@ -895,7 +896,7 @@ __device__ __forceinline__ uint32_t pack_planes(const PlaneIO<kVec>& io, const S
 }
 
 template <int kVec>
-__global__ void __launch_bounds__(kSzThreads, 3) sz_pack_kernel(const __grid_constant__ SzLocalArgs a) {
+__global__ void __launch_bounds__(kSzThreads, kVec == 1 ? 4 : 3) sz_pack_kernel(const __grid_constant__ SzLocalArgs a) {
   __shared__ __align__(16) unsigned char stage[kClusterSize][kWarpStage];
   __shared__ __align__(16) float plane[kVec == 1 ? kClusterSize : 1][kVec == 1 ? kTX * kTY : 4];
   __shared__ uint32_t s_size[kClusterSize];
@@ -1099,9 +1100,18 @@ __global__ void __launch_bounds__(kSzThreads, kVec == 1 ? 4 : 5) sz_unpack_kerne
 // offsets[ngroups + 1] = the largest size as it stands. `sizes` (u32 each) or, without them, the
 // groups' own headers in `slots`. One CTA: a few thousand groups at most in use, and the copy
 // that follows is the larger part.
+// With `head` (the start of a container, the sizes behind it) the number of groups is what the header
+// says, if no more than `ngroups`; otherwise nothing is scanned. Header and the two sums then go to
+// `found` besides, to be read back in one piece.
 constexpr int kScanThreads = 1024;
 __global__ void __launch_bounds__(kScanThreads) container_scan_kernel(const char* __restrict__ slots, const uint32_t* __restrict__ sizes,
-                                                                      unsigned int ngroups, unsigned long long* offsets) {
+                                                                      unsigned int ngroups, unsigned long long* offsets,
+                                                                      const uint32_t* __restrict__ head = nullptr, uint32_t* found = nullptr) {
+  if (head) {
+    const uint32_t said = head[7];
+    ngroups = said <= ngroups ? said : 0u;
+    if (threadIdx.x < 10) found[threadIdx.x] = head[threadIdx.x];
+  }
   __shared__ unsigned long long part[kScanThreads / 32];
   __shared__ uint32_t largest[kScanThreads / 32];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1145,6 +1155,10 @@ __global__ void __launch_bounds__(kScanThreads) container_scan_kernel(const char
     for (int k = 1; k < kScanThreads / 32; ++k) most = max(most, largest[k]);
     offsets[ngroups] = carry;
     offsets[ngroups + 1] = most;
+    if (head) {
+      reinterpret_cast<unsigned long long*>(found)[5] = carry;
+      reinterpret_cast<unsigned long long*>(found)[6] = most;
+    }
   }
 }
 
@@ -1316,16 +1330,9 @@ static int sz_launch(SzArgs& a, int nlocal, int num_sms, cudaStream_t stream) {
   return CCB_OK;
 }
 
-static int device_sms() {
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  return sms;
-}
-
 // Eight CTAs of 256 threads fill an SM; a group is a few KB, so a CTA takes several in turn.
 static unsigned int container_grid(uint64_t ngroups) {
-  const uint64_t most = (uint64_t)device_sms() * 8;
+  const uint64_t most = (uint64_t)sm_count() * 8;
   return (unsigned int)(ngroups < most ? ngroups : most);
 }
 // See PlaneIO.
@@ -1409,6 +1416,21 @@ extern "C" int ccb_sz_container_scan(const void* slots, const uint32_t* sizes, u
   return launched("ccb_sz_container_scan");
 }
 
+// The scan of a container of `bytes` bytes whose header is still on the device: offsets for at most
+// `room` groups (room + 2 words); found (56 bytes, 8-byte aligned) takes the header, the sum of the
+// group sizes and the largest. Nothing is scanned where the header speaks of more groups than `room`.
+extern "C" int ccb_sz_container_open(const void* blob, uint64_t bytes, uint64_t room, unsigned long long* offsets, void* found, ccb_stream_t stream) {
+  if (!blob || !offsets || !found || room == 0 || (room >> 31) || bytes < sizeof(ContainerHead) + 4 * room || (reinterpret_cast<uintptr_t>(blob) & 3) ||
+      (reinterpret_cast<uintptr_t>(found) & 7)) {
+    set_error("ccb_sz_container_open: bad arguments");
+    return CCB_ERR_ARG;
+  }
+  const uint32_t* head = static_cast<const uint32_t*>(blob);
+  container_scan_kernel<<<1, kScanThreads, 0, static_cast<cudaStream_t>(stream)>>>(nullptr, head + sizeof(ContainerHead) / 4, (unsigned int)room, offsets, head,
+                                                                                  static_cast<uint32_t*>(found));
+  return launched("ccb_sz_container_open");
+}
+
 // out: 40 + 4 * ngroups + offsets[ngroups] bytes, 4-byte aligned.
 extern "C" int ccb_sz_container_pack(const void* slots, const unsigned long long* offsets, int nx, int ny, int nz, float eb, uint64_t ngroups, void* out,
                                      ccb_stream_t stream) {
@@ -1482,5 +1504,5 @@ extern "C" int ccb_sz_collective(ccb_comm* c, const float* const* send, float* c
     a.bcast_waves = (unsigned int)waves;
   }
   if (d_used) cudaMemsetAsync(d_used, 0, sizeof(unsigned long long) * nlocal, stream);
-  return sz_launch(a, nlocal, device_sms(), stream);
+  return sz_launch(a, nlocal, sm_count(), stream);
 }

@@ -132,6 +132,19 @@ static const char* cu_err(CUresult r) {
 
 static size_t round_up(size_t x, size_t m) { return (x + m - 1) / m * m; }
 
+// Asked once for each device: the two runtime calls are a tenth of a small call's host time.
+int sm_count() {
+  static std::atomic<int> known[64];
+  int dev = 0, sms = 148;
+  if (cudaGetDevice(&dev) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return sms;
+  }
+  if (dev >= 0 && dev < 64 && known[dev].load(std::memory_order_relaxed)) return known[dev].load(std::memory_order_relaxed);
+  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && dev >= 0 && dev < 64) known[dev].store(sms, std::memory_order_relaxed);
+  return sms;
+}
+
 }  // namespace ccb
 
 using namespace ccb;

@@ -9,6 +9,7 @@ struct ccb_comm;
 namespace ccb {
 void set_error(const char* fmt, ...);
 void count_launch();
+int sm_count();   // of the current device
 CommDev comm_dev(ccb_comm* c, uint32_t epoch);
 uint32_t next_epoch(ccb_comm* c);
 int grid_cap(ccb_comm* c, const void* kernel, int threads = 512);

@@ -35,6 +35,7 @@ int ccb_sz_decompress(const void* in, int nx, int ny, int nz, float eb, float* o
  * the largest group's (ngroups + 2 words); from the groups' own headers (slots) or from a list of
  * sizes, exactly one of the two given. pack writes 40 + 4 * ngroups + offsets[ngroups] bytes;
  * unpack takes the payload behind a container's size list and fills ngroups whole slots. */
+int ccb_sz_container_open(const void* blob, uint64_t bytes, uint64_t room, unsigned long long* offsets, void* found, ccb_stream_t stream);
 int ccb_sz_container_scan(const void* slots, const uint32_t* sizes, uint64_t ngroups, unsigned long long* offsets, ccb_stream_t stream);
 int ccb_sz_container_pack(const void* slots, const unsigned long long* offsets, int nx, int ny, int nz, float eb, uint64_t ngroups, void* out,
                           ccb_stream_t stream);

@@ -28,3 +28,30 @@ def test_bytes_and_values_at_every_line_width(shape, start, scale):
     torch.cuda.synchronize()
     assert np.array_equal(target.view(shape).cpu().numpy(), sz.decode_cpu(want))
     assert (out[:start] == 7).all() and (out[start + n:] == 7).all()
+
+
+@pytest.mark.parametrize("damage", ["none", "short", "groups", "size", "payload", "magic"])
+def test_container_opened_on_the_device(damage):
+    shape, eb = (20, 30, 70), 1e-2
+    field = torch.randn(shape, generator=torch.Generator().manual_seed(1)).cuda()
+    buf, _ = sz.compress(field, eb)
+    blob = sz.to_container(buf, shape, eb)
+    words = blob[:sz.HEADER_BYTES + 8].view(torch.int32)
+    if damage == "short":
+        blob = blob[:sz.HEADER_BYTES + 60].clone()
+    elif damage == "groups":      # more than the blob has room for
+        words[7] = 1 << 30
+    elif damage == "size":        # of the first group
+        words[10] += 4
+    elif damage == "payload":
+        blob = blob[:-4].clone()
+    elif damage == "magic":
+        words[0] += 1
+    if damage == "none":
+        back, got_shape, got_eb = sz.from_container(blob)
+        assert got_shape == shape and abs(got_eb - eb) < 1e-9
+        assert torch.equal(sz.decompress(back, shape, got_eb), sz.decompress(buf, shape, eb))
+        assert torch.equal(sz.to_container(back, shape, eb), blob)
+    else:
+        with pytest.raises(ValueError):
+            sz.from_container(blob)
