@@ -29,7 +29,6 @@ _DTYPES = {torch.float32: K.F32, torch.bfloat16: K.BF16, torch.float16: K.F16}
 
 # Not in every torch: an inner function of the package, and absent from builds without CUDA.
 _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
-_device = getattr(torch._C, "_cuda_getDevice", torch.cuda.current_device)   # without the check for a first use of CUDA
 
 
 def current_stream_ptr() -> ctypes.c_void_p:
@@ -38,7 +37,7 @@ def current_stream_ptr() -> ctypes.c_void_p:
     where torch does not have the shorter one."""
     if _raw_stream is None:
         return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
-    return ctypes.c_void_p(_raw_stream(_device()))
+    return ctypes.c_void_p(_raw_stream(torch.cuda.current_device()))
 
 
 class CcbError(RuntimeError):
