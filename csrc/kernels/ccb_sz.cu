@@ -963,12 +963,21 @@ __global__ void __launch_bounds__(kSzThreads, kVec == 1 ? 4 : 5) sz_unpack_kerne
   const unsigned char* src = reinterpret_cast<const unsigned char*>(group) + kGroupHeader + off;
   const uint32_t hw = lane < 16 ? ldg_cg_u32(src + 4 * lane) : 0u;   // the row widths, four a word
   if ((__shfl_sync(0xffffffffu, hw, 0) & 0xffu) == 255u) {
-    const float4* raw = reinterpret_cast<const float4*>(src + kRows);
+    const uint32_t* raw = reinterpret_cast<const uint32_t*>(src + kRows) + 8 * lane;
+    const bool wide = (reinterpret_cast<uintptr_t>(raw) & 15) == 0;   // a buffer is promised to start on 4 bytes, no more
 #pragma unroll 1
-    for (int z = 0; z < kTZ; ++z) {
-      const uint4 p = ldg_cg(raw + 2 * (32 * z + lane)), q = ldg_cg(raw + 2 * (32 * z + lane) + 1);
-      const float v[8] = {__uint_as_float(p.x), __uint_as_float(p.y), __uint_as_float(p.z), __uint_as_float(p.w),
-                          __uint_as_float(q.x), __uint_as_float(q.y), __uint_as_float(q.z), __uint_as_float(q.w)};
+    for (int z = 0; z < kTZ; ++z, raw += kTX * kTY) {
+      uint32_t w[8];
+      if (wide) {
+        const uint4 p = ldg_cg(raw), q = ldg_cg(raw + 4);
+        w[0] = p.x; w[1] = p.y; w[2] = p.z; w[3] = p.w; w[4] = q.x; w[5] = q.y; w[6] = q.z; w[7] = q.w;
+      } else {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) w[e] = ldg_cg_u32(raw + e);
+      }
+      float v[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) v[e] = __uint_as_float(w[e]);
       io.store(z, v);
     }
     return;

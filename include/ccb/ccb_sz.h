@@ -22,10 +22,9 @@ uint64_t ccb_sz_capacity(int nx, int ny, int nz);
  * kernel's clusters and the cooperative attribute together, 2 = it refused the pair and the kernel
  * was launched plainly (grid bounded by the resident-cluster count). */
 int ccb_sz_launch_path(void);
-/* |in - decompress(compress(in))| <= eb for every finite element. `d_used` (device
- * memory, optional) receives the number of compressed bytes produced. Should a bounded wait of the
- * kernel ever give up, its top bit is set, a tile that never arrived is NaN, and the size words of
- * the groups concerned are larger than a group can be, so that no container is made of them. */
+/* |in - decompress(compress(in))| <= eb for every finite element. `out` starts on 16 bytes, the fields
+ * and a buffer to be read on 4. `d_used` (device memory, optional) receives the number of compressed
+ * bytes produced (those of the tiles, without the groups' size words). */
 int ccb_sz_compress(const float* in, int nx, int ny, int nz, float eb, void* out, unsigned long long* d_used,
                     ccb_stream_t stream);
 int ccb_sz_decompress(const void* in, int nx, int ny, int nz, float eb, float* out, ccb_stream_t stream);
@@ -34,7 +33,10 @@ int ccb_sz_decompress(const void* in, int nx, int ny, int nz, float eb, float* o
  * scan: offsets[g] = used bytes before group g, offsets[ngroups] their total, offsets[ngroups + 1]
  * the largest group's (ngroups + 2 words); from the groups' own headers (slots) or from a list of
  * sizes, exactly one of the two given. pack writes 40 + 4 * ngroups + offsets[ngroups] bytes;
- * unpack takes the payload behind a container's size list and fills ngroups whole slots. */
+ * unpack takes the payload behind a container's size list and fills ngroups whole slots.
+ * open: the scan of a container of `bytes` bytes whose header has not been read yet. `found` (56 bytes, on
+ * 8) takes the header, then the total and the largest as u64; offsets has room + 2 words, and nothing is
+ * scanned where the header speaks of more than `room` groups (40 + 4 * room <= bytes). */
 int ccb_sz_container_open(const void* blob, uint64_t bytes, uint64_t room, unsigned long long* offsets, void* found, ccb_stream_t stream);
 int ccb_sz_container_scan(const void* slots, const uint32_t* sizes, uint64_t ngroups, unsigned long long* offsets, ccb_stream_t stream);
 int ccb_sz_container_pack(const void* slots, const unsigned long long* offsets, int nx, int ny, int nz, float eb, uint64_t ngroups, void* out,

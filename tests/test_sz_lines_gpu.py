@@ -55,3 +55,14 @@ def test_container_opened_on_the_device(damage):
     else:
         with pytest.raises(ValueError):
             sz.from_container(blob)
+
+
+@pytest.mark.parametrize("start", [4, 8, 16])
+def test_packed_and_raw_tiles_from_a_buffer_on_four_bytes(start):
+    shape, eb = (17, 20, 96), 1e-2
+    field = torch.randn(shape, generator=torch.Generator().manual_seed(2))
+    field[:8, :8, 32:64] = 1e30
+    buf, _ = sz.compress(field.cuda(), eb)
+    moved = torch.empty(buf.numel() + start, dtype=torch.uint8, device="cuda")[start:]
+    moved.copy_(buf)
+    assert torch.equal(sz.decompress(moved, shape, eb), sz.decompress(buf, shape, eb))
