@@ -25,14 +25,14 @@
 // so a receiver finds every tile without any size exchange, while only the used
 // bytes are ever written (and cross NVLink).
 //
-// Kernel shape: one thread-block cluster of 8 CTAs per group. Each CTA fetches its
-// tile with ONE 3-D TMA copy (cp.async.bulk.tensor, no multicast) tracked by an
-// mbarrier, packs it in shared memory, the cluster exchanges the 8 sizes through
-// distributed shared memory to place the tiles back to back, and the packed tile is
-// copied out with 16-byte stores, to local memory (ccb_sz_compress) or straight
-// into every peer's arena (ccb_sz_all_gather), where the same CTAs decode what
-// arrives. Fields whose x extent is not a multiple of 4 elements (TMA needs 16-byte
-// row strides) take a plain-load path.
+// Kernel shapes: local buffers (ccb_sz_compress, ccb_sz_decompress) take a CTA a group, a
+// warp a tile (sz_pack_kernel, sz_unpack_kernel). The collectives take one thread-block
+// cluster of 8 CTAs per group: each CTA fetches its tile with ONE 3-D TMA copy
+// (cp.async.bulk.tensor, no multicast) tracked by an mbarrier, packs it in shared memory,
+// the cluster exchanges the 8 sizes through distributed shared memory to place the tiles
+// back to back, and the packed tile is copied out with 16-byte stores straight into every
+// peer's arena, where the same CTAs decode what arrives. Fields whose x extent is not a
+// multiple of 4 elements (TMA needs 16-byte row strides) take a plain-load path there.
 //
 // The reference has no GPU error-bounded codec: it reaches SZ3 through dlopen on the
 // CPU (userconfig/wrapper_code_examples/compression/sz3/mpi_sz3_wrapper.c:57-101,
