@@ -91,11 +91,17 @@ def _collective(comm, send, recv, eb, root, used):
 #   [u64 payload bytes][u32 used bytes of each group (header included)] [the used bytes of every group]
 MAGIC, VERSION = 0x5A534343, 2
 GROUP_STRIDE, GROUP_HEADER, HEADER_BYTES = 66112, 32, 40
-_LEAST_GROUP = 4 + GROUP_HEADER + 64   # its size word, the tiles' size words, the row widths of one tile
+ROWS, TILE_CAP = 64, 64 + 4 * TX * TY * TZ
+_LEAST_GROUP = 4 + GROUP_HEADER + ROWS   # its size word, the tiles' size words, the row widths of one tile
 
 
 def _by_kernel(t: torch.Tensor, align: int) -> bool:
     return t.is_cuda and t.dtype == torch.uint8 and t.is_contiguous() and t.data_ptr() % align == 0
+
+
+def _sound(sizes) -> bool:
+    """Whether tiles can have these sizes (csrc/kernels/ccb_sz_layout.h; 0: beyond the field)."""
+    return bool((((sizes == 0) | (sizes >= ROWS)) & (sizes <= TILE_CAP) & (sizes % 16 == 0)).all())
 
 
 def to_container(buf: torch.Tensor, shape, eb: float) -> torch.Tensor:
@@ -111,14 +117,15 @@ def to_container(buf: torch.Tensor, shape, eb: float) -> torch.Tensor:
             _check(L.ccb_sz_container_scan(buf.data_ptr(), None, ngroups, offsets.data_ptr(), _stream()))
             total, largest = offsets[ngroups:].tolist()
             if largest > GROUP_STRIDE:
-                raise ValueError("a group of the buffer was given up in compression, or is damaged")
+                raise ValueError("a group of the buffer is damaged")
             blob = torch.empty(HEADER_BYTES + 4 * ngroups + total, dtype=torch.uint8, device=buf.device)
             _check(L.ccb_sz_container_pack(buf.data_ptr(), offsets.data_ptr(), nx, ny, nz, eb, ngroups, blob.data_ptr(), _stream()))
         return blob
     slots = buf.view(ngroups, GROUP_STRIDE)
-    sizes = slots[:, :GROUP_HEADER].contiguous().view(torch.int32).to(torch.int64).sum(dim=1) + GROUP_HEADER
-    if ngroups and int(sizes.max()) > GROUP_STRIDE:
-        raise ValueError("a group of the buffer was given up in compression, or is damaged")
+    tiles = slots[:, :GROUP_HEADER].contiguous().view(torch.int32)
+    if not _sound(tiles):
+        raise ValueError("a group of the buffer is damaged")
+    sizes = tiles.to(torch.int64).sum(dim=1) + GROUP_HEADER
     keep = torch.arange(GROUP_STRIDE, device=buf.device).unsqueeze(0) < sizes.unsqueeze(1)
     payload = slots[keep]
     step = torch.tensor(2.0 * eb, dtype=torch.float32) * (1 - 2.0 ** -10)
@@ -132,14 +139,13 @@ def to_container(buf: torch.Tensor, shape, eb: float) -> torch.Tensor:
 
 def from_container(blob: torch.Tensor):
     """Inverse of to_container: returns (buffer of group slots, shape, eb)."""
-    opened = None
-    if _by_kernel(blob, 8) and blob.numel() >= HEADER_BYTES + _LEAST_GROUP:
-        # header, scan of the sizes and its sums in one read-back; no group is smaller than an empty tile's
+    by_kernel = _by_kernel(blob, 4) and blob.numel() >= HEADER_BYTES + _LEAST_GROUP
+    if by_kernel:   # header, scan of the sizes and its sums in one read-back; no group is smaller than an empty tile's
         with torch.cuda.device(blob.device):
             room = (blob.numel() - HEADER_BYTES) // _LEAST_GROUP
-            opened = torch.empty(room + 2 + 7, dtype=torch.int64, device=blob.device)
-            _check(_decl().ccb_sz_container_open(blob.data_ptr(), blob.numel(), room, opened.data_ptr(), opened.data_ptr() + 8 * (room + 2), _stream()))
-            found = opened[room + 2:].cpu()
+            offsets = torch.empty(room + 2 + 7, dtype=torch.int64, device=blob.device)
+            _check(_decl().ccb_sz_container_open(blob.data_ptr(), blob.numel(), room, offsets.data_ptr(), offsets.data_ptr() + 8 * (room + 2), _stream()))
+            found = offsets[room + 2:].cpu()
             head = found.view(torch.uint8)[:HEADER_BYTES]
     else:
         head = blob[:HEADER_BYTES].cpu()
@@ -151,24 +157,15 @@ def from_container(blob: torch.Tensor):
     nbytes = head[32:40].view(torch.int64).item()
     if ngroups * GROUP_STRIDE != capacity((nz, ny, nx)):
         raise ValueError("container header does not match its dimensions")
-    if _by_kernel(blob, 4) and ngroups and blob.numel() >= HEADER_BYTES + 4 * ngroups:
-        if opened is not None and ngroups > room:
-            opened = None
-        if blob.numel() - HEADER_BYTES - 4 * ngroups != nbytes:
+    if by_kernel:
+        if ngroups > room or blob.numel() - HEADER_BYTES - 4 * ngroups != nbytes:
+            raise ValueError("container payload is damaged")
+        total, largest = found[5:].tolist()
+        if total != nbytes or largest > GROUP_STRIDE:
             raise ValueError("container payload is damaged")
         with torch.cuda.device(blob.device):
-            L = _decl()
-            if opened is not None:
-                offsets = opened
-                total, largest = found[5:].tolist()
-            else:
-                offsets = torch.empty(ngroups + 2, dtype=torch.int64, device=blob.device)
-                _check(L.ccb_sz_container_scan(None, blob.data_ptr() + HEADER_BYTES, ngroups, offsets.data_ptr(), _stream()))
-                total, largest = offsets[ngroups:].tolist()
-            if total != nbytes or largest > GROUP_STRIDE:
-                raise ValueError("container payload is damaged")
             buf = torch.empty(ngroups * GROUP_STRIDE, dtype=torch.uint8, device=blob.device)
-            _check(L.ccb_sz_container_unpack(blob.data_ptr() + HEADER_BYTES + 4 * ngroups, offsets.data_ptr(), ngroups, buf.data_ptr(), _stream()))
+            _check(_decl().ccb_sz_container_unpack(blob.data_ptr() + HEADER_BYTES + 4 * ngroups, offsets.data_ptr(), ngroups, buf.data_ptr(), _stream()))
         return buf, (nz, ny, nx), eb
     sizes = blob[HEADER_BYTES:HEADER_BYTES + 4 * ngroups].contiguous().view(torch.int32).to(torch.int64)
     payload = blob[HEADER_BYTES + 4 * ngroups:]
@@ -177,6 +174,9 @@ def from_container(blob: torch.Tensor):
     buf = torch.zeros(ngroups, GROUP_STRIDE, dtype=torch.uint8, device=blob.device)
     keep = torch.arange(GROUP_STRIDE, device=blob.device).unsqueeze(0) < sizes.unsqueeze(1)
     buf[keep] = payload
+    tiles = buf[:, :GROUP_HEADER].contiguous().view(torch.int32)
+    if not _sound(tiles) or not torch.equal(tiles.to(torch.int64).sum(dim=1) + GROUP_HEADER, sizes):
+        raise ValueError("container payload is damaged")
     return buf.view(-1), (nz, ny, nx), eb
 
 
@@ -289,6 +289,8 @@ def decode_cpu(blob: np.ndarray) -> np.ndarray:
     for g in range(ngroups):
         grp = body[pos:pos + int(used[g])]
         pos += int(used[g])
+        if grp.size < GROUP_HEADER or not _sound(grp[:GROUP_HEADER].view("<u4")) or int(grp[:GROUP_HEADER].view("<u4").sum()) + GROUP_HEADER != grp.size:
+            raise ValueError("container payload is damaged")
         sizes = grp[:GROUP_HEADER].view("<u4")
         off = GROUP_HEADER
         for k in range(8):
@@ -297,6 +299,8 @@ def decode_cpu(blob: np.ndarray) -> np.ndarray:
                 continue
             t = grp[off:off + int(sizes[k])]
             off += int(sizes[k])
+            if t.size < (TILE_CAP if t[0] == 255 else ROWS + 4 * int(t[:ROWS].sum())) or (t[0] != 255 and t[:ROWS].max() > 32):
+                raise ValueError("container payload is damaged")
             if t[0] == 255:
                 vals = t[64:64 + 4 * TZ * TY * TX].view("<f4").reshape(TZ, TY, TX)
             else:

@@ -50,6 +50,7 @@
 #include "../rt/ccb_rt_internal.h"
 #include "ccb/ccb_sz.h"
 #include "ccb_fastdiv.h"
+#include "ccb_sz_layout.h"
 #include "ccb_bits.cuh"
 #include "ccb_reduce.cuh"
 
@@ -59,12 +60,13 @@ namespace ccb {
 
 constexpr int kTX = 32, kTY = 8, kTZ = 8;
 constexpr int kTileVals = kTX * kTY * kTZ;        // 2048
-constexpr int kRows = kTY * kTZ;                  // 64
+constexpr int kRows = CCB_SZ_ROWS;                // kTY * kTZ
 constexpr int kSzThreads = 256;                   // warp = z plane, lane = x
-constexpr int kClusterSize = 8;
-constexpr int kTileCap = kRows + kTileVals * 4;   // 8256 bytes, worst case (w = 32 everywhere)
-constexpr int kGroupHeader = 32;
-constexpr int kGroupStride = kGroupHeader + kClusterSize * kTileCap + 32;  // 66112, multiple of 16
+constexpr int kClusterSize = CCB_SZ_TILES;
+constexpr int kTileCap = CCB_SZ_TILE_CAP;         // 8256 bytes, worst case (w = 32 everywhere)
+constexpr int kGroupHeader = CCB_SZ_GROUP_HEADER;
+constexpr int kGroupStride = CCB_SZ_GROUP_STRIDE;   // 66112, multiple of 16
+static_assert(kRows == kTY * kTZ && kTileCap == kRows + kTileVals * 4, "the tile that ccb_sz_layout.h describes");
 static_assert(kGroupStride % 16 == 0, "slots must keep 16-byte alignment");
 constexpr float kQMax = 4194304.f;                // 2^22: |q| beyond this stores the tile raw
 
@@ -338,17 +340,20 @@ __device__ __forceinline__ uint32_t pack_tile(float* vals, unsigned char* pk, in
 // `qs2` is two times 8 KB of shared scratch, of which a packed tile takes the one that the packed
 // tile before it did not (`scratch`: 0 or 1). A raw tile takes none and needs no barrier. (512^3
 // fields, B200: raw tiles only 407 us, packed tiles only 324; with a scratch for every tile and a
-// barrier in the raw ones it was 432 and 321.)
-__device__ __forceinline__ void unpack_tile(const unsigned char* src, int* qs2, int& scratch, const SzArgs& a, float* out, const TileCoord& t) {
+// barrier in the raw ones it was 432 and 321.) A tile whose widths cannot be (or `sound` false: whose
+// place cannot) becomes NaN, without an access through its words.
+__device__ __forceinline__ void unpack_tile(const unsigned char* src, bool sound, int* qs2, int& scratch, const SzArgs& a, float* out, const TileCoord& t) {
   const int lane = threadIdx.x & 31, z = threadIdx.x >> 5;
   // the 16 words of row widths, one per lane, and their running word count
-  const uint32_t hw = lane < 16 ? ldg_cg_u32(src + 4 * lane) : 0u;
-  if ((__shfl_sync(0xffffffffu, hw, 0) & 0xffu) == 255u) {
+  const uint32_t hw = sound && lane < 16 ? ldg_cg_u32(src + 4 * lane) : 0u;
+  const bool raw_tile = (__shfl_sync(0xffffffffu, hw, 0) & 0xffu) == 255u;
+  sound = sound && (raw_tile || !__any_sync(0xffffffffu, !ccb_sz_widths_ok(hw)));
+  if (raw_tile || !sound) {
     const float* raw = reinterpret_cast<const float*>(src + kRows);
     for (int i = threadIdx.x; i < kTileVals; i += kSzThreads) {
       const int gx = t.x0 + (i % kTX), gy = t.y0 + (i / kTX) % kTY, gz = t.z0 + i / (kTX * kTY);
       if (gx < a.nx && gy < a.ny && gz < a.nz)
-        out[((size_t)gz * a.ny + gy) * a.nx + gx] = __uint_as_float(ldg_cg_u32(raw + i));
+        out[((size_t)gz * a.ny + gy) * a.nx + gx] = __uint_as_float(sound ? ldg_cg_u32(raw + i) : 0x7fffffffu);
     }
     return;
   }
@@ -661,14 +666,12 @@ __global__ void __cluster_dims__(kClusterSize, 1, 1) __launch_bounds__(kSzThread
                           (mode == 3 && dwave < kBcastWaves && (dwave ? dwave_end(dwave - 1) : 0u) <= f + 1);
     sz_next = boundary ? 0u : sizes_of(f + 1);
     if (!valid(f)) continue;
-    uint32_t off = __reduce_add_sync(0xffffffffu, sz);
-    if (off > (uint32_t)(kClusterSize * kTileCap)) {   // damaged size words: stay inside the slot and flag it
-      off = 0;
-      if (threadIdx.x == 0 && a.c.status) atomicOr(a.c.status + CCB_STATUS_FLAGS, CCB_ST_TIMEOUT);
-    }
+    const uint32_t off = __reduce_add_sync(0xffffffffu, sz);
+    const bool sound = ccb_sz_offset_ok(off, k);
+    if (!sound && threadIdx.x == 0 && a.c.status) atomicOr(a.c.status + CCB_STATUS_FLAGS, CCB_ST_TIMEOUT);   // damaged size words
     const int q = mode == 2 ? (r + 1 + (int)(f / per_src)) % n : a.root;
     float* out = a.f[lr].out + (mode == 2 ? (size_t)q * a.nx * a.ny * a.nz : 0);
-    unpack_tile(reinterpret_cast<const unsigned char*>(group_of(f)) + kGroupHeader + off, reinterpret_cast<int*>(vals2[0]), scratch, a,
+    unpack_tile(reinterpret_cast<const unsigned char*>(group_of(f)) + kGroupHeader + off, sound, reinterpret_cast<int*>(vals2[0]), scratch, a,
                 out, tile_coord(a, (cl + (f % per_src) * ncl) * kClusterSize + k));
   }
   trace_mark(a.c, 4);
@@ -959,9 +962,11 @@ __global__ void __launch_bounds__(kSzThreads, kVec == 1 ? 4 : 5) sz_unpack_kerne
   const char* group = a.slots + (size_t)blockIdx.x * kGroupStride;
   const PlaneIO<kVec> io(a.out, a, tile_coord(a, tile), plane[kVec == 1 ? k : 0]);
   uint32_t off = __reduce_add_sync(0xffffffffu, lane < k ? ldg_cg_u32(group + 4 * lane) : 0u);
-  if (off > (uint32_t)(kClusterSize * kTileCap)) off = 0;   // damaged size words: stay inside the slot
+  const bool there = ccb_sz_offset_ok(off, k);
+  if (!there) off = 0;
   const unsigned char* src = reinterpret_cast<const unsigned char*>(group) + kGroupHeader + off;
-  const uint32_t hw = lane < 16 ? ldg_cg_u32(src + 4 * lane) : 0u;   // the row widths, four a word
+  uint32_t hw = lane < 16 ? ldg_cg_u32(src + 4 * lane) : 0u;   // the row widths, four a word
+  if (!there) hw = 0xfefefefeu;
   if ((__shfl_sync(0xffffffffu, hw, 0) & 0xffu) == 255u) {
     const uint32_t* raw = reinterpret_cast<const uint32_t*>(src + kRows) + 8 * lane;
     const bool wide = (reinterpret_cast<uintptr_t>(raw) & 15) == 0;   // a buffer is promised to start on 4 bytes, no more
@@ -980,6 +985,14 @@ __global__ void __launch_bounds__(kSzThreads, kVec == 1 ? 4 : 5) sz_unpack_kerne
       for (int e = 0; e < 8; ++e) v[e] = __uint_as_float(w[e]);
       io.store(z, v);
     }
+    return;
+  }
+  if (__any_sync(0xffffffffu, !ccb_sz_widths_ok(hw))) {   // a tile whose place or widths cannot be: NaN, nothing is read through its words
+    float v[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) v[e] = __int_as_float(0x7fffffff);
+#pragma unroll 1
+    for (int z = 0; z < kTZ; ++z) io.store(z, v);
     return;
   }
   uint32_t* words = reinterpret_cast<uint32_t*>(const_cast<unsigned char*>(src) + kRows);
@@ -1105,17 +1118,34 @@ __global__ void __launch_bounds__(kSzThreads, kVec == 1 ? 4 : 5) sz_unpack_kerne
 // several times: a field of 130 x 201 x 258 took 819 us through compress, pack, unpack and
 // decompress, 159 us since (B200).
 
+struct ContainerHead {   // 40 bytes, as in a file
+  uint32_t magic, version;
+  int nx, ny, nz;
+  float eb, step;
+  uint32_t ngroups;
+  unsigned long long payload;
+};
+static_assert(sizeof(ContainerHead) == 40, "container header layout");
+
 // offsets[g] = sum of the (clipped) sizes before group g; offsets[ngroups] = their total,
-// offsets[ngroups + 1] = the largest size as it stands. `sizes` (u32 each) or, without them, the
+// offsets[ngroups + 1] = the largest size as it stands, or 2^32 - 1 where a group's tiles cannot have the
+// sizes that its header gives them. `sizes` (u32 each) or, without them, the
 // groups' own headers in `slots`. One CTA: a few thousand groups at most in use, and the copy
 // that follows is the larger part.
 // With `head` (the start of a container, the sizes behind it) the number of groups is what the header
 // says, if no more than `ngroups`; otherwise nothing is scanned. Header and the two sums then go to
-// `found` besides, to be read back in one piece.
+// `found` besides, to be read back in one piece, and the groups' headers, in the `bytes` bytes from
+// `head` on, are held against the list.
 constexpr int kScanThreads = 1024;
+__device__ __forceinline__ bool sizes_sound(const uint4& x, const uint4& y) {
+  return ccb_sz_size_ok(x.x) && ccb_sz_size_ok(x.y) && ccb_sz_size_ok(x.z) && ccb_sz_size_ok(x.w) && ccb_sz_size_ok(y.x) && ccb_sz_size_ok(y.y) &&
+         ccb_sz_size_ok(y.z) && ccb_sz_size_ok(y.w);
+}
+__device__ __forceinline__ uint32_t sizes_sum(const uint4& x, const uint4& y) { return x.x + x.y + x.z + x.w + y.x + y.y + y.z + y.w; }
 __global__ void __launch_bounds__(kScanThreads) container_scan_kernel(const char* __restrict__ slots, const uint32_t* __restrict__ sizes,
                                                                       unsigned int ngroups, unsigned long long* offsets,
-                                                                      const uint32_t* __restrict__ head = nullptr, uint32_t* found = nullptr) {
+                                                                      const uint32_t* __restrict__ head = nullptr, uint32_t* found = nullptr,
+                                                                      unsigned long long bytes = 0) {
   if (head) {
     const uint32_t said = head[7];
     ngroups = said <= ngroups ? said : 0u;
@@ -1135,7 +1165,8 @@ __global__ void __launch_bounds__(kScanThreads) container_scan_kernel(const char
       } else {
         const uint4* h = reinterpret_cast<const uint4*>(slots + (size_t)g * kGroupStride);
         const uint4 x = h[0], y = h[1];
-        size = x.x + x.y + x.z + x.w + y.x + y.y + y.z + y.w + kGroupHeader;
+        size = sizes_sum(x, y) + kGroupHeader;
+        if (!sizes_sound(x, y)) most = 0xffffffffu;
       }
     }
     most = max(most, size);
@@ -1154,6 +1185,16 @@ __global__ void __launch_bounds__(kScanThreads) container_scan_kernel(const char
       all += part[k];
     }
     if (g < ngroups) offsets[g] = before + incl - clipped;
+    if (head && g < ngroups) {   // (a list that does not add up to what is there is refused by its total)
+      const unsigned long long at = sizeof(ContainerHead) + 4ull * ngroups + before + incl - clipped;
+      if ((at & 3u) == 0 && at + kGroupHeader <= bytes) {
+        const uint32_t* h = head + at / 4;
+        const uint4 x = make_uint4(h[0], h[1], h[2], h[3]), y = make_uint4(h[4], h[5], h[6], h[7]);
+        if (!sizes_sound(x, y) || sizes_sum(x, y) + kGroupHeader != size) most = 0xffffffffu;
+      } else {
+        most = 0xffffffffu;
+      }
+    }
     carry += all;
     __syncthreads();
   }
@@ -1189,14 +1230,6 @@ __device__ __forceinline__ void copy_bytes(char* dst, const char* src, uint32_t 
   for (uint32_t i = done + threadIdx.x; i < n; i += blockDim.x) dst[i] = src[i];
 }
 
-struct ContainerHead {   // 40 bytes, as in a file
-  uint32_t magic, version;
-  int nx, ny, nz;
-  float eb, step;
-  uint32_t ngroups;
-  unsigned long long payload;
-};
-static_assert(sizeof(ContainerHead) == 40, "container header layout");
 constexpr uint32_t kContainerMagic = 0x5A534343u, kContainerVersion = 2u;
 
 __global__ void __launch_bounds__(256) container_pack_kernel(const char* __restrict__ slots, const unsigned long long* __restrict__ offsets,
@@ -1436,7 +1469,7 @@ extern "C" int ccb_sz_container_open(const void* blob, uint64_t bytes, uint64_t 
   }
   const uint32_t* head = static_cast<const uint32_t*>(blob);
   container_scan_kernel<<<1, kScanThreads, 0, static_cast<cudaStream_t>(stream)>>>(nullptr, head + sizeof(ContainerHead) / 4, (unsigned int)room, offsets, head,
-                                                                                  static_cast<uint32_t*>(found));
+                                                                                  static_cast<uint32_t*>(found), bytes);
   return launched("ccb_sz_container_open");
 }
 

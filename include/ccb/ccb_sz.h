@@ -24,18 +24,22 @@ uint64_t ccb_sz_capacity(int nx, int ny, int nz);
 int ccb_sz_launch_path(void);
 /* |in - decompress(compress(in))| <= eb for every finite element. `out` starts on 16 bytes, the fields
  * and a buffer to be read on 4. `d_used` (device memory, optional) receives the number of compressed
- * bytes produced (those of the tiles, without the groups' size words). */
+ * bytes produced (those of the tiles, without the groups' size words). A tile of a damaged buffer whose
+ * size words put it outside its group, or whose rows are wider than 32 bits, is decompressed to NaN;
+ * what else a damaged buffer holds is decoded as it stands, from inside its slots. */
 int ccb_sz_compress(const float* in, int nx, int ny, int nz, float eb, void* out, unsigned long long* d_used,
                     ccb_stream_t stream);
 int ccb_sz_decompress(const void* in, int nx, int ny, int nz, float eb, float* out, ccb_stream_t stream);
 /* The packed container of a compressed buffer: a 40-byte header, the used bytes of each group as u32,
  * then the used bytes of every group. All pointers device memory.
  * scan: offsets[g] = used bytes before group g, offsets[ngroups] their total, offsets[ngroups + 1]
- * the largest group's (ngroups + 2 words); from the groups' own headers (slots) or from a list of
+ * the largest group's (ngroups + 2 words; 2^32 - 1 where a group's header holds sizes that tiles cannot
+ * have); from the groups' own headers (slots) or from a list of
  * sizes, exactly one of the two given. pack writes 40 + 4 * ngroups + offsets[ngroups] bytes;
  * unpack takes the payload behind a container's size list and fills ngroups whole slots.
  * open: the scan of a container of `bytes` bytes whose header has not been read yet. `found` (56 bytes, on
- * 8) takes the header, then the total and the largest as u64; offsets has room + 2 words, and nothing is
+ * 8) takes the header, then the total and the largest as u64 (2^32 - 1 also where a group's header does not
+ * add up to its size in the list); offsets has room + 2 words, and nothing is
  * scanned where the header speaks of more than `room` groups (40 + 4 * room <= bytes). */
 int ccb_sz_container_open(const void* blob, uint64_t bytes, uint64_t room, unsigned long long* offsets, void* found, ccb_stream_t stream);
 int ccb_sz_container_scan(const void* slots, const uint32_t* sizes, uint64_t ngroups, unsigned long long* offsets, ccb_stream_t stream);

@@ -66,3 +66,63 @@ def test_packed_and_raw_tiles_from_a_buffer_on_four_bytes(start):
     moved = torch.empty(buf.numel() + start, dtype=torch.uint8, device="cuda")[start:]
     moved.copy_(buf)
     assert torch.equal(sz.decompress(moved, shape, eb), sz.decompress(buf, shape, eb))
+
+
+@pytest.mark.parametrize("shape", [(17, 20, 96), (9, 9, 258)])
+@pytest.mark.parametrize("word,value", [(0, 8 * 8256), (1, 12), (2, 1 << 31), (6, 7), (3, 0xfffffff0)])
+def test_damaged_tile_sizes_stay_inside_the_slot(shape, word, value):
+    """A size word that puts the tiles behind it where none can lie: those become NaN, the rest stay."""
+    eb = 1e-2
+    field = torch.randn(shape, generator=torch.Generator().manual_seed(3)).cuda()
+    buf, _ = sz.compress(field, eb)
+    want = sz.decompress(buf, shape, eb)
+    bad = buf.clone()
+    group = buf.numel() // sz.GROUP_STRIDE - 1
+    sizes = bad[group * sz.GROUP_STRIDE:][:sz.GROUP_HEADER].view(torch.int32)
+    sizes[word] = value if value < 1 << 31 else value - (1 << 32)
+    words = [w & 0xffffffff for w in sizes.tolist()]
+    got = sz.decompress(bad, shape, eb)
+    with pytest.raises(ValueError):
+        sz.to_container(bad, shape, eb)
+    tx, ty = -(-shape[2] // 32), -(-shape[1] // 8)
+    tiles = tx * ty * -(-shape[0] // 8)
+    off = 0
+    for t in range(tiles):
+        z, y, x = 8 * (t // (tx * ty)), 8 * (t // tx % ty), 32 * (t % tx)
+        box = (slice(z, z + 8), slice(y, y + 8), slice(x, x + 32))
+        k = t % 8
+        if t < 8 * group or k <= word:
+            assert torch.equal(got[box], want[box]), t
+        elif off > k * sz.TILE_CAP or off % 16:
+            assert got[box].isnan().all(), t
+        off = (0 if k == 7 else off + words[k]) & 0xffffffff if t >= 8 * group else 0
+
+
+@pytest.mark.parametrize("row", [0, 1, 31, 63])
+@pytest.mark.parametrize("width", [33, 128, 254])
+def test_damaged_row_widths_make_their_tile_nan(row, width):
+    shape, eb = (8, 8, 64), 1e-2
+    field = torch.randn(shape, generator=torch.Generator().manual_seed(4)).cuda()
+    buf, _ = sz.compress(field, eb)
+    want = sz.decompress(buf, shape, eb)
+    first = int(buf[:4].view(torch.int32))
+    buf[sz.GROUP_HEADER + first + row] = width
+    got = sz.decompress(buf, shape, eb)
+    assert torch.equal(got[..., :32], want[..., :32]) and got[..., 32:].isnan().all()
+
+
+@pytest.mark.parametrize("start", [0, 4])
+@pytest.mark.parametrize("word,change", [(0, 4), (1, 16), (5, 1 << 20)])
+def test_container_with_damaged_tile_sizes_is_refused_on_the_device(start, word, change):
+    shape, eb = (20, 30, 70), 1e-2
+    field = torch.randn(shape, generator=torch.Generator().manual_seed(1)).cuda()
+    buf, _ = sz.compress(field, eb)
+    blob = sz.to_container(buf, shape, eb)
+    moved = torch.empty(blob.numel() + start, dtype=torch.uint8, device="cuda")[start:]
+    moved.copy_(blob)
+    assert torch.equal(sz.from_container(moved)[0], sz.from_container(blob)[0])
+    first = int(blob[sz.HEADER_BYTES:][:4].view(torch.int32))
+    at = sz.HEADER_BYTES + 4 * (buf.numel() // sz.GROUP_STRIDE) + first + 4 * word   # group 1
+    moved[at:at + 4].view(torch.int32).add_(change)
+    with pytest.raises(ValueError):
+        sz.from_container(moved)
