@@ -33,6 +33,7 @@
 #include "../rt/ccb_rt_internal.h"
 #include "ccb_device.cuh"
 #include "ccb_bits.cuh"
+#include "ccb_lossless_layout.h"
 
 namespace ccb {
 
@@ -272,9 +273,9 @@ __global__ void __launch_bounds__(kLlThreads, kLlCtas) lossless_decode_kernel(co
     Body b;
     const char* slot = slot_of(t);
     const uint32_t wsel = warp < 4 ? d.h.y : d.h.z;
-    b.w = (int)((wsel >> sh) & 0xffu);
+    b.w = (int)ccb_ll_planes((wsel >> sh) & 0xffu, Tr::kExpBits);
     b.kmin = ((warp < 4 ? d.h.w : d.high_min) >> sh) & 0xffu;
-    const uint32_t off = __dp4a(wsel & ((1u << sh) - 1u), 0x01010101u, warp < 4 ? 0u : __dp4a(d.h.y, 0x01010101u, 0u));
+    const uint32_t off = ccb_ll_first_plane(__dp4a(wsel & ((1u << sh) - 1u), 0x01010101u, warp < 4 ? 0u : __dp4a(d.h.y, 0x01010101u, 0u)), warp, Tr::kExpBits);
     b.planes = fetch_planes(reinterpret_cast<const uint32_t*>(slot + 32 + Tr::kRestBytesPerTile) + off * 16, b.w, lane);
 #pragma unroll
     for (int p = 0; p < kRest; ++p) b.rest[p] = *reinterpret_cast<const uint4*>(slot + 32 + warp * kWarpElems + lane * 16 + (size_t)p * kLlTileElems);

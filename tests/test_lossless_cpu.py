@@ -60,3 +60,36 @@ def test_ratio_tool_on_the_numpy_codec(tmp_path, capsys):
     assert all(0.5 < r["ratio"] < 1.0 for r in rows), rows
     assert R.main([str(tmp_path), "--cpu", "--sizes", "64K"]) == 0
     assert "ratio below 1.0" in capsys.readouterr().out
+
+
+def test_planes_of_damaged_widths_stay_inside_their_slot(tmp_path):
+    """csrc/kernels/ccb_lossless_layout.h, which the decoder reads a slot by: any eight width bytes, for
+    each type's slot; and sound ones keep their places."""
+    import os
+    import shutil
+    import subprocess
+
+    if not shutil.which("gcc"):
+        pytest.skip("no C compiler")
+    src = tmp_path / "t.c"
+    src.write_text(r'''
+#include <stdlib.h>
+#include "ccb_lossless_layout.h"
+int main(void) {
+    const uint32_t bits[3] = {8, 8, 5}, rest[3] = {3 * 4096, 4096, 4096 + 1536}, slot[3] = {32 + 16384, 32 + 8192, 32 + 8192};
+    for (int t = 0; t < 3; ++t)
+        for (int i = 0; i < 200000; ++i) {
+            uint32_t sum = 0;
+            for (uint32_t b = 0; b < 8; ++b) {
+                const uint32_t w = i == 0 ? 255u : i < 100000 ? (uint32_t)rand() % 256u : (uint32_t)rand() % (bits[t] + 1);
+                const uint32_t first = ccb_ll_first_plane(sum, b, bits[t]), n = ccb_ll_planes(w, bits[t]);
+                if (32 + rest[t] + 64 * (first + n) > slot[t]) return 1;
+                if (i >= 100000 && (first != sum || n != w)) return 2;
+                sum += w;
+            }
+        }
+    return 0;
+}''')
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    subprocess.run(["gcc", "-O2", "-I" + os.path.join(root, "csrc", "kernels"), str(src), "-o", str(tmp_path / "t")], check=True)
+    assert subprocess.run([str(tmp_path / "t")]).returncode == 0

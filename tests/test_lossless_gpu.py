@@ -118,3 +118,17 @@ def test_hook_library_round_trip_and_reduce():
     assert torch.equal(acc, x + 2.0)
     v = x.view(chunks, per)
     assert torch.equal(one, (v[0] + v[1]) + v[2])
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("block,width", [(0, 255), (3, 9), (7, 255)])
+def test_damaged_widths_leave_the_blocks_before_them(dtype, block, width):
+    code = {torch.float32: 0, torch.bfloat16: 1, torch.float16: 2}[dtype]
+    x = torch.randn(2 * LL.TILE, generator=torch.Generator().manual_seed(1)).to(dtype).cuda()
+    comp = LL.encode(x)
+    at = LL.HEADER + LL.slot_bytes(code) + 4 + block   # of the last slot
+    comp[at] = width
+    got = LL.decode(comp, x.numel(), dtype)
+    sound = LL.TILE + block * LL.BLOCK
+    bits = torch.int32 if dtype == torch.float32 else torch.int16
+    assert torch.equal(got[:sound].view(bits), x[:sound].view(bits))
