@@ -24,7 +24,9 @@ extern "C" {
  * combine: rank r (expert side) sends the rows of `y` that came from origin q (the
  *   block starting at row sum_{s<q} counts[s][r]) back to q; origin q computes
  *   out[t] = sum_k gate[t*topk+k] * row(from rank dest_rank[t*topk+k], position pos[t*topk+k])
- *   where pos is the index of (t,k) inside the block q sent to that rank.
+ *   where pos is the index of (t,k) inside the block q sent to that rank. A pair whose dest_rank is
+ *   no rank, or whose pos is not below counts[q][dest_rank], contributes nothing: a plan marks the
+ *   pairs that it dropped (an expert's capacity) with pos = -1, and leaves them out of perm and counts.
  * Arrays are per local rank like everywhere else. */
 int ccb_moe_dispatch(ccb_comm* c, const void* const* x, void* const* recv, const int32_t* const* perm,
                      const uint64_t* counts, uint64_t hidden, int dtype, int codec, ccb_stream_t stream);

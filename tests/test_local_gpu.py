@@ -218,3 +218,42 @@ def test_moe(dtype, codec, n, tokens, hidden, topk):
 
         _both(comm, onto)
     comm.close()
+
+
+@pytest.mark.parametrize("codec", ["none", "fp8", "int4"])
+@pytest.mark.parametrize("n,tokens,hidden,topk", [(2, 33, 512, 1), (4, 130, 1536, 2)])
+def test_moe_with_dropped_pairs(codec, n, tokens, hidden, topk):
+    """Experts that take so many pairs of each rank and no more: what is beyond is left out of perm and
+    counts, and marked in pos or dest_rank."""
+    keep = tokens * topk // n // 2 + 1
+    comm = Communicator.local(n, arena_bytes=64 << 20)
+    g = torch.Generator(device="cuda").manual_seed(tokens)
+    xs = [_values(tokens * hidden, torch.bfloat16, r).view(tokens, hidden) for r in range(n)]
+    routes, counts, gates = [], [], []
+    for r in range(n):
+        w, ids = torch.topk(torch.softmax(torch.rand(tokens, 8, generator=g, device="cuda"), -1), topk, -1)
+        full = moe.plan_route(ids, w, n)
+        sent = full.send_counts.tolist()
+        kept = [min(c, keep) for c in sent]
+        perm = torch.cat([full.perm[sum(sent[:d]):][:kept[d]] for d in range(n)])
+        dropped = full.pos >= keep
+        assert dropped.any()
+        pos = torch.where(dropped, torch.full_like(full.pos, -1 if r % 2 else keep), full.pos)
+        dest = torch.where(dropped & (torch.arange(tokens * topk, device="cuda") % 3 == 0), torch.full_like(full.dest_rank, -1 if r % 2 else n), full.dest_rank)
+        routes.append(moe.Route(perm.contiguous(), dest, pos, full.gate, torch.tensor(kept), topk))
+        counts.append(kept)
+        gates.append(torch.where(dropped, torch.zeros_like(full.gate), full.gate).view(tokens, topk).sum(1, keepdim=True))
+    rows = [sum(counts[q][d] for q in range(n)) for d in range(n)]
+
+    def call():
+        recv = [torch.full((rows[d] + 1, hidden), 7.0, dtype=torch.bfloat16, device="cuda") for d in range(n)]
+        out = [torch.full((tokens, hidden), 7.0, dtype=torch.bfloat16, device="cuda") for _ in range(n)]
+        moe.dispatch(comm, xs, recv, routes, counts, codec=codec)
+        moe.combine(comm, recv, out, routes, counts, codec=codec)
+        if codec == "none":   # every kept copy of a token is the token; topk products and sums in fp32, one rounding to bf16
+            for o, x, gate in zip(out, xs, gates):
+                assert ((o.float() - x.float() * gate).abs() <= 2.0 ** -8 * (x.float() * gate).abs() + 1e-30).all()
+        return recv + out
+
+    _both(comm, call)
+    comm.close()
