@@ -14,6 +14,7 @@
 // CTAs in the order of the addresses.
 #pragma once
 #include "ccb_codec.cuh"
+#include "ccb_grid.h"
 
 namespace ccb {
 
@@ -273,7 +274,7 @@ __device__ __forceinline__ void local_reduce_unit(const LocalReduceArgs& a, uint
 
 template <class T, class C, int ALGO, bool kEf, bool kAnyOffset>
 __global__ void __launch_bounds__(kLocalThreads, LocalShape<T, ALGO, kEf, kAnyOffset>::kCtas) local_reduce_kernel(const __grid_constant__ LocalReduceArgs a) {
-  const uint32_t u = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const uint32_t u = ccb_grid_warp(blockIdx.x, blockDim.x, threadIdx.x);
   if (u >= a.units) return;
   const uint32_t s = ALGO == kLocalTwoShot || ALGO == kLocalRing || ALGO == kLocalScatter ? u / a.shard_units : 0u;
   const size_t e0 = (size_t)(ALGO == kLocalScatter ? u - s * a.shard_units : u) * kWarpElems, idx = e0 + (threadIdx.x & 31) * kLaneElems;
@@ -334,7 +335,7 @@ template <class T, class C, bool kAnyOffset>
 __global__ void __launch_bounds__(kLocalThreads, kAnyOffset ? (sizeof(T) == 4 ? 2 : 3) : 6) local_exchange_kernel(const __grid_constant__ LocalExchangeArgs a) {
   constexpr int W = 4 * (int)sizeof(T), kPer = 4 / (int)sizeof(T);   // words of a lane, elements of a word
   const int lane = threadIdx.x & 31;
-  const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const uint32_t w = ccb_grid_warp(blockIdx.x, blockDim.x, threadIdx.x);
   if (w >= a.first_run[a.nblocks]) return;
   int b = 0;
   while (w >= a.first_run[b + 1]) ++b;

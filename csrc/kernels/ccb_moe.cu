@@ -240,7 +240,7 @@ __global__ void __launch_bounds__(kMoeLocalThreads, 6) moe_local_dispatch_kernel
 template <class T, class C>
 __global__ void __launch_bounds__(kMoeLocalThreads, sizeof(T) == 4 ? 3 : 5) moe_local_combine_kernel(const __grid_constant__ MoeLocalArgs a) {
   const uint32_t lane = threadIdx.x & 31, upr = a.row_units, per_rank = a.tokens * upr;
-  const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const uint32_t w = ccb_grid_warp(blockIdx.x, blockDim.x, threadIdx.x);
   if (w >= per_rank * (uint32_t)a.n) return;
   const uint32_t r = w / per_rank, u = w - r * per_rank, tok = u / upr;
   const size_t col = (size_t)(u - tok * upr) * kWarpElems + lane * kLaneElems, pair0 = (size_t)tok * a.topk;

@@ -407,3 +407,26 @@ int main(void) {
     out = subprocess.run([str(exe)], capture_output=True, text=True)
     assert out.returncode == 0, out.stdout
     assert int(out.stdout.split()[0]) > 100_000_000
+
+
+def test_warps_of_a_grid_are_numbered_past_two_to_the_27(tmp_path):
+    """csrc/kernels/ccb_grid.h: what the kernels that take a unit a warp find it by, up to the 2^31 units
+    that their launches let through."""
+    import shutil
+    import subprocess
+
+    if not shutil.which("gcc"):
+        pytest.skip("no C compiler")
+    src = tmp_path / "t.c"
+    src.write_text(r'''
+#include "ccb_grid.h"
+int main(void) {
+    for (uint32_t threads = 32; threads <= 256; threads *= 2)
+        for (uint64_t warp = 0; warp < (1ull << 31); warp += warp < 5000 || warp > (1ull << 31) - 5000 || (warp >> 12) == (1u << 15) ? 1 : 4099) {
+            const uint32_t per = threads / 32;
+            if (ccb_grid_warp((uint32_t)(warp / per), threads, (uint32_t)(warp % per) * 32 + 31) != warp) return 1;
+        }
+    return 0;
+}''')
+    subprocess.run(["gcc", "-O2", "-I" + os.path.join(ROOT, "csrc", "kernels"), str(src), "-o", str(tmp_path / "t")], check=True)
+    assert subprocess.run([str(tmp_path / "t")]).returncode == 0
