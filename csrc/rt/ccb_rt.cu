@@ -1413,11 +1413,14 @@ extern "C" int ccb_exchange(ccb_comm* c, const void* const* send, void* const* r
     out[i] = r1 ? span_of(recv[i], r0 * es, r1 * es) : Span{0, 0};
     // a rank's own buffers may meet too, if its own block stays where it is (the calls in place)
     const bool meet = in[i].lo < out[i].hi && out[i].lo < in[i].hi;
-    const Span mine = span_of(send[i], a.send_off[r][r] * es, (a.send_off[r][r] + a.cnt[r][r]) * es);
-    const bool in_place = a.cnt[r][r] && mine.lo == span_of(recv[i], a.recv_off[r][r] * es, 0).lo;
+    const bool in_place = a.cnt[r][r] && span_of(send[i], a.send_off[r][r] * es, 0).lo == span_of(recv[i], a.recv_off[r][r] * es, 0).lo;
     if (a.cnt[r][r] && meet && !in_place) own_direct = false;
-    // without an arena all that this rank sends has to be its own block (an all-gather in place)
-    if (meet && !(in_place && in[i].lo == mine.lo && in[i].hi == mine.hi)) in_registers = false;
+    // Without an arena all that this rank sends has to be its own block, to every rank that gets any (an
+    // all-gather in place): a part of it sent by itself would be read while the block goes through the codec.
+    bool one_block = true;
+    for (int p = 0; p < n; ++p)
+      one_block = one_block && (!a.cnt[r][p] || (a.cnt[r][p] == a.cnt[r][r] && a.send_off[r][p] == a.send_off[r][r]));
+    if (meet && !(in_place && one_block)) in_registers = false;
   }
   const bool apart = ranks_apart(in, out, c->nlocal);
   own_direct = own_direct && apart;

@@ -68,3 +68,25 @@ def test_gathered_blocks_shared_and_moved():
     torch.cuda.synchronize()
     assert torch.equal(buf[0].cpu(), torch.cat([torch.arange(16.0), torch.arange(32.0), torch.arange(48.0, 64.0)]))
     comm.close()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("codec", ["int8", "fp8"])
+@pytest.mark.parametrize("count", [700, 148 * 24 * 512 + 9])   # one CTA; more units than warps at once
+def test_block_in_place_whose_start_is_sent_too(dtype, codec, count):
+    """Every rank's own block stays where it is and goes through the codec there; the others get the
+    first part of it as it was before, its last group by itself."""
+    n, part = 3, count - 70
+    comm = Communicator.local(n, arena_bytes=128 << 20)
+    xs = _inputs(n, count, dtype)
+    counts = [[count if p == r else part for p in range(n)] for r in range(n)]
+    recv_off = [[0 if q == r else count + ((q - r - 1) % n) * part for q in range(n)] for r in range(n)]
+    trip = lambda x: C.roundtrip(x.float(), codec, dtype).to(dtype)
+    for _ in range(4):
+        bufs = [torch.cat([x, torch.zeros((n - 1) * part, dtype=dtype)]).cuda() for x in xs]
+        comm.exchange(bufs, bufs, counts, [[0] * n] * n, recv_off, codec=codec)
+        torch.cuda.synchronize()
+        for r in range(n):
+            want = torch.cat([trip(xs[r])] + [trip(xs[(r + 1 + j) % n][:part]) for j in range(n - 1)])
+            assert torch.equal(bufs[r].cpu(), want), r
+    comm.close()
