@@ -397,7 +397,7 @@ def _check(rc: int) -> None:
         raise CcbError(rc, (lib().ccb_last_error() or b"").decode(errors="replace"))
 
 
-@functools.lru_cache(maxsize=1024)   # the same few sizes come again and again
+@functools.lru_cache(maxsize=1024, typed=True)   # the same few sizes come again and again (typed: 1000.0 stays refused)
 def wire_bytes(codec, dtype: torch.dtype, count: int) -> int:
     return int(lib().ccb_wire_bytes(_code(codec, K.CODECS), _DTYPES[dtype], count))
 

@@ -81,3 +81,13 @@ def test_int4_restatement_properties():
     assert ((x - y).abs() <= 0.5 * step + 1e-7).all()
     assert torch.equal(C.roundtrip(y, "int4"), y)          # idempotent: codes survive a second trip
     assert abs(C.wire_ratio("int4", torch.bfloat16) - 2 / (0.5 + 4 / 128)) < 1e-9
+
+
+def test_wire_bytes_refuses_a_count_that_is_no_integer_after_an_equal_one_too():
+    import ctypes
+
+    from ccbench_b200.comm import wire_bytes
+
+    assert wire_bytes("int8", torch.float32, 1000) > 1000
+    with pytest.raises(ctypes.ArgumentError):
+        wire_bytes("int8", torch.float32, 1000.0)
