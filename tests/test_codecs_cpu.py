@@ -1,4 +1,5 @@
 """CPU checks of the torch restatements of the codecs and algorithms."""
+import pytest
 import torch
 
 from ccbench_b200.ops import codecs as C
