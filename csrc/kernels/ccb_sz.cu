@@ -43,6 +43,8 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include <atomic>
+
 #include <map>
 #include <mutex>
 #include <utility>
@@ -699,8 +701,6 @@ struct SzLocalArgs {
   float eb, two_eb, inv_two_eb;
   unsigned long long magic_x, magic_xy;
 };
-constexpr int kWarpStage = 4096;   // bytes of a packed tile that a warp stages; what is larger is packed a second time, to its place
-
 // How a lane's eight values lie in memory: every line on 32 bytes (kVec 8), on 16 (4), or anywhere
 // (1: a plane goes through shared memory, so that the accesses of a warp lie side by side).
 template <int kVec>
@@ -806,13 +806,14 @@ __device__ __forceinline__ void plane_codes(const float (&x)[8], const SzLocalAr
       bad |= fabsf(__fsub_rn(x[e], __fmul_rn(rf, a.two_eb))) > a.eb;
       q[e] = (int)rf + kCodeBias;
     }
+    bad = __any_sync(0xffffffffu, bad);
   }
 }
 
-// Packs the warp's tile to `pk` (64 width bytes, then the planes). Returns its words and whether it
-// has to be stored raw. Words beyond `room` are counted and not written.
+// Packs the warp's tile to `pk` (64 width bytes, then the planes). Returns its words, or 0 and `bad` as
+// soon as a plane shows that it has to be stored raw.
 template <int kVec>
-__device__ __forceinline__ uint32_t pack_planes(const PlaneIO<kVec>& io, const SzLocalArgs& a, unsigned char* pk, uint32_t room, bool& bad) {
+__device__ __forceinline__ uint32_t pack_planes(const PlaneIO<kVec>& io, const SzLocalArgs& a, unsigned char* pk, bool& bad) {
   const int lane = io.lane;
   uint32_t* words = reinterpret_cast<uint32_t*>(pk + kRows);
   int before[8];
@@ -821,7 +822,7 @@ __device__ __forceinline__ uint32_t pack_planes(const PlaneIO<kVec>& io, const S
   uint32_t run = 0;
   float ahead[8];
   io.load(0, ahead);
-  constexpr int kTurns = kVec == 1 ? 1 : 2;   // with two the form for any line spills (511 x 512 x 512: 282 us, 250 with one)
+  constexpr int kTurns = kVec == 1 ? 1 : 2;   // 300 x 300 x 403, tiles of 7 KB: 120 us with one turn at a time, 124 with two
 #pragma unroll kTurns
   for (int z = 0; z < kTZ; ++z) {
     float x[8];
@@ -831,6 +832,7 @@ __device__ __forceinline__ uint32_t pack_planes(const PlaneIO<kVec>& io, const S
     io.settle(x);
     int q[8], d[8];
     plane_codes(x, a, q, bad);
+    if (bad) return 0;
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
       d[e] = q[e] - before[e];
@@ -868,11 +870,9 @@ __device__ __forceinline__ uint32_t pack_planes(const PlaneIO<kVec>& io, const S
       if (lane < 8) pk[8 * z + lane] = (unsigned char)__popc(((lane < 4 ? W0 : W1) >> (8 * (lane & 3))) & 0xffu);
       tot_lo = __popc(W0);
       tot = tot_lo + __popc(W1);
-      if (run + tot <= room) {
-        const uint32_t below = (1u << lane) - 1u;
-        if ((W0 >> lane) & 1u) words[run + __popc(W0 & below)] = u[0];
-        if ((W1 >> lane) & 1u) words[run + tot_lo + __popc(W1 & below)] = u[1];
-      }
+      const uint32_t below = (1u << lane) - 1u;
+      if ((W0 >> lane) & 1u) words[run + __popc(W0 & below)] = u[0];
+      if ((W1 >> lane) & 1u) words[run + tot_lo + __popc(W1 & below)] = u[1];
     } else {
 #pragma unroll
       for (int e = 0; e < 8; ++e) u[e] = ((uint32_t)d[e] << 1) ^ (uint32_t)(d[e] >> 31);
@@ -885,71 +885,67 @@ __device__ __forceinline__ uint32_t pack_planes(const PlaneIO<kVec>& io, const S
       tot_lo = bytesum(W0);
       tot = tot_lo + bytesum(W1);
       if (lane == 0) reinterpret_cast<uint2*>(pk)[z] = make_uint2(W0, W1);
-      if (run + tot <= room) {
-        uint32_t ua[4] = {u[0], u[1], u[2], u[3]}, ub[4] = {u[4], u[5], u[6], u[7]};
-        wide_planes4<true>(ua, W0, run, words, lane);
-        wide_planes4<true>(ub, W1, run + tot_lo, words, lane);
-      }
+      uint32_t ua[4] = {u[0], u[1], u[2], u[3]}, ub[4] = {u[4], u[5], u[6], u[7]};
+      wide_planes4<true>(ua, W0, run, words, lane);
+      wide_planes4<true>(ub, W1, run + tot_lo, words, lane);
     }
     run += tot;
   }
   const uint32_t pad = (0u - run) & 3u;   // the tile ends on 16 bytes (64 width bytes before the words)
-  if ((uint32_t)lane < pad && run + pad <= room) words[run + lane] = 0u;
+  if ((uint32_t)lane < pad) words[run + lane] = 0u;
   return run;
 }
 
+// A warp stages the whole of its tile, 8256 bytes at most, three CTAs an SM. With 4 KiB each, tiles that
+// were larger went through the codec a second time, to their places: 512^3 values of white noise, bound
+// 1e-5 of their range (2.05 bytes a value) 470 us, 267 so; 1e-6 (3.4 bytes) 440 and 281. Where lines
+// lie anywhere (kVec 1) a plane passes through the last KB of the stage, which only the words of the
+// last plane can reach, after it has passed; three CTAs of 80 registers are the faster ones there too
+// (130 x 201 x 258, bound 1e-4: 24.7 us with four of 64, 22.7 so). A tile that turns out raw is left at
+// that plane and copied (bound 1e-7, all raw: 317 us with all eight planes looked at first, 235 so). B200.
 template <int kVec>
-__global__ void __launch_bounds__(kSzThreads, kVec == 1 ? 4 : 3) sz_pack_kernel(const __grid_constant__ SzLocalArgs a) {
-  __shared__ __align__(16) unsigned char stage[kClusterSize][kWarpStage];
-  __shared__ __align__(16) float plane[kVec == 1 ? kClusterSize : 1][kVec == 1 ? kTX * kTY : 4];
+__global__ void __launch_bounds__(kSzThreads, 3) sz_pack_kernel(const __grid_constant__ SzLocalArgs a) {
+  extern __shared__ __align__(16) unsigned char stages[];   // kClusterSize * kTileCap
   __shared__ uint32_t s_size[kClusterSize];
   const int lane = threadIdx.x & 31, k = threadIdx.x >> 5;
   const unsigned int tile = blockIdx.x * kClusterSize + k;
   char* group = a.slots + (size_t)blockIdx.x * kGroupStride;
-  const PlaneIO<kVec> io(a.in, a, tile_coord(a, tile), plane[kVec == 1 ? k : 0]);
-  unsigned char* pk = stage[k];
-  uint32_t room = (kWarpStage - kRows) / 4;
-  for (bool first = true;; first = false) {   // a second turn for a tile that was too large for its stage: to its place
-    uint32_t size = 0;
-    bool raw = false;
-    if (tile < (unsigned)a.tiles_x * a.tiles_y * a.tiles_z) {
-      bool bad = false;
-      const uint32_t words = pack_planes<kVec>(io, a, pk, room, bad);
-      raw = __any_sync(0xffffffffu, bad);
-      size = raw ? kRows + kTileVals * 4u : (kRows + 4u * words + 15u) & ~15u;
-    }
-    if (!first) return;
-    if (lane == 0) s_size[k] = size;
-    __syncthreads();
-    const uint32_t of = lane < kClusterSize ? s_size[lane] : 0u;
-    const uint32_t off = __reduce_add_sync(0xffffffffu, lane < k ? of : 0u);
-    if (k == 0) {
-      const uint32_t all = __reduce_add_sync(0xffffffffu, of);
-      if (lane < kClusterSize) reinterpret_cast<uint32_t*>(group)[lane] = of;
-      if (lane == 0 && a.used_bytes) atomicAdd(a.used_bytes, (unsigned long long)all);
-    }
-    if (size == 0) return;
-    char* dst = group + kGroupHeader + off;
-    if (!raw && size > (uint32_t)kWarpStage) {
-      pk = reinterpret_cast<unsigned char*>(dst);
-      room = kTileVals;
-      continue;
-    }
-    if (!raw) {
-      for (uint32_t i = lane; i < size / 16; i += 32) stg(dst + 16 * i, reinterpret_cast<const uint4*>(stage[k])[i]);
-      return;
-    }
-    reinterpret_cast<uint16_t*>(dst)[lane] = lane == 0 ? 255 : 0;   // marker, then the fp32 values
-#pragma unroll 1
-    for (int z = 0; z < kTZ; ++z) {
-      float x[8];
-      io.load(z, x);
-      io.settle(x);
-      float4* to = reinterpret_cast<float4*>(dst + kRows) + 2 * (32 * z + lane);
-      to[0] = make_float4(x[0], x[1], x[2], x[3]);
-      to[1] = make_float4(x[4], x[5], x[6], x[7]);
-    }
+  unsigned char* stage = stages + k * kTileCap;
+  const PlaneIO<kVec> io(a.in, a, tile_coord(a, tile), reinterpret_cast<float*>(stage + kTileCap - 4 * kTX * kTY));
+  uint32_t size = 0;
+  bool raw = false;
+  if (tile < (unsigned)a.tiles_x * a.tiles_y * a.tiles_z) {
+    const uint32_t words = pack_planes<kVec>(io, a, stage, raw);
+    size = raw ? kTileCap : (kRows + 4u * words + 15u) & ~15u;
+  }
+  if (lane == 0) s_size[k] = size;
+  __syncthreads();
+  const uint32_t of = lane < kClusterSize ? s_size[lane] : 0u;
+  const uint32_t off = __reduce_add_sync(0xffffffffu, lane < k ? of : 0u);
+  if (k == 0) {
+    const uint32_t all = __reduce_add_sync(0xffffffffu, of);
+    if (lane < kClusterSize) reinterpret_cast<uint32_t*>(group)[lane] = of;
+    if (lane == 0 && a.used_bytes) atomicAdd(a.used_bytes, (unsigned long long)all);
+  }
+  if (size == 0) return;
+  char* dst = group + kGroupHeader + off;
+  if (!raw) {
+    for (uint32_t i = lane; i < size / 16; i += 32) stg(dst + 16 * i, reinterpret_cast<const uint4*>(stage)[i]);
     return;
+  }
+  reinterpret_cast<uint16_t*>(dst)[lane] = lane == 0 ? 255 : 0;   // marker, then the fp32 values
+  float ahead[8];
+  io.load(0, ahead);
+#pragma unroll 2
+  for (int z = 0; z < kTZ; ++z) {
+    float x[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) x[e] = ahead[e];
+    if (z + 1 < kTZ) io.load(z + 1, ahead);
+    io.settle(x);
+    float4* to = reinterpret_cast<float4*>(dst + kRows) + 2 * (32 * z + lane);
+    to[0] = make_float4(x[0], x[1], x[2], x[3]);
+    to[1] = make_float4(x[4], x[5], x[6], x[7]);
   }
 }
 
@@ -1382,6 +1378,20 @@ static int line_width(const void* field, int nx) {
   const uintptr_t at = reinterpret_cast<uintptr_t>(field);
   return nx % 8 == 0 && at % 32 == 0 ? 8 : nx % 4 == 0 && at % 16 == 0 ? 4 : 1;
 }
+// More shared memory than a kernel may have unasked: allowed once for each device.
+template <int kVec>
+static void launch_pack(const SzLocalArgs& a, cudaStream_t stream) {
+  constexpr int kBytes = kClusterSize * kTileCap;
+  static std::atomic<uint64_t> allowed{0};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  const uint64_t bit = dev >= 0 && dev < 64 ? 1ull << dev : 0ull;
+  if (!(allowed.load(std::memory_order_relaxed) & bit)) {
+    if (cudaFuncSetAttribute(sz_pack_kernel<kVec>, cudaFuncAttributeMaxDynamicSharedMemorySize, kBytes) == cudaSuccess)
+      allowed.fetch_or(bit, std::memory_order_relaxed);
+  }
+  sz_pack_kernel<kVec><<<a.ngroups, kSzThreads, kBytes, stream>>>(a);
+}
 static int launched(const char* what) {
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {
@@ -1420,9 +1430,9 @@ extern "C" int ccb_sz_compress(const float* in, int nx, int ny, int nz, float eb
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (d_used) cudaMemsetAsync(d_used, 0, sizeof(unsigned long long), s);
   switch (line_width(in, nx)) {
-    case 8: sz_pack_kernel<8><<<a.ngroups, kSzThreads, 0, s>>>(a); break;
-    case 4: sz_pack_kernel<4><<<a.ngroups, kSzThreads, 0, s>>>(a); break;
-    default: sz_pack_kernel<1><<<a.ngroups, kSzThreads, 0, s>>>(a);
+    case 8: launch_pack<8>(a, s); break;
+    case 4: launch_pack<4>(a, s); break;
+    default: launch_pack<1>(a, s);
   }
   return launched("ccb_sz_compress");
 }

@@ -1,6 +1,6 @@
 """The error-bounded codec where its accesses to a field change: lines on 32 bytes, on 16 and anywhere
 (extents and a start of the buffer that allow no wider), tiles cut off in each direction, and packed
-tiles from a few bytes to more than a warp stages (4 KiB), against the host codec byte for byte."""
+tiles from a few bytes to the largest that a warp stages (8256), against the host codec byte for byte."""
 import numpy as np
 import pytest
 import torch
@@ -126,3 +126,14 @@ def test_container_with_damaged_tile_sizes_is_refused_on_the_device(start, word,
     moved[at:at + 4].view(torch.int32).add_(change)
     with pytest.raises(ValueError):
         sz.from_container(moved)
+
+
+@pytest.mark.parametrize("nx", [64, 68, 65])
+@pytest.mark.parametrize("z", [0, 1, 6, 7])
+def test_tile_that_turns_out_raw_at_any_plane(nx, z):
+    field = torch.randn(8, 8, nx, generator=torch.Generator().manual_seed(z)) * 1e4   # rows of about 22 bits before it
+    field[z, 5, 37] = float("nan")
+    buf, _ = sz.compress(field.cuda(), 1e-2)
+    want = sz.encode_cpu(field.numpy(), 1e-2)
+    assert np.array_equal(sz.to_container(buf, field.shape, 1e-2).cpu().numpy(), want)
+    assert np.array_equal(sz.decompress(buf, field.shape, 1e-2).cpu().numpy(), sz.decode_cpu(want), equal_nan=True)
