@@ -344,7 +344,8 @@ __device__ __forceinline__ uint32_t pack_tile(float* vals, unsigned char* pk, in
 // fields, B200: raw tiles only 407 us, packed tiles only 324; with a scratch for every tile and a
 // barrier in the raw ones it was 432 and 321.) A tile whose widths cannot be (or `sound` false: whose
 // place cannot) becomes NaN, without an access through its words.
-__device__ __forceinline__ void unpack_tile(const unsigned char* src, bool sound, int* qs2, int& scratch, const SzArgs& a, float* out, const TileCoord& t) {
+template <class Args>
+__device__ __forceinline__ void unpack_tile(const unsigned char* src, bool sound, int* qs2, int& scratch, const Args& a, float* out, const TileCoord& t) {
   const int lane = threadIdx.x & 31, z = threadIdx.x >> 5;
   // the 16 words of row widths, one per lane, and their running word count
   const uint32_t hw = sound && lane < 16 ? ldg_cg_u32(src + 4 * lane) : 0u;
@@ -1106,6 +1107,17 @@ __global__ void __launch_bounds__(kSzThreads, kVec == 1 ? 4 : 5) sz_unpack_kerne
   }
 }
 
+// A field of few tiles leaves most of the chip idle with a warp a tile, and what counts is how long a
+// tile takes: here a CTA a tile, a plane a warp (unpack_tile), six CTAs an SM.
+__global__ void __launch_bounds__(kSzThreads, 6) sz_unpack_few_kernel(const __grid_constant__ SzLocalArgs a) {
+  __shared__ __align__(16) int codes[kTileVals];
+  const unsigned int k = blockIdx.x % kClusterSize, lane = threadIdx.x & 31;
+  const char* group = a.slots + (size_t)(blockIdx.x / kClusterSize) * kGroupStride;
+  const uint32_t off = __reduce_add_sync(0xffffffffu, lane < k ? ldg_cg_u32(group + 4 * lane) : 0u);
+  int scratch = 1;
+  unpack_tile(reinterpret_cast<const unsigned char*>(group) + kGroupHeader + off, ccb_sz_offset_ok(off, k), codes, scratch, a, a.out, tile_coord(a, blockIdx.x));
+}
+
 // ----------------------------------------------------------------- container ----
 // The contiguous form of a compressed field: [40-byte header][u32 used bytes of each group]
 // [the used bytes of every group]. Packing and unpacking are a scan over the groups' sizes and
@@ -1392,6 +1404,12 @@ static void launch_pack(const SzLocalArgs& a, cudaStream_t stream) {
   }
   sz_pack_kernel<kVec><<<a.ngroups, kSzThreads, kBytes, stream>>>(a);
 }
+// Tiles up to which a CTA a tile unpacks a field faster than a warp a tile, us, CTA / warp, B200. Lines on
+// 16 bytes: 64^3 (128 tiles) 7.5 / 7.5 to 12.4 by the widths of its rows, 128 x 128 x 256 (2048) 10.4 /
+// 10.3 at 0.75 bytes a value, 12.4 / 16.5 at 2; 160 x 160 x 256 (3200) 14.5 / 12.4 and 16.5 / 18.6.
+// Lines anywhere: 130 x 201 x 258 (3978) 16.5 / 18.6 and 20.6 / 27, 176 x 200 x 258 (4950) 20.6 / 22.7
+// and 24.7 / 30.9, 256 x 256 x 257 (9216) 35 / 33 and 43 / 48.
+static unsigned int few_tiles(int width) { return width == 1 ? 5120u : 2560u; }
 static int launched(const char* what) {
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {
@@ -1448,7 +1466,13 @@ extern "C" int ccb_sz_decompress(const void* in, int nx, int ny, int nz, float e
   a.out = out;
   a.slots = const_cast<char*>(static_cast<const char*>(in));
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  switch (line_width(out, nx)) {
+  const unsigned int ntiles = (unsigned)a.tiles_x * a.tiles_y * a.tiles_z;
+  const int width = line_width(out, nx);
+  if (ntiles <= few_tiles(width)) {
+    sz_unpack_few_kernel<<<ntiles, kSzThreads, 0, s>>>(a);
+    return launched("ccb_sz_decompress");
+  }
+  switch (width) {
     case 8: sz_unpack_kernel<8><<<a.ngroups, kSzThreads, 0, s>>>(a); break;
     case 4: sz_unpack_kernel<4><<<a.ngroups, kSzThreads, 0, s>>>(a); break;
     default: sz_unpack_kernel<1><<<a.ngroups, kSzThreads, 0, s>>>(a);

@@ -68,7 +68,7 @@ def test_packed_and_raw_tiles_from_a_buffer_on_four_bytes(start):
     assert torch.equal(sz.decompress(moved, shape, eb), sz.decompress(buf, shape, eb))
 
 
-@pytest.mark.parametrize("shape", [(17, 20, 96), (9, 9, 258)])
+@pytest.mark.parametrize("shape", [(17, 20, 96), (9, 9, 258), (9, 9, 32 * 1300), (9, 9, 32 * 1300 + 5)])   # a CTA a tile, a warp a tile
 @pytest.mark.parametrize("word,value", [(0, 8 * 8256), (1, 12), (2, 1 << 31), (6, 7), (3, 0xfffffff0)])
 def test_damaged_tile_sizes_stay_inside_the_slot(shape, word, value):
     """A size word that puts the tiles behind it where none can lie: those become NaN, the rest stay."""
@@ -91,24 +91,29 @@ def test_damaged_tile_sizes_stay_inside_the_slot(shape, word, value):
         z, y, x = 8 * (t // (tx * ty)), 8 * (t // tx % ty), 32 * (t % tx)
         box = (slice(z, z + 8), slice(y, y + 8), slice(x, x + 32))
         k = t % 8
-        if t < 8 * group or k <= word:
+        if t < 8 * group:
+            continue
+        if k <= word:
             assert torch.equal(got[box], want[box]), t
         elif off > k * sz.TILE_CAP or off % 16:
             assert got[box].isnan().all(), t
-        off = (0 if k == 7 else off + words[k]) & 0xffffffff if t >= 8 * group else 0
+        got[box] = want[box]
+        off = (off + words[k]) & 0xffffffff
+    assert torch.equal(got, want)   # the groups before
 
 
 @pytest.mark.parametrize("row", [0, 1, 31, 63])
 @pytest.mark.parametrize("width", [33, 128, 254])
-def test_damaged_row_widths_make_their_tile_nan(row, width):
-    shape, eb = (8, 8, 64), 1e-2
+@pytest.mark.parametrize("nx", [64, 32 * 5200, 32 * 5200 - 3])
+def test_damaged_row_widths_make_their_tile_nan(row, width, nx):
+    shape, eb = (8, 8, nx), 1e-2
     field = torch.randn(shape, generator=torch.Generator().manual_seed(4)).cuda()
     buf, _ = sz.compress(field, eb)
     want = sz.decompress(buf, shape, eb)
     first = int(buf[:4].view(torch.int32))
     buf[sz.GROUP_HEADER + first + row] = width
     got = sz.decompress(buf, shape, eb)
-    assert torch.equal(got[..., :32], want[..., :32]) and got[..., 32:].isnan().all()
+    assert torch.equal(got[..., :32], want[..., :32]) and got[..., 32:64].isnan().all() and torch.equal(got[..., 64:], want[..., 64:])
 
 
 @pytest.mark.parametrize("start", [0, 4])
@@ -137,3 +142,26 @@ def test_tile_that_turns_out_raw_at_any_plane(nx, z):
     want = sz.encode_cpu(field.numpy(), 1e-2)
     assert np.array_equal(sz.to_container(buf, field.shape, 1e-2).cpu().numpy(), want)
     assert np.array_equal(sz.decompress(buf, field.shape, 1e-2).cpu().numpy(), sz.decode_cpu(want), equal_nan=True)
+
+
+@pytest.mark.parametrize("ny", [8, 11])
+@pytest.mark.parametrize("tail", [0, 8, 12, 31])   # lines on 32 bytes, on 16 and anywhere
+@pytest.mark.parametrize("scale", [1e-3, 1.0, 400.0, 1e5])
+@pytest.mark.parametrize("start", [0, 4])
+def test_many_tiles_are_unpacked_as_few_are(ny, tail, scale, start):
+    """A field that repeats a small one along x: more tiles than the kernel for few takes, each the tile
+    of the small field (whose values are held against the host codec above). The last column is cut off."""
+    nz, period, eb = 9, 64, 1e-2
+    base = torch.randn((nz, ny, period), generator=torch.Generator().manual_seed(ny + tail)) * scale
+    base[:8, :8, 32:] *= 1e-2
+    base[8, 5, 40] = 1e30   # a raw tile
+    repeats = 5200 // (2 * -(-nz // 8) * -(-ny // 8)) + 1
+    field = torch.cat([base.repeat(1, 1, repeats), base[..., :tail]], -1).cuda()
+    got_base = sz.decompress(sz.compress(base.cuda(), eb)[0], base.shape, eb)
+    want = [got_base.repeat(1, 1, repeats)]
+    if tail:
+        want.append(sz.decompress(sz.compress(base[..., :tail].contiguous().cuda(), eb)[0], (nz, ny, tail), eb))
+    buf, _ = sz.compress(field.contiguous(), eb)
+    moved = torch.empty(buf.numel() + start, dtype=torch.uint8, device="cuda")[start:]
+    moved.copy_(buf)
+    assert torch.equal(sz.decompress(moved, field.shape, eb), torch.cat(want, -1))
