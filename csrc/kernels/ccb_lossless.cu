@@ -42,7 +42,7 @@ constexpr int kLlBlocksPerTile = kLlThreads / 32;          // 8
 constexpr int kLlTileElems = kLlBlocksPerTile * kWarpElems;  // 4096
 constexpr uint32_t kLlMagic = 0x4C424343u;                 // "CCBL"
 constexpr int kLlHeader = 32;
-constexpr int kLlCtas = 4;   // resident on an SM, and launched: each takes its tiles in turn
+constexpr int kLlCtas = 4;   // resident on an SM
 
 template <class T> struct LlTraits;
 template <> struct LlTraits<float> {
@@ -135,16 +135,17 @@ __device__ __forceinline__ void pairs_of_planes(const uint32_t (&u)[4], uint32_t
   }
 }
 
-// Both directions were bound by the pipe of the logical and byte operations (encoding 85 % busy, ncu),
-// and work on four values at a time as far as they can: the exponents and the bytes of sign and
-// mantissa of four values are one word each. A tile's values are requested while the tile before is
-// packed, and one barrier per tile passes the widths round. The decoder has the planes of the next
-// tile and the head of the one after on their way. 32 Mi bf16 values, encoding and decoding: 29.2 and
-// 27.5 us with two values at a time and four transposes a block, 24.9 and 24.7 so; 16 Mi fp32 values
-// 22.0 and 20.7. (B200; the memory needs 18 and 19 us at 6.55 TB/s. Five or six resident CTAs, with
-// the fewer registers that leaves them, are slower: fp32 24 and 28 us, 33 and 33.)
+// Both directions are bound by the pipe of the logical and byte operations or by their memory, and work
+// on four values at a time as far as they can: the exponents and the bytes of sign and mantissa of four
+// values are one word each. A tile's values are requested while the tile before is packed, and one
+// barrier per tile passes the widths round. The decoder has the planes of the next tile and the head of
+// the one after on their way; adding to fp32 values it has no registers for that (a 4 MiB chunk 5.2 us
+// with, 4.4 without). 32 Mi bf16 values, encoding and decoding: 23.1 and 22.6 us (27.2 and 28.7 with two
+// values at a time and four transposes a block); 32 Mi fp32 values 42.3 and 40.9. The memory needs 18
+// and 38 each way. An fp32 encoder with 64 registers for a fourth CTA takes 43.3 us, on random bits 48 instead
+// of 44; five or six CTAs of any kind are slower. (B200.)
 template <class T>
-__global__ void __launch_bounds__(kLlThreads, kLlCtas) lossless_encode_kernel(const T* __restrict__ in, size_t count, char* out, size_t ntiles) {
+__global__ void __launch_bounds__(kLlThreads, sizeof(T) == 4 ? 3 : kLlCtas) lossless_encode_kernel(const T* __restrict__ in, size_t count, char* out, size_t ntiles) {
   using Tr = LlTraits<T>;
   __shared__ uint2 info[2][kLlBlocksPerTile];   // (width, minimum) of each block, by parity of the tile
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -284,18 +285,26 @@ __global__ void __launch_bounds__(kLlThreads, kLlCtas) lossless_decode_kernel(co
   };
   size_t t = blockIdx.x;
   if (!mine(t)) return;   // only the last tile has blocks that hold nothing
+  constexpr bool kAhead = sizeof(T) == 2 || MODE == 0;
   Head head = head_of(t);
-  Body next = body_of(t, head);
-  if (mine(t + gridDim.x)) head = head_of(t + gridDim.x);
+  Body next;
+  if (kAhead) {
+    next = body_of(t, head);
+    if (mine(t + gridDim.x)) head = head_of(t + gridDim.x);
+  }
   for (;;) {
+    if (!kAhead) next = body_of(t, head);
     const Body b = next;
     const size_t idx = t * kLlTileElems + (size_t)warp * kWarpElems + (size_t)lane * kLaneElems;
     t += gridDim.x;
     const bool more = mine(t);
-    if (more) {
+    if (kAhead && more) {
       next = body_of(t, head);
       if (mine(t + gridDim.x)) head = head_of(t + gridDim.x);
     }
+    if (!kAhead && more) head = head_of(t);
+    [[maybe_unused]] Wide16<T> have;
+    if constexpr (MODE == 1 && sizeof(T) == 2) load16_wide<T>(out, idx, count, have);
     uint32_t u[4];
     values_of_planes(b.planes, u, b.w, lane);
     Wide16<T> raw;
@@ -334,8 +343,7 @@ __global__ void __launch_bounds__(kLlThreads, kLlCtas) lossless_decode_kernel(co
       }
     }
     if constexpr (MODE == 1) {
-      Wide16<T> have;
-      load16_wide<T>(out, idx, count, have);
+      if constexpr (sizeof(T) == 4) load16_wide<T>(out, idx, count, have);
       float x[16], y[16];
       wide16_to_f<T>(raw, x);
       wide16_to_f<T>(have, y);
@@ -351,10 +359,13 @@ __global__ void __launch_bounds__(kLlThreads, kLlCtas) lossless_decode_kernel(co
 
 static size_t ll_tiles(size_t count) { return (count + kLlTileElems - 1) / kLlTileElems; }
 static size_t ll_slot(int dtype) { return dtype == CCB_F32 ? ll_slot_bytes<float>() : ll_slot_bytes<__half>(); }
-static int ll_grid(size_t ntiles) {
-  const int sms = sm_count();
-  const size_t cap = (size_t)sms * kLlCtas;
-  return (int)(ntiles < cap ? (ntiles ? ntiles : 1) : cap);
+// Up to eight tiles an SM each has a CTA. Beyond that CTAs take several in turn, in grids of as many an
+// SM as were fastest of 4, 8 and 16 (32 Mi values encoded / decoded, us: bf16 23.1 / 22.6, 23.1 / 22.8 and
+// 24.7 / 24.6; f16 31.4 / 30.6, 30.8 / 28.8, 30.8 / 30.0; fp32 46.9 / 44.5, 43.3 / 41.1, 42.3 / 40.9): what
+// a first tile costs against a last turn that only some have. B200.
+static int ll_grid(size_t ntiles, int dtype) {
+  const size_t sms = (size_t)sm_count(), cap = sms * (dtype == CCB_F32 ? 16 : dtype == CCB_F16 ? 8 : 4);
+  return (int)(ntiles == 0 ? 1 : ntiles <= 8 * sms || ntiles < cap ? ntiles : cap);
 }
 
 }  // namespace ccb
@@ -380,7 +391,7 @@ extern "C" int ccb_lossless_encode(int dtype, const void* in, uint64_t count, vo
     return CCB_ERR_CUDA;
   }
   const size_t nt = ll_tiles(count);
-  const int g = ll_grid(nt);
+  const int g = ll_grid(nt, dtype);
   if (dtype == CCB_F32) lossless_encode_kernel<float><<<g, kLlThreads, 0, s>>>((const float*)in, count, (char*)out, nt);
   else if (dtype == CCB_BF16) lossless_encode_kernel<__nv_bfloat16><<<g, kLlThreads, 0, s>>>((const __nv_bfloat16*)in, count, (char*)out, nt);
   else lossless_encode_kernel<__half><<<g, kLlThreads, 0, s>>>((const __half*)in, count, (char*)out, nt);
@@ -401,7 +412,7 @@ extern "C" int ccb_lossless_decode(int dtype, const void* in, uint64_t count, vo
   const size_t nt = ll_tiles(count);
   if (nt == 0) return CCB_OK;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  const int g = ll_grid(nt);
+  const int g = ll_grid(nt, dtype);
 #define CCB_LL_DEC(T)                                                                                          \
   do {                                                                                                         \
     if (accumulate) lossless_decode_kernel<T, 1><<<g, kLlThreads, 0, s>>>((const char*)in, count, (T*)out, nt); \
