@@ -216,7 +216,7 @@ struct CodecInt4 {
 #pragma unroll
     for (int i = 0; i < 16; ++i) v[i] = (float)((int)(w[i >> 3] << (28 - 4 * (i & 7))) >> 28) * pk.scale;
   }
-  // v - decode(pk) in one rounding, as the product and the difference come out where nothing else uses the product.
+  // v - decode(pk) in one rounding.
   static __device__ __forceinline__ void residual(const Packet& pk, const float (&v)[16], float (&e)[16]) {
     const uint32_t w[2] = {pk.q.x, pk.q.y};
 #pragma unroll
@@ -240,6 +240,19 @@ struct CodecInt4 {
     if ((threadIdx.x & (kLanes - 1)) == 0) mc_st4(slot + pad / 2 + (idx / kGroup) * 4, __float_as_uint(pk.scale));
   }
 };
+
+// What a sender's residual is where it does not need the decoded packet for anything else. (Where it
+// does, the residual is the difference to those values.)
+template <class C>
+__device__ __forceinline__ void residual_of_sent(const typename C::Packet& pk, const float (&v)[16], float (&e)[16]) {
+  if constexpr (C::kId == CCB_CODEC_INT4) {
+    C::residual(pk, v, e);
+  } else {
+    C::decode(pk, e);
+#pragma unroll
+    for (int i = 0; i < 16; ++i) e[i] = __fsub_rn(v[i], e[i]);
+  }
+}
 
 struct CodecFp8 {
   static constexpr int kId = CCB_CODEC_FP8;

@@ -532,7 +532,7 @@ __device__ __forceinline__ float apply_op(int op, float a, float b) {
     case CCB_OP_PROD: return a * b;
     case CCB_OP_MAX: return fmaxf(a, b);
     case CCB_OP_MIN: return fminf(a, b);
-    default: return a + b;
+    default: return __fadd_rn(a, b);   // never fused with a decoder's product
   }
 }
 

@@ -129,7 +129,7 @@ __device__ __forceinline__ void combine16(int op, float (&a)[16], const float (&
 }
 
 // v becomes what a receiver of the packet decodes; with a residual, v - that is kept for the next call.
-// kSentOnly: the kernels over peer memory decode this packet for the residual alone (see CodecInt4::residual).
+// kSentOnly: where the kernels over peer memory decode this packet for the residual alone (see residual_of_sent).
 template <class C, bool kEf, bool kAnyOffset = false, bool kSentOnly = false>
 __device__ __forceinline__ void through_codec(float (&v)[16], float* ef, size_t idx, size_t limit, bool inside) {
   if constexpr (!kEf) {

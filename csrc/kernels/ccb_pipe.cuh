@@ -225,7 +225,7 @@ __global__ void __launch_bounds__(kPipeThreads, 1) pipe_kernel(const __grid_cons
   auto accumulate = [&](float (&acc)[16], const float (&d)[16]) {
     if (sum) {
 #pragma unroll
-      for (int k = 0; k < 16; ++k) acc[k] += d[k];
+      for (int k = 0; k < 16; ++k) acc[k] = __fadd_rn(acc[k], d[k]);
     } else {
 #pragma unroll
       for (int k = 0; k < 16; ++k) acc[k] = apply_op(a.op, acc[k], d[k]);
@@ -266,9 +266,7 @@ __global__ void __launch_bounds__(kPipeThreads, 1) pipe_kernel(const __grid_cons
         C::store(dst, pad, idx, pk);
         if (efs) {
           float d[16];
-          C::decode(pk, d);
-#pragma unroll
-          for (int q = 0; q < 16; ++q) d[q] = v[q] - d[q];
+          residual_of_sent<C>(pk, v, d);
           store16f_plain(efs, idx, valid, d);
         }
       }
@@ -323,7 +321,7 @@ __global__ void __launch_bounds__(kPipeThreads, 1) pipe_kernel(const __grid_cons
       if (efs) {
         float e[16];
 #pragma unroll
-        for (int k = 0; k < 16; ++k) e[k] = acc[k] - d[k];
+        for (int k = 0; k < 16; ++k) e[k] = __fsub_rn(acc[k], d[k]);
         store16f_plain(efs, idx, valid, e);
       }
       store16<T>(out, idx, valid, d);

@@ -133,9 +133,7 @@ __global__ void __launch_bounds__(kThreads, 2) reduce_kernel(const __grid_consta
       }
       if (ef) {
         float d[16];
-        C::decode(pk, d);
-#pragma unroll
-        for (int i = 0; i < 16; ++i) d[i] = v[i] - d[i];
+        residual_of_sent<C>(pk, v, d);
         store16f_plain(ef, idx, a.count, d);
       }
     }
@@ -231,9 +229,7 @@ __global__ void __launch_bounds__(kThreads, 2) reduce_kernel(const __grid_consta
             C::store(dst, pad, idx, pk);
             if (efs) {
               float d[16];
-              C::decode(pk, d);
-#pragma unroll
-              for (int i = 0; i < 16; ++i) d[i] = v[i] - d[i];
+              residual_of_sent<C>(pk, v, d);
               store16f_plain(efs, idx, valid, d);
             }
           }
@@ -287,7 +283,7 @@ __global__ void __launch_bounds__(kThreads, 2) reduce_kernel(const __grid_consta
           if (efs) {
             float e[16];
 #pragma unroll
-            for (int i = 0; i < 16; ++i) e[i] = acc[i] - d[i];
+            for (int i = 0; i < 16; ++i) e[i] = __fsub_rn(acc[i], d[i]);
             store16f_plain(efs, idx, valid, e);
           }
           store16<T>(recv + (size_t)s * a.shard_elems, idx, valid, d);
@@ -384,7 +380,7 @@ __global__ void __launch_bounds__(kAny ? (kEf || sizeof(T) == 4 ? 768 : 640) : k
     store16_wide<T>(recv, idx, count, d);
     if constexpr (kEf) {
 #pragma unroll
-      for (int i = 0; i < 16; ++i) d[i] = v[i] - d[i];
+      for (int i = 0; i < 16; ++i) d[i] = __fsub_rn(v[i], d[i]);
       store16_wide<float>(ef, idx, count, d);
     }
   }

@@ -100,7 +100,7 @@ __global__ void __launch_bounds__(kThreads, 2) ring_kernel(const __grid_constant
         if (last) store16<T>(recv + (size_t)cs * a.shard_elems, idx, valid, d);
         if (efs) {
 #pragma unroll
-          for (int i = 0; i < 16; ++i) d[i] = v[i] - d[i];
+          for (int i = 0; i < 16; ++i) d[i] = __fsub_rn(v[i], d[i]);
           store16f_plain(efs, idx, valid, d);
         }
       }
@@ -214,7 +214,7 @@ __global__ void __launch_bounds__(kThreads, 2) tree_kernel(const __grid_constant
       if (!parent) store16<T>(recv, idx, valid, d);
       if (ef) {
 #pragma unroll
-        for (int i = 0; i < 16; ++i) d[i] = v[i] - d[i];
+        for (int i = 0; i < 16; ++i) d[i] = __fsub_rn(v[i], d[i]);
         store16f_plain(ef, idx, valid, d);
       }
     }
