@@ -1,7 +1,8 @@
 """Numerics of the fused collective kernels against plain PyTorch fp32 restatements.
 
-All ranks are played on ONE GPU by a single cooperative launch
-(`Communicator.local`), so the full flag protocol runs on a one-GPU box."""
+All ranks are played on ONE GPU (`Communicator.local`), whose collectives run in registers; what is
+named _over_the_arena asks for the kernels of ranks on several GPUs, with their flags, and
+test_local_gpu.py holds those against the ones in registers bit for bit."""
 import pytest
 import torch
 
@@ -227,6 +228,19 @@ def test_large_message_is_sliced(comms):
     torch.cuda.synchronize()
     assert comm.status()[0] == 0
     assert xg[0][::4097].eq(3.0).all() and xg[1][-5:].eq(3.0).all()
+
+
+def test_large_message_is_sliced_over_the_arena(comms):
+    n = 2
+    comm = comms(n)
+    count = 40 << 20
+    xg = [torch.full((count,), float(r + 1), device="cuda") for r in range(n)]
+    comm.set_trace(True)
+    comm.all_reduce(xg, codec="none", algo="twoshot")
+    comm.set_trace(False)
+    torch.cuda.synchronize()
+    assert comm.status()[0] == 0
+    assert xg[0].eq(3.0).all() and xg[1].eq(3.0).all()
 
 
 def test_wait_timeout_reports_status_and_leaves_the_context_usable():

@@ -7,6 +7,7 @@ import pytest
 import torch
 
 from ccbench_b200 import Communicator
+from ccbench_b200.comm import launch_count
 from ccbench_b200.parallel import moe
 
 pytestmark = pytest.mark.gpu
@@ -254,6 +255,50 @@ def test_moe_with_dropped_pairs(codec, n, tokens, hidden, topk):
             for o, x, gate in zip(out, xs, gates):
                 assert ((o.float() - x.float() * gate).abs() <= 2.0 ** -8 * (x.float() * gate).abs() + 1e-30).all()
         return recv + out
+
+    _both(comm, call)
+    comm.close()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("codec", ["none", "int8", "int4"])
+@pytest.mark.parametrize("algo", ["oneshot", "twoshot", "ring", "tree"])
+@pytest.mark.parametrize("ef", [False, True])
+def test_messages_cut_to_a_small_arena(dtype, codec, algo, ef):
+    """Several launches a call: the halves of the arena and the flag rows taken in turn, residuals and
+    results at the slices' places. (An arena of 4 MiB, half of it for a call; these messages would need 2.8 MB and more.)"""
+    n, count = 3, 4_000_003
+    comm = Communicator.local(n, arena_bytes=4 << 20)
+    xs = [_values(count, dtype, r + n) for r in range(n)]
+
+    def call():
+        before = launch_count()
+        res = [torch.linspace(-1, 1, count, device="cuda") * (r + 1) for r in range(n)] if ef else None
+        out = [torch.empty_like(x) for x in xs]
+        for _ in range(2):
+            comm.all_reduce(xs, out, codec=codec, algo=algo, error_feedback=res)
+        assert launch_count() - before >= 4
+        return out + (res or [])
+
+    _both(comm, call)
+    comm.close()
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("n", [2, 5])
+@pytest.mark.parametrize("overlap", [False, True])
+def test_one_shot_that_reads_its_own_values_again(dtype, n, overlap):
+    """From 8 MiB over the ranks played a rank's own uncompressed values are read from `send` and not
+    from its arena, unless another rank's result lies there."""
+    count = (8 << 20) // n // torch.empty((), dtype=dtype).element_size() + 700
+    comm = Communicator.local(n, arena_bytes=160 << 20)
+    xs = [_values(count, dtype, r + n) for r in range(n)]
+
+    def call():
+        bufs = [x.clone() for x in xs]
+        out = bufs[1:] + bufs[:1] if overlap else [torch.empty_like(x) for x in xs]
+        comm.all_reduce(bufs, out, codec="none", algo="oneshot")
+        return out + bufs
 
     _both(comm, call)
     comm.close()

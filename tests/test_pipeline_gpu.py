@@ -1,7 +1,7 @@
 """The warp-specialised pipelined two-shot kernel against the plain two-shot kernel and the
-PyTorch restatement. Both kernels do the same arithmetic in the same order; the compiler
-contracts multiply-add pairs differently in the two, so results agree to the last bits of
-fp32, and an occasional code lands on the other side of a rounding boundary. The pipelined
+PyTorch restatement. Both kernels do the same arithmetic in the same order, each rounding of a
+codec's products, sums and residuals written down; the bounds here leave room for sums in another
+order, which moves an occasional code across a rounding boundary. The pipelined
 kernel is forced on (mode 2) so that small, odd-sized messages exercise partial chunks,
 empty waves and every role split."""
 import pytest
