@@ -34,7 +34,8 @@ struct LocalReduceArgs {
 };
 
 // Ranks whose values are requested before the first is used, and CTAs of 256 threads on an SM: what
-// was fastest of one, two and four ranks at 40 to 128 registers a thread, where nothing spills.
+// was fastest of one, two and four ranks at 40 to 128 registers a thread. (At these nothing spills but 4
+// to 8 bytes in one-shots and trees of 16-bit types.)
 // (B200. 4 ranks of 64 MiB of bf16, two-shot int8: two ranks at 64 registers 82.4 us, at 48, which
 // spill, 105, four at 80 123. 8 ranks of 25 MiB to their owners: 43.3; one rank at 48 53. Shards at
 // odd places: one at 64 registers 66, two 70. 2 ranks of 5,000,011 fp32 values: one at 64 10.5, two

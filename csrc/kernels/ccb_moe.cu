@@ -234,8 +234,9 @@ __global__ void __launch_bounds__(kMoeLocalThreads, 6) moe_local_dispatch_kernel
 
 // Combine: a warp takes 512 elements of one token and fetches them from the topk rows that hold it, one
 // after the other: what a warp waits for in turn, indices and rows, is hidden by as many warps as fit.
-// (8 ranks, 8192 x 4096 bf16, top 2, fp8: 323 us with 40 warps an SM; 337 with two rows at once and 32
-// warps, 380 with two and 24. Top 4 of 2048 x 2048 80 and 79, top 1 33 and 41. B200.)
+// (8 ranks, 8192 x 4096 bf16, top 2, fp8: 323 us with 40 warps an SM, whose 48 registers spill 32 to 44
+// bytes but for no codec; 337 with two rows at once and 32 warps, 380 with two and 24. Top 4 of 2048 x
+// 2048 80 and 79, top 1 33 and 41. B200.)
 // An index outside its block (the entry of a dropped pair) contributes nothing.
 template <class T, class C>
 __global__ void __launch_bounds__(kMoeLocalThreads, sizeof(T) == 4 ? 3 : 5) moe_local_combine_kernel(const __grid_constant__ MoeLocalArgs a) {

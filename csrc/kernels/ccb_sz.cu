@@ -26,7 +26,8 @@
 // bytes are ever written (and cross NVLink).
 //
 // Kernel shapes: local buffers (ccb_sz_compress, ccb_sz_decompress) take a CTA a group, a
-// warp a tile (sz_pack_kernel, sz_unpack_kernel). The collectives take one thread-block
+// warp a tile (sz_pack_kernel, sz_unpack_kernel; fields of few tiles are unpacked by a CTA a
+// tile, sz_unpack_few_kernel). The collectives take one thread-block
 // cluster of 8 CTAs per group: each CTA fetches its tile with ONE 3-D TMA copy
 // (cp.async.bulk.tensor, no multicast) tracked by an mbarrier, packs it in shared memory,
 // the cluster exchanges the 8 sizes through distributed shared memory to place the tiles
@@ -687,11 +688,11 @@ __global__ void __cluster_dims__(kClusterSize, 1, 1) __launch_bounds__(kSzThread
 // before stays in its registers, y and x neighbours come by shuffles, and the words of a plane go
 // behind those of the plane before. So nothing of a tile is exchanged between warps, there is one
 // barrier a GROUP (a CTA of eight warps), for the tiles' sizes, and no cluster. Both directions are
-// bound by instructions (packing: the pipe of logical operations 69 % busy, 84 % of the issue slots)
-// and the latency of a tile's first loads. (512^3 field, bound 1e-4 of its range, B200: packing 181 us
-// and unpacking 162; with a CTA a tile, its planes on eight warps, three barriers a tile and the sizes
-// sent round a cluster it was 332 and 279. Packing with 64 registers instead of 80 187 us, unpacking
-// with 64 instead of 48 170.)
+// bound by instructions (ncu, 384^3: packing keeps the pipe of logical operations 61 % busy and 76 % of
+// the issue slots, unpacking 76 % and 76 %) and the latency of a tile's first loads. (512^3 field, bound
+// 1e-4 of its range, B200: packing 177 us and unpacking 163; with a CTA a tile, its planes on eight
+// warps, three barriers a tile and the sizes sent round a cluster it was 332 and 279. Packing with 64
+// registers instead of 80 took 6 us more, unpacking with 64 instead of 48 8.)
 struct SzLocalArgs {
   const float* in;
   float* out;
