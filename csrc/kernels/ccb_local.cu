@@ -57,6 +57,9 @@ static bool reduce_aligned(const ReduceArgs& r, size_t es, bool* ef) {
   return aligned;
 }
 
+// Residuals want every buffer on 32 bytes; the others have forms for any offset. (4 ranks of 25 MiB of
+// bf16 in int8 with residuals: 96 us so; by the kernels over peer memory 159 with values on 16 bytes,
+// 326 with residuals on 4, 490 with values on 2. Without residuals, values on 2 bytes, 58 here. B200.)
 bool local_reduce_takes(const ReduceArgs& r, int dtype) {
   bool ef;
   return reduce_aligned(r, elem_size(dtype), &ef) || !ef;

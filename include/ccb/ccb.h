@@ -84,7 +84,11 @@ int ccb_comm_status(ccb_comm* c, uint32_t* words);
 /* Device-side phase tracing: when on, every CTA of the two-shot kernels records
  * globaltimer nanoseconds at its phase boundaries (slots: 0 start, 1 first phase-1
  * done, 2 first phase-2 done, 3 all phase-2 done, 4 end); so does the kernel of a
- * communicator of one rank, where 1 follows 0 and 2, 3, 4 mark the end. */
+ * communicator of one rank, where 1 follows 0 and 2, 3, 4 mark the end. A communicator of
+ * ccb_comm_create_local() runs other kernels while it is on: those of ranks on several
+ * GPUs, over its arenas, with the same results. What is traced there is those kernels and
+ * not the calls as they run without a trace (nor are those traced); the one-rank kernel
+ * too is another one. */
 int ccb_comm_set_trace(ccb_comm* c, int on);
 int ccb_comm_read_trace(ccb_comm* c, unsigned long long* out, int ctas);
 /* Wire bytes a call moves per rank for `count` elements (for ratio reporting). */
