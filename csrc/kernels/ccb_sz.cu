@@ -689,10 +689,10 @@ __global__ void __cluster_dims__(kClusterSize, 1, 1) __launch_bounds__(kSzThread
 // behind those of the plane before. So nothing of a tile is exchanged between warps, there is one
 // barrier a GROUP (a CTA of eight warps), for the tiles' sizes, and no cluster. Both directions are
 // bound by instructions (ncu, 384^3: packing keeps the pipe of logical operations 61 % busy and 76 % of
-// the issue slots, unpacking 76 % and 76 %) and the latency of a tile's first loads. (512^3 field, bound
+// the issue slots) and the latency of a tile's first loads. (512^3 field, bound
 // 1e-4 of its range, B200: packing 177 us and unpacking 163; with a CTA a tile, its planes on eight
 // warps, three barriers a tile and the sizes sent round a cluster it was 332 and 279. Packing with 64
-// registers instead of 80 took 6 us more, unpacking with 64 instead of 48 8.)
+// registers instead of 80 took 6 us more. Unpacking by matrix products: 122, see PlanePrefix.)
 struct SzLocalArgs {
   const float* in;
   float* out;
@@ -951,24 +951,221 @@ __global__ void __launch_bounds__(kSzThreads, 3) sz_pack_kernel(const __grid_con
   }
 }
 
+// Unpacking sums a plane's residuals along x and y and adds the plane before: with the plane as a matrix D (8
+// lines of 32) and triangular matrices of ones, L D U + previous. The tensor cores do it. As fp16 pairs a
+// lane's eight residuals of its line are the fragment of D^T (k = x, n = y) that it has to hold. U^T D^T, for
+// the two halves of x apart, comes out in fp16 (sums of 16 residuals of 8 bits, 2048 at most: exact), is the
+// left operand of the product with L^T as it stands, and that adds to the codes of the plane before in fp32
+// (whole numbers, exact). Residuals of 9 to 15 bits go through in two digits, 7 bits and the rest, those of up to
+// 22 that a first plane has where the values are far from 0 in three.
+__device__ __forceinline__ void mma_x(uint32_t& d0, uint32_t& d1, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f16.f16.f16.f16 {%0, %1}, {%2, %3, %4, %5}, {%6, %7}, {%8, %8};"
+      : "=r"(d0), "=r"(d1) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(0));
+}
+__device__ __forceinline__ void mma_y(float (&c)[4], const uint32_t (&a)[4], uint32_t b) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %8}, {%0, %1, %2, %3};"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b));
+}
+struct PlanePrefix {
+  // [x_in <= x_out] for x_in = 8 t .. + 7 and x_out = 4 g .. + 3 (g = lane / 4, t = lane % 4) as pairs of fp16 ones
+  // and zeros: what the difference of 8 t and 4 g, a multiple of 4, leaves of it.
+  uint32_t p0, p4, p8, q0, q4;
+  uint32_t lines;     // [y_in <= y_out], L^T
+  float code[2][4];   // [m][2 h + j]: x = 4 g + 2 m + h, y = 2 t + j
+  __device__ __forceinline__ explicit PlanePrefix(int lane) {
+    const int g = lane >> 2, t = lane & 3, e = 8 * t - 4 * g;
+    auto ones = [](bool lo, bool hi) { return (lo ? 0x3c00u : 0u) | (hi ? 0x3c000000u : 0u); };
+    p0 = ones(e <= 0, e <= 0);
+    p4 = ones(e <= -4, e <= -4);
+    p8 = ones(e <= -8, e <= -8);
+    q0 = ones(e <= 0, e <= -4);
+    q4 = ones(e <= -4, e <= -8);
+    lines = ones(2 * t <= g, 2 * t + 1 <= g);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) code[i >> 2][i & 3] = 0.f;
+  }
+  // h[i]: residuals 2 i and 2 i + 1 of the lane's eight; `weighted`: L^T times the weight of the digit that they are.
+  __device__ __forceinline__ void add(float (&to)[2][4], const uint32_t (&h)[4], uint32_t weighted) const {
+    uint32_t d[4], f[4];
+    mma_x(d[0], d[1], q0, p0, p4, p4, h[0], h[1]);
+    mma_x(d[2], d[3], q4, p4, p8, p8, h[2], h[3]);
+    mma_x(f[0], f[1], p0, p0, q0, p0, h[0], h[1]);
+    mma_x(f[2], f[3], p4, p4, q4, p4, h[2], h[3]);
+    mma_y(to[0], d, weighted);
+    mma_y(to[1], f, weighted);
+  }
+};
+// fp16 pairs of a lane's eight residuals, held as bytes plus a bias in b[0] and b[1]: a byte is the low mantissa of 1024.
+__device__ __forceinline__ void halves_of(const uint32_t (&b)[2], uint32_t bias, uint32_t (&h)[4]) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const uint32_t w = __byte_perm(b[i >> 1], 0x64646464u, i & 1 ? 0x4342 : 0x4140);
+    const __half2 d = __hsub2(*reinterpret_cast<const __half2*>(&w), *reinterpret_cast<const __half2*>(&bias));
+    h[i] = *reinterpret_cast<const uint32_t*>(&d);
+  }
+}
+// 255 in the bytes whose highest bit is set, 0 in the others.
+__device__ __forceinline__ uint32_t byte_signs(uint32_t v) {
+  uint32_t m;
+  asm("prmt.b32 %0, %1, 0, 0xba98;" : "=r"(m) : "r"(v));
+  return m;
+}
+
+// Where a lane writes the codes of PlanePrefix: x = 4 g .. + 3 of the lines y = 2 t and 2 t + 1. kAligned: every line
+// on 16 bytes, a warp writes four of 128 bytes at a time; otherwise a plane goes through shared memory, line by line.
+template <bool kAligned>
+struct PlaneOut {
+  float* at;
+  size_t stride;     // of a plane
+  int line;          // of a line
+  int planes, more;  // planes of the tile that the lane writes; kAligned: of its second line; otherwise lines of the tile
+  float* sh;
+  __device__ __forceinline__ PlaneOut(const SzLocalArgs& a, TileCoord t, float* shared) {
+    const int lane = threadIdx.x & 31;
+    sh = shared;
+    line = a.nx;
+    stride = (size_t)a.ny * a.nx;
+    const int gx = kAligned ? t.x0 + (lane & ~3) : t.x0 + lane, gy = kAligned ? t.y0 + 2 * (lane & 3) : t.y0;
+    at = a.out + ((size_t)t.z0 * a.ny + gy) * a.nx + gx;
+    const int depth = gx < a.nx ? min(kTZ, a.nz - t.z0) : 0;
+    planes = gy < a.ny ? depth : 0;
+    more = !kAligned ? a.ny - t.y0 : gy + 1 < a.ny ? depth : 0;
+  }
+  __device__ __forceinline__ void store(int z, const float (&code)[2][4], float step) const {
+    float* p = at + z * stride;
+    float4 v[2];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) v[j] = make_float4(__fmul_rn(code[0][j], step), __fmul_rn(code[0][2 + j], step), __fmul_rn(code[1][j], step), __fmul_rn(code[1][2 + j], step));
+    if constexpr (kAligned) {
+      if (z < planes) stg_stream(p, *reinterpret_cast<const uint4*>(&v[0]));
+      if (z < more) stg_stream(p + line, *reinterpret_cast<const uint4*>(&v[1]));
+    } else {
+      const int lane = threadIdx.x & 31;
+#pragma unroll
+      for (int j = 0; j < 2; ++j) reinterpret_cast<float4*>(sh)[8 * (2 * (lane & 3) + j) + (lane >> 2)] = v[j];
+      __syncwarp();
+#pragma unroll
+      for (int y = 0; y < kTY; ++y)
+        if (z < planes && y < more) p[(size_t)y * line] = sh[kTX * y + lane];
+      __syncwarp();
+    }
+  }
+};
+
+// A packed tile in shared memory whose residuals have at most 15 bits, those of its first plane 22.
+template <bool kAligned>
+__device__ __forceinline__ void unpack_digits(const PlaneOut<kAligned>& io, const unsigned char* tile, uint32_t small, float step) {
+  const int lane = threadIdx.x & 31, j = lane & 7;
+  const uint32_t* words = reinterpret_cast<const uint32_t*>(tile + kRows);
+  // Lane 8 r + j fetches bit planes of row r: for j = 7 the first, which holds the signs, so that it comes to the
+  // highest bit of a byte; else plane j + 1, and of wider rows j + 8.
+  const uint32_t below = (1u << (lane & 24)) - 1u, first = (uint32_t)(j + 1) & 7u, pick = 0x4440u | (uint32_t)(lane >> 3);
+  PlanePrefix sums(lane);
+  uint32_t run = 0;   // words before the plane
+  auto plane = [&](int z, auto narrow) {
+    const uint2 W = reinterpret_cast<const uint2*>(tile)[z];
+    const uint32_t half = __dp4a(W.x, 0x01010101u, run);
+    const uint32_t at0 = __dp4a(W.x & below, 0x01010101u, run) + first, at1 = __dp4a(W.y & below, 0x01010101u, half) + first;
+    const uint32_t w0 = __byte_perm(W.x, 0u, pick), w1 = __byte_perm(W.y, 0u, pick);
+    run = __dp4a(W.y, 0x01010101u, half);
+    const uint32_t X0 = first < w0 ? words[at0] : 0u, X1 = first < w1 ? words[at1] : 0u;
+    const uint32_t x0 = transpose32(X0, lane), x1 = transpose32(X1, lane), s0 = byte_signs(x0), s1 = byte_signs(x1);
+    uint32_t h[4];
+    if (decltype(narrow)::value || ((small >> (2 * z)) & 3u) == 3u) {   // zig-zag undone: a negative residual is the complement; plus 128
+      const uint32_t b[2] = {(x0 | 0x80808080u) ^ s0, (x1 | 0x80808080u) ^ s1};
+      halves_of(b, 0x64806480u, h);
+      sums.add(sums.code, h, sums.lines);
+    } else {   // the low seven bits, and 128 times the others with the sign
+      uint32_t y0 = X0, y1 = X1;
+      if (j < 7) {
+        y0 = first + 7u < w0 ? words[at0 + 7u] : 0u;
+        y1 = first + 7u < w1 ? words[at1 + 7u] : 0u;
+      }
+      const uint32_t lo[2] = {(x0 ^ s0) & 0x7f7f7f7fu, (x1 ^ s1) & 0x7f7f7f7fu};
+      halves_of(lo, 0x64006400u, h);
+      sums.add(sums.code, h, sums.lines);
+      y0 = transpose32(y0, lane);
+      y1 = transpose32(y1, lane);
+      const bool third = z == 0 && __any_sync(0xffffffffu, max(w0, w1) > 15u);
+      const uint32_t mid[2] = {third ? (y0 ^ s0) & 0x7f7f7f7fu : (y0 | 0x80808080u) ^ s0, third ? (y1 ^ s1) & 0x7f7f7f7fu : (y1 | 0x80808080u) ^ s1};
+      halves_of(mid, third ? 0x64006400u : 0x64806480u, h);
+      sums.add(sums.code, h, (sums.lines & 0x04000400u) * 0x16u);   // 128 for 1
+      if (third) {   // 16384 times these in one rounding of what is a whole number below 2^23 again
+        y0 = X0;
+        y1 = X1;
+        if (j < 7) {
+          y0 = first + 14u < w0 ? words[at0 + 14u] : 0u;
+          y1 = first + 14u < w1 ? words[at1 + 14u] : 0u;
+        }
+        const uint32_t hi[2] = {(transpose32(y0, lane) | 0x80808080u) ^ s0, (transpose32(y1, lane) | 0x80808080u) ^ s1};
+        halves_of(hi, 0x64806480u, h);
+        float top[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+        sums.add(top, h, sums.lines);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) sums.code[e >> 2][e & 3] = __fmaf_rn(top[e >> 2][e & 3], 16384.f, sums.code[e >> 2][e & 3]);
+      }
+    }
+    io.store(z, sums.code, step);
+  };
+  if ((small | 3u) == 0xffffffffu) {   // nearly always: beyond the first plane no residual of more than 8 bits
+    plane(0, Int<0>{});
+#pragma unroll
+    for (int z = 1; z < kTZ; ++z) plane(z, Int<1>{});
+  } else {
+#pragma unroll 1
+    for (int z = 0; z < kTZ; ++z) plane(z, Int<0>{});
+  }
+}
+
+// A warp brings a packed tile of up to 2304 bytes to shared memory, all of it under way at once, and takes its planes
+// from there by the tensor cores; larger ones, raw ones, and those with wider residuals are read where they are, from L2 where
+// a prefetch puts them, and summed by shuffles. (B200, us, the whole by shuffles with one plane requested ahead / so: 512^3
+// field, bound 1e-4 of its range, 163 / 122; 1e-3 154 / 115; 1e-5 183 / 140; the first with 30 added to its values 165 / 131;
+// 300 x 300 x 404 49.5 / 33.5, x 403 61.8 / 55; 512^3 of white noise, 1e-6 189 / 177, 1e-5 277 / 279. Stages of 4608 bytes took
+// as long on the fields and 12 us more on the noise at 1e-6; five CTAs of 48 registers spill, 129 instead of 120, three of
+// 80 138. Lanes that hold 32 bytes of a line: as fast at 512^3, 45 instead of 33 where lines lie on 16 bytes. B200.)
+// What is left of the 94 us that the memory needs is the latency of a tile's size, then its words.
+constexpr int kUnpackStage = 2304;
+
 template <int kVec>
-__global__ void __launch_bounds__(kSzThreads, kVec == 1 ? 4 : 5) sz_unpack_kernel(const __grid_constant__ SzLocalArgs a) {
+__global__ void __launch_bounds__(kSzThreads, 4) sz_unpack_kernel(const __grid_constant__ SzLocalArgs a) {
   __shared__ __align__(16) float plane[kVec == 1 ? kClusterSize : 1][kVec == 1 ? kTX * kTY : 4];
+  __shared__ __align__(16) unsigned char stages[kClusterSize][kUnpackStage];
   const int lane = threadIdx.x & 31, k = threadIdx.x >> 5;
   const unsigned int tile = blockIdx.x * kClusterSize + k;
   if (tile >= (unsigned)a.tiles_x * a.tiles_y * a.tiles_z) return;
   const char* group = a.slots + (size_t)blockIdx.x * kGroupStride;
-  const PlaneIO<kVec> io(a.out, a, tile_coord(a, tile), plane[kVec == 1 ? k : 0]);
-  uint32_t off = __reduce_add_sync(0xffffffffu, lane < k ? ldg_cg_u32(group + 4 * lane) : 0u);
+  const uint32_t size_word = lane < kClusterSize ? ldg_cg_u32(group + 4 * lane) : 0u;
+  const TileCoord coord = tile_coord(a, tile);
+  uint32_t off = __reduce_add_sync(0xffffffffu, lane < k ? size_word : 0u);
+  const uint32_t size = __shfl_sync(0xffffffffu, size_word, k);
   const bool there = ccb_sz_offset_ok(off, k);
   if (!there) off = 0;
   const unsigned char* src = reinterpret_cast<const unsigned char*>(group) + kGroupHeader + off;
-  uint32_t hw = lane < 16 ? ldg_cg_u32(src + 4 * lane) : 0u;   // the row widths, four a word
+  // (a buffer is promised to start on 4 bytes, no more)
+  const bool staged = size >= kRows && size <= kUnpackStage && (size & 15u) == 0 && (reinterpret_cast<uintptr_t>(src) & 15) == 0;
+  if (staged) {
+    const uint32_t to = smem_u32(stages[k]);
+    for (uint32_t i = 16u * lane; i < size; i += 512u) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to + i), "l"(src + i) : "memory");
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncwarp();
+  } else {
+    for (uint32_t i = 128u * lane; i < min(size, (uint32_t)kTileCap); i += 4096u) asm volatile("prefetch.global.L2 [%0];" ::"l"(src + i));
+  }
+  uint32_t hw = 0u;   // the row widths, four a word
+  if (lane < 16) hw = staged ? reinterpret_cast<const uint32_t*>(stages[k])[lane] : ldg_cg_u32(src + 4 * lane);
   if (!there) hw = 0xfefefefeu;
+  if (staged && !__any_sync(0xffffffffu, ((hw + (lane < 2 ? 0x69696969u : 0x70707070u)) | hw) & 0x80808080u) && kRows + 4u * __reduce_add_sync(0xffffffffu, bytesum(hw)) <= size) {
+    const PlaneOut<kVec != 1> out(a, coord, plane[kVec == 1 ? k : 0]);
+    unpack_digits(out, stages[k], __ballot_sync(0xffffffffu, bytes_le8(hw)), a.two_eb);
+    return;
+  }
+  const PlaneIO<kVec> io(a.out, a, coord, plane[kVec == 1 ? k : 0]);
   if ((__shfl_sync(0xffffffffu, hw, 0) & 0xffu) == 255u) {
     const uint32_t* raw = reinterpret_cast<const uint32_t*>(src + kRows) + 8 * lane;
-    const bool wide = (reinterpret_cast<uintptr_t>(raw) & 15) == 0;   // a buffer is promised to start on 4 bytes, no more
-#pragma unroll 1
+    const bool wide = (reinterpret_cast<uintptr_t>(raw) & 15) == 0;
+    constexpr int kRawTurns = kVec == 1 ? 2 : 4;
+#pragma unroll kRawTurns
     for (int z = 0; z < kTZ; ++z, raw += kTX * kTY) {
       uint32_t w[8];
       if (wide) {
@@ -1405,11 +1602,11 @@ static void launch_pack(const SzLocalArgs& a, cudaStream_t stream) {
   }
   sz_pack_kernel<kVec><<<a.ngroups, kSzThreads, kBytes, stream>>>(a);
 }
-// Tiles up to which a CTA a tile unpacks a field faster than a warp a tile, us, CTA / warp, B200. Lines on
-// 16 bytes: 64^3 (128 tiles) 7.5 / 7.5 to 12.4 by the widths of its rows, 128 x 128 x 256 (2048) 10.4 /
-// 10.3 at 0.75 bytes a value, 12.4 / 16.5 at 2; 160 x 160 x 256 (3200) 14.5 / 12.4 and 16.5 / 18.6.
-// Lines anywhere: 130 x 201 x 258 (3978) 16.5 / 18.6 and 20.6 / 27, 176 x 200 x 258 (4950) 20.6 / 22.7
-// and 24.7 / 30.9, 256 x 256 x 257 (9216) 35 / 33 and 43 / 48.
+// Tiles up to which a CTA a tile unpacks a field faster than a warp a tile, us, CTA / warp, at bounds of 1e-4
+// and 1e-5 of the range (0.6 and 1 byte a value), B200. Lines on 16 bytes: 64^3 (128 tiles) 6.0 / 8.6 and
+// 5.9 / 13.8, 128 x 128 x 256 (2048) 10.6 / 10.4 and 10.6 / 14.7, 160 x 160 x 256 (3200) 14.7 / 10.6 and
+// 14.9 / 16.7. Lines anywhere: 130 x 130 x 258 (2601) 12.8 / 14.6 and 12.7 / 18.9, 176 x 176 x 258 (4356)
+// 18.8 / 16.7 and 19.2 / 20.8, 256 x 256 x 257 (9216) 35 / 29 and 37 / 34.
 static unsigned int few_tiles(int width) { return width == 1 ? 5120u : 2560u; }
 static int launched(const char* what) {
   const cudaError_t e = cudaGetLastError();

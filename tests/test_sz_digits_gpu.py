@@ -1,0 +1,50 @@
+"""Unpacking of fields of many tiles, whose prefix sums run on the tensor cores in digits of seven and eight bits:
+residuals on either side of each number of digits, in first planes and in others, and the largest sums."""
+import pytest
+import torch
+
+from ccbench_b200.ops import sz
+
+pytestmark = pytest.mark.gpu
+
+EB = 2.0 ** -6
+
+
+def _residuals(first, other, g):
+    """One tile [8, 8, 32]: residuals of `other` bits (zig-zag), `first` bits in the corner value."""
+    half = 1 << other >> 1
+    d = torch.randint(-half, max(half, 1), (8, 8, 32), generator=g) if other else torch.zeros(8, 8, 32, dtype=torch.int64)
+    if other:
+        d.view(-1)[1 + torch.randperm(2047, generator=g)[:2]] = torch.tensor([-half, half - 1])
+    if first:
+        d[0, 0, 0] = -(1 << first >> 1)
+    return d
+
+
+@pytest.mark.parametrize("shape", [(160, 168, 256), (161, 163, 260), (200, 201, 257)])   # lines on 32 bytes, on 16, anywhere
+def test_every_width_of_residuals_comes_back(shape):
+    g = torch.Generator().manual_seed(5)
+    kinds = [_residuals(first, other, g) for first in (0, 8, 9, 15, 16, 22) for other in (0, 1, 2, 7, 8, 9, 13, 14, 15, 16)]
+    kinds += [torch.full((8, 8, 32), -128), torch.full((8, 8, 32), 127), _residuals(22, 8, g)]   # sums of 2048 residuals
+    codes = torch.stack([k.cumsum(0).cumsum(1).cumsum(2) for k in kinds])
+    codes = codes[codes.abs().amax((1, 2, 3)) < 1 << 21]
+    assert len(codes) > 40
+    tz, ty, tx = (-(-n // t) for n, t in zip(shape, (8, 8, 32)))
+    pick = torch.randint(0, len(codes), (tz, ty, tx), generator=g)
+    q = codes[pick].permute(0, 3, 1, 4, 2, 5).reshape(8 * tz, 8 * ty, 32 * tx)[:shape[0], :shape[1], :shape[2]]
+    step = torch.tensor(2 * EB, dtype=torch.float32) * (1 - 2.0 ** -10)   # what the decoder multiplies with, exact here
+    field = (q.float() * step).cuda()
+    buf, _ = sz.compress(field, EB)
+    assert torch.equal(sz.decompress(buf, shape, EB), field)
+    tiles = buf.view(-1, sz.GROUP_STRIDE)[:, :sz.GROUP_HEADER].contiguous().view(torch.int32)
+    assert int((tiles == sz.TILE_CAP).sum()) == 0 and int((tiles > 2304).sum()) > 0 and int((tiles[tiles > 0] <= 2304).sum()) > 0
+
+
+def test_a_buffer_on_four_bytes_is_unpacked_where_it_lies():
+    shape = (160, 168, 256)
+    f = torch.randn(shape, generator=torch.Generator().manual_seed(1)).cuda().cumsum(2)
+    buf, _ = sz.compress(f, 1e-2)
+    want = sz.decompress(buf, shape, 1e-2)
+    moved = torch.empty(buf.numel() + 16, dtype=torch.uint8, device="cuda")[4:4 + buf.numel()]
+    moved.copy_(buf)
+    assert torch.equal(sz.decompress(moved, shape, 1e-2), want)
