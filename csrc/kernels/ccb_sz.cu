@@ -684,15 +684,11 @@ __global__ void __cluster_dims__(kClusterSize, 1, 1) __launch_bounds__(kSzThread
 
 // ------------------------------------------------------- local buffers, a warp a tile --
 // Compression into and decompression from a buffer of this GPU. A warp owns a tile and walks its
-// eight planes: a lane holds eight consecutive x of line y = lane / 4 (the mapping above), the plane
-// before stays in its registers, y and x neighbours come by shuffles, and the words of a plane go
-// behind those of the plane before. So nothing of a tile is exchanged between warps, there is one
-// barrier a GROUP (a CTA of eight warps), for the tiles' sizes, and no cluster. Both directions are
-// bound by instructions (ncu, 384^3: packing keeps the pipe of logical operations 61 % busy and 76 % of
-// the issue slots) and the latency of a tile's first loads. (512^3 field, bound
-// 1e-4 of its range, B200: packing 177 us and unpacking 163; with a CTA a tile, its planes on eight
-// warps, three barriers a tile and the sizes sent round a cluster it was 332 and 279. Packing with 64
-// registers instead of 80 took 6 us more. Unpacking by matrix products: 122, see PlanePrefix.)
+// eight planes: a lane holds eight consecutive x of line y = lane / 4 (the mapping above), and the words of a
+// plane go behind those of the plane before. So nothing of a tile is exchanged between warps, there is one
+// barrier a GROUP (a CTA of eight warps), for the tiles' sizes, and no cluster. (With a CTA a tile, its planes on
+// eight warps, three barriers a tile and the sizes sent round a cluster, a 512^3 field, bound 1e-4 of its
+// range, took 332 us to pack and 279 to unpack; B200.)
 struct SzLocalArgs {
   const float* in;
   float* out;
@@ -701,6 +697,7 @@ struct SzLocalArgs {
   int nx, ny, nz, tiles_x, tiles_y, tiles_z;
   unsigned int ngroups;
   float eb, two_eb, inv_two_eb;
+  float one;   // 1, which the compiler must not know: see pack_halves
   unsigned long long magic_x, magic_xy;
 };
 // How a lane's eight values lie in memory: every line on 32 bytes (kVec 8), on 16 (4), or anywhere
@@ -776,8 +773,84 @@ struct PlaneIO {
   }
 };
 
-// Codes of one plane, 2^21 added to each; the arithmetic and its result are pack_tile's. Codes that
-// far from 0 and values that are not finite show in the codes' high bits and take the exact tests.
+// The largest magnitude of three, NaN if any is.
+__device__ __forceinline__ float max_abs3(float a, float b, float c) {
+  float m;
+  asm("max.NaN.abs.f32 %0, %1, %2, %3;" : "=f"(m) : "f"(a), "f"(b), "f"(c));
+  return m;
+}
+// The packer brings the values of a tile to shared memory, [z][y][x] behind the 64 bytes of its widths, all planes under
+// way at once, and packs it in place: the words of planes 0 to z end where plane z + 1 begins, or before. Two
+// neighbouring pieces of 16 bytes change places on odd lines, for a lane reads two of them and eight lanes at a time
+// should find theirs in different banks. What lies outside the field is 0.
+template <int kVec>
+__device__ __forceinline__ void stage_tile(const SzLocalArgs& a, TileCoord t, unsigned char* tile) {
+  const int lane = threadIdx.x & 31, depth = min(kTZ, a.nz - t.z0);
+  const size_t stride = (size_t)a.ny * a.nx;
+  const uint32_t to = smem_u32(tile + kRows);
+  auto bring = [&](auto width, uint32_t dst, const float* src, bool on) {
+    constexpr int kBytes = decltype(width)::value;
+    const int n = on ? kBytes : 0;
+    if constexpr (kBytes == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(n) : "memory");
+    else asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(n) : "memory");
+  };
+  constexpr int kParts = kVec == 1 ? kTY : 2;
+  const float* from[2];
+  bool on[2];
+  if constexpr (kVec != 1) {
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int x = t.x0 + 4 * (lane & 7), y = t.y0 + (lane >> 3) + 4 * i;
+      on[i] = x < a.nx && y < a.ny;
+      from[i] = on[i] ? a.in + ((size_t)t.z0 * a.ny + y) * a.nx + x : a.in;
+    }
+  } else {
+    on[0] = t.x0 + lane < a.nx;
+    from[0] = on[0] ? a.in + ((size_t)t.z0 * a.ny + t.y0) * a.nx + t.x0 + lane : a.in;
+  }
+#pragma unroll
+  for (int z = 0; z < kTZ; ++z) {
+#pragma unroll
+    for (int i = 0; i < kParts; ++i) {
+      if constexpr (kVec != 1) {
+        const bool in = on[i] && z < depth;
+        bring(Int<16>{}, to + 1024 * z + 512 * i + 16 * (lane ^ (lane >> 3 & 1)), in ? from[i] + z * stride : a.in, in);
+      } else {
+        const bool in = on[0] && z < depth && t.y0 + i < a.ny;
+        bring(Int<4>{}, to + 1024 * z + 128 * i + 4 * (lane ^ (4 * (i & 1))), in ? from[0] + z * stride + (size_t)i * a.nx : a.in, in);
+      }
+    }
+    if (z == 1 || z + 1 == kTZ) asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+}
+// The lane's eight values of plane z: x = 8 (lane % 4) .. + 7 of line lane / 4. The words of this plane may follow.
+__device__ __forceinline__ void staged_plane(const unsigned char* tile, int z, float (&x)[8]) {
+  const int lane = threadIdx.x & 31;
+  const float4* at = reinterpret_cast<const float4*>(tile + kRows + 1024 * z) + 2 * lane;
+  const float4 p = at[lane >> 2 & 1], q = at[~lane >> 2 & 1];
+  x[0] = p.x; x[1] = p.y; x[2] = p.z; x[3] = p.w; x[4] = q.x; x[5] = q.y; x[6] = q.z; x[7] = q.w;
+  __syncwarp();
+}
+
+// Codes of one plane where the nearest grid point may be another or none is near enough: the arithmetic and
+// its result are pack_tile's. `base` is added to each.
+__device__ __forceinline__ void exact_codes(const float (&x)[8], const SzLocalArgs& a, int base, int (&q)[8], bool& bad) {
+  const float half = 0.5f * a.two_eb;
+#pragma unroll
+  for (int e = 0; e < 8; ++e) {
+    const float se = __fmul_rn(x[e], a.inv_two_eb);
+    bad |= !(fabsf(se) < kQMax);
+    float rf = __fadd_rn(__fadd_rn(se, kRoundMagic), -kRoundMagic);
+    const float diff = __fsub_rn(x[e], __fmul_rn(rf, a.two_eb));
+    rf += diff > half ? 1.f : 0.f;
+    rf -= -diff > half ? 1.f : 0.f;
+    bad |= fabsf(__fsub_rn(x[e], __fmul_rn(rf, a.two_eb))) > a.eb;
+    q[e] = (int)rf + base;
+  }
+  bad = __any_sync(0xffffffffu, bad);
+}
+// Codes of one plane, 2^21 added to each. Codes that far from 0 and values that are not finite show in the
+// codes' high bits and take the exact tests.
 constexpr int kCodeBias = 1 << 21;
 __device__ __forceinline__ void plane_codes(const float (&x)[8], const SzLocalArgs& a, int (&q)[8], bool& bad) {
   const float half = 0.5f * a.two_eb;
@@ -796,42 +869,240 @@ __device__ __forceinline__ void plane_codes(const float (&x)[8], const SzLocalAr
     worst = fmaxf(worst, fmaxf(fabsf(__fsub_rn(x[e], p0)), fabsf(__fsub_rn(x[e + 1], p1))));
   }
   const bool wild = (high >> 22) != 0u;   // NaN and infinities among them, so `worst` may pass them over
-  if (__any_sync(0xffffffffu, wild || worst > half)) {
+  if (__any_sync(0xffffffffu, wild || worst > half)) exact_codes(x, a, kCodeBias, q, bad);
+}
+
+// 255 in the bytes whose highest bit is set, 0 in the others.
+__device__ __forceinline__ uint32_t byte_signs(uint32_t v) {
+  uint32_t m;
+  asm("prmt.b32 %0, %1, 0, 0xba98;" : "=r"(m) : "r"(v));
+  return m;
+}
+// A plane of wider residuals to `words`: W0 and W1 become the widths of its rows, a byte each. Returns its words.
+__device__ __forceinline__ uint32_t wide_plane(const int (&d)[8], uint32_t* words, uint32_t& W0, uint32_t& W1, int lane) {
+  uint32_t u[8];
+  W0 = W1 = 0u;
 #pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      const float se = __fmul_rn(x[e], a.inv_two_eb);
-      bad |= !(fabsf(se) < kQMax);
-      float rf = __fadd_rn(__fadd_rn(se, kRoundMagic), -kRoundMagic);
-      const float diff = __fsub_rn(x[e], __fmul_rn(rf, a.two_eb));
-      rf += diff > half ? 1.f : 0.f;
-      rf -= -diff > half ? 1.f : 0.f;
-      bad |= fabsf(__fsub_rn(x[e], __fmul_rn(rf, a.two_eb))) > a.eb;
-      q[e] = (int)rf + kCodeBias;
-    }
-    bad = __any_sync(0xffffffffu, bad);
+  for (int e = 0; e < 8; ++e) u[e] = ((uint32_t)d[e] << 1) ^ (uint32_t)(d[e] >> 31);
+#pragma unroll
+  for (int e = 0; e < 8; ++e) {
+    const uint32_t w = 32 - __clz((int)__reduce_or_sync(0xffffffffu, u[e]));
+    if (e < 4) W0 |= w << (8 * e);
+    else W1 |= w << (8 * (e - 4));
   }
+  const uint32_t lo = bytesum(W0);
+  uint32_t ua[4] = {u[0], u[1], u[2], u[3]}, ub[4] = {u[4], u[5], u[6], u[7]};
+  wide_planes4<true>(ua, W0, 0u, words, lane);
+  wide_planes4<true>(ub, W1, lo, words, lane);
+  return lo + bytesum(W1);
+}
+
+// Which of the planes up to 8 of four rows are stored, from the bits that occur: all up to the highest of a row.
+__device__ __forceinline__ uint32_t planes_up_to(uint32_t any) {
+  any |= (any >> 1) & 0x7f7f7f7fu;
+  any |= (any >> 2) & 0x3f3f3f3fu;
+  return any | ((any >> 4) & 0x0f0f0f0fu);
+}
+__device__ __forceinline__ uint32_t byte_bits(uint32_t v) {   // the bits set in each byte
+  v -= (v >> 1) & 0x55555555u;
+  v = (v & 0x33333333u) + ((v >> 2) & 0x33333333u);
+  return (v + (v >> 4)) & 0x0f0f0f0fu;
+}
+// Bytes `at` and `at` + 2 of four words that hold elements i and 4 + i: of elements 0 to 3, of 4 to 7.
+__device__ __forceinline__ void bytes_of_halves(const uint32_t (&t)[4], int at, uint32_t& u0, uint32_t& u1) {
+  const uint32_t sel = 0x6240u + 0x1111u * at, lo = __byte_perm(t[0], t[1], sel), hi = __byte_perm(t[2], t[3], sel);
+  u0 = __byte_perm(lo, hi, 0x5410);
+  u1 = __byte_perm(lo, hi, 0x7632);
+}
+
+// Packs the warp's tile as pack_planes does, if its codes lie within 4094 of the first: then two residuals share a word,
+// a + 65536 b, whose sums and differences are those of the pairs whatever carries between the halves, since in
+// the end a is below 2^15 either way (8 x 4095). All codes are taken relative to the first, which
+// leaves only the first residual other than it is. Returns the tile's words; kNoHalves where it is not such a tile (`whole`:
+// its values are all there still).
+// Additions of 1.5 * 2^23 are multiply-adds by a.one, two at a time: as additions they could be fused with the
+// products before them (see f32x2).
+constexpr uint32_t kNoHalves = 0xffffffffu;
+__device__ __forceinline__ uint32_t pack_halves(const SzLocalArgs& a, unsigned char* pk, bool& bad, bool& whole) {
+  const int lane = threadIdx.x & 31;
+  uint32_t* words = reinterpret_cast<uint32_t*>(pk + kRows);
+  const float half = 0.5f * a.two_eb;
+  const f32x2 inv2 = pair2(a.inv_two_eb, a.inv_two_eb), step2 = pair2(a.two_eb, a.two_eb), one2 = pair2(a.one, a.one), less2 = pair2(-a.one, -a.one);
+  const f32x2 magic2 = pair2(kRoundMagic, kRoundMagic), back2 = pair2(-kRoundMagic, -kRoundMagic);
+  const Transpose32 transposed((uint32_t)lane);
+  const int below_line = lane >= 4 ? -1 : 0;
+  const uint32_t self = 1u << lane, below = self - 1u, below_row = (1u << (lane & 24)) - 1u, from_mine = 0xffu >> (lane & 7);
+  uint32_t before[4], run = 0, wide = 0;   // wide: planes whose rows' widths are stored as such, not yet as the bit planes that they have
+  f32x2 first2 = 0;
+  bool far = false;   // the first code is not within 16 bits
+  auto plane = [&](int z, const float (&x)[8], auto first_too) -> bool {
+    int q[8];
+    float diff[8], away[8];
+    f32x2 r2[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const f32x2 x2 = pair2(x[2 * i], x[2 * i + 1]);
+      float r0, r1;
+      r2[i] = fma2(mul2(x2, inv2), one2, magic2);
+      split2(r2[i], r0, r1);
+      q[2 * i] = __float_as_int(r0);
+      q[2 * i + 1] = __float_as_int(r1);
+      split2(fma2(mul2(add2(r2[i], back2), step2), less2, x2), diff[2 * i], diff[2 * i + 1]);
+    }
+    uint32_t bias0 = 0x80808080u;
+    int corner = 0;
+    if (decltype(first_too)::value && z == 0) {
+      const int first = __shfl_sync(0xffffffffu, q[0], 0);
+      corner = first - __float_as_int(kRoundMagic);
+      far = abs(corner) >= 32000;
+      if (lane == 0) bias0 += far ? 1 << 14 : corner;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) before[i] = (uint32_t)first * 65537u;
+      first2 = pair2(-__int_as_float(first), -__int_as_float(first));
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) split2(add2(r2[i], first2), away[2 * i], away[2 * i + 1]);
+    const float worst = max_abs3(max_abs3(diff[0], diff[1], diff[2]), max_abs3(diff[3], diff[4], diff[5]), max_abs3(diff[6], diff[7], 0.f));
+    const float apart = max_abs3(max_abs3(away[0], away[1], away[2]), max_abs3(away[3], away[4], away[5]), max_abs3(away[6], away[7], 0.f));
+    if (__any_sync(0xffffffffu, !(worst <= half && apart <= 4094.f) || abs(corner) > kCodeBias - 4096)) {
+      if (__any_sync(0xffffffffu, !(apart <= 4094.f) || abs(corner) > kCodeBias - 4096)) return false;
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {   // the nearest grid point by the decoder's own product, as in exact_codes: nearly always one of 256
+        const bool off = fabsf(diff[e]) > half;
+        if (__any_sync(0xffffffffu, off) && off) {
+          q[e] += diff[e] > 0.f ? 1 : -1;
+          bad |= !(fabsf(__fsub_rn(x[e], __fmul_rn(__fadd_rn(__int_as_float(q[e]), -kRoundMagic), a.two_eb))) <= a.eb);
+        }
+      }
+      bad = __any_sync(0xffffffffu, bad);
+      if (bad) return false;
+    }
+    uint32_t d[4], t[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const uint32_t w = (uint32_t)q[4 + i] * 65536u + (uint32_t)q[i];
+      d[i] = w - before[i];
+      before[i] = w;
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) d[i] += (uint32_t)below_line * __shfl_up_sync(0xffffffffu, d[i], 4);
+    // what stands left of elements 0 and 4: the left lane's 7 and this lane's 3
+    const uint32_t last = d[3] + 0x80008000u;
+    uint32_t left = __shfl_up_sync(0xffffffffu, last, 1);
+    if ((lane & 3) == 0) left = 0x80000000u;
+    t[0] = d[0] - __byte_perm(left, last, 0x5432) + bias0;
+#pragma unroll
+    for (int i = 1; i < 4; ++i) t[i] = d[i] - d[i - 1] + 0x00800080u;
+    if (!__any_sync(0xffffffffu, ((t[0] | t[1] | t[2] | t[3]) & 0xff00ff00u) != 0u)) {
+      // nearly always: residuals as bytes d + 128, whose zig-zag is twice d, complemented where d is negative
+      uint32_t u0, u1;
+      bytes_of_halves(t, 0, u0, u1);
+      u0 = ((u0 + u0) & 0xfefefefeu) ^ ~byte_signs(u0);
+      u1 = ((u1 + u1) & 0xfefefefeu) ^ ~byte_signs(u1);
+      const uint32_t any0 = __reduce_or_sync(0xffffffffu, u0), any1 = __reduce_or_sync(0xffffffffu, u1);
+      // a lane, plane j of its row, is stored if any plane from j up of that row holds a bit
+      const uint32_t W0 = __ballot_sync(0xffffffffu, ((any0 >> lane) & from_mine) != 0u), W1 = __ballot_sync(0xffffffffu, ((any1 >> lane) & from_mine) != 0u);
+      u0 = transposed(u0);
+      u1 = transposed(u1);
+      if (lane == 0) reinterpret_cast<uint2*>(pk)[z] = make_uint2(W0, W1);
+      const uint32_t mid = run + __popc(W0);
+      if (W0 & self) words[run + __popc(W0 & below)] = u0;
+      if (W1 & self) words[mid + __popc(W1 & below)] = u1;
+      run = mid + __popc(W1);
+    } else if (!(decltype(first_too)::value && far && z == 0)) {
+      // up to 16 bits: the same in halves, whose lower and upper bytes are transposed by themselves
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const uint32_t v = t[i] + 0x7f807f80u;
+        uint32_t minus;
+        asm("prmt.b32 %0, %1, 0, 0xbb99;" : "=r"(minus) : "r"(v));
+        t[i] = ((v + v) & 0xfffefffeu) ^ ~minus;
+      }
+      uint32_t u0, u1, y0, y1;
+      bytes_of_halves(t, 0, u0, u1);
+      bytes_of_halves(t, 1, y0, y1);
+      const uint32_t V0 = planes_up_to(__reduce_or_sync(0xffffffffu, y0)), V1 = planes_up_to(__reduce_or_sync(0xffffffffu, y1));
+      // a row with an upper plane has all the lower ones
+      const uint32_t W0 = planes_up_to(__reduce_or_sync(0xffffffffu, u0)) | (V0 & 0x01010101u) * 0xffu;
+      const uint32_t W1 = planes_up_to(__reduce_or_sync(0xffffffffu, u1)) | (V1 & 0x01010101u) * 0xffu;
+      u0 = transposed(u0);
+      u1 = transposed(u1);
+      y0 = transposed(y0);
+      y1 = transposed(y1);
+      const uint32_t mid = run + __popc(W0) + __popc(V0);
+      uint32_t* row0 = words + run + __popc(W0 & below_row) + __popc(V0 & below_row) + (lane & 7);
+      uint32_t* row1 = words + mid + __popc(W1 & below_row) + __popc(V1 & below_row) + (lane & 7);
+      if (W0 & self) row0[0] = u0;
+      if (V0 & self) row0[8] = y0;
+      if (W1 & self) row1[0] = u1;
+      if (V1 & self) row1[8] = y1;
+      run = mid + __popc(W1) + __popc(V1);
+      if (lane == 0) reinterpret_cast<uint2*>(pk)[z] = make_uint2(byte_bits(W0) + byte_bits(V0), byte_bits(W1) + byte_bits(V1));
+      wide |= 1u << z;
+    } else {
+      int e[8];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int lo = (int)(t[i] << 16) >> 16;
+        e[i] = lo - 128;
+        e[4 + i] = ((int)(t[i] - (uint32_t)lo) >> 16) - 128;
+      }
+      if (lane == 0) e[0] += corner - (1 << 14);
+      uint32_t W0, W1;
+      run = wide_plane(e, words, W0, W1, lane);
+      if (lane == 0) reinterpret_cast<uint2*>(pk)[0] = make_uint2(W0, W1);
+      wide = 1u;
+    }
+    return true;
+  };
+  asm volatile("cp.async.wait_group 1;" ::: "memory");
+  __syncwarp();
+#pragma unroll 1
+  for (int z = 0; z < kTZ; z += 2) {
+    float x[8];
+    if (z == 2) {
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+      __syncwarp();
+    }
+    staged_plane(pk, z, x);
+    if (!plane(z, x, Int<1>{})) {
+      whole = z == 0;
+      return bad ? 0 : kNoHalves;
+    }
+    staged_plane(pk, z + 1, x);
+    if (!plane(z + 1, x, Int<0>{})) return bad ? 0 : kNoHalves;
+  }
+  __syncwarp();
+  if (lane < 16 && !((wide >> (lane >> 1)) & 1u)) {
+    uint32_t* rows = reinterpret_cast<uint32_t*>(pk) + lane;
+    *rows = byte_bits(*rows);
+  }
+  const uint32_t pad = (0u - run) & 3u;
+  if ((uint32_t)lane < pad) words[run + lane] = 0u;
+  return run;
+}
+
+// Planes of four rows of at most eight bits each, the zig-zag residuals of a lane in the bytes of u: the words, one
+// bit plane a lane, and which lanes hold one that is stored.
+__device__ __forceinline__ uint32_t row_planes(uint32_t& u, int lane) {
+  const uint32_t stored = planes_up_to(__reduce_or_sync(0xffffffffu, u));
+  u = transpose32(u, lane);
+  return stored;
 }
 
 // Packs the warp's tile to `pk` (64 width bytes, then the planes). Returns its words, or 0 and `bad` as
 // soon as a plane shows that it has to be stored raw.
-template <int kVec>
-__device__ __forceinline__ uint32_t pack_planes(const PlaneIO<kVec>& io, const SzLocalArgs& a, unsigned char* pk, bool& bad) {
-  const int lane = io.lane;
+__device__ __forceinline__ uint32_t pack_planes(const SzLocalArgs& a, unsigned char* pk, bool& bad) {
+  const int lane = threadIdx.x & 31;
   uint32_t* words = reinterpret_cast<uint32_t*>(pk + kRows);
   int before[8];
 #pragma unroll
   for (int e = 0; e < 8; ++e) before[e] = kCodeBias;
   uint32_t run = 0;
-  float ahead[8];
-  io.load(0, ahead);
-  constexpr int kTurns = kVec == 1 ? 1 : 2;   // 300 x 300 x 403, tiles of 7 KB: 120 us with one turn at a time, 124 with two
-#pragma unroll kTurns
+#pragma unroll 1
   for (int z = 0; z < kTZ; ++z) {
     float x[8];
-#pragma unroll
-    for (int e = 0; e < 8; ++e) x[e] = ahead[e];
-    if (z + 1 < kTZ) io.load(z + 1, ahead);   // the next plane is on its way while this one is packed
-    io.settle(x);
+    staged_plane(pk, z, x);
     int q[8], d[8];
     plane_codes(x, a, q, bad);
     if (bad) return 0;
@@ -857,39 +1128,24 @@ __device__ __forceinline__ uint32_t pack_planes(const PlaneIO<kVec>& io, const S
       t[e] = (uint32_t)(d[e] + 128);
       high |= t[e];
     }
-    uint32_t W0 = 0u, W1 = 0u, u[8], tot_lo, tot;
-    const bool narrow = !__any_sync(0xffffffffu, high > 0xffu);
-    if (narrow) {
+    uint32_t W0, W1, tot;
+    if (!__any_sync(0xffffffffu, high > 0xffu)) {
+      uint32_t u[2];
 #pragma unroll
       for (int k = 0; k < 2; ++k) {
         const uint32_t b = __byte_perm(__byte_perm(t[4 * k], t[4 * k + 1], 0x0040), __byte_perm(t[4 * k + 2], t[4 * k + 3], 0x0040), 0x5410);
-        const uint32_t minus = ((b >> 7) & 0x01010101u) ^ 0x01010101u;
-        u[k] = transpose32(((b << 1) & 0xfefefefeu) ^ (minus * 0xffu), lane);
+        u[k] = ((b + b) & 0xfefefefeu) ^ ~byte_signs(b);
       }
-      // a lane, plane j of its row, is there if any plane from j up of that row holds a bit
-      W0 = __ballot_sync(0xffffffffu, ((__ballot_sync(0xffffffffu, u[0] != 0u) >> lane) & (0xffu >> (lane & 7))) != 0u);
-      W1 = __ballot_sync(0xffffffffu, ((__ballot_sync(0xffffffffu, u[1] != 0u) >> lane) & (0xffu >> (lane & 7))) != 0u);
+      W0 = row_planes(u[0], lane);
+      W1 = row_planes(u[1], lane);
       if (lane < 8) pk[8 * z + lane] = (unsigned char)__popc(((lane < 4 ? W0 : W1) >> (8 * (lane & 3))) & 0xffu);
-      tot_lo = __popc(W0);
+      const uint32_t tot_lo = __popc(W0), below = (1u << lane) - 1u;
       tot = tot_lo + __popc(W1);
-      const uint32_t below = (1u << lane) - 1u;
       if ((W0 >> lane) & 1u) words[run + __popc(W0 & below)] = u[0];
       if ((W1 >> lane) & 1u) words[run + tot_lo + __popc(W1 & below)] = u[1];
     } else {
-#pragma unroll
-      for (int e = 0; e < 8; ++e) u[e] = ((uint32_t)d[e] << 1) ^ (uint32_t)(d[e] >> 31);
-#pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        const uint32_t w = 32 - __clz((int)__reduce_or_sync(0xffffffffu, u[e]));
-        if (e < 4) W0 |= w << (8 * e);
-        else W1 |= w << (8 * (e - 4));
-      }
-      tot_lo = bytesum(W0);
-      tot = tot_lo + bytesum(W1);
+      tot = wide_plane(d, words + run, W0, W1, lane);
       if (lane == 0) reinterpret_cast<uint2*>(pk)[z] = make_uint2(W0, W1);
-      uint32_t ua[4] = {u[0], u[1], u[2], u[3]}, ub[4] = {u[4], u[5], u[6], u[7]};
-      wide_planes4<true>(ua, W0, run, words, lane);
-      wide_planes4<true>(ub, W1, run + tot_lo, words, lane);
     }
     run += tot;
   }
@@ -898,13 +1154,15 @@ __device__ __forceinline__ uint32_t pack_planes(const PlaneIO<kVec>& io, const S
   return run;
 }
 
-// A warp stages the whole of its tile, 8256 bytes at most, three CTAs an SM. With 4 KiB each, tiles that
-// were larger went through the codec a second time, to their places: 512^3 values of white noise, bound
-// 1e-5 of their range (2.05 bytes a value) 470 us, 267 so; 1e-6 (3.4 bytes) 440 and 281. Where lines
-// lie anywhere (kVec 1) a plane passes through the last KB of the stage, which only the words of the
-// last plane can reach, after it has passed; three CTAs of 80 registers are the faster ones there too
-// (130 x 201 x 258, bound 1e-4: 24.7 us with four of 64, 22.7 so). A tile that turns out raw is left at
-// that plane and copied (bound 1e-7, all raw: 317 us with all eight planes looked at first, 235 so). B200.
+// A warp stages the whole of its tile, 8256 bytes at most, three CTAs an SM; with less of it, tiles that were larger
+// went through the codec a second time, to their places (512^3 values of white noise, bound 1e-5 of their range,
+// 470 us). Bound by instructions at 24 warps an SM: ncu, 384^3, 47.9 M of them, 217 a plane with all that a tile needs
+// besides, 68 % of the issue slots, 54 % of the pipe of logical operations. With planes loaded to registers one ahead
+// (moves of eight registers a plane), residuals one to a word, the masks of the bit transpose chosen at each use and planes
+// of 9 to 16 bits a row at a time it was 62.3 M. (B200, us, that / so: 512^3 field, bound 1e-4 of its range, 173 / 146;
+// 1e-3 168 / 140; 1e-5 189 / 180; with 30 added to its values 179 / 154; 300 x 300 x 404 55.5 / 53.5, x 403 67 / 64; 130
+// x 201 x 258 22.8 / 18.6; white noise 512^3, 1e-5 266 / 268, 1e-6 265 / 248, 1e-7, all raw, 238 / 209.) Operands of the
+// packed operations kept in registers, or given as pairs of arguments, changed nothing; one vote for both tests neither.
 template <int kVec>
 __global__ void __launch_bounds__(kSzThreads, 3) sz_pack_kernel(const __grid_constant__ SzLocalArgs a) {
   extern __shared__ __align__(16) unsigned char stages[];   // kClusterSize * kTileCap
@@ -913,11 +1171,23 @@ __global__ void __launch_bounds__(kSzThreads, 3) sz_pack_kernel(const __grid_con
   const unsigned int tile = blockIdx.x * kClusterSize + k;
   char* group = a.slots + (size_t)blockIdx.x * kGroupStride;
   unsigned char* stage = stages + k * kTileCap;
-  const PlaneIO<kVec> io(a.in, a, tile_coord(a, tile), reinterpret_cast<float*>(stage + kTileCap - 4 * kTX * kTY));
+  const TileCoord coord = tile_coord(a, tile);
   uint32_t size = 0;
   bool raw = false;
   if (tile < (unsigned)a.tiles_x * a.tiles_y * a.tiles_z) {
-    const uint32_t words = pack_planes<kVec>(io, a, stage, raw);
+    stage_tile<kVec>(a, coord, stage);
+    bool whole = false;
+    uint32_t words = pack_halves(a, stage, raw, whole);
+    if (words == kNoHalves) {
+      if (!whole) {
+        __syncwarp();
+        stage_tile<kVec>(a, coord, stage);
+      }
+      asm volatile("cp.async.wait_all;" ::: "memory");
+      __syncwarp();
+      words = pack_planes(a, stage, raw);
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");   // of a tile that was left early
     size = raw ? kTileCap : (kRows + 4u * words + 15u) & ~15u;
   }
   if (lane == 0) s_size[k] = size;
@@ -936,6 +1206,8 @@ __global__ void __launch_bounds__(kSzThreads, 3) sz_pack_kernel(const __grid_con
     return;
   }
   reinterpret_cast<uint16_t*>(dst)[lane] = lane == 0 ? 255 : 0;   // marker, then the fp32 values
+  __syncwarp();
+  const PlaneIO<kVec> io(a.in, a, coord, reinterpret_cast<float*>(stage + kRows));
   float ahead[8];
   io.load(0, ahead);
 #pragma unroll 2
@@ -1003,12 +1275,6 @@ __device__ __forceinline__ void halves_of(const uint32_t (&b)[2], uint32_t bias,
     const __half2 d = __hsub2(*reinterpret_cast<const __half2*>(&w), *reinterpret_cast<const __half2*>(&bias));
     h[i] = *reinterpret_cast<const uint32_t*>(&d);
   }
-}
-// 255 in the bytes whose highest bit is set, 0 in the others.
-__device__ __forceinline__ uint32_t byte_signs(uint32_t v) {
-  uint32_t m;
-  asm("prmt.b32 %0, %1, 0, 0xba98;" : "=r"(m) : "r"(v));
-  return m;
 }
 
 // Where a lane writes the codes of PlanePrefix: x = 4 g .. + 3 of the lines y = 2 t and 2 t + 1. kAligned: every line
@@ -1641,6 +1907,7 @@ extern "C" int ccb_sz_compress(const float* in, int nx, int ny, int nz, float eb
   memset(&a, 0, sizeof(a));
   fill_geometry(a, nx, ny, nz, eb);
   a.in = in;
+  a.one = 1.f;
   a.slots = static_cast<char*>(out);
   a.used_bytes = d_used;
   cudaStream_t s = static_cast<cudaStream_t>(stream);

@@ -48,3 +48,29 @@ def test_a_buffer_on_four_bytes_is_unpacked_where_it_lies():
     moved = torch.empty(buf.numel() + 16, dtype=torch.uint8, device="cuda")[4:4 + buf.numel()]
     moved.copy_(buf)
     assert torch.equal(sz.decompress(moved, shape, 1e-2), want)
+
+
+@pytest.mark.parametrize("nx", [0, 4, 5])   # off a whole number of tiles: lines on 32 bytes, on 16, anywhere
+def test_tiles_packed_in_halves_end_where_they_should(nx):
+    """Codes on either side of where two residuals no longer share a word: far from a tile's first code, first
+    codes of more than 8, 16 and 22 bits, in the first plane and in the last."""
+    g = torch.Generator().manual_seed(9)
+    tiles = []
+    for corner in (0, 127, -128, 128, 31999, -32000, 32000, (1 << 21) - 4097, (1 << 21) - 4095, -(1 << 21) - 5, (1 << 22) - 3):
+        for spread in (3, 4093, 4094, 4095, 40000):
+            t = torch.randint(-1, 2, (8, 8, 32), generator=g) + corner
+            t[0, 0, 0] = corner
+            t[0 if spread % 2 else 7, 5, 31] = corner + spread if corner < 0 or spread < 5 else corner - spread
+            tiles.append(t)
+    alternating = torch.where((torch.arange(8)[:, None, None] + torch.arange(8)[:, None] + torch.arange(32)) % 2 == 0, 4094, -4094)
+    alternating[0, 0, 0] = 0
+    tiles.append(alternating)   # residuals of 8 x 4094
+    tiles.append(torch.zeros(8, 8, 32, dtype=torch.int64))
+    q = torch.cat(tiles, dim=2)
+    step = torch.tensor(2 * EB, dtype=torch.float32) * (1 - 2.0 ** -10)
+    f = q.float() * step
+    f += (torch.rand(f.shape, generator=g) - 0.5) * step * (q.abs() < 4000)   # off the grid, near ties among them
+    f = f[:, :, :f.shape[2] - (32 - nx if nx else 0)].contiguous()
+    buf, _ = sz.compress(f.cuda(), EB)
+    want = sz.encode_cpu(f.numpy(), EB)
+    assert (sz.to_container(buf, f.shape, EB).cpu().numpy() == want).all()
