@@ -142,11 +142,12 @@ int local_exchange(ccb_comm* c, const ExchangeArgs& x, int dtype, int codec, cud
       }
       a.dst[dsts] = static_cast<char*>(x.recv[p]) + x.recv_off[p][r] * es;
       aligned = aligned && on32(a.dst[dsts]);
+      if (a.dst[dsts] == a.src[a.nblocks - 1]) a.in_place |= 1ull << (a.nblocks - 1);
       ++dsts;
     }
   }
   a.first_dst[a.nblocks] = (uint8_t)dsts;
-  // At any offset every run ends in element stores: runs as long as leave every warp slot of the chip
+  // At any offset a run reads the unit before it once more: runs as long as leave every warp slot of the chip
   // its own. Aligned units have nothing to do with one another.
   const uint64_t slots = (uint64_t)comm_sms(c) * 24;
   a.run = 1;

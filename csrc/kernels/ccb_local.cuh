@@ -324,14 +324,17 @@ struct LocalExchangeArgs {
   void* dst[CCB_MAX_RANKS * CCB_MAX_RANKS];                // of all blocks, in their order
   uint32_t first_run[CCB_MAX_RANKS * CCB_MAX_RANKS + 1];   // runs before each block
   uint8_t first_dst[CCB_MAX_RANKS * CCB_MAX_RANKS + 1];
+  uint64_t in_place;   // blocks that are their own destination, a bit each
   int nblocks;
   uint32_t run;
 };
 
 // kAnyOffset: blocks may start anywhere. Where the destinations of a block lie alike on their
 // 32-byte sectors the warp rotates a unit once for all of them, and the first sector of a unit is
-// completed with what the unit before left over, so that only the ends of a run are written
-// element by element. (Without kAnyOffset a run is one unit.)
+// completed with what the unit before left over; a run begins with that unit, of which it stores nothing
+// else, so that only the ends of a block are written element by element. (With the ends of runs of four written so,
+// 64 stores of an element for eight of a lane's 32 bytes, an all-gather of 8 x 1,638,401 bf16 in fp8 took 50 us, 46 so; B200.)
+// A block in place keeps to its own units: the one before may have been written. (Without kAnyOffset a run is one unit.)
 template <class T, class C, bool kAnyOffset>
 __global__ void __launch_bounds__(kLocalThreads, kAnyOffset ? (sizeof(T) == 4 ? 2 : 3) : 6) local_exchange_kernel(const __grid_constant__ LocalExchangeArgs a) {
   constexpr int W = 4 * (int)sizeof(T), kPer = 4 / (int)sizeof(T);   // words of a lane, elements of a word
@@ -371,9 +374,12 @@ __global__ void __launch_bounds__(kLocalThreads, kAnyOffset ? (sizeof(T) == 4 ? 
       for (size_t u = u0; u < u1; ++u) plain(u * kWarpElems, Int<1>{});
     } else if (u0 < u1) {
       Wide16<T> next, left;   // left, in lane 0: the last `mis` elements of the unit before
-      local_load<T, true>(src, u0 * kWarpElems + lane * kLaneElems, cnt, true, next);
+      const bool apart = !(a.in_place >> b & 1u);
+      const size_t start = apart && mis && u0 ? u0 - 1 : u0;
+      size_t u = start;
+      local_load<T, true>(src, u * kWarpElems + lane * kLaneElems, cnt, true, next);
 #pragma unroll 1
-      for (size_t u = u0; u < u1; ++u) {
+      for (; u < u1; ++u) {
         const size_t idx = u * kWarpElems + lane * kLaneElems;
         float v[16];
         wide16_to_f<T>(next, v);
@@ -383,16 +389,16 @@ __global__ void __launch_bounds__(kLocalThreads, kAnyOffset ? (sizeof(T) == 4 ? 
         pack16<T>(v, o);
         rotate_up<T>(o.w, mis, lane);
         const Wide16<T> mine = o;   // lane 0: this unit's last `mis` elements, then its first 16 - mis
-        if (lane == 0 && u > u0) {
+        if (lane == 0 && u > start) {
 #pragma unroll
           for (int k = 0; k < W; ++k) {
             if ((uint32_t)(kPer * k + kPer - 1) < mis) o.w[k] = left.w[k];
             else if (kPer == 2 && (uint32_t)(2 * k) < mis) o.w[k] = __byte_perm(left.w[k], o.w[k], 0x7610);
           }
         }
-        const bool sector = lane != 0 || u > u0 || mis == 0;
+        const bool sector = lane != 0 || u > start || mis == 0;
 #pragma unroll 1
-        for (int d = d0; d < d1; ++d) {
+        for (int d = u < u0 ? d1 : d0; d < d1; ++d) {
           T* p = static_cast<T*>(a.dst[d]) + idx - mis;
           if (sector) {
 #pragma unroll
@@ -405,7 +411,7 @@ __global__ void __launch_bounds__(kLocalThreads, kAnyOffset ? (sizeof(T) == 4 ? 
         }
         left = mine;
       }
-      if (lane == 0) {   // behind the last whole unit of the run
+      if (lane == 0 && (u1 == whole || !apart)) {   // behind the last whole unit of the block
 #pragma unroll 1
         for (int d = d0; d < d1; ++d) {
           T* p = static_cast<T*>(a.dst[d]) + u1 * kWarpElems - mis;

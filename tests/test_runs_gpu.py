@@ -1,0 +1,46 @@
+"""Exchanges of ranks of one GPU at odd offsets, in runs of one to eight units a warp: the sectors where runs
+meet, and blocks in place. Against the kernels of ranks on several GPUs: same inputs, same bits."""
+import pytest
+import torch
+
+from ccbench_b200 import Communicator
+
+pytestmark = pytest.mark.gpu
+
+
+def _values(count, dtype, seed):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    x = torch.randn(count, generator=g, device="cuda").to(dtype)
+    x[::97] *= 100
+    return x
+
+
+def _both(comm, call):
+    got = call()
+    comm.set_trace(True)
+    want = call()
+    comm.set_trace(False)
+    torch.cuda.synchronize()
+    assert comm.status()[0] == 0
+    for a, b in zip(got, want):
+        assert torch.equal(a.view(torch.uint8), b.view(torch.uint8))
+
+
+@pytest.mark.parametrize("dtype,codec", [(torch.bfloat16, "fp8"), (torch.float16, "int4"), (torch.float32, "int8")])
+@pytest.mark.parametrize("n,count", [(2, 400_001), (8, 600_003), (8, 1_000_007), (4, 3_700_001)])
+@pytest.mark.parametrize("in_place", [False, True])
+def test_all_gather_of_odd_blocks(dtype, codec, n, count, in_place):
+    comm = Communicator.local(n, arena_bytes=160 << 20)
+    xs = [_values(count, dtype, r) for r in range(n)]
+
+    def call():
+        out = [torch.full((n * count + 3,), 7.0, dtype=dtype, device="cuda")[1:-2] for _ in range(n)]
+        if in_place:
+            for r in range(n):
+                out[r][r * count:(r + 1) * count] = xs[r]
+        comm.all_gather([o[r * count:(r + 1) * count] for r, o in enumerate(out)] if in_place else xs, out, codec=codec)
+        return out
+
+    _both(comm, call)
+    comm.close()
+
