@@ -123,6 +123,13 @@ __device__ __forceinline__ float absmax16(const float (&v)[16]) {
   return m;
 }
 
+// The largest magnitude of three, NaN if any is.
+__device__ __forceinline__ float max3_abs_nan(float a, float b, float c) {
+  float m;
+  asm("max.NaN.abs.f32 %0, %1, %2, %3;" : "=f"(m) : "f"(a), "f"(b), "f"(c));
+  return m;
+}
+
 template <int G>
 struct CodecInt8 {
   static_assert(G == 128 || G == 256, "group must be 128 or 256");
@@ -205,21 +212,40 @@ struct CodecInt4 {
   static constexpr int kLanes = kGroup / 16;
   struct Packet { uint2 q; float scale; };
   static __host__ __device__ size_t slot_bytes(size_t pad) { return pad / 2 + pad / kGroup * 4; }
-  static __device__ __forceinline__ void encode(const float (&v)[16], Packet& pk) {
+  static __device__ __forceinline__ float absmax(const float (&v)[16]) {
     float m = absmax16(v);
 #pragma unroll
     for (int d = 1; d < kLanes; d <<= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, d));
+    return m;
+  }
+  // Whether every product v * (7 / absmax) of the warp is a number of at most 7 in magnitude, which adding 1.5 * 2^23
+  // rounds as the conversion does. NaN (which absmax passes over), infinities and groups of values so small that
+  // 7 / absmax overflows take the conversion, for what it makes of them.
+  static __device__ __forceinline__ bool usual(const float (&v)[16], float m) {
+    float worst = 0.f;   // NaN if any is
+#pragma unroll
+    for (int i = 0; i < 16; i += 2) worst = max3_abs_nan(worst, v[i], v[i + 1]);
+    return !__any_sync(0xffffffffu, !(m < 1e37f) || (m > 0.f && m < 1e-36f) || worst != worst);
+  }
+  static __device__ __forceinline__ void encode(const float (&v)[16], Packet& pk) {
+    const float m = absmax(v);
     const float inv = m > 0.f ? 7.f / m : 0.f;
     pk.scale = m / 7.f;
     uint32_t w[2] = {0u, 0u};
+    if (usual(v, m)) {
 #pragma unroll
-    for (int i = 0; i < 16; ++i) w[i >> 3] |= ((uint32_t)__float2int_rn(v[i] * inv) & 0xfu) << (4 * (i & 7));
+      for (int i = 0; i < 16; ++i) w[i >> 3] |= (__float_as_uint(__fadd_rn(__fmul_rn(v[i], inv), 12582912.f)) & 0xfu) << (4 * (i & 7));
+    } else {
+#pragma unroll
+      for (int i = 0; i < 16; ++i) w[i >> 3] |= ((uint32_t)__float2int_rn(v[i] * inv) & 0xfu) << (4 * (i & 7));
+    }
     pk.q = make_uint2(w[0], w[1]);
   }
   static __device__ __forceinline__ void decode(const Packet& pk, float (&v)[16]) {
     const uint32_t w[2] = {pk.q.x, pk.q.y};
 #pragma unroll
-    for (int i = 0; i < 16; ++i) v[i] = (float)((int)(w[i >> 3] << (28 - 4 * (i & 7))) >> 28) * pk.scale;
+    for (int i = 0; i < 16; ++i)   // the nibble, biased by 8, in the low mantissa bits of 1.5 * 2^23
+      v[i] = __fadd_rn(__uint_as_float(((w[i >> 3] >> (4 * (i & 7))) & 0xfu) ^ 0x4B400008u), -12582920.f) * pk.scale;
   }
   // v - decode(pk) in one rounding.
   static __device__ __forceinline__ void residual(const Packet& pk, const float (&v)[16], float (&e)[16]) {
@@ -227,10 +253,25 @@ struct CodecInt4 {
 #pragma unroll
     for (int i = 0; i < 16; ++i) e[i] = __fmaf_rn(-(float)((int)(w[i >> 3] << (28 - 4 * (i & 7))) >> 28), pk.scale, v[i]);
   }
+  // The rounded multiples themselves, without the conversions to integers and back that four-bit codes take
+  // (8 ranks of 32 MiB of f16 reduced to their owners 65 us with them, 55 so; a ring of 8 x 16 MiB of bf16 46.7
+  // and 44.6; B200).
   static __device__ __forceinline__ void round_trip(float (&v)[16]) {
-    Packet pk;
-    encode(v, pk);
-    decode(pk, v);
+    const float m = absmax(v);
+    if (usual(v, m)) {
+      const float inv = m > 0.f ? 7.f / m : 0.f, scale = m / 7.f;
+      const f32x2 inv2 = pair2(inv, inv), scale2 = pair2(scale, scale), back2 = pair2(-12582912.f, -12582912.f);
+#pragma unroll
+      for (int i = 0; i < 16; i += 2) {
+        float a, b;
+        split2(mul2(pair2(v[i], v[i + 1]), inv2), a, b);
+        split2(mul2(add2(pair2(__fadd_rn(a, 12582912.f), __fadd_rn(b, 12582912.f)), back2), scale2), v[i], v[i + 1]);
+      }
+    } else {
+      Packet pk;
+      encode(v, pk);
+      decode(pk, v);
+    }
   }
   static __device__ __forceinline__ void store(char* slot, size_t pad, size_t idx, const Packet& pk) {
     stg8(slot + idx / 2, pk.q);

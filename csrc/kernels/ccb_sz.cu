@@ -773,12 +773,6 @@ struct PlaneIO {
   }
 };
 
-// The largest magnitude of three, NaN if any is.
-__device__ __forceinline__ float max_abs3(float a, float b, float c) {
-  float m;
-  asm("max.NaN.abs.f32 %0, %1, %2, %3;" : "=f"(m) : "f"(a), "f"(b), "f"(c));
-  return m;
-}
 // The packer brings the values of a tile to shared memory, [z][y][x] behind the 64 bytes of its widths, all planes under
 // way at once, and packs it in place: the words of planes 0 to z end where plane z + 1 begins, or before. Two
 // neighbouring pieces of 16 bytes change places on odd lines, for a lane reads two of them and eight lanes at a time
@@ -962,8 +956,8 @@ __device__ __forceinline__ uint32_t pack_halves(const SzLocalArgs& a, unsigned c
     }
 #pragma unroll
     for (int i = 0; i < 4; ++i) split2(add2(r2[i], first2), away[2 * i], away[2 * i + 1]);
-    const float worst = max_abs3(max_abs3(diff[0], diff[1], diff[2]), max_abs3(diff[3], diff[4], diff[5]), max_abs3(diff[6], diff[7], 0.f));
-    const float apart = max_abs3(max_abs3(away[0], away[1], away[2]), max_abs3(away[3], away[4], away[5]), max_abs3(away[6], away[7], 0.f));
+    const float worst = max3_abs_nan(max3_abs_nan(diff[0], diff[1], diff[2]), max3_abs_nan(diff[3], diff[4], diff[5]), max3_abs_nan(diff[6], diff[7], 0.f));
+    const float apart = max3_abs_nan(max3_abs_nan(away[0], away[1], away[2]), max3_abs_nan(away[3], away[4], away[5]), max3_abs_nan(away[6], away[7], 0.f));
     if (__any_sync(0xffffffffu, !(worst <= half && apart <= 4094.f) || abs(corner) > kCodeBias - 4096)) {
       if (__any_sync(0xffffffffu, !(apart <= 4094.f) || abs(corner) > kCodeBias - 4096)) return false;
 #pragma unroll
