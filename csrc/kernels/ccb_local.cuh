@@ -106,6 +106,30 @@ __device__ __forceinline__ void local_store(T* base, size_t idx, size_t limit, b
   }
 }
 
+// Units of 512 elements on 32 bytes by way of shared memory: what a warp has under way does not take registers
+// there. kUnitPieces pieces of 16 bytes each; a lane reads sizeof(T) of them that follow one another, and they change
+// places so that eight lanes at a time find theirs in different banks.
+template <class T> constexpr int kUnitPieces = 32 * (int)sizeof(T);
+template <class T> __device__ __forceinline__ uint32_t unit_piece(uint32_t c) { return c ^ (c >> 3 & (sizeof(T) == 4 ? 3u : 1u)); }
+template <class T>
+__device__ __forceinline__ void bring_unit(uint4* to, const T* from) {   // to be waited for by the lane, then met by the warp
+  const uint32_t lane = threadIdx.x & 31, at = (uint32_t)__cvta_generic_to_shared(to);
+#pragma unroll
+  for (int i = 0; i < (int)sizeof(T); ++i)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(at + 16u * unit_piece<T>(lane + 32 * i)), "l"(reinterpret_cast<const char*>(from) + 16 * (lane + 32 * i)) : "memory");
+}
+template <class T>
+__device__ __forceinline__ void brought_unit(const uint4* unit, float (&v)[16]) {   // the lane's 16 elements
+  const uint32_t lane = threadIdx.x & 31;
+  Wide16<T> raw;
+#pragma unroll
+  for (int i = 0; i < (int)sizeof(T); ++i) {
+    const uint4 p = unit[unit_piece<T>(sizeof(T) * lane + i)];
+    raw.w[4 * i] = p.x; raw.w[4 * i + 1] = p.y; raw.w[4 * i + 2] = p.z; raw.w[4 * i + 3] = p.w;
+  }
+  wide16_to_f<T>(raw, v);
+}
+
 template <class T>
 __device__ __forceinline__ void pack16(const float (&v)[16], Wide16<T>& o) {
   if constexpr (sizeof(T) == 4) {

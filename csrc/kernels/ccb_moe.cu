@@ -201,72 +201,120 @@ struct MoeLocalArgs {
   uint32_t first_out[CCB_MAX_RANKS][CCB_MAX_RANKS];  // [src][dst]: first entry of that block in perm
   uint64_t hidden;
   uint32_t tokens, row_units, chunk_rows, chunks;   // a chunk of a block: its rows for one CTA
+  uint32_t batch_units, groups;                     // units of a row for a warp, such groups of units in a row
   int topk, n;
 };
-constexpr int kMoeLocalThreads = 256;
+// Both ways a warp brings what it works on to shared memory first, up to 4 KiB under way at once.
+constexpr int kMoeLocalThreads = 128, kMoeStage = 4096;
+template <class T> constexpr int kMoeSlots = kMoeStage / 16 / kUnitPieces<T>;   // units of 512 elements in it
+template <class T>
+__device__ __forceinline__ void moe_bring(uint4* stage, const char* from, uint32_t units) {   // consecutive units
+#pragma unroll 1
+  for (uint32_t u = 0; u < units; ++u, from += kWarpElems * sizeof(T), stage += kUnitPieces<T>) bring_unit<T>(stage, reinterpret_cast<const T*>(from));
+}
+__device__ __forceinline__ void moe_brought() {
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  __syncwarp();
+}
 
 // Dispatch. The rows of a rank are sorted by destination, and within one by token. A CTA takes
-// `chunk_rows` rows of one block, a warp one unit at a time; the blocks of a rank take turns chunk by
+// `chunk_rows` rows of one block, a warp some units of a row at a time; the blocks of a rank take turns chunk by
 // chunk, so that the topk copies of a token, which lie at about the same depth of their blocks, are
 // read from memory once and from L2 after that.
 template <class T, class C>
-__global__ void __launch_bounds__(kMoeLocalThreads, 6) moe_local_dispatch_kernel(const __grid_constant__ MoeLocalArgs a) {
-  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, upr = a.row_units;
+__global__ void __launch_bounds__(kMoeLocalThreads, 12) moe_local_dispatch_kernel(const __grid_constant__ MoeLocalArgs a) {
+  __shared__ uint4 stages[kMoeLocalThreads / 32][kMoeStage / 16];
+  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t n = (uint32_t)a.n, p = blockIdx.x % n, c = blockIdx.x / n % a.chunks, r = blockIdx.x / n / a.chunks;
   const uint32_t j0 = c * a.chunk_rows, rows = a.cnt[r][p];
   if (j0 >= rows) return;
-  const uint32_t units = min(a.chunk_rows, rows - j0) * upr;
-  const T* src = static_cast<const T*>(a.src[r]);
+  const uint32_t items = min(a.chunk_rows, rows - j0) * a.groups;
   const int32_t* perm = a.perm[r] + a.first_out[r][p] + j0;
-  T* dst = static_cast<T*>(a.dst[p]) + (size_t)(a.first_in[p][r] + j0) * a.hidden;   // unit u of whole rows starts at element 512 u
+  T* dst = static_cast<T*>(a.dst[p]) + (size_t)(a.first_in[p][r] + j0) * a.hidden;
 #pragma unroll 1
-  for (uint32_t u = warp; u < units; u += kMoeLocalThreads / 32) {
-    const uint32_t j = u / upr;
-    Wide16<T> raw;
-    local_load<T>(src + (size_t)perm[j] * a.hidden, (size_t)(u - j * upr) * kWarpElems + lane * kLaneElems, 0, true, raw);
-    float v[16];
-    wide16_to_f<T>(raw, v);
-    C::round_trip(v);
-    pack16<T>(v, raw);
-    local_store<T>(dst, (size_t)u * kWarpElems + lane * kLaneElems, 0, true, raw);
+  for (uint32_t i = warp; i < items; i += blockDim.x / 32) {
+    const uint32_t j = i / a.groups, u0 = (i - j * a.groups) * a.batch_units, units = min(a.batch_units, a.row_units - u0);
+    moe_bring<T>(stages[warp], reinterpret_cast<const char*>(static_cast<const T*>(a.src[r]) + (size_t)perm[j] * a.hidden + (size_t)u0 * kWarpElems), units);
+    moe_brought();
+    T* out = dst + (size_t)j * a.hidden + (size_t)u0 * kWarpElems;
+#pragma unroll 1
+    for (uint32_t u = 0; u < units; ++u) {
+      float v[16];
+      brought_unit<T>(stages[warp] + u * kUnitPieces<T>, v);
+      C::round_trip(v);
+      Wide16<T> o;
+      pack16<T>(v, o);
+      local_store<T>(out, (size_t)u * kWarpElems + lane * kLaneElems, 0, true, o);
+    }
+    __syncwarp();
   }
 }
 
-// Combine: a warp takes 512 elements of one token and fetches them from the topk rows that hold it, one
-// after the other: what a warp waits for in turn, indices and rows, is hidden by as many warps as fit.
-// (8 ranks, 8192 x 4096 bf16, top 2, fp8: 323 us with 40 warps an SM, whose 48 registers spill 32 to 44
-// bytes but for no codec; 337 with two rows at once and 32 warps, 380 with two and 24. Top 4 of 2048 x
-// 2048 80 and 79, top 1 33 and 41. B200.)
-// An index outside its block (the entry of a dropped pair) contributes nothing.
+// Combine: a warp takes some units of 512 elements of one token and brings them from all rows that hold the token to
+// shared memory, 4 KiB under way at once, where a row at a time in registers left a warp waiting for one row after
+// the other, 1 KiB each. An index outside its block (the entry of a dropped pair) contributes nothing.
+// (8 ranks, 8192 x 4096 bf16, top 2, fp8: 328 us a row at a time with 40 warps an SM, 267 so, of 246 that the memory
+// needs; 2048 x 4096 fp32, top 2, int8 162 and 131; top 1 of 4096 x 4096 62 and 47.5; top 4 of 2048 x 2048 in int8, bound by
+// its codec, 84 and 84. 36 warps an SM, 56 registers: with 40, which spill, 265 but 98 at top 4, with 32 276. B200.)
 template <class T, class C>
-__global__ void __launch_bounds__(kMoeLocalThreads, sizeof(T) == 4 ? 3 : 5) moe_local_combine_kernel(const __grid_constant__ MoeLocalArgs a) {
-  const uint32_t lane = threadIdx.x & 31, upr = a.row_units, per_rank = a.tokens * upr;
-  const uint32_t w = ccb_grid_warp(blockIdx.x, blockDim.x, threadIdx.x);
+__global__ void __launch_bounds__(kMoeLocalThreads, 9) moe_local_combine_kernel(const __grid_constant__ MoeLocalArgs a) {
+  constexpr int kSlots = kMoeSlots<T>;
+  __shared__ uint4 stages[kMoeLocalThreads / 32][kMoeStage / 16];
+  const uint32_t lane = threadIdx.x & 31;
+  uint4* stage = stages[threadIdx.x >> 5];
+  const uint32_t w = ccb_grid_warp(blockIdx.x, blockDim.x, threadIdx.x), per_rank = a.tokens * a.groups;
   if (w >= per_rank * (uint32_t)a.n) return;
-  const uint32_t r = w / per_rank, u = w - r * per_rank, tok = u / upr;
-  const size_t col = (size_t)(u - tok * upr) * kWarpElems + lane * kLaneElems, pair0 = (size_t)tok * a.topk;
+  const uint32_t r = w / per_rank, item = w - r * per_rank, tok = item / a.groups, u0 = (item - tok * a.groups) * a.batch_units;
+  const uint32_t units = min(a.batch_units, a.row_units - u0);
+  const size_t pair0 = (size_t)tok * a.topk;
   const int32_t* dest = a.dest_rank[r] + pair0;
   const int32_t* pos = a.pos[r] + pair0;
   const float* gate = a.gate[r] + pair0;
+  T* out = static_cast<T*>(a.dst[r]) + (size_t)tok * a.hidden + (size_t)u0 * kWarpElems;
   float acc[16];
 #pragma unroll
   for (int i = 0; i < 16; ++i) acc[i] = 0.f;
 #pragma unroll 1
-  for (int k = 0; k < a.topk; ++k) {
-    const uint32_t q = (uint32_t)dest[k], j = (uint32_t)pos[k];
-    const float g = gate[k];
-    if (q >= (uint32_t)a.n || j >= a.cnt[r][q]) continue;
-    Wide16<T> raw;
-    local_load<T>(static_cast<const T*>(a.src[q]) + (size_t)(a.first_in[q][r] + j) * a.hidden, col, 0, true, raw);
-    float d[16];
-    wide16_to_f<T>(raw, d);
-    C::round_trip(d);
+  for (int k0 = 0; k0 < a.topk; k0 += kSlots) {   // more than one turn: units is 1
+    const uint32_t rows = (uint32_t)min(kSlots, a.topk - k0);
+    const char* row = nullptr;   // lane k: the k-th row from the unit on
+    float gate_k = 0.f;
+    bool held = false;
+    if (lane < rows) {
+      const uint32_t q = (uint32_t)dest[k0 + lane], j = (uint32_t)pos[k0 + lane];
+      gate_k = gate[k0 + lane];
+      held = q < (uint32_t)a.n && j < a.cnt[r][q];
+      if (held) row = reinterpret_cast<const char*>(static_cast<const T*>(a.src[q]) + (size_t)(a.first_in[q][r] + j) * a.hidden + (size_t)u0 * kWarpElems);
+    }
+    const uint32_t all = __ballot_sync(0xffffffffu, held);
+#pragma unroll 1
+    for (uint32_t k = 0; k < rows; ++k) {
+      const char* from = reinterpret_cast<const char*>(__shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(row), k));
+      if (all >> k & 1u) moe_bring<T>(stage + k * a.batch_units * kUnitPieces<T>, from, units);
+    }
+    moe_brought();
+#pragma unroll 1
+    for (uint32_t u = 0; u < units; ++u) {
+#pragma unroll 1
+      for (uint32_t k = 0; k < rows; ++k) {
+        const float g = __shfl_sync(0xffffffffu, gate_k, k);
+        if (!(all >> k & 1u)) continue;
+        float d[16];
+        brought_unit<T>(stage + (k * a.batch_units + u) * kUnitPieces<T>, d);
+        C::round_trip(d);
 #pragma unroll
-    for (int e = 0; e < 16; ++e) acc[e] += g * d[e];
+        for (int e = 0; e < 16; ++e) acc[e] += g * d[e];
+      }
+      if (k0 + kSlots >= a.topk) {
+        Wide16<T> o;
+        pack16<T>(acc, o);
+        local_store<T>(out + (size_t)u * kWarpElems, lane * kLaneElems, 0, true, o);
+#pragma unroll
+        for (int e = 0; e < 16; ++e) acc[e] = 0.f;
+      }
+    }
+    __syncwarp();
   }
-  Wide16<T> o;
-  pack16<T>(acc, o);
-  local_store<T>(static_cast<T*>(a.dst[r]) + (size_t)tok * a.hidden, col, 0, true, o);
 }
 
 template <template <class, class> class K>
@@ -316,15 +364,18 @@ static int moe_local_launch(ccb_comm* c, const MoeArgs& m, bool combine, int dty
   a.row_units = (uint32_t)(m.hidden / kWarpElems);
   a.tokens = (uint32_t)m.tokens;
   a.topk = m.topk;
+  const uint32_t slots = dtype == CCB_F32 ? kMoeSlots<float> : kMoeSlots<__half>, rows = combine ? (uint32_t)m.topk < slots ? (uint32_t)m.topk : slots : 1u;
+  a.batch_units = rows ? slots / rows : 1u;
+  if (a.batch_units > a.row_units) a.batch_units = a.row_units;
+  a.groups = (a.row_units + a.batch_units - 1) / a.batch_units;
   uint64_t ctas, warps = kMoeLocalThreads / 32;
   if (combine) {
-    const uint64_t units = (uint64_t)a.n * m.tokens * a.row_units, sms = (uint64_t)comm_sms(c);
-    while (warps > 1 && units / warps < sms) warps >>= 1;
-    ctas = (units + warps - 1) / warps;
+    const uint64_t items = (uint64_t)a.n * m.tokens * a.groups, sms = (uint64_t)comm_sms(c);
+    while (warps > 1 && items / warps < sms) --warps;
+    ctas = (items + warps - 1) / warps;
   } else {
-    const uint64_t rows = warps > a.row_units ? warps / a.row_units : 1;   // about a unit a warp
-    a.chunk_rows = (uint32_t)rows;
-    a.chunks = (uint32_t)((max_rows + rows - 1) / rows);
+    a.chunk_rows = warps > a.groups ? (uint32_t)(warps / a.groups) : 1u;   // about an item a warp
+    a.chunks = (uint32_t)((max_rows + a.chunk_rows - 1) / a.chunk_rows);
     ctas = (uint64_t)a.n * a.n * a.chunks;
   }
   if (ctas == 0) return CCB_OK;

@@ -1,9 +1,11 @@
 """Exchanges of ranks of one GPU at odd offsets, in runs of one to eight units a warp: the sectors where runs
-meet, and blocks in place. Against the kernels of ranks on several GPUs: same inputs, same bits."""
+meet, blocks in place, and rows of experts in groups of units that do not divide them. Against the kernels of
+ranks on several GPUs: same inputs, same bits."""
 import pytest
 import torch
 
 from ccbench_b200 import Communicator
+from ccbench_b200.parallel import moe
 
 pytestmark = pytest.mark.gpu
 
@@ -44,3 +46,32 @@ def test_all_gather_of_odd_blocks(dtype, codec, n, count, in_place):
     _both(comm, call)
     comm.close()
 
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("codec", ["none", "int8", "int4"])
+@pytest.mark.parametrize("topk", [1, 2, 3, 5, 9])   # beyond eight the rows of a token take several turns
+@pytest.mark.parametrize("hidden", [512, 1536, 3584])
+def test_rows_in_groups_of_units(dtype, codec, topk, hidden):
+    n, tokens = 3, 61
+    comm = Communicator.local(n, arena_bytes=96 << 20)
+    g = torch.Generator().manual_seed(topk)
+    xs = [_values(tokens * hidden, dtype, r).view(tokens, hidden) for r in range(n)]
+    routes, counts = [], []
+    for r in range(n):
+        ids = torch.randint(0, n, (tokens, topk), generator=g).cuda()
+        routes.append(moe.plan_route(ids, torch.rand(tokens, topk, generator=g).cuda(), n))
+        counts.append(routes[r].send_counts.tolist())
+    pairs = torch.arange(0, tokens * topk, 7, device="cuda")
+    for r in range(n):
+        routes[r].pos[pairs] = -1   # dropped on the way back
+    rows_in = [sum(counts[s][d] for s in range(n)) for d in range(n)]
+
+    def call():
+        recv = [torch.zeros(max(k, 1), hidden, dtype=dtype, device="cuda") for k in rows_in]
+        out = [torch.full_like(x, 3.0) for x in xs]
+        moe.dispatch(comm, xs, recv, routes, counts, codec=codec)
+        moe.combine(comm, recv, out, routes, counts, codec=codec)
+        return recv + out
+
+    _both(comm, call)
+    comm.close()
