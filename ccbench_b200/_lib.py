@@ -7,14 +7,19 @@ no JIT cache is involved and the built file travels with the source tree.
 from __future__ import annotations
 
 import ctypes
+import functools
+import importlib.machinery
+import importlib.util
 import os
 import shutil
 import subprocess
+import sysconfig
 from pathlib import Path
 
 ROOT = Path(__file__).resolve().parent.parent
 NATIVE_DIR = Path(__file__).resolve().parent / "_native"
 LIBCCB = NATIVE_DIR / "libccb.so"
+CALLS, CALLS_SOURCE = NATIVE_DIR / "ccb_calls.so", ROOT / "csrc/py/ccb_calls.cpp"
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -52,6 +57,47 @@ def build_native(force: bool = False, verbose: bool = False) -> Path:
             print(" ".join(cmd))
         subprocess.run(cmd, check=True, cwd=ROOT)
     return LIBCCB
+
+
+def build_calls(force: bool = False, verbose: bool = False) -> Path:
+    """Compile the native side of the frequent calls (csrc/py/ccb_calls.cpp) against the torch that is installed,
+    if it is missing or older than its sources. Processes that build at once each make their own file."""
+    import torch
+
+    NATIVE_DIR.mkdir(parents=True, exist_ok=True)
+    if force or _stale(CALLS, [CALLS_SOURCE, *(ROOT / "include").rglob("*.h")]):
+        home, cuda = Path(torch.__file__).parent, Path(os.environ.get("CUDA_HOME", "/usr/local/cuda"))
+        made = CALLS.with_name(f"{CALLS.name}.{os.getpid()}")
+        include = [home / "include", home / "include/torch/csrc/api/include", sysconfig.get_paths()["include"], cuda / "include", ROOT / "include"]
+        cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", *(f"-I{i}" for i in include), str(CALLS_SOURCE), "-o", str(made), f"-L{home / 'lib'}",
+               "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda", f"-L{cuda / 'lib64'}", "-lcudart"]
+        if verbose:
+            print(" ".join(cmd))
+        subprocess.run(cmd, check=True, cwd=ROOT)
+        os.replace(made, CALLS)
+    return CALLS
+
+
+@functools.cache
+def calls():
+    """The native side of the frequent calls, or None where it cannot be had (no compiler, another torch than it was
+    built with): every call has a way without it."""
+    import torch
+
+    from . import constants as K
+
+    try:
+        if not CALLS.exists():
+            build_calls()
+        spec = importlib.util.spec_from_file_location("ccb_calls", CALLS, loader=importlib.machinery.ExtensionFileLoader("ccb_calls", str(CALLS)))
+        module = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(module)
+    except (ImportError, OSError, subprocess.CalledProcessError):
+        return None
+    L = lib()
+    where = {name: ctypes.cast(getattr(L, name), ctypes.c_void_p).value for name in module.names().split()}
+    module.setup(where, K.OPS, K.CODECS, K.ALGOS, torch.nn.Parameter)
+    return module
 
 
 _lib = None

@@ -3,9 +3,10 @@ from __future__ import annotations
 
 
 def build_all(verbose: bool = False) -> None:
-    from ._lib import build_native
+    from ._lib import build_calls, build_native
 
     build_native(verbose=verbose)
+    build_calls(verbose=verbose)
     try:
         from .native_build import build_c_targets
     except ImportError:

@@ -20,7 +20,7 @@ from typing import Optional, Sequence, Union
 import torch
 
 from . import constants as K
-from ._lib import lib
+from ._lib import calls, lib
 
 Tensors = Union[torch.Tensor, Sequence[torch.Tensor]]
 
@@ -59,6 +59,8 @@ class Communicator:
         self.nranks = L.ccb_comm_nranks(self._h)
         self.nlocal = L.ccb_comm_nlocal(self._h)
         self._pointers = ctypes.c_void_p * self.nlocal
+        self._calls, self._handle = calls(), handle   # see csrc/py/ccb_calls.cpp: None from it means the general way
+        self._tuned = {}
 
     # ------------------------------------------------------------ creation --
     @classmethod
@@ -99,7 +101,7 @@ class Communicator:
     def close(self) -> None:
         if self._h:
             lib().ccb_comm_destroy(self._h)
-            self._h = None
+            self._h, self._handle = None, 0
 
     def __del__(self):
         try:
@@ -228,6 +230,11 @@ class Communicator:
         recv is None. `error_feedback` is one fp32 tensor per rank of the same element
         count that carries the quantisation residual from call to call."""
         recv = send if recv is None else recv
+        if self._calls is not None and algo != "nvls" and not (self._tuned and algo == "auto"):
+            rc = self._calls.all_reduce(self._handle, self.nlocal, send, recv, error_feedback, op, codec, algo)
+            if rc is not None:
+                _check(rc)
+                return recv
         sp, st = self._ptrs(send, "send")
         rp, rt = self._ptrs(recv, "recv")
         ep, et = self._ptrs(error_feedback, "error_feedback")
@@ -242,7 +249,7 @@ class Communicator:
                 _check(L.ccb_all_reduce_symm(self._h, so, ro, st[0].numel(), self._dtype(st), self._stream()))
                 return recv
         if algo == "auto":   # a measured choice for this shape, when tune_all_reduce() made one
-            algo = getattr(self, "_tuned", {}).get((st[0].numel(), st[0].dtype, codec), "auto")
+            algo = self._tuned.get((st[0].numel(), st[0].dtype, codec), "auto")
         _check(lib().ccb_all_reduce(self._h, sp, rp, st[0].numel(), self._dtype(st), _code(op, K.OPS),
                                     _code(codec, K.CODECS), _code(algo, K.ALGOS), ep, self._stream()))
         return recv
@@ -291,13 +298,16 @@ class Communicator:
         best = min(seen, key=lambda a: seen[a]["ms"]) if seen else "auto"
         if prefer in seen and best != prefer and seen[best]["ms"] > (1.0 - margin) * seen[prefer]["ms"]:
             best = prefer
-        if not hasattr(self, "_tuned"):
-            self._tuned = {}
         self._tuned[(st[0].numel(), st[0].dtype, codec)] = best
         return (best, seen) if report else best
 
     def reduce_scatter(self, send: Tensors, recv: Tensors, *, op="sum", codec="int8",
                        error_feedback: Optional[Tensors] = None):
+        if self._calls is not None and error_feedback is None:
+            rc = self._calls.reduce_scatter(self._handle, self.nlocal, self.nranks, send, recv, op, codec)
+            if rc is not None:
+                _check(rc)
+                return recv
         sp, st = self._ptrs(send, "send")
         rp, rt = self._ptrs(recv, "recv")
         ep, _ = self._ptrs(error_feedback, "error_feedback")
@@ -315,6 +325,11 @@ class Communicator:
         return recv
 
     def all_gather(self, send: Tensors, recv: Tensors, *, codec="int8"):
+        if self._calls is not None:
+            rc = self._calls.all_gather(self._handle, self.nlocal, self.nranks, send, recv, codec)
+            if rc is not None:
+                _check(rc)
+                return recv
         sp, st = self._ptrs(send, "send")
         rp, rt = self._ptrs(recv, "recv")
         if rt[0].numel() != st[0].numel() * self.nranks:
@@ -395,6 +410,13 @@ class _P2pOp(ctypes.Structure):
 def _check(rc: int) -> None:
     if rc != K.OK:
         raise CcbError(rc, (lib().ccb_last_error() or b"").decode(errors="replace"))
+
+
+def taken(answer):
+    """What a native call made; raises where that is the library's code."""
+    if answer.__class__ is int:
+        _check(answer)
+    return answer
 
 
 @functools.lru_cache(maxsize=1024, typed=True)   # the same few sizes come again and again (typed: 1000.0 stays refused)

@@ -153,8 +153,22 @@ def _gpu():
     return torch, L, _DTYPES, _check, current_stream_ptr
 
 
+def _calls():
+    from .._lib import calls
+
+    return calls()
+
+
+def _taken(made):
+    from ..comm import taken
+
+    return taken(made)
+
+
 def encode(x):
     """x: contiguous CUDA tensor (float32, bfloat16 or float16) -> container (uint8 CUDA tensor)."""
+    if (c := _calls()) is not None and (made := c.lossless_encode(x)) is not None:
+        return _taken(made)
     torch, L, DT, check, stream = _gpu()
     out = torch.empty(int(L.ccb_lossless_max_bytes(DT[x.dtype], x.numel())), dtype=torch.uint8, device=x.device)
     check(L.ccb_lossless_encode(DT[x.dtype], x.data_ptr(), x.numel(), out.data_ptr(), stream()))
@@ -162,6 +176,8 @@ def encode(x):
 
 
 def decode(comp, count: int, dtype, out=None, accumulate: bool = False):
+    if out is None and not accumulate and (c := _calls()) is not None and (made := c.lossless_decode(comp, count, dtype)) is not None:
+        return _taken(made)
     torch, L, DT, check, stream = _gpu()
     out = torch.empty(count, dtype=dtype, device=comp.device) if out is None else out
     check(L.ccb_lossless_decode(DT[dtype], comp.data_ptr(), count, out.data_ptr(), 1 if accumulate else 0,

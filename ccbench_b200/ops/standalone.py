@@ -9,8 +9,8 @@ import functools
 import torch
 
 from .. import constants as K
-from .._lib import lib
-from ..comm import _check, _DTYPES, current_stream_ptr as _stream, wire_bytes
+from .._lib import calls, lib
+from ..comm import _check, _DTYPES, current_stream_ptr as _stream, taken, wire_bytes
 
 
 @functools.cache   # the declarations once: plain integers then go straight through
@@ -26,12 +26,16 @@ def _lib():
 
 def encode(x: torch.Tensor, codec: str) -> torch.Tensor:
     """Returns the wire bytes (uint8 tensor) of a contiguous CUDA tensor."""
+    if (c := calls()) is not None and (made := c.encode(x, codec)) is not None:
+        return taken(made)
     wire = torch.empty(wire_bytes(codec, x.dtype, x.numel()), dtype=torch.uint8, device=x.device)
     _check(_lib().ccb_encode(K.CODECS[codec], _DTYPES[x.dtype], x.data_ptr(), x.numel(), wire.data_ptr(), _stream()))
     return wire
 
 
 def decode(wire: torch.Tensor, codec: str, count: int, dtype: torch.dtype) -> torch.Tensor:
+    if (c := calls()) is not None and (made := c.decode(wire, codec, count, dtype)) is not None:
+        return taken(made)
     out = torch.empty(count, dtype=dtype, device=wire.device)
     _check(_lib().ccb_decode(K.CODECS[codec], _DTYPES[dtype], wire.data_ptr(), count, out.data_ptr(), _stream()))
     return out
@@ -46,6 +50,8 @@ def decode_reduce(wire: torch.Tensor, codec: str, inout: torch.Tensor) -> torch.
 
 def reduce_recode(wires, codec: str, count: int) -> torch.Tensor:
     """encode(sum_k decode(wires[k])) without leaving the compressed domain in memory."""
+    if (c := calls()) is not None and (made := c.reduce_recode(wires, codec, count)) is not None:
+        return taken(made)
     arr = (ctypes.c_void_p * len(wires))(*[w.data_ptr() for w in wires])
     out = torch.empty_like(wires[0])
     _check(_lib().ccb_reduce_recode(K.CODECS[codec], arr, len(wires), count, out.data_ptr(), _stream()))

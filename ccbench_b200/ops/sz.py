@@ -5,12 +5,13 @@ from __future__ import annotations
 
 import ctypes
 import functools
+import struct
 
 import numpy as np
 import torch
 
-from .._lib import lib
-from ..comm import Communicator, _check, current_stream_ptr
+from .._lib import calls, lib
+from ..comm import Communicator, _check, current_stream_ptr, taken
 
 TX, TY, TZ = 32, 8, 8
 
@@ -42,6 +43,8 @@ def capacity(shape) -> int:
 
 def compress(field: torch.Tensor, eb: float):
     """Returns (buffer uint8 [capacity], used_bytes int). field: fp32 CUDA tensor [nz, ny, nx]."""
+    if (c := calls()) is not None and (made := c.sz_compress(field, eb)) is not None:
+        return taken(made)
     assert field.is_cuda and field.dtype == torch.float32 and field.dim() == 3 and field.is_contiguous()
     nz, ny, nx = field.shape
     buf = torch.empty(capacity(field.shape), dtype=torch.uint8, device=field.device)
@@ -51,6 +54,8 @@ def compress(field: torch.Tensor, eb: float):
 
 
 def decompress(buf: torch.Tensor, shape, eb: float) -> torch.Tensor:
+    if (c := calls()) is not None and (made := c.sz_decompress(buf, shape, eb)) is not None:
+        return taken(made)
     nz, ny, nx = shape
     out = torch.empty(shape, dtype=torch.float32, device=buf.device)
     _check(_decl().ccb_sz_decompress(buf.data_ptr(), nx, ny, nz, eb, out.data_ptr(), _stream()))
@@ -110,6 +115,12 @@ def to_container(buf: torch.Tensor, shape, eb: float) -> torch.Tensor:
     of the total between them), plain tensor operations for a host buffer."""
     nz, ny, nx = shape
     ngroups = buf.numel() // GROUP_STRIDE
+    if (c := calls()) is not None and (scan := c.sz_scan(buf, GROUP_STRIDE)) is not None:
+        offsets, total, largest = taken(scan)
+        if largest > GROUP_STRIDE:
+            raise ValueError("a group of the buffer is damaged")
+        if (blob := c.sz_pack(buf, offsets, tuple(shape), eb, ngroups, HEADER_BYTES + 4 * ngroups + total)) is not None:
+            return taken(blob)
     if _by_kernel(buf, 16) and ngroups and buf.numel() == ngroups * GROUP_STRIDE:
         with torch.cuda.device(buf.device):
             L = _decl()
@@ -141,28 +152,31 @@ def from_container(blob: torch.Tensor):
     """Inverse of to_container: returns (buffer of group slots, shape, eb)."""
     by_kernel = _by_kernel(blob, 4) and blob.numel() >= HEADER_BYTES + _LEAST_GROUP
     if by_kernel:   # header, scan of the sizes and its sums in one read-back; no group is smaller than an empty tile's
-        with torch.cuda.device(blob.device):
-            room = (blob.numel() - HEADER_BYTES) // _LEAST_GROUP
-            offsets = torch.empty(room + 2 + 7, dtype=torch.int64, device=blob.device)
-            _check(_decl().ccb_sz_container_open(blob.data_ptr(), blob.numel(), room, offsets.data_ptr(), offsets.data_ptr() + 8 * (room + 2), _stream()))
-            found = offsets[room + 2:].cpu()
-            head = found.view(torch.uint8)[:HEADER_BYTES]
+        room = (blob.numel() - HEADER_BYTES) // _LEAST_GROUP
+        if (c := calls()) is not None and (opened := c.sz_open(blob, room)) is not None:
+            offsets, head = taken(opened)
+        else:
+            with torch.cuda.device(blob.device):
+                offsets = torch.empty(room + 2 + 7, dtype=torch.int64, device=blob.device)
+                _check(_decl().ccb_sz_container_open(blob.data_ptr(), blob.numel(), room, offsets.data_ptr(), offsets.data_ptr() + 8 * (room + 2), _stream()))
+                head = offsets[room + 2:].cpu().numpy().tobytes()
     else:
-        head = blob[:HEADER_BYTES].cpu()
-    magic, version, nx, ny, nz = head[0:20].view(torch.int32).tolist()
+        head = blob[:HEADER_BYTES].cpu().numpy().tobytes()
+    if len(head) < HEADER_BYTES:
+        raise ValueError("container payload is damaged")
+    magic, version, nx, ny, nz, eb, _, ngroups, nbytes = struct.unpack_from("<5i2fiq", head)
     if magic != MAGIC or version != VERSION:
         raise ValueError(f"not a ccb-sz v{VERSION} container (magic {magic:#x}, version {version})")
-    eb = head[20:24].view(torch.float32).item()
-    ngroups = head[28:32].view(torch.int32).item()
-    nbytes = head[32:40].view(torch.int64).item()
     if ngroups * GROUP_STRIDE != capacity((nz, ny, nx)):
         raise ValueError("container header does not match its dimensions")
     if by_kernel:
         if ngroups > room or blob.numel() - HEADER_BYTES - 4 * ngroups != nbytes:
             raise ValueError("container payload is damaged")
-        total, largest = found[5:].tolist()
+        total, largest = struct.unpack_from("<2q", head, HEADER_BYTES)
         if total != nbytes or largest > GROUP_STRIDE:
             raise ValueError("container payload is damaged")
+        if c is not None and (buf := c.sz_unpack(blob, HEADER_BYTES + 4 * ngroups, offsets, ngroups, GROUP_STRIDE)) is not None:
+            return taken(buf), (nz, ny, nx), eb
         with torch.cuda.device(blob.device):
             buf = torch.empty(ngroups * GROUP_STRIDE, dtype=torch.uint8, device=blob.device)
             _check(_decl().ccb_sz_container_unpack(blob.data_ptr() + HEADER_BYTES + 4 * ngroups, offsets.data_ptr(), ngroups, buf.data_ptr(), _stream()))

@@ -65,6 +65,11 @@ def _counts(count_matrix):
 def dispatch(comm: Communicator, x, recv, routes, count_matrix, *, codec="fp8"):
     """x, recv, routes: one per local rank. count_matrix[src][dst] rows (the same on every
     rank: all-gather the per-rank send_counts first). recv needs sum_s count[s][me] rows."""
+    if comm._calls is not None:
+        rc = comm._calls.moe_dispatch(comm._handle, comm.nlocal, comm.nranks, x, recv, routes, count_matrix, codec)
+        if rc is not None:
+            _check(rc)
+            return recv
     xs = [x] if isinstance(x, torch.Tensor) else list(x)
     rs = [recv] if isinstance(recv, torch.Tensor) else list(recv)
     rt = [routes] if isinstance(routes, Route) else list(routes)
@@ -74,6 +79,11 @@ def dispatch(comm: Communicator, x, recv, routes, count_matrix, *, codec="fp8"):
 
 
 def combine(comm: Communicator, y, out, routes, count_matrix, *, codec="fp8"):
+    if comm._calls is not None:
+        rc = comm._calls.moe_combine(comm._handle, comm.nlocal, comm.nranks, y, out, routes, count_matrix, codec)
+        if rc is not None:
+            _check(rc)
+            return out
     ys = [y] if isinstance(y, torch.Tensor) else list(y)
     os_ = [out] if isinstance(out, torch.Tensor) else list(out)
     rt = [routes] if isinstance(routes, Route) else list(routes)
