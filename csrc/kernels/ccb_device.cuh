@@ -135,6 +135,11 @@ template <> struct Elem<__half> {
   static __device__ __forceinline__ __half from_f(float x) { return __float2half_rn(x); }
 };
 
+// The first thing in a kernel that launch_next() launches, before it touches memory: the kernel before it on the
+// stream has then ended, and what it wrote is there. (None of them lets the one behind it begin early: a kernel may
+// follow that does not wait, see launch(), and it gained nothing.)
+__device__ __forceinline__ void after_kernel_before() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 __device__ __forceinline__ uint4 ldg_stream(const void* p) {
   uint4 v;
   asm volatile("ld.global.cs.v4.u32 {%0,%1,%2,%3}, [%4];"

@@ -28,7 +28,7 @@ static int local_launch(ccb_comm* c, const void* fn, void* args, uint64_t warps,
   per = per < 1 ? 1 : per > kLocalThreads / 32 ? kLocalThreads / 32 : per;
   const uint64_t ctas = (warps + per - 1) / per;
   void* params[] = {args};
-  const cudaError_t e = cudaLaunchKernel(fn, dim3((unsigned)(ctas ? ctas : 1)), dim3((unsigned)(32 * per)), params, 0, stream);
+  const cudaError_t e = launch_next(fn, dim3((unsigned)(ctas ? ctas : 1)), dim3((unsigned)(32 * per)), params, 0, stream);
   if (e != cudaSuccess) {
     set_error("kernel launch failed: %s", cudaGetErrorString(e));
     return CCB_ERR_CUDA;

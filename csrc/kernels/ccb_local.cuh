@@ -299,6 +299,7 @@ __device__ __forceinline__ void local_reduce_unit(const LocalReduceArgs& a, uint
 
 template <class T, class C, int ALGO, bool kEf, bool kAnyOffset>
 __global__ void __launch_bounds__(kLocalThreads, LocalShape<T, ALGO, kEf, kAnyOffset>::kCtas) local_reduce_kernel(const __grid_constant__ LocalReduceArgs a) {
+  after_kernel_before();
   const uint32_t u = ccb_grid_warp(blockIdx.x, blockDim.x, threadIdx.x);
   if (u >= a.units) return;
   const uint32_t s = ALGO == kLocalTwoShot || ALGO == kLocalRing || ALGO == kLocalScatter ? u / a.shard_units : 0u;
@@ -332,6 +333,7 @@ __device__ __forceinline__ void local_solo_unit(const LocalReduceArgs& a, size_t
 }
 template <class T, class C, bool kEf, bool kAnyOffset>
 __global__ void __launch_bounds__(kLocalThreads, kEf ? 4 : sizeof(T) == 4 ? (kAnyOffset ? 4 : 6) : kAnyOffset ? 6 : 8) local_solo_kernel(const __grid_constant__ LocalReduceArgs a) {
+  after_kernel_before();
   const size_t e0 = (((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * kWarpElems, idx = e0 + (threadIdx.x & 31) * kLaneElems;
   if (e0 >= a.count) return;
   if (e0 + kWarpElems <= a.count) local_solo_unit<T, C, kEf, kAnyOffset, true>(a, idx);
@@ -361,6 +363,7 @@ struct LocalExchangeArgs {
 // A block in place keeps to its own units: the one before may have been written. (Without kAnyOffset a run is one unit.)
 template <class T, class C, bool kAnyOffset>
 __global__ void __launch_bounds__(kLocalThreads, kAnyOffset ? (sizeof(T) == 4 ? 2 : 3) : 6) local_exchange_kernel(const __grid_constant__ LocalExchangeArgs a) {
+  after_kernel_before();
   constexpr int W = 4 * (int)sizeof(T), kPer = 4 / (int)sizeof(T);   // words of a lane, elements of a word
   const int lane = threadIdx.x & 31;
   const uint32_t w = ccb_grid_warp(blockIdx.x, blockDim.x, threadIdx.x);

@@ -146,6 +146,7 @@ __device__ __forceinline__ void pairs_of_planes(const uint32_t (&u)[4], uint32_t
 // of 44; five or six CTAs of any kind are slower. (B200.)
 template <class T>
 __global__ void __launch_bounds__(kLlThreads, sizeof(T) == 4 ? 3 : kLlCtas) lossless_encode_kernel(const T* __restrict__ in, size_t count, char* out, size_t ntiles) {
+  after_kernel_before();
   using Tr = LlTraits<T>;
   __shared__ uint2 info[2][kLlBlocksPerTile];   // (width, minimum) of each block, by parity of the tile
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -260,6 +261,7 @@ __global__ void __launch_bounds__(kLlThreads, sizeof(T) == 4 ? 3 : kLlCtas) loss
 // MODE 0: out = decoded values; MODE 1: out += decoded values (in T, one rounding)
 template <class T, int MODE>
 __global__ void __launch_bounds__(kLlThreads, kLlCtas) lossless_decode_kernel(const char* __restrict__ in, size_t count, T* out, size_t ntiles) {
+  after_kernel_before();
   using Tr = LlTraits<T>;
   constexpr int kRest = sizeof(T) == 4 ? 3 : 1;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, sh = 8 * (warp & 3);
@@ -386,15 +388,15 @@ extern "C" int ccb_lossless_encode(int dtype, const void* in, uint64_t count, vo
   if (dtype != CCB_F32 && dtype != CCB_BF16 && dtype != CCB_F16) return CCB_ERR_UNSUPPORTED;
   // the kernel writes the header (a copy from the host would be a staged transfer per call) and
   // adds up its byte count, which has to start at zero
-  if (cudaMemsetAsync(out, 0, kLlHeader, s) != cudaSuccess) {
+  if (launch_clear(out, kLlHeader, s) != cudaSuccess) {
     set_error("ccb_lossless_encode: clearing the header failed: %s", cudaGetErrorString(cudaGetLastError()));
     return CCB_ERR_CUDA;
   }
   const size_t nt = ll_tiles(count);
   const int g = ll_grid(nt, dtype);
-  if (dtype == CCB_F32) lossless_encode_kernel<float><<<g, kLlThreads, 0, s>>>((const float*)in, count, (char*)out, nt);
-  else if (dtype == CCB_BF16) lossless_encode_kernel<__nv_bfloat16><<<g, kLlThreads, 0, s>>>((const __nv_bfloat16*)in, count, (char*)out, nt);
-  else lossless_encode_kernel<__half><<<g, kLlThreads, 0, s>>>((const __half*)in, count, (char*)out, nt);
+  if (dtype == CCB_F32) launch_next(lossless_encode_kernel<float>, g, kLlThreads, 0, s, (const float*)in, count, (char*)out, nt);
+  else if (dtype == CCB_BF16) launch_next(lossless_encode_kernel<__nv_bfloat16>, g, kLlThreads, 0, s, (const __nv_bfloat16*)in, count, (char*)out, nt);
+  else launch_next(lossless_encode_kernel<__half>, g, kLlThreads, 0, s, (const __half*)in, count, (char*)out, nt);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {
     set_error("ccb_lossless_encode: %s", cudaGetErrorString(e));
@@ -415,8 +417,8 @@ extern "C" int ccb_lossless_decode(int dtype, const void* in, uint64_t count, vo
   const int g = ll_grid(nt, dtype);
 #define CCB_LL_DEC(T)                                                                                          \
   do {                                                                                                         \
-    if (accumulate) lossless_decode_kernel<T, 1><<<g, kLlThreads, 0, s>>>((const char*)in, count, (T*)out, nt); \
-    else lossless_decode_kernel<T, 0><<<g, kLlThreads, 0, s>>>((const char*)in, count, (T*)out, nt);            \
+    if (accumulate) launch_next(lossless_decode_kernel<T, 1>, g, kLlThreads, 0, s, (const char*)in, count, (T*)out, nt); \
+    else launch_next(lossless_decode_kernel<T, 0>, g, kLlThreads, 0, s, (const char*)in, count, (T*)out, nt);            \
   } while (0)
   if (dtype == CCB_F32) CCB_LL_DEC(float);
   else if (dtype == CCB_BF16) CCB_LL_DEC(__nv_bfloat16);

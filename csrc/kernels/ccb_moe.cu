@@ -223,6 +223,7 @@ __device__ __forceinline__ void moe_brought() {
 // read from memory once and from L2 after that.
 template <class T, class C>
 __global__ void __launch_bounds__(kMoeLocalThreads, 12) moe_local_dispatch_kernel(const __grid_constant__ MoeLocalArgs a) {
+  after_kernel_before();
   __shared__ uint4 stages[kMoeLocalThreads / 32][kMoeStage / 16];
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t n = (uint32_t)a.n, p = blockIdx.x % n, c = blockIdx.x / n % a.chunks, r = blockIdx.x / n / a.chunks;
@@ -258,6 +259,7 @@ __global__ void __launch_bounds__(kMoeLocalThreads, 12) moe_local_dispatch_kerne
 // its codec, 84 and 84. 36 warps an SM, 56 registers: with 40, which spill, 265 but 98 at top 4, with 32 276. B200.)
 template <class T, class C>
 __global__ void __launch_bounds__(kMoeLocalThreads, 9) moe_local_combine_kernel(const __grid_constant__ MoeLocalArgs a) {
+  after_kernel_before();
   constexpr int kSlots = kMoeSlots<T>;
   __shared__ uint4 stages[kMoeLocalThreads / 32][kMoeStage / 16];
   const uint32_t lane = threadIdx.x & 31;
@@ -381,7 +383,7 @@ static int moe_local_launch(ccb_comm* c, const MoeArgs& m, bool combine, int dty
   if (ctas == 0) return CCB_OK;
   const void* fn = combine ? moe_by_type<MoeLocalCombine>(dtype, codec) : moe_by_type<MoeLocalDispatch>(dtype, codec);
   void* params[] = {&a};
-  const cudaError_t e = cudaLaunchKernel(fn, dim3((unsigned)ctas), dim3((unsigned)(32 * warps)), params, 0, stream);
+  const cudaError_t e = launch_next(fn, dim3((unsigned)ctas), dim3((unsigned)(32 * warps)), params, 0, stream);
   if (e != cudaSuccess) {
     set_error("kernel launch failed: %s", cudaGetErrorString(e));
     return CCB_ERR_CUDA;

@@ -26,6 +26,7 @@ constexpr int kSaThreads = 256;
 template <class T, class C, bool kBy16>
 __global__ void __launch_bounds__(kSaThreads) encode_kernel(const T* __restrict__ in, size_t count, char* wire, size_t pad,
                                                             size_t in_stride, size_t wire_stride) {
+  after_kernel_before();
   in += (size_t)blockIdx.y * in_stride;
   wire += (size_t)blockIdx.y * wire_stride;
   const size_t units = pad / kWarpElems;
@@ -47,6 +48,7 @@ __global__ void __launch_bounds__(kSaThreads) encode_kernel(const T* __restrict_
 template <class T, class C, int MODE>
 __global__ void __launch_bounds__(kSaThreads) decode_kernel(const char* wire, size_t count, T* out, size_t pad,
                                                             size_t wire_stride, size_t out_stride) {
+  after_kernel_before();
   wire += (size_t)blockIdx.y * wire_stride;
   out += (size_t)blockIdx.y * out_stride;
   const size_t units = pad / kWarpElems;
@@ -75,6 +77,7 @@ __global__ void __launch_bounds__(kSaThreads) decode_kernel(const char* wire, si
 // decodes into a temporary (coccl_wrapper_template.cu:258-272 add_*_kernel in the reference).
 template <class T>
 __global__ void __launch_bounds__(kSaThreads) accumulate_kernel(const T* __restrict__ src, T* inout, size_t count) {
+  after_kernel_before();
   const size_t units = (count + kWarpElems - 1) / kWarpElems;
   const size_t warp = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = ((size_t)gridDim.x * blockDim.x) >> 5;
   const int lane = threadIdx.x & 31;
@@ -101,6 +104,7 @@ struct WireList {
 // wire_out = encode(sum_k decode(wires[k]))
 template <class C>
 __global__ void __launch_bounds__(kSaThreads) reduce_recode_kernel(const __grid_constant__ WireList wl, size_t count, char* wire_out, size_t pad) {
+  after_kernel_before();
   const size_t units = pad / kWarpElems;
   const size_t warp = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = ((size_t)gridDim.x * blockDim.x) >> 5;
   const int lane = threadIdx.x & 31;
@@ -126,6 +130,7 @@ __global__ void __launch_bounds__(kSaThreads) reduce_recode_kernel(const __grid_
 // Reference wire v0: scales[g] = 127/absmax (1.0 when absmax < 1e-10), then int8 payload.
 template <class T>
 __global__ void __launch_bounds__(kSaThreads) refwire_encode_kernel(const T* __restrict__ in, size_t count, int group, float* scales, int8_t* q) {
+  after_kernel_before();
   // one warp per group; group <= 4096
   const size_t warp = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = ((size_t)gridDim.x * blockDim.x) >> 5;
   const int lane = threadIdx.x & 31;
@@ -146,6 +151,7 @@ __global__ void __launch_bounds__(kSaThreads) refwire_encode_kernel(const T* __r
 }
 template <class T>
 __global__ void __launch_bounds__(kSaThreads) refwire_decode_kernel(const float* scales, const int8_t* q, size_t count, int group, T* out) {
+  after_kernel_before();
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += (size_t)gridDim.x * blockDim.x)
     out[i] = Elem<T>::from_f((float)q[i] * (1.0f / scales[i / group]));
 }
@@ -156,6 +162,7 @@ __global__ void __launch_bounds__(kSaThreads) refwire_decode_kernel(const float*
 template <class T>
 __global__ void __launch_bounds__(kSaThreads) fold_kernel(const T* __restrict__ parts, size_t stride, int nparts, size_t count, int op,
                                                           T* __restrict__ out) {
+  after_kernel_before();
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += (size_t)gridDim.x * blockDim.x) {
     T acc = parts[i];
     for (int p = 1; p < nparts; ++p) {
@@ -165,6 +172,14 @@ __global__ void __launch_bounds__(kSaThreads) fold_kernel(const T* __restrict__ 
     if (op == 4) acc = (T)(acc / (T)nparts);
     out[i] = acc;
   }
+}
+
+__global__ void __launch_bounds__(32) clear_kernel(uint32_t* words, int n) {
+  after_kernel_before();
+  if ((int)threadIdx.x < n) words[threadIdx.x] = 0u;
+}
+cudaError_t launch_clear(void* words, size_t bytes, cudaStream_t stream) {
+  return launch_next(clear_kernel, 1, 32, 0, stream, static_cast<uint32_t*>(words), (int)(bytes / 4));
 }
 
 static int sa_grid(size_t units) {
@@ -194,7 +209,7 @@ static int encode_t(int codec, const void* in, size_t count, void* wire, size_t 
                     size_t in_stride = 0, size_t wire_stride = 0) {
   const dim3 g = sa_grid2(pad / kWarpElems, nchunks);
   const bool by16 = sizeof(T) == 2 || count * nchunks < ((size_t)32 << 20);
-#define CCB_ENC(C, BY16) encode_kernel<T, C, BY16><<<g, kSaThreads, 0, s>>>((const T*)in, count, (char*)wire, pad, in_stride, wire_stride)
+#define CCB_ENC(C, BY16) launch_next(encode_kernel<T, C, BY16>, g, kSaThreads, 0, s, (const T*)in, count, (char*)wire, pad, in_stride, wire_stride)
 #define CCB_ENC_CODEC(C)                              \
   do {                                                \
     if (by16) CCB_ENC(C, true);                       \
@@ -219,7 +234,7 @@ template <class T, int MODE>
 static int decode_t(int codec, const void* wire, size_t count, void* out, size_t pad, cudaStream_t s, size_t nchunks = 1,
                     size_t wire_stride = 0, size_t out_stride = 0) {
   const dim3 g = sa_grid2(pad / kWarpElems, nchunks);
-#define CCB_DEC(C) decode_kernel<T, C, MODE><<<g, kSaThreads, 0, s>>>((const char*)wire, count, (T*)out, pad, wire_stride, out_stride)
+#define CCB_DEC(C) launch_next(decode_kernel<T, C, MODE>, g, kSaThreads, 0, s, (const char*)wire, count, (T*)out, pad, wire_stride, out_stride)
   switch (codec) {
     case CCB_CODEC_NONE: CCB_DEC(CodecNone<T>); break;
     case CCB_CODEC_INT8: CCB_DEC(CodecInt8<128>); break;
@@ -324,9 +339,9 @@ extern "C" int ccb_accumulate(int dtype, const void* src, void* inout, uint64_t 
   if (!count) return CCB_OK;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const int g = sa_grid((count + kWarpElems - 1) / kWarpElems);
-  if (dtype == CCB_F32) accumulate_kernel<float><<<g, kSaThreads, 0, s>>>((const float*)src, (float*)inout, count);
-  else if (dtype == CCB_BF16) accumulate_kernel<__nv_bfloat16><<<g, kSaThreads, 0, s>>>((const __nv_bfloat16*)src, (__nv_bfloat16*)inout, count);
-  else if (dtype == CCB_F16) accumulate_kernel<__half><<<g, kSaThreads, 0, s>>>((const __half*)src, (__half*)inout, count);
+  if (dtype == CCB_F32) launch_next(accumulate_kernel<float>, g, kSaThreads, 0, s, (const float*)src, (float*)inout, count);
+  else if (dtype == CCB_BF16) launch_next(accumulate_kernel<__nv_bfloat16>, g, kSaThreads, 0, s, (const __nv_bfloat16*)src, (__nv_bfloat16*)inout, count);
+  else if (dtype == CCB_F16) launch_next(accumulate_kernel<__half>, g, kSaThreads, 0, s, (const __half*)src, (__half*)inout, count);
   else return CCB_ERR_UNSUPPORTED;
   return finish("ccb_accumulate");
 }
@@ -344,11 +359,11 @@ extern "C" int ccb_reduce_recode(int codec, const void* const* wires, int nwires
   const int g = sa_grid(pad / kWarpElems);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   switch (codec) {
-    case CCB_CODEC_INT8: reduce_recode_kernel<CodecInt8<128>><<<g, kSaThreads, 0, s>>>(wl, count, (char*)wire_out, pad); break;
-    case CCB_CODEC_INT8_G256: reduce_recode_kernel<CodecInt8<256>><<<g, kSaThreads, 0, s>>>(wl, count, (char*)wire_out, pad); break;
-    case CCB_CODEC_FP8: reduce_recode_kernel<CodecFp8><<<g, kSaThreads, 0, s>>>(wl, count, (char*)wire_out, pad); break;
-    case CCB_CODEC_INT4: reduce_recode_kernel<CodecInt4><<<g, kSaThreads, 0, s>>>(wl, count, (char*)wire_out, pad); break;
-    case CCB_CODEC_NONE: reduce_recode_kernel<CodecNone<float>><<<g, kSaThreads, 0, s>>>(wl, count, (char*)wire_out, pad); break;
+    case CCB_CODEC_INT8: launch_next(reduce_recode_kernel<CodecInt8<128>>, g, kSaThreads, 0, s, wl, count, (char*)wire_out, pad); break;
+    case CCB_CODEC_INT8_G256: launch_next(reduce_recode_kernel<CodecInt8<256>>, g, kSaThreads, 0, s, wl, count, (char*)wire_out, pad); break;
+    case CCB_CODEC_FP8: launch_next(reduce_recode_kernel<CodecFp8>, g, kSaThreads, 0, s, wl, count, (char*)wire_out, pad); break;
+    case CCB_CODEC_INT4: launch_next(reduce_recode_kernel<CodecInt4>, g, kSaThreads, 0, s, wl, count, (char*)wire_out, pad); break;
+    case CCB_CODEC_NONE: launch_next(reduce_recode_kernel<CodecNone<float>>, g, kSaThreads, 0, s, wl, count, (char*)wire_out, pad); break;
     default: return CCB_ERR_UNSUPPORTED;
   }
   return finish("ccb_reduce_recode");
@@ -359,7 +374,7 @@ extern "C" int ccb_fold(int xtype, int op, const void* parts, uint64_t stride, i
   if (nparts < 1 || op < 0 || op > 4) return CCB_ERR_ARG;
   const int g = sa_grid((count + 31) / 32);  // one thread per element, grid-stride beyond the cap
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-#define CCB_FOLD(T) fold_kernel<T><<<g, kSaThreads, 0, s>>>((const T*)parts, stride, nparts, count, op, (T*)out)
+#define CCB_FOLD(T) launch_next(fold_kernel<T>, g, kSaThreads, 0, s, (const T*)parts, stride, nparts, count, op, (T*)out)
   switch (xtype) {
     case CCB_X_I8: CCB_FOLD(int8_t); break;
     case CCB_X_U8: CCB_FOLD(uint8_t); break;
@@ -383,9 +398,9 @@ extern "C" int ccb_refwire_encode(int dtype, const void* in, uint64_t count, int
   int8_t* q = reinterpret_cast<int8_t*>(scales + ng);
   const int g = sa_grid(ng);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (dtype == CCB_F32) refwire_encode_kernel<float><<<g, kSaThreads, 0, s>>>((const float*)in, count, group, scales, q);
-  else if (dtype == CCB_F16) refwire_encode_kernel<__half><<<g, kSaThreads, 0, s>>>((const __half*)in, count, group, scales, q);
-  else if (dtype == CCB_BF16) refwire_encode_kernel<__nv_bfloat16><<<g, kSaThreads, 0, s>>>((const __nv_bfloat16*)in, count, group, scales, q);
+  if (dtype == CCB_F32) launch_next(refwire_encode_kernel<float>, g, kSaThreads, 0, s, (const float*)in, count, group, scales, q);
+  else if (dtype == CCB_F16) launch_next(refwire_encode_kernel<__half>, g, kSaThreads, 0, s, (const __half*)in, count, group, scales, q);
+  else if (dtype == CCB_BF16) launch_next(refwire_encode_kernel<__nv_bfloat16>, g, kSaThreads, 0, s, (const __nv_bfloat16*)in, count, group, scales, q);
   else return CCB_ERR_UNSUPPORTED;
   return finish("ccb_refwire_encode");
 }
@@ -397,9 +412,9 @@ extern "C" int ccb_refwire_decode(int dtype, const void* wire, uint64_t count, i
   const int8_t* q = reinterpret_cast<const int8_t*>(scales + ng);
   const int g = sa_grid((count + 255) / 256);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (dtype == CCB_F32) refwire_decode_kernel<float><<<g, kSaThreads, 0, s>>>(scales, q, count, group, (float*)out);
-  else if (dtype == CCB_F16) refwire_decode_kernel<__half><<<g, kSaThreads, 0, s>>>(scales, q, count, group, (__half*)out);
-  else if (dtype == CCB_BF16) refwire_decode_kernel<__nv_bfloat16><<<g, kSaThreads, 0, s>>>(scales, q, count, group, (__nv_bfloat16*)out);
+  if (dtype == CCB_F32) launch_next(refwire_decode_kernel<float>, g, kSaThreads, 0, s, scales, q, count, group, (float*)out);
+  else if (dtype == CCB_F16) launch_next(refwire_decode_kernel<__half>, g, kSaThreads, 0, s, scales, q, count, group, (__half*)out);
+  else if (dtype == CCB_BF16) launch_next(refwire_decode_kernel<__nv_bfloat16>, g, kSaThreads, 0, s, scales, q, count, group, (__nv_bfloat16*)out);
   else return CCB_ERR_UNSUPPORTED;
   return finish("ccb_refwire_decode");
 }

@@ -1159,6 +1159,7 @@ __device__ __forceinline__ uint32_t pack_planes(const SzLocalArgs& a, unsigned c
 // packed operations kept in registers, or given as pairs of arguments, changed nothing; one vote for both tests neither.
 template <int kVec>
 __global__ void __launch_bounds__(kSzThreads, 3) sz_pack_kernel(const __grid_constant__ SzLocalArgs a) {
+  after_kernel_before();
   extern __shared__ __align__(16) unsigned char stages[];   // kClusterSize * kTileCap
   __shared__ uint32_t s_size[kClusterSize];
   const int lane = threadIdx.x & 31, k = threadIdx.x >> 5;
@@ -1389,6 +1390,7 @@ constexpr int kUnpackStage = 2304;
 
 template <int kVec>
 __global__ void __launch_bounds__(kSzThreads, 4) sz_unpack_kernel(const __grid_constant__ SzLocalArgs a) {
+  after_kernel_before();
   __shared__ __align__(16) float plane[kVec == 1 ? kClusterSize : 1][kVec == 1 ? kTX * kTY : 4];
   __shared__ __align__(16) unsigned char stages[kClusterSize][kUnpackStage];
   const int lane = threadIdx.x & 31, k = threadIdx.x >> 5;
@@ -1568,6 +1570,7 @@ __global__ void __launch_bounds__(kSzThreads, 4) sz_unpack_kernel(const __grid_c
 // A field of few tiles leaves most of the chip idle with a warp a tile, and what counts is how long a
 // tile takes: here a CTA a tile, a plane a warp (unpack_tile), six CTAs an SM.
 __global__ void __launch_bounds__(kSzThreads, 6) sz_unpack_few_kernel(const __grid_constant__ SzLocalArgs a) {
+  after_kernel_before();
   __shared__ __align__(16) int codes[kTileVals];
   const unsigned int k = blockIdx.x % kClusterSize, lane = threadIdx.x & 31;
   const char* group = a.slots + (size_t)(blockIdx.x / kClusterSize) * kGroupStride;
@@ -1612,6 +1615,7 @@ __global__ void __launch_bounds__(kScanThreads) container_scan_kernel(const char
                                                                       unsigned int ngroups, unsigned long long* offsets,
                                                                       const uint32_t* __restrict__ head = nullptr, uint32_t* found = nullptr,
                                                                       unsigned long long bytes = 0) {
+  after_kernel_before();
   if (head) {
     const uint32_t said = head[7];
     ngroups = said <= ngroups ? said : 0u;
@@ -1700,6 +1704,7 @@ constexpr uint32_t kContainerMagic = 0x5A534343u, kContainerVersion = 2u;
 
 __global__ void __launch_bounds__(256) container_pack_kernel(const char* __restrict__ slots, const unsigned long long* __restrict__ offsets,
                                                              ContainerHead head, char* out) {
+  after_kernel_before();
   char* payload = out + sizeof(ContainerHead) + 4 * (size_t)head.ngroups;
   for (unsigned int g = blockIdx.x; g < head.ngroups; g += gridDim.x) {
     const char* slot = slots + (size_t)g * kGroupStride;
@@ -1721,6 +1726,7 @@ __global__ void __launch_bounds__(256) container_pack_kernel(const char* __restr
 // The inverse; the rest of every slot is cleared.
 __global__ void __launch_bounds__(256) container_unpack_kernel(const char* __restrict__ payload, const unsigned long long* __restrict__ offsets,
                                                                unsigned int ngroups, char* slots) {
+  after_kernel_before();
   for (unsigned int g = blockIdx.x; g < ngroups; g += gridDim.x) {
     char* slot = slots + (size_t)g * kGroupStride;
     const unsigned long long at = offsets[g];
@@ -1860,7 +1866,7 @@ static void launch_pack(const SzLocalArgs& a, cudaStream_t stream) {
     if (cudaFuncSetAttribute(sz_pack_kernel<kVec>, cudaFuncAttributeMaxDynamicSharedMemorySize, kBytes) == cudaSuccess)
       allowed.fetch_or(bit, std::memory_order_relaxed);
   }
-  sz_pack_kernel<kVec><<<a.ngroups, kSzThreads, kBytes, stream>>>(a);
+  launch_next(sz_pack_kernel<kVec>, a.ngroups, kSzThreads, kBytes, stream, a);
 }
 // Tiles up to which a CTA a tile unpacks a field faster than a warp a tile, us, CTA / warp, at bounds of 1e-4
 // and 1e-5 of the range (0.6 and 1 byte a value), B200. Lines on 16 bytes: 64^3 (128 tiles) 6.0 / 8.6 and
@@ -1905,7 +1911,7 @@ extern "C" int ccb_sz_compress(const float* in, int nx, int ny, int nz, float eb
   a.slots = static_cast<char*>(out);
   a.used_bytes = d_used;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (d_used) cudaMemsetAsync(d_used, 0, sizeof(unsigned long long), s);
+  if (d_used) launch_clear(d_used, sizeof(unsigned long long), s);
   switch (line_width(in, nx)) {
     case 8: launch_pack<8>(a, s); break;
     case 4: launch_pack<4>(a, s); break;
@@ -1928,13 +1934,13 @@ extern "C" int ccb_sz_decompress(const void* in, int nx, int ny, int nz, float e
   const unsigned int ntiles = (unsigned)a.tiles_x * a.tiles_y * a.tiles_z;
   const int width = line_width(out, nx);
   if (ntiles <= few_tiles(width)) {
-    sz_unpack_few_kernel<<<ntiles, kSzThreads, 0, s>>>(a);
+    launch_next(sz_unpack_few_kernel, ntiles, kSzThreads, 0, s, a);
     return launched("ccb_sz_decompress");
   }
   switch (width) {
-    case 8: sz_unpack_kernel<8><<<a.ngroups, kSzThreads, 0, s>>>(a); break;
-    case 4: sz_unpack_kernel<4><<<a.ngroups, kSzThreads, 0, s>>>(a); break;
-    default: sz_unpack_kernel<1><<<a.ngroups, kSzThreads, 0, s>>>(a);
+    case 8: launch_next(sz_unpack_kernel<8>, a.ngroups, kSzThreads, 0, s, a); break;
+    case 4: launch_next(sz_unpack_kernel<4>, a.ngroups, kSzThreads, 0, s, a); break;
+    default: launch_next(sz_unpack_kernel<1>, a.ngroups, kSzThreads, 0, s, a);
   }
   return launched("ccb_sz_decompress");
 }
@@ -1947,7 +1953,8 @@ extern "C" int ccb_sz_container_scan(const void* slots, const uint32_t* sizes, u
     set_error("ccb_sz_container_scan: bad arguments");
     return CCB_ERR_ARG;
   }
-  container_scan_kernel<<<1, kScanThreads, 0, static_cast<cudaStream_t>(stream)>>>(static_cast<const char*>(slots), sizes, (unsigned int)ngroups, offsets);
+  launch_next(container_scan_kernel, 1, kScanThreads, 0, static_cast<cudaStream_t>(stream), static_cast<const char*>(slots), sizes, (unsigned int)ngroups, offsets,
+              nullptr, nullptr, 0ull);
   return launched("ccb_sz_container_scan");
 }
 
@@ -1961,7 +1968,7 @@ extern "C" int ccb_sz_container_open(const void* blob, uint64_t bytes, uint64_t 
     return CCB_ERR_ARG;
   }
   const uint32_t* head = static_cast<const uint32_t*>(blob);
-  container_scan_kernel<<<1, kScanThreads, 0, static_cast<cudaStream_t>(stream)>>>(nullptr, head + sizeof(ContainerHead) / 4, (unsigned int)room, offsets, head,
+  launch_next(container_scan_kernel, 1, kScanThreads, 0, static_cast<cudaStream_t>(stream), nullptr, head + sizeof(ContainerHead) / 4, (unsigned int)room, offsets, head,
                                                                                   static_cast<uint32_t*>(found), bytes);
   return launched("ccb_sz_container_open");
 }
@@ -1974,7 +1981,7 @@ extern "C" int ccb_sz_container_pack(const void* slots, const unsigned long long
     return CCB_ERR_ARG;
   }
   const ContainerHead head = {kContainerMagic, kContainerVersion, nx, ny, nz, eb, 2.f * eb * (1.f - 0.0009765625f), (uint32_t)ngroups, 0};
-  container_pack_kernel<<<container_grid(ngroups), 256, 0, static_cast<cudaStream_t>(stream)>>>(static_cast<const char*>(slots), offsets, head, static_cast<char*>(out));
+  launch_next(container_pack_kernel, container_grid(ngroups), 256, 0, static_cast<cudaStream_t>(stream), static_cast<const char*>(slots), offsets, head, static_cast<char*>(out));
   return launched("ccb_sz_container_pack");
 }
 
@@ -1984,7 +1991,7 @@ extern "C" int ccb_sz_container_unpack(const void* payload, const unsigned long 
     set_error("ccb_sz_container_unpack: bad arguments");
     return CCB_ERR_ARG;
   }
-  container_unpack_kernel<<<container_grid(ngroups), 256, 0, static_cast<cudaStream_t>(stream)>>>(static_cast<const char*>(payload), offsets,
+  launch_next(container_unpack_kernel, container_grid(ngroups), 256, 0, static_cast<cudaStream_t>(stream), static_cast<const char*>(payload), offsets,
                                                                                                    (unsigned int)ngroups, static_cast<char*>(slots));
   return launched("ccb_sz_container_unpack");
 }

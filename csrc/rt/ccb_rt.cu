@@ -17,6 +17,7 @@
 #include <atomic>
 #include <map>
 #include <mutex>
+#include <set>
 #include <tuple>
 #include <string>
 #include <vector>
@@ -284,6 +285,43 @@ int grid_cap(ccb_comm* c, const void* kernel, int threads) {
   return cap < 1 ? 1 : cap;
 }
 
+// Streams whose last launch here was an overlapping one (see launch()). What comes next on them waits for more than
+// that kernel: the one before it, for which it did not wait, may still run. Rare, so that others look at a counter alone.
+static std::atomic<int> g_overlapped_count{0};
+static std::mutex g_overlapped_lock;
+static std::set<cudaStream_t> g_overlapped;
+static bool g_overlapped_all = false;   // too many streams to tell apart
+static void note_overlapped(cudaStream_t stream) {
+  std::lock_guard<std::mutex> hold(g_overlapped_lock);
+  if (g_overlapped.size() < 4096) g_overlapped.insert(stream);
+  else g_overlapped_all = true;
+  g_overlapped_count.store((int)g_overlapped.size());
+}
+static bool behind_overlapped(cudaStream_t stream) {
+  if (g_overlapped_count.load() == 0) return false;
+  std::lock_guard<std::mutex> hold(g_overlapped_lock);
+  if (g_overlapped_all) return true;
+  const bool hit = g_overlapped.erase(stream) != 0;
+  g_overlapped_count.store((int)g_overlapped.size());
+  return hit;
+}
+
+cudaError_t launch_next(const void* kernel, dim3 grid, dim3 block, void** params, size_t shared, cudaStream_t stream) {
+  if (behind_overlapped(stream)) return cudaLaunchKernel(kernel, grid, block, params, shared, stream);
+  cudaLaunchConfig_t cfg;
+  memset(&cfg, 0, sizeof(cfg));
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = shared;
+  cfg.stream = stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelExC(&cfg, kernel, params);
+}
+
 int launch(ccb_comm* c, const void* kernel, int ctas, void* args, cudaStream_t stream, int threads, bool may_overlap) {
   dim3 grid((unsigned)ctas, (unsigned)c->nlocal, 1), block((unsigned)threads, 1, 1);
   void* params[] = {args};
@@ -310,6 +348,7 @@ int launch(ccb_comm* c, const void* kernel, int ctas, void* args, cudaStream_t s
       set_error("kernel launch failed: %s", cudaGetErrorString(e));
       return CCB_ERR_CUDA;
     }
+    note_overlapped(stream);
     count_launch();
     return CCB_OK;
   }

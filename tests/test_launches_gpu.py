@@ -1,0 +1,57 @@
+"""Launches that are got ready while the kernel before them runs: a chain in which every kernel reads what the one
+before it wrote, ours and torch's in turn, on the default stream, on another, and as a graph."""
+import pytest
+import torch
+
+from ccbench_b200 import Communicator
+from ccbench_b200.ops import lossless, standalone, sz
+
+pytestmark = pytest.mark.gpu
+
+
+def _chain(comm, x, wait):
+    out = []
+    for k in range(6):
+        x = standalone.decode(standalone.encode(x, ("int8", "fp8", "int4")[k % 3]), ("int8", "fp8", "int4")[k % 3], x.numel(), x.dtype)
+        wait()
+        ys = [torch.empty_like(x) for _ in range(2)]
+        comm.all_reduce([x, x.flip(0)], ys, codec="int8")
+        wait()
+        x = ys[1] * 0.5
+        wait()
+        x = lossless.decode(lossless.encode(x), x.numel(), x.dtype)
+        wait()
+        f = x[:x.numel() // 2048 * 2048].view(-1, 32, 64)
+        packed, used = sz.compress(f, 1e-3)
+        wait()
+        f = sz.decompress(packed, f.shape, 1e-3)
+        wait()
+        x = torch.cat([f.reshape(-1), x[f.numel():]])
+        out += [x, used]
+    return out
+
+
+@pytest.mark.parametrize("count", [5_000, 300_001, 6_000_003])
+def test_a_chain_waits_for_what_it_reads(count):
+    comm = Communicator.local(2, arena_bytes=64 << 20)
+    x = torch.randn(count, generator=torch.Generator(device="cuda").manual_seed(count), device="cuda")
+    want = _chain(comm, x, torch.cuda.synchronize)
+    side = torch.cuda.Stream()
+    for _ in range(5):
+        for stream in (torch.cuda.current_stream(), side):
+            stream.wait_stream(torch.cuda.current_stream())
+            with torch.cuda.stream(stream):
+                got = _chain(comm, x, lambda: None)
+            torch.cuda.synchronize()
+            assert all(torch.equal(a, b) for a, b in zip(got, want))
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = _chain(comm, x, lambda: None)
+    for _ in range(3):
+        for t in got:
+            t.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert all(torch.equal(a, b) for a, b in zip(got, want))
+    del graph
+    comm.close()
