@@ -1600,10 +1600,9 @@ static_assert(sizeof(ContainerHead) == 40, "container header layout");
 // offsets[ngroups + 1] = the largest size as it stands, or 2^32 - 1 where a group's tiles cannot have the
 // sizes that its header gives them. `sizes` (u32 each) or, without them, the
 // groups' own headers in `slots`. One CTA: a few thousand groups at most in use, and the copy
-// that follows is the larger part.
+// that follows is the larger part. The last two go to `sums` as well, if given, to be read back.
 // With `head` (the start of a container, the sizes behind it) the number of groups is what the header
-// says, if no more than `ngroups`; otherwise nothing is scanned. Header and the two sums then go to
-// `found` besides, to be read back in one piece, and the groups' headers, in the `bytes` bytes from
+// says, if no more than `ngroups`; otherwise nothing is scanned. The header then goes to `found`, and the groups' headers, in the `bytes` bytes from
 // `head` on, are held against the list.
 constexpr int kScanThreads = 1024;
 __device__ __forceinline__ bool sizes_sound(const uint4& x, const uint4& y) {
@@ -1613,8 +1612,8 @@ __device__ __forceinline__ bool sizes_sound(const uint4& x, const uint4& y) {
 __device__ __forceinline__ uint32_t sizes_sum(const uint4& x, const uint4& y) { return x.x + x.y + x.z + x.w + y.x + y.y + y.z + y.w; }
 __global__ void __launch_bounds__(kScanThreads) container_scan_kernel(const char* __restrict__ slots, const uint32_t* __restrict__ sizes,
                                                                       unsigned int ngroups, unsigned long long* offsets,
-                                                                      const uint32_t* __restrict__ head = nullptr, uint32_t* found = nullptr,
-                                                                      unsigned long long bytes = 0) {
+                                                                      const uint32_t* __restrict__ head, uint32_t* found, unsigned long long bytes,
+                                                                      unsigned long long* sums) {
   after_kernel_before();
   if (head) {
     const uint32_t said = head[7];
@@ -1675,9 +1674,9 @@ __global__ void __launch_bounds__(kScanThreads) container_scan_kernel(const char
     for (int k = 1; k < kScanThreads / 32; ++k) most = max(most, largest[k]);
     offsets[ngroups] = carry;
     offsets[ngroups + 1] = most;
-    if (head) {
-      reinterpret_cast<unsigned long long*>(found)[5] = carry;
-      reinterpret_cast<unsigned long long*>(found)[6] = most;
+    if (sums) {   // of a container: behind the header in `found`
+      sums[0] = carry;
+      sums[1] = most;
     }
   }
 }
@@ -1945,17 +1944,23 @@ extern "C" int ccb_sz_decompress(const void* in, int nx, int ny, int nz, float e
   return launched("ccb_sz_decompress");
 }
 
-// offsets: ngroups + 2 words of 64 bits (see container_scan_kernel). Exactly one of slots and
-// sizes is given.
-extern "C" int ccb_sz_container_scan(const void* slots, const uint32_t* sizes, uint64_t ngroups, unsigned long long* offsets, ccb_stream_t stream) {
+static int container_scan(const void* slots, const uint32_t* sizes, uint64_t ngroups, unsigned long long* offsets, unsigned long long* sums, ccb_stream_t stream) {
   if (!offsets || (slots != nullptr) == (sizes != nullptr) || ngroups == 0 || (ngroups >> 31) || (reinterpret_cast<uintptr_t>(slots) & 15) ||
-      (reinterpret_cast<uintptr_t>(sizes) & 3)) {
+      (reinterpret_cast<uintptr_t>(sizes) & 3) || (reinterpret_cast<uintptr_t>(sums) & 7)) {
     set_error("ccb_sz_container_scan: bad arguments");
     return CCB_ERR_ARG;
   }
-  launch_next(container_scan_kernel, 1, kScanThreads, 0, static_cast<cudaStream_t>(stream), static_cast<const char*>(slots), sizes, (unsigned int)ngroups, offsets,
-              nullptr, nullptr, 0ull);
+  launch_next(container_scan_kernel, 1, kScanThreads, 0, static_cast<cudaStream_t>(stream), static_cast<const char*>(slots), sizes, (unsigned int)ngroups, offsets, nullptr, nullptr,
+              0ull, sums);
   return launched("ccb_sz_container_scan");
+}
+// offsets: ngroups + 2 words of 64 bits (see container_scan_kernel). Exactly one of slots and
+// sizes is given.
+extern "C" int ccb_sz_container_scan(const void* slots, const uint32_t* sizes, uint64_t ngroups, unsigned long long* offsets, ccb_stream_t stream) {
+  return container_scan(slots, sizes, ngroups, offsets, nullptr, stream);
+}
+extern "C" int ccb_sz_container_sums(const void* slots, uint64_t ngroups, unsigned long long* offsets, unsigned long long* sums, ccb_stream_t stream) {
+  return container_scan(slots, nullptr, ngroups, offsets, sums, stream);
 }
 
 // The scan of a container of `bytes` bytes whose header is still on the device: offsets for at most
@@ -1969,7 +1974,7 @@ extern "C" int ccb_sz_container_open(const void* blob, uint64_t bytes, uint64_t 
   }
   const uint32_t* head = static_cast<const uint32_t*>(blob);
   launch_next(container_scan_kernel, 1, kScanThreads, 0, static_cast<cudaStream_t>(stream), nullptr, head + sizeof(ContainerHead) / 4, (unsigned int)room, offsets, head,
-                                                                                  static_cast<uint32_t*>(found), bytes);
+              static_cast<uint32_t*>(found), bytes, static_cast<unsigned long long*>(found) + 5);
   return launched("ccb_sz_container_open");
 }
 

@@ -31,7 +31,7 @@ namespace {
 #define CCB_CALLS(X)                                                                                                          \
   X(ccb_all_reduce) X(ccb_reduce_scatter) X(ccb_all_gather) X(ccb_moe_dispatch) X(ccb_moe_combine) X(ccb_wire_bytes)           \
   X(ccb_encode) X(ccb_decode) X(ccb_reduce_recode) X(ccb_lossless_max_bytes) X(ccb_lossless_encode) X(ccb_lossless_decode)     \
-  X(ccb_sz_capacity) X(ccb_sz_compress) X(ccb_sz_decompress) X(ccb_sz_container_scan) X(ccb_sz_container_open)                 \
+  X(ccb_sz_capacity) X(ccb_sz_compress) X(ccb_sz_decompress) X(ccb_sz_container_sums) X(ccb_sz_container_open)                 \
   X(ccb_sz_container_pack) X(ccb_sz_container_unpack)
 struct Library {
 #define CCB_FIELD(f) decltype(&::f) f;
@@ -364,11 +364,7 @@ FUNCTION(sz_decompress, 3)
   return result(unlocked([&] { return lib.ccb_sz_decompress(in, e[2], e[1], e[0], eb, to, st); }), out);
 END
 
-// `bytes` bytes from the device to pinned memory, waited for.
-int read_back(const at::Tensor& to, const void* from, size_t bytes, cudaStream_t st) {
-  void* host = to.data_ptr();
-  return unlocked([&] { return cudaMemcpyAsync(host, from, bytes, cudaMemcpyDeviceToHost, st) == cudaSuccess && cudaStreamSynchronize(st) == cudaSuccess ? 0 : CCB_ERR_CUDA; });
-}
+int ended(cudaStream_t st) { return cudaStreamSynchronize(st) == cudaSuccess ? 0 : CCB_ERR_CUDA; }
 at::Tensor pinned(int64_t words) { return at::empty({words}, at::TensorOptions().dtype(at::kLong).pinned_memory(true)); }
 
 // (slots, stride of a group) -> (offsets, total, largest): the scan of a buffer's groups
@@ -382,8 +378,11 @@ FUNCTION(sz_scan, 2)
   const void* slots = buf->data_ptr();
   unsigned long long* at = static_cast<unsigned long long*>(offsets.data_ptr());
   const cudaStream_t st = stream();
-  int rc = unlocked([&] { return lib.ccb_sz_container_scan(slots, nullptr, groups, at, st); });
-  if (!rc) rc = read_back(host, at + groups, 16, st);
+  unsigned long long* sums = static_cast<unsigned long long*>(host.data_ptr());   // see sz_open
+  const int rc = unlocked([&] {
+    const int code = lib.ccb_sz_container_sums(slots, groups, at, sums, st);
+    return code ? code : ended(st);
+  });
   if (rc) return PyLong_FromLong(rc);
   const int64_t* v = static_cast<const int64_t*>(host.data_ptr());
   return Py_BuildValue("NLL", THPVariable_Wrap(offsets), (long long)v[0], (long long)v[1]);
@@ -399,8 +398,11 @@ FUNCTION(sz_open, 2)
   const uint64_t bytes = (uint64_t)blob->numel();
   unsigned long long* at = static_cast<unsigned long long*>(offsets.data_ptr());
   const cudaStream_t st = stream();
-  int rc = unlocked([&] { return lib.ccb_sz_container_open(in, bytes, room, at, at + room + 2, st); });
-  if (!rc) rc = read_back(host, at + room + 2, 56, st);
+  void* found = host.data_ptr();   // pinned memory is the device's as well: the kernel's last words, without a copy
+  const int rc = unlocked([&] {
+    const int code = lib.ccb_sz_container_open(in, bytes, room, at, found, st);
+    return code ? code : ended(st);
+  });
   if (rc) return PyLong_FromLong(rc);
   return Py_BuildValue("Ny#", THPVariable_Wrap(offsets), static_cast<const char*>(host.data_ptr()), (Py_ssize_t)56);
 END

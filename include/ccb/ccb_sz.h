@@ -43,6 +43,8 @@ int ccb_sz_decompress(const void* in, int nx, int ny, int nz, float eb, float* o
  * scanned where the header speaks of more than `room` groups (40 + 4 * room <= bytes). */
 int ccb_sz_container_open(const void* blob, uint64_t bytes, uint64_t room, unsigned long long* offsets, void* found, ccb_stream_t stream);
 int ccb_sz_container_scan(const void* slots, const uint32_t* sizes, uint64_t ngroups, unsigned long long* offsets, ccb_stream_t stream);
+/* The scan of slots, its last two words to `sums` as well: device memory or pinned host memory, 8-byte aligned. */
+int ccb_sz_container_sums(const void* slots, uint64_t ngroups, unsigned long long* offsets, unsigned long long* sums, ccb_stream_t stream);
 int ccb_sz_container_pack(const void* slots, const unsigned long long* offsets, int nx, int ny, int nz, float eb, uint64_t ngroups, void* out,
                           ccb_stream_t stream);
 int ccb_sz_container_unpack(const void* payload, const unsigned long long* offsets, uint64_t ngroups, void* slots, ccb_stream_t stream);
