@@ -788,7 +788,6 @@ __device__ __forceinline__ void stage_tile(const SzLocalArgs& a, TileCoord t, un
     if constexpr (kBytes == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(n) : "memory");
     else asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(n) : "memory");
   };
-  constexpr int kParts = kVec == 1 ? kTY : 2;
   const float* from[2];
   bool on[2];
   if constexpr (kVec != 1) {
@@ -802,17 +801,25 @@ __device__ __forceinline__ void stage_tile(const SzLocalArgs& a, TileCoord t, un
     on[0] = t.x0 + lane < a.nx;
     from[0] = on[0] ? a.in + ((size_t)t.z0 * a.ny + t.y0) * a.nx + t.x0 + lane : a.in;
   }
+  const size_t step0 = on[0] ? stride : 0;   // what lies outside is not read: its address stays
+  [[maybe_unused]] size_t step1 = 0;
+  if constexpr (kVec != 1) step1 = on[1] ? stride : 0;
 #pragma unroll
   for (int z = 0; z < kTZ; ++z) {
+    const bool deep = z < depth;
+    if constexpr (kVec != 1) {
 #pragma unroll
-    for (int i = 0; i < kParts; ++i) {
-      if constexpr (kVec != 1) {
-        const bool in = on[i] && z < depth;
-        bring(Int<16>{}, to + 1024 * z + 512 * i + 16 * (lane ^ (lane >> 3 & 1)), in ? from[i] + z * stride : a.in, in);
-      } else {
-        const bool in = on[0] && z < depth && t.y0 + i < a.ny;
-        bring(Int<4>{}, to + 1024 * z + 128 * i + 4 * (lane ^ (4 * (i & 1))), in ? from[0] + z * stride + (size_t)i * a.nx : a.in, in);
+      for (int i = 0; i < 2; ++i) {
+        bring(Int<16>{}, to + 1024 * z + 512 * i + 16 * (lane ^ (lane >> 3 & 1)), from[i], on[i] && deep);
+        if (z + 1 < depth) from[i] += i ? step1 : step0;
       }
+    } else {
+#pragma unroll
+      for (int i = 0; i < kTY; ++i) {
+        const bool in = on[0] && deep && t.y0 + i < a.ny;
+        bring(Int<4>{}, to + 1024 * z + 128 * i + 4 * (lane ^ (4 * (i & 1))), in ? from[0] + (size_t)i * a.nx : a.in, in);
+      }
+      if (z + 1 < depth) from[0] += step0;
     }
     if (z == 1 || z + 1 == kTZ) asm volatile("cp.async.commit_group;" ::: "memory");
   }
@@ -1150,12 +1157,13 @@ __device__ __forceinline__ uint32_t pack_planes(const SzLocalArgs& a, unsigned c
 
 // A warp stages the whole of its tile, 8256 bytes at most, three CTAs an SM; with less of it, tiles that were larger
 // went through the codec a second time, to their places (512^3 values of white noise, bound 1e-5 of their range,
-// 470 us). Bound by instructions at 24 warps an SM: ncu, 384^3, 47.9 M of them, 217 a plane with all that a tile needs
+// 470 us). Bound by instructions at 24 warps an SM: ncu, 384^3, 48.8 M of them, 221 a plane with all that a tile needs
 // besides, 68 % of the issue slots, 54 % of the pipe of logical operations. With planes loaded to registers one ahead
 // (moves of eight registers a plane), residuals one to a word, the masks of the bit transpose chosen at each use and planes
-// of 9 to 16 bits a row at a time it was 62.3 M. (B200, us, that / so: 512^3 field, bound 1e-4 of its range, 173 / 146;
-// 1e-3 168 / 140; 1e-5 189 / 180; with 30 added to its values 179 / 154; 300 x 300 x 404 55.5 / 53.5, x 403 67 / 64; 130
-// x 201 x 258 22.8 / 18.6; white noise 512^3, 1e-5 266 / 268, 1e-6 265 / 248, 1e-7, all raw, 238 / 209.) Operands of the
+// of 9 to 16 bits a row at a time it was 62.3 M. (B200, us, that / so: 512^3 field, bound 1e-4 of its range, 173 / 138;
+// 1e-3 168 / 133; 1e-5 190 / 175; with 30 added to its values 179 / 148; 300 x 300 x 404 55.6 / 49.4, x 403 68 / 61; 130
+// x 201 x 258 22.8 / 16; white noise 512^3, 1e-5 266 / 262, 1e-6 265 / 245, 1e-7, all raw, 239 / 206. An address computed
+// afresh for each piece that is staged 143.) Operands of the
 // packed operations kept in registers, or given as pairs of arguments, changed nothing; one vote for both tests neither.
 template <int kVec>
 __global__ void __launch_bounds__(kSzThreads, 3) sz_pack_kernel(const __grid_constant__ SzLocalArgs a) {
