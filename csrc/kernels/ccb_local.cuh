@@ -18,7 +18,7 @@
 
 namespace ccb {
 
-constexpr int kLocalThreads = 256;
+constexpr int kLocalThreads = 128;   // with 256 the slots of an SM come free in larger pieces (B200, us, 256 / 128: reduce-scatter of 8 x 32 MiB of bf16 in int8 53.2 / 52.3, tree of 3 x 40 MiB of f16 51.0 / 49.3, gather of 8 x 400,003 fp32 21.7 / 20.9)
 
 enum { kLocalTwoShot = 0, kLocalOneShot = 1, kLocalRing = 2, kLocalTree = 3, kLocalScatter = 4 };
 
@@ -33,7 +33,7 @@ struct LocalReduceArgs {
   int n, op, root;             // root: kLocalScatter delivers to this rank alone (>= 0), or shard s to rank s (< 0)
 };
 
-// Ranks whose values are requested before the first is used, and CTAs of 256 threads on an SM: what
+// Ranks whose values are requested before the first is used, and CTAs of 128 threads on an SM: what
 // was fastest of one, two and four ranks at 40 to 128 registers a thread. (At these nothing spills but 4
 // to 8 bytes in one-shots and trees of 16-bit types.)
 // (B200. 4 ranks of 64 MiB of bf16, two-shot int8: two ranks at 64 registers 82.4 us, at 48, which
@@ -42,7 +42,7 @@ struct LocalReduceArgs {
 // at 128 12.6. 4 ranks of 25 MiB of bf16 with residuals: two at 128 registers 96.7, one 100.6.)
 template <class T, int ALGO, bool kEf, bool kAnyOffset> struct LocalShape {
   static constexpr int kBatch = sizeof(T) == 4 || kAnyOffset ? 1 : 2;
-  static constexpr int kCtas = kEf ? 2 : (ALGO == kLocalTree ? 3 : 4) - (sizeof(T) == 4 && (kAnyOffset || ALGO == kLocalTree) ? 1 : 0);
+  static constexpr int kCtas = kEf ? 4 : (ALGO == kLocalTree ? 6 : 8) - (sizeof(T) == 4 && (kAnyOffset || ALGO == kLocalTree) ? 2 : 0);
 };
 
 template <class T>
@@ -332,7 +332,7 @@ __device__ __forceinline__ void local_solo_unit(const LocalReduceArgs& a, size_t
   local_store<T, kAnyOffset>(static_cast<T*>(a.recv[0]), idx, a.count, inside, o);
 }
 template <class T, class C, bool kEf, bool kAnyOffset>
-__global__ void __launch_bounds__(kLocalThreads, kEf ? 4 : sizeof(T) == 4 ? (kAnyOffset ? 4 : 6) : kAnyOffset ? 6 : 8) local_solo_kernel(const __grid_constant__ LocalReduceArgs a) {
+__global__ void __launch_bounds__(kLocalThreads, kEf ? 8 : sizeof(T) == 4 ? (kAnyOffset ? 8 : 12) : kAnyOffset ? 12 : 16) local_solo_kernel(const __grid_constant__ LocalReduceArgs a) {
   after_kernel_before();
   const size_t e0 = (((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * kWarpElems, idx = e0 + (threadIdx.x & 31) * kLaneElems;
   if (e0 >= a.count) return;
@@ -362,7 +362,7 @@ struct LocalExchangeArgs {
 // 64 stores of an element for eight of a lane's 32 bytes, an all-gather of 8 x 1,638,401 bf16 in fp8 took 50 us, 46 so; B200.)
 // A block in place keeps to its own units: the one before may have been written. (Without kAnyOffset a run is one unit.)
 template <class T, class C, bool kAnyOffset>
-__global__ void __launch_bounds__(kLocalThreads, kAnyOffset ? (sizeof(T) == 4 ? 2 : 3) : 6) local_exchange_kernel(const __grid_constant__ LocalExchangeArgs a) {
+__global__ void __launch_bounds__(kLocalThreads, kAnyOffset ? (sizeof(T) == 4 ? 4 : 6) : 12) local_exchange_kernel(const __grid_constant__ LocalExchangeArgs a) {
   after_kernel_before();
   constexpr int W = 4 * (int)sizeof(T), kPer = 4 / (int)sizeof(T);   // words of a lane, elements of a word
   const int lane = threadIdx.x & 31;
