@@ -1300,11 +1300,16 @@ struct PlaneOut {
     planes = gy < a.ny ? depth : 0;
     more = !kAligned ? a.ny - t.y0 : gy + 1 < a.ny ? depth : 0;
   }
-  __device__ __forceinline__ void store(int z, const float (&code)[2][4], float step) const {
-    float* p = at + z * stride;
+  // The planes in turn: the address moves on.
+  __device__ __forceinline__ void store(int z, const float (&code)[2][4], f32x2 step2) {
+    float* p = at;
+    at += stride;
     float4 v[2];
 #pragma unroll
-    for (int j = 0; j < 2; ++j) v[j] = make_float4(__fmul_rn(code[0][j], step), __fmul_rn(code[0][2 + j], step), __fmul_rn(code[1][j], step), __fmul_rn(code[1][2 + j], step));
+    for (int j = 0; j < 2; ++j) {
+      split2(mul2(pair2(code[0][j], code[0][2 + j]), step2), v[j].x, v[j].y);
+      split2(mul2(pair2(code[1][j], code[1][2 + j]), step2), v[j].z, v[j].w);
+    }
     if constexpr (kAligned) {
       if (z < planes) stg_stream(p, *reinterpret_cast<const uint4*>(&v[0]));
       if (z < more) stg_stream(p + line, *reinterpret_cast<const uint4*>(&v[1]));
@@ -1323,13 +1328,14 @@ struct PlaneOut {
 
 // A packed tile in shared memory whose residuals have at most 15 bits, those of its first plane 22.
 template <bool kAligned>
-__device__ __forceinline__ void unpack_digits(const PlaneOut<kAligned>& io, const unsigned char* tile, uint32_t small, float step) {
+__device__ __forceinline__ void unpack_digits(PlaneOut<kAligned>& io, const unsigned char* tile, uint32_t small, float step) {
   const int lane = threadIdx.x & 31, j = lane & 7;
   const uint32_t* words = reinterpret_cast<const uint32_t*>(tile + kRows);
   // Lane 8 r + j fetches bit planes of row r: for j = 7 the first, which holds the signs, so that it comes to the
   // highest bit of a byte; else plane j + 1, and of wider rows j + 8.
   const uint32_t below = (1u << (lane & 24)) - 1u, first = (uint32_t)(j + 1) & 7u, pick = 0x4440u | (uint32_t)(lane >> 3);
   PlanePrefix sums(lane);
+  const f32x2 step2 = pair2(step, step);
   uint32_t run = 0;   // words before the plane
   auto plane = [&](int z, auto narrow) {
     const uint2 W = reinterpret_cast<const uint2*>(tile)[z];
@@ -1374,7 +1380,7 @@ __device__ __forceinline__ void unpack_digits(const PlaneOut<kAligned>& io, cons
         for (int e = 0; e < 8; ++e) sums.code[e >> 2][e & 3] = __fmaf_rn(top[e >> 2][e & 3], 16384.f, sums.code[e >> 2][e & 3]);
       }
     }
-    io.store(z, sums.code, step);
+    io.store(z, sums.code, step2);
   };
   if ((small | 3u) == 0xffffffffu) {   // nearly always: beyond the first plane no residual of more than 8 bits
     plane(0, Int<0>{});
@@ -1389,11 +1395,13 @@ __device__ __forceinline__ void unpack_digits(const PlaneOut<kAligned>& io, cons
 // A warp brings a packed tile of up to 2304 bytes to shared memory, all of it under way at once, and takes its planes
 // from there by the tensor cores; larger ones, raw ones, and those with wider residuals are read where they are, from L2 where
 // a prefetch puts them, and summed by shuffles. (B200, us, the whole by shuffles with one plane requested ahead / so: 512^3
-// field, bound 1e-4 of its range, 163 / 122; 1e-3 154 / 115; 1e-5 183 / 140; the first with 30 added to its values 165 / 131;
-// 300 x 300 x 404 49.5 / 33.5, x 403 61.8 / 55; 512^3 of white noise, 1e-6 189 / 177, 1e-5 277 / 279. Stages of 4608 bytes took
-// as long on the fields and 12 us more on the noise at 1e-6; five CTAs of 48 registers spill, 129 instead of 120, three of
-// 80 138. Lanes that hold 32 bytes of a line: as fast at 512^3, 45 instead of 33 where lines lie on 16 bytes. B200.)
-// What is left of the 94 us that the memory needs is the latency of a tile's size, then its words.
+// field, bound 1e-4 of its range, 163 / 111; 1e-3 154 / 105; 1e-5 183 / 129; the first with 30 added to its values 165 / 118;
+// 300 x 300 x 404 49.5 / 32, x 403 62 / 51; 512^3 of white noise, 1e-6 190 / 173, 1e-5 277 / 258. Stages of 4608 bytes took
+// as long on the fields and 12 us more on the noise at 1e-6; five CTAs of 48 registers spill and take 10 us more, three of 80
+// 18. Lanes that hold 32 bytes of a line: as fast at 512^3, 45 instead of 33 where lines lie on 16 bytes. Resident CTAs that
+// take groups in turn with the next tile under way: 209 instead of 119. Addresses moved on instead of computed, values
+// scaled in pairs: 119 and 111.) ncu, 384^3: 33.6 M instructions, 58.2 M by shuffles. What is left of the 94 us that the memory
+// needs is the latency of a tile's size, then its words.
 constexpr int kUnpackStage = 2304;
 
 template <int kVec>
@@ -1426,7 +1434,7 @@ __global__ void __launch_bounds__(kSzThreads, 4) sz_unpack_kernel(const __grid_c
   if (lane < 16) hw = staged ? reinterpret_cast<const uint32_t*>(stages[k])[lane] : ldg_cg_u32(src + 4 * lane);
   if (!there) hw = 0xfefefefeu;
   if (staged && !__any_sync(0xffffffffu, ((hw + (lane < 2 ? 0x69696969u : 0x70707070u)) | hw) & 0x80808080u) && kRows + 4u * __reduce_add_sync(0xffffffffu, bytesum(hw)) <= size) {
-    const PlaneOut<kVec != 1> out(a, coord, plane[kVec == 1 ? k : 0]);
+    PlaneOut<kVec != 1> out(a, coord, plane[kVec == 1 ? k : 0]);
     unpack_digits(out, stages[k], __ballot_sync(0xffffffffu, bytes_le8(hw)), a.two_eb);
     return;
   }
