@@ -919,12 +919,17 @@ __device__ __forceinline__ void bytes_of_halves(const uint32_t (&t)[4], int at, 
 // Packs the warp's tile as pack_planes does, if its codes lie within 4094 of the first: then two residuals share a word,
 // a + 65536 b, whose sums and differences are those of the pairs whatever carries between the halves, since in
 // the end a is below 2^15 either way (8 x 4095). All codes are taken relative to the first, which
-// leaves only the first residual other than it is. Returns the tile's words; kNoHalves where it is not such a tile (`whole`:
-// its values are all there still).
+// leaves only the first residual other than it is. Returns the tile's words; kNoHalves where a plane is not such a one:
+// `left` then says where pack_planes goes on.
 // Additions of 1.5 * 2^23 are multiply-adds by a.one, two at a time: as additions they could be fused with the
 // products before them (see f32x2).
 constexpr uint32_t kNoHalves = 0xffffffffu;
-__device__ __forceinline__ uint32_t pack_halves(const SzLocalArgs& a, unsigned char* pk, bool& bad, bool& whole) {
+struct TileLeft {
+  int z;            // planes that are packed
+  uint32_t run;     // their words
+  int before[8];    // codes of the last of them, 2^21 added
+};
+__device__ __forceinline__ uint32_t pack_halves(const SzLocalArgs& a, unsigned char* pk, bool& bad, TileLeft& left) {
   const int lane = threadIdx.x & 31;
   uint32_t* words = reinterpret_cast<uint32_t*>(pk + kRows);
   const float half = 0.5f * a.two_eb;
@@ -1065,18 +1070,33 @@ __device__ __forceinline__ uint32_t pack_halves(const SzLocalArgs& a, unsigned c
       asm volatile("cp.async.wait_group 0;" ::: "memory");
       __syncwarp();
     }
+    left.z = z;
     staged_plane(pk, z, x);
-    if (!plane(z, x, Int<1>{})) {
-      whole = z == 0;
-      return bad ? 0 : kNoHalves;
-    }
+    if (!plane(z, x, Int<1>{})) break;
+    left.z = z + 1;
     staged_plane(pk, z + 1, x);
-    if (!plane(z + 1, x, Int<0>{})) return bad ? 0 : kNoHalves;
+    if (!plane(z + 1, x, Int<0>{})) break;
+    left.z = z + 2;
   }
+  if (bad) return 0;
   __syncwarp();
-  if (lane < 16 && !((wide >> (lane >> 1)) & 1u)) {
+  if (lane < 2 * left.z && !((wide >> (lane >> 1)) & 1u)) {
     uint32_t* rows = reinterpret_cast<uint32_t*>(pk) + lane;
     *rows = byte_bits(*rows);
+  }
+  if (left.z < kTZ) {
+    left.run = run;
+    float first, unused;
+    split2(first2, first, unused);
+    const int code = __float_as_int(-first);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const uint32_t two = before[i] - (uint32_t)code * 65537u;
+      const int lo = (int)(two << 16) >> 16, hi = (int)(two - (uint32_t)lo) >> 16, base = code - __float_as_int(kRoundMagic) + kCodeBias;
+      left.before[i] = left.z ? base + lo : kCodeBias;
+      left.before[4 + i] = left.z ? base + hi : kCodeBias;
+    }
+    return kNoHalves;
   }
   const uint32_t pad = (0u - run) & 3u;
   if ((uint32_t)lane < pad) words[run + lane] = 0u;
@@ -1091,17 +1111,17 @@ __device__ __forceinline__ uint32_t row_planes(uint32_t& u, int lane) {
   return stored;
 }
 
-// Packs the warp's tile to `pk` (64 width bytes, then the planes). Returns its words, or 0 and `bad` as
+// Packs what is left of the warp's tile to `pk` (64 width bytes, then the planes). Returns the tile's words, or 0 and `bad` as
 // soon as a plane shows that it has to be stored raw.
-__device__ __forceinline__ uint32_t pack_planes(const SzLocalArgs& a, unsigned char* pk, bool& bad) {
+__device__ __forceinline__ uint32_t pack_planes(const SzLocalArgs& a, unsigned char* pk, bool& bad, const TileLeft& left) {
   const int lane = threadIdx.x & 31;
   uint32_t* words = reinterpret_cast<uint32_t*>(pk + kRows);
   int before[8];
 #pragma unroll
-  for (int e = 0; e < 8; ++e) before[e] = kCodeBias;
-  uint32_t run = 0;
+  for (int e = 0; e < 8; ++e) before[e] = left.before[e];
+  uint32_t run = left.run;
 #pragma unroll 1
-  for (int z = 0; z < kTZ; ++z) {
+  for (int z = left.z; z < kTZ; ++z) {
     float x[8];
     staged_plane(pk, z, x);
     int q[8], d[8];
@@ -1161,9 +1181,10 @@ __device__ __forceinline__ uint32_t pack_planes(const SzLocalArgs& a, unsigned c
 // besides, 68 % of the issue slots, 54 % of the pipe of logical operations. With planes loaded to registers one ahead
 // (moves of eight registers a plane), residuals one to a word, the masks of the bit transpose chosen at each use and planes
 // of 9 to 16 bits a row at a time it was 62.3 M. (B200, us, that / so: 512^3 field, bound 1e-4 of its range, 173 / 138;
-// 1e-3 168 / 133; 1e-5 190 / 175; with 30 added to its values 179 / 148; 300 x 300 x 404 55.6 / 49.4, x 403 68 / 61; 130
+// 1e-3 168 / 132; 1e-5 190 / 166; with 30 added to its values 179 / 148; 300 x 300 x 404 55.6 / 49.4, x 403 68 / 61; 130
 // x 201 x 258 22.8 / 16; white noise 512^3, 1e-5 266 / 262, 1e-6 265 / 245, 1e-7, all raw, 239 / 206. An address computed
-// afresh for each piece that is staged 143.) Operands of the
+// afresh for each piece that is staged 143; tiles begun again by the general way where a plane is not one for halves, 175 at
+// 1e-5. Two planes at a time, with one vote and their transposes interleaved, 135.5 at 1e-4 but 202 at 1e-5.) Operands of the
 // packed operations kept in registers, or given as pairs of arguments, changed nothing; one vote for both tests neither.
 template <int kVec>
 __global__ void __launch_bounds__(kSzThreads, 3) sz_pack_kernel(const __grid_constant__ SzLocalArgs a) {
@@ -1179,16 +1200,12 @@ __global__ void __launch_bounds__(kSzThreads, 3) sz_pack_kernel(const __grid_con
   bool raw = false;
   if (tile < (unsigned)a.tiles_x * a.tiles_y * a.tiles_z) {
     stage_tile<kVec>(a, coord, stage);
-    bool whole = false;
-    uint32_t words = pack_halves(a, stage, raw, whole);
+    TileLeft left;
+    uint32_t words = pack_halves(a, stage, raw, left);
     if (words == kNoHalves) {
-      if (!whole) {
-        __syncwarp();
-        stage_tile<kVec>(a, coord, stage);
-      }
       asm volatile("cp.async.wait_all;" ::: "memory");
       __syncwarp();
-      words = pack_planes(a, stage, raw);
+      words = pack_planes(a, stage, raw, left);
     }
     asm volatile("cp.async.wait_all;" ::: "memory");   // of a tile that was left early
     size = raw ? kTileCap : (kRows + 4u * words + 15u) & ~15u;
