@@ -20,7 +20,7 @@ static const void* find(int dtype, const LocalKey& k) {
 }
 
 // One unit (or run) a warp (ring, 4 ranks of 64 MiB of bf16 in fp8: 83 us so, 97 with resident CTAs
-// that loop). CTAs of up to 256 threads; a call of few units gets narrower ones, to be spread over
+// that loop). CTAs of up to 128 threads; a call of few units gets narrower ones, to be spread over
 // the chip all the same.
 static int local_launch(ccb_comm* c, const void* fn, void* args, uint64_t warps, cudaStream_t stream) {
   const uint64_t sms = (uint64_t)comm_sms(c);

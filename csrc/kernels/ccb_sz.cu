@@ -1178,7 +1178,7 @@ __device__ __forceinline__ uint32_t pack_planes(const SzLocalArgs& a, unsigned c
 // A warp stages the whole of its tile, 8256 bytes at most, three CTAs an SM; with less of it, tiles that were larger
 // went through the codec a second time, to their places (512^3 values of white noise, bound 1e-5 of their range,
 // 470 us). Bound by instructions at 24 warps an SM: ncu, 384^3, 48.8 M of them, 221 a plane with all that a tile needs
-// besides, 68 % of the issue slots, 54 % of the pipe of logical operations. With planes loaded to registers one ahead
+// besides, 73 % of the issue slots, 60 % of the pipe of logical operations. With planes loaded to registers one ahead
 // (moves of eight registers a plane), residuals one to a word, the masks of the bit transpose chosen at each use and planes
 // of 9 to 16 bits a row at a time it was 62.3 M. (B200, us, that / so: 512^3 field, bound 1e-4 of its range, 173 / 138;
 // 1e-3 168 / 132; 1e-5 190 / 166; with 30 added to its values 179 / 148; 300 x 300 x 404 55.6 / 49.4, x 403 68 / 61; 130
@@ -1343,9 +1343,21 @@ struct PlaneOut {
   }
 };
 
-// A packed tile in shared memory whose residuals have at most 15 bits, those of its first plane 22.
-template <bool kAligned>
-__device__ __forceinline__ void unpack_digits(PlaneOut<kAligned>& io, const unsigned char* tile, uint32_t small, float step) {
+// Bytes of a packed tile that a warp holds in shared memory: with residuals of at most 8 bits, those of the first plane
+// 22, all of it; with at most 15 bits its planes in two turns.
+constexpr int kUnpackStage = 2816, kDigitsMost = kRows + 4 * (8 * 22 + 7 * 8 * 15);
+static_assert(kRows + 4 * (8 * 22 + 7 * 8 * 8) <= kUnpackStage && kDigitsMost % 16 == 0, "tiles of small residuals are held whole");
+static_assert(kDigitsMost - (kUnpackStage - 4 * 8 * 22) + 16 <= kUnpackStage - kRows, "what a first turn leaves fits a second one");
+__device__ __forceinline__ void bring_tile(unsigned char* to, const unsigned char* from, uint32_t bytes, int lane) {
+  for (uint32_t i = 16u * lane; i < bytes; i += 512u) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(to) + i), "l"(from + i) : "memory");
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  __syncwarp();
+}
+
+// A packed tile whose residuals have at most 15 bits, those of its first plane 22, in shared memory; kWhole false: the first
+// kUnpackStage bytes of it, of the `size` at `src`.
+template <bool kWhole, bool kAligned>
+__device__ __forceinline__ void unpack_digits(PlaneOut<kAligned>& io, unsigned char* tile, const unsigned char* src, uint32_t size, uint32_t small, float step) {
   const int lane = threadIdx.x & 31, j = lane & 7;
   const uint32_t* words = reinterpret_cast<const uint32_t*>(tile + kRows);
   // Lane 8 r + j fetches bit planes of row r: for j = 7 the first, which holds the signs, so that it comes to the
@@ -1399,7 +1411,21 @@ __device__ __forceinline__ void unpack_digits(PlaneOut<kAligned>& io, const unsi
     }
     io.store(z, sums.code, step2);
   };
-  if ((small | 3u) == 0xffffffffu) {   // nearly always: beyond the first plane no residual of more than 8 bits
+  if constexpr (!kWhole) {
+    uint32_t held = (kUnpackStage - kRows) / 4;   // words before the end of what is in shared memory
+#pragma unroll 1
+    for (int z = 0; z < kTZ; ++z) {
+      const uint2 W = reinterpret_cast<const uint2*>(tile)[z];
+      if (__dp4a(W.y, 0x01010101u, __dp4a(W.x, 0x01010101u, run)) > held) {
+        const uint32_t gone = run & ~3u, at = kRows + 4u * gone;
+        __syncwarp();
+        bring_tile(tile + kRows, src + at, min(size - at, (uint32_t)(kUnpackStage - kRows)), lane);
+        words = reinterpret_cast<const uint32_t*>(tile + kRows) - gone;
+        held = size;
+      }
+      plane(z, Int<0>{});
+    }
+  } else if ((small | 3u) == 0xffffffffu) {   // nearly always: beyond the first plane no residual of more than 8 bits
     plane(0, Int<0>{});
 #pragma unroll
     for (int z = 1; z < kTZ; ++z) plane(z, Int<1>{});
@@ -1409,18 +1435,19 @@ __device__ __forceinline__ void unpack_digits(PlaneOut<kAligned>& io, const unsi
   }
 }
 
-// A warp brings a packed tile of up to 2304 bytes to shared memory, all of it under way at once, and takes its planes
-// from there by the tensor cores; larger ones, raw ones, and those with wider residuals are read where they are, from L2 where
-// a prefetch puts them, and summed by shuffles. (B200, us, the whole by shuffles with one plane requested ahead / so: 512^3
-// field, bound 1e-4 of its range, 163 / 111; 1e-3 154 / 105; 1e-5 183 / 129; the first with 30 added to its values 165 / 118;
-// 300 x 300 x 404 49.5 / 32, x 403 62 / 51; 512^3 of white noise, 1e-6 190 / 173, 1e-5 277 / 258. Stages of 4608 bytes took
-// as long on the fields and 12 us more on the noise at 1e-6; five CTAs of 48 registers spill and take 10 us more, three of 80
-// 18. Lanes that hold 32 bytes of a line: as fast at 512^3, 45 instead of 33 where lines lie on 16 bytes. Resident CTAs that
-// take groups in turn with the next tile under way: 209 instead of 119. Addresses moved on instead of computed, values
-// scaled in pairs: 119 and 111.) ncu, 384^3: 33.6 M instructions, 58.2 M by shuffles. What is left of the 94 us that the memory
-// needs is the latency of a tile's size, then its words.
-constexpr int kUnpackStage = 2304;
-
+// A warp brings a packed tile to shared memory, all of it under way at once or, above 2816 bytes, in two turns, and
+// takes its planes from there by the tensor cores; raw ones, and those with residuals of more than 15 bits, are read
+// where they are, from L2 where a prefetch puts them, and summed by shuffles. (B200, us, the whole by shuffles with
+// one plane requested ahead / so: 512^3 field, bound 1e-4 of its range, 163 / 111; 1e-3 154 / 105; 1e-5 183 / 129;
+// the first with 30 added to its values 165 / 118; 300 x 300 x 404 49.5 / 32, x 403 62 / 51; 512^3 of white noise,
+// 1e-6 190 / 173, 1e-5 277 / 258. Stages of 4608 bytes took as long on the fields and 12 us more on the noise at
+// 1e-6, of 3328 10 us more there; of 2304, with larger tiles by shuffles, a field at 3e-6, 1.3 bytes a value, 242
+// instead of 175, 256^3 white noise of 1.65 bytes a value 41 instead of 27, 256^3 at 1e-5 21.5 instead of 22.4 (one
+// loop for both kinds of wide tiles 23.1). Five CTAs of 48 registers spill and take 10 us more, three of 80 18. Lanes
+// that hold 32 bytes of a line: as fast at 512^3, 45 instead of 33 where lines lie on 16 bytes. Resident CTAs that
+// take groups in turn with the next tile under way: 209 instead of 119. Addresses moved on instead of computed,
+// values scaled in pairs: 119 and 111.) ncu, 384^3: 30.8 M instructions, 58.2 M by shuffles. What is left of the 94
+// us that the memory needs is the latency of a tile's size, then its words.
 template <int kVec>
 __global__ void __launch_bounds__(kSzThreads, 4) sz_unpack_kernel(const __grid_constant__ SzLocalArgs a) {
   after_kernel_before();
@@ -1438,12 +1465,10 @@ __global__ void __launch_bounds__(kSzThreads, 4) sz_unpack_kernel(const __grid_c
   if (!there) off = 0;
   const unsigned char* src = reinterpret_cast<const unsigned char*>(group) + kGroupHeader + off;
   // (a buffer is promised to start on 4 bytes, no more)
-  const bool staged = size >= kRows && size <= kUnpackStage && (size & 15u) == 0 && (reinterpret_cast<uintptr_t>(src) & 15) == 0;
+  const bool staged = size >= kRows && size <= kDigitsMost && (size & 15u) == 0 && (reinterpret_cast<uintptr_t>(src) & 15) == 0;
   if (staged) {
-    const uint32_t to = smem_u32(stages[k]);
-    for (uint32_t i = 16u * lane; i < size; i += 512u) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to + i), "l"(src + i) : "memory");
-    asm volatile("cp.async.wait_all;" ::: "memory");
-    __syncwarp();
+    if (kUnpackStage + 128u * lane < size) asm volatile("prefetch.global.L2 [%0];" ::"l"(src + kUnpackStage + 128 * lane));
+    bring_tile(stages[k], src, min(size, (uint32_t)kUnpackStage), lane);
   } else {
     for (uint32_t i = 128u * lane; i < min(size, (uint32_t)kTileCap); i += 4096u) asm volatile("prefetch.global.L2 [%0];" ::"l"(src + i));
   }
@@ -1452,7 +1477,9 @@ __global__ void __launch_bounds__(kSzThreads, 4) sz_unpack_kernel(const __grid_c
   if (!there) hw = 0xfefefefeu;
   if (staged && !__any_sync(0xffffffffu, ((hw + (lane < 2 ? 0x69696969u : 0x70707070u)) | hw) & 0x80808080u) && kRows + 4u * __reduce_add_sync(0xffffffffu, bytesum(hw)) <= size) {
     PlaneOut<kVec != 1> out(a, coord, plane[kVec == 1 ? k : 0]);
-    unpack_digits(out, stages[k], __ballot_sync(0xffffffffu, bytes_le8(hw)), a.two_eb);
+    const uint32_t small = __ballot_sync(0xffffffffu, bytes_le8(hw));
+    if (size <= kUnpackStage) unpack_digits<true>(out, stages[k], src, size, small, a.two_eb);
+    else unpack_digits<false>(out, stages[k], src, size, small, a.two_eb);
     return;
   }
   const PlaneIO<kVec> io(a.out, a, coord, plane[kVec == 1 ? k : 0]);

@@ -37,7 +37,7 @@ def test_every_width_of_residuals_comes_back(shape):
     buf, _ = sz.compress(field, EB)
     assert torch.equal(sz.decompress(buf, shape, EB), field)
     tiles = buf.view(-1, sz.GROUP_STRIDE)[:, :sz.GROUP_HEADER].contiguous().view(torch.int32)
-    assert int((tiles == sz.TILE_CAP).sum()) == 0 and int((tiles > 2304).sum()) > 0 and int((tiles[tiles > 0] <= 2304).sum()) > 0
+    assert int((tiles == sz.TILE_CAP).sum()) == 0 and int(((tiles > 2816) & (tiles <= 4128)).sum()) > 0 and int((tiles[tiles > 0] <= 2816).sum()) > 0
 
 
 def test_a_buffer_on_four_bytes_is_unpacked_where_it_lies():
