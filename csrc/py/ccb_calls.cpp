@@ -364,6 +364,11 @@ FUNCTION(sz_decompress, 3)
   return result(unlocked([&] { return lib.ccb_sz_decompress(in, e[2], e[1], e[0], eb, to, st); }), out);
 END
 
+// A capture cannot be read back from: the general way says so.
+bool capturing(cudaStream_t st) {
+  cudaStreamCaptureStatus now;
+  return cudaStreamIsCapturing(st, &now) != cudaSuccess || now != cudaStreamCaptureStatusNone;
+}
 int ended(cudaStream_t st) { return cudaStreamSynchronize(st) == cudaSuccess ? 0 : CCB_ERR_CUDA; }
 at::Tensor pinned(int64_t words) { return at::empty({words}, at::TensorOptions().dtype(at::kLong).pinned_memory(true)); }
 
@@ -374,10 +379,11 @@ FUNCTION(sz_scan, 2)
   if (!buf || buf->scalar_type() != at::kByte || !number(a[1], stride)) NOT_TAKEN;
   const uint64_t groups = (uint64_t)buf->numel() / stride;
   if (!groups || groups * stride != (uint64_t)buf->numel() || (reinterpret_cast<uintptr_t>(buf->data_ptr()) & 15)) NOT_TAKEN;
+  const cudaStream_t st = stream();
+  if (capturing(st)) NOT_TAKEN;
   const at::Tensor offsets = made({(int64_t)groups + 2}, at::kLong, *buf), host = pinned(2);
   const void* slots = buf->data_ptr();
   unsigned long long* at = static_cast<unsigned long long*>(offsets.data_ptr());
-  const cudaStream_t st = stream();
   unsigned long long* sums = static_cast<unsigned long long*>(host.data_ptr());   // see sz_open
   const int rc = unlocked([&] {
     const int code = lib.ccb_sz_container_sums(slots, groups, at, sums, st);
@@ -393,11 +399,12 @@ FUNCTION(sz_open, 2)
   const at::Tensor* blob = plain(a[0]);
   uint64_t room;
   if (!blob || blob->scalar_type() != at::kByte || !number(a[1], room) || !room || room >> 31) NOT_TAKEN;
+  const cudaStream_t st = stream();
+  if (capturing(st)) NOT_TAKEN;
   const at::Tensor offsets = made({(int64_t)room + 2 + 7}, at::kLong, *blob), host = pinned(7);
   const void* in = blob->data_ptr();
   const uint64_t bytes = (uint64_t)blob->numel();
   unsigned long long* at = static_cast<unsigned long long*>(offsets.data_ptr());
-  const cudaStream_t st = stream();
   void* found = host.data_ptr();   // pinned memory is the device's as well: the kernel's last words, without a copy
   const int rc = unlocked([&] {
     const int code = lib.ccb_sz_container_open(in, bytes, room, at, found, st);
