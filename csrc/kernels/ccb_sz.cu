@@ -923,7 +923,7 @@ __device__ __forceinline__ void bytes_of_halves(const uint32_t (&t)[4], int at, 
 // `left` then says where pack_planes goes on.
 // Additions of 1.5 * 2^23 are multiply-adds by a.one, two at a time: as additions they could be fused with the
 // products before them (see f32x2).
-constexpr uint32_t kNoHalves = 0xffffffffu;
+constexpr uint32_t kNoHalves = 0xffffffffu, kFirstMost = kCodeBias - 4096;   // kFirstMost: of the first code, so that all are below 2^21
 struct TileLeft {
   int z;            // planes that are packed
   uint32_t run;     // their words
@@ -956,12 +956,12 @@ __device__ __forceinline__ uint32_t pack_halves(const SzLocalArgs& a, unsigned c
       split2(fma2(mul2(add2(r2[i], back2), step2), less2, x2), diff[2 * i], diff[2 * i + 1]);
     }
     uint32_t bias0 = 0x80808080u;
-    int corner = 0;
+    uint32_t corner = 0;
     if (decltype(first_too)::value && z == 0) {
       const int first = __shfl_sync(0xffffffffu, q[0], 0);
-      corner = first - __float_as_int(kRoundMagic);
-      far = abs(corner) >= 32000;
-      if (lane == 0) bias0 += far ? 1 << 14 : corner;
+      corner = (uint32_t)first - __float_as_uint(kRoundMagic);
+      far = !ccb_sz_code_within(corner, 31999u);
+      if (lane == 0) bias0 += far ? 1u << 14 : corner;
 #pragma unroll
       for (int i = 0; i < 4; ++i) before[i] = (uint32_t)first * 65537u;
       first2 = pair2(-__int_as_float(first), -__int_as_float(first));
@@ -970,8 +970,8 @@ __device__ __forceinline__ uint32_t pack_halves(const SzLocalArgs& a, unsigned c
     for (int i = 0; i < 4; ++i) split2(add2(r2[i], first2), away[2 * i], away[2 * i + 1]);
     const float worst = max3_abs_nan(max3_abs_nan(diff[0], diff[1], diff[2]), max3_abs_nan(diff[3], diff[4], diff[5]), max3_abs_nan(diff[6], diff[7], 0.f));
     const float apart = max3_abs_nan(max3_abs_nan(away[0], away[1], away[2]), max3_abs_nan(away[3], away[4], away[5]), max3_abs_nan(away[6], away[7], 0.f));
-    if (__any_sync(0xffffffffu, !(worst <= half && apart <= 4094.f) || abs(corner) > kCodeBias - 4096)) {
-      if (__any_sync(0xffffffffu, !(apart <= 4094.f) || abs(corner) > kCodeBias - 4096)) return false;
+    if (__any_sync(0xffffffffu, !(worst <= half && apart <= 4094.f) || !ccb_sz_code_within(corner, kFirstMost))) {
+      if (__any_sync(0xffffffffu, !(apart <= 4094.f) || !ccb_sz_code_within(corner, kFirstMost))) return false;
 #pragma unroll
       for (int e = 0; e < 8; ++e) {   // the nearest grid point by the decoder's own product, as in exact_codes: nearly always one of 256
         const bool off = fabsf(diff[e]) > half;
@@ -1053,7 +1053,7 @@ __device__ __forceinline__ uint32_t pack_halves(const SzLocalArgs& a, unsigned c
         e[i] = lo - 128;
         e[4 + i] = ((int)(t[i] - (uint32_t)lo) >> 16) - 128;
       }
-      if (lane == 0) e[0] += corner - (1 << 14);
+      if (lane == 0) e[0] += (int)corner - (1 << 14);
       uint32_t W0, W1;
       run = wide_plane(e, words, W0, W1, lane);
       if (lane == 0) reinterpret_cast<uint2*>(pk)[0] = make_uint2(W0, W1);
@@ -1088,11 +1088,11 @@ __device__ __forceinline__ uint32_t pack_halves(const SzLocalArgs& a, unsigned c
     left.run = run;
     float first, unused;
     split2(first2, first, unused);
-    const int code = __float_as_int(-first);
+    const uint32_t code = __float_as_uint(-first);
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      const uint32_t two = before[i] - (uint32_t)code * 65537u;
-      const int lo = (int)(two << 16) >> 16, hi = (int)(two - (uint32_t)lo) >> 16, base = code - __float_as_int(kRoundMagic) + kCodeBias;
+      const uint32_t two = before[i] - code * 65537u;
+      const int lo = (int)(two << 16) >> 16, hi = (int)(two - (uint32_t)lo) >> 16, base = (int)(code - __float_as_uint(kRoundMagic) + kCodeBias);
       left.before[i] = left.z ? base + lo : kCodeBias;
       left.before[4 + i] = left.z ? base + hi : kCodeBias;
     }

@@ -28,5 +28,9 @@ CCB_SZ_LAYOUT_FN int ccb_sz_offset_ok(uint32_t off, unsigned k) { return off <= 
 CCB_SZ_LAYOUT_FN int ccb_sz_size_ok(uint32_t size) { return size == 0 || (size >= CCB_SZ_ROWS && size <= CCB_SZ_TILE_CAP && (size & 15u) == 0); }
 /* Is every byte of a word of four row widths at most 32? */
 CCB_SZ_LAYOUT_FN int ccb_sz_widths_ok(uint32_t four) { return ((four | ((four & 0x7f7f7f7fu) + 0x5f5f5f5fu)) & 0x80808080u) == 0; }
+/* The packer adds 1.5 * 2^23 to a value in steps and takes how far the sum's bits are above that number's as the
+ * code (mod 2^32): is it within `most` (below 2^22) of 0? Without a sign, because -1.5 * 2^23, the sum of a value 1.5 * 2^24
+ * steps below 0, lies 2^31 away, which has no magnitude in 32 bits. */
+CCB_SZ_LAYOUT_FN int ccb_sz_code_within(uint32_t code, uint32_t most) { return code + most <= 2u * most; }
 
 #endif

@@ -74,3 +74,17 @@ def test_tiles_packed_in_halves_end_where_they_should(nx):
     buf, _ = sz.compress(f.cuda(), EB)
     want = sz.encode_cpu(f.numpy(), EB)
     assert (sz.to_container(buf, f.shape, EB).cpu().numpy() == want).all()
+
+
+@pytest.mark.parametrize("value,eb", [(-50282496.0, 1.0), (-5028.2495, 1e-4)])   # 1.5 * 2^24 steps below 0: a tile of them has no codes
+@pytest.mark.parametrize("nx", [256, 260, 257])
+def test_tiles_that_begin_far_outside_the_codes_are_stored_raw(value, eb, nx):
+    f = torch.randn((16, 24, nx), generator=torch.Generator().manual_seed(3)).cumsum(2) * (20 * eb)
+    f[:8, 8:16, 32:64] = value
+    f[8:, :8, 64:96] += value   # not constant, within 4094 codes of the first
+    f[8:, 16:, 0] = value
+    f[0, 0, 128] = value        # the first value alone
+    f[1, 16, 200] = value       # another alone
+    buf, _ = sz.compress(f.cuda(), eb)
+    assert (sz.to_container(buf, f.shape, eb).cpu().numpy() == sz.encode_cpu(f.numpy(), eb)).all()
+    assert (sz.decompress(buf, f.shape, eb).cpu() - f).abs().max() <= eb
