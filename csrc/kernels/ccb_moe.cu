@@ -276,8 +276,9 @@ __global__ void __launch_bounds__(kMoeLocalThreads, 9) moe_local_combine_kernel(
   float acc[16];
 #pragma unroll
   for (int i = 0; i < 16; ++i) acc[i] = 0.f;
+  int k0 = 0;
 #pragma unroll 1
-  for (int k0 = 0; k0 < a.topk; k0 += kSlots) {   // more than one turn: units is 1
+  do {   // more than one turn: units is 1; one all the same where a token has no rows, whose sum is 0
     const uint32_t rows = (uint32_t)min(kSlots, a.topk - k0);
     const char* row = nullptr;   // lane k: the k-th row from the unit on
     float gate_k = 0.f;
@@ -316,7 +317,8 @@ __global__ void __launch_bounds__(kMoeLocalThreads, 9) moe_local_combine_kernel(
       }
     }
     __syncwarp();
-  }
+    k0 += kSlots;
+  } while (k0 < a.topk);
 }
 
 template <template <class, class> class K>
@@ -365,8 +367,8 @@ static int moe_local_launch(ccb_comm* c, const MoeArgs& m, bool combine, int dty
   a.hidden = m.hidden;
   a.row_units = (uint32_t)(m.hidden / kWarpElems);
   a.tokens = (uint32_t)m.tokens;
-  a.topk = m.topk;
-  const uint32_t slots = dtype == CCB_F32 ? kMoeSlots<float> : kMoeSlots<__half>, rows = combine ? (uint32_t)m.topk < slots ? (uint32_t)m.topk : slots : 1u;
+  a.topk = m.topk > 0 ? m.topk : 0;
+  const uint32_t slots = dtype == CCB_F32 ? kMoeSlots<float> : kMoeSlots<__half>, rows = combine ? (uint32_t)a.topk < slots ? (uint32_t)a.topk : slots : 1u;
   a.batch_units = rows ? slots / rows : 1u;
   if (a.batch_units > a.row_units) a.batch_units = a.row_units;
   a.groups = (a.row_units + a.batch_units - 1) / a.batch_units;

@@ -49,7 +49,7 @@ def test_all_gather_of_odd_blocks(dtype, codec, n, count, in_place):
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("codec", ["none", "int8", "int4"])
-@pytest.mark.parametrize("topk", [1, 2, 3, 5, 9])   # beyond eight the rows of a token take several turns
+@pytest.mark.parametrize("topk", [1, 2, 3, 5, 9])   # beyond four (fp32: two) the rows of a token take several turns
 @pytest.mark.parametrize("hidden", [512, 1536, 3584])
 def test_rows_in_groups_of_units(dtype, codec, topk, hidden):
     n, tokens = 3, 61
@@ -72,6 +72,25 @@ def test_rows_in_groups_of_units(dtype, codec, topk, hidden):
         moe.dispatch(comm, xs, recv, routes, counts, codec=codec)
         moe.combine(comm, recv, out, routes, counts, codec=codec)
         return recv + out
+
+    _both(comm, call)
+    comm.close()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("hidden", [512, 1536, 4096])
+def test_a_token_of_no_rows_is_zero(dtype, hidden):
+    n, tokens = 2, 37
+    comm = Communicator.local(n, arena_bytes=32 << 20)
+    routes = [moe.plan_route(torch.empty(tokens, 0, dtype=torch.int64, device="cuda"), torch.empty(tokens, 0, device="cuda"), n) for _ in range(n)]
+    counts = [r.send_counts.tolist() for r in routes]
+
+    def call():
+        xs, recv, out = ([torch.full((rows, hidden), 3.0, dtype=dtype, device="cuda") for _ in range(n)] for rows in (tokens, 1, tokens))
+        moe.dispatch(comm, xs, recv, routes, counts)
+        moe.combine(comm, recv, out, routes, counts)
+        assert all(bool((o == 0).all()) for o in out) and all(bool((r == 3).all()) for r in recv)
+        return out
 
     _both(comm, call)
     comm.close()
