@@ -137,7 +137,8 @@ template <> struct Elem<__half> {
 
 // The first thing in a kernel that launch_next() launches, before it touches memory: the kernel before it on the
 // stream has then ended, and what it wrote is there. (None of them lets the one behind it begin early: a kernel may
-// follow that does not wait, see launch(), and it gained nothing.)
+// follow that does not wait, see launch(), and it gained nothing. Nor does any other kernel here but the pipelined one
+// of calls that overlap.)
 __device__ __forceinline__ void after_kernel_before() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 __device__ __forceinline__ uint4 ldg_stream(const void* p) {

@@ -322,7 +322,10 @@ cudaError_t launch_next(const void* kernel, dim3 grid, dim3 block, void** params
   return cudaLaunchKernelExC(&cfg, kernel, params);
 }
 
-int launch(ccb_comm* c, const void* kernel, int ctas, void* args, cudaStream_t stream, int threads, bool may_overlap) {
+// Whether consecutive calls of this communicator's pipelined kernel may overlap: a rank a GPU, and the caller says so.
+static bool overlaps(const ccb_comm* c) { return c->call_overlap && c->nlocal == 1; }
+
+int launch(ccb_comm* c, const void* kernel, int ctas, void* args, cudaStream_t stream, int threads, bool overlapping) {
   dim3 grid((unsigned)ctas, (unsigned)c->nlocal, 1), block((unsigned)threads, 1, 1);
   void* params[] = {args};
   // Consecutive calls may overlap tail and head (ccb_comm_set_call_overlap): the launch is
@@ -332,7 +335,7 @@ int launch(ccb_comm* c, const void* kernel, int ctas, void* args, cudaStream_t s
   // caller has promised that consecutive calls touch different user buffers, and the staging
   // halves and flags alternate by epoch. One CTA of 1024 threads fills an SM, so the call
   // after the next cannot start before this one has left the device.
-  if (may_overlap && c->call_overlap && c->nlocal == 1) {
+  if (overlapping) {
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof(cfg));
     cudaLaunchAttribute attr[1];
@@ -1103,7 +1106,7 @@ static int reduce_launch(ccb_comm* c, const void* const* send, void* const* recv
       if (w > most) w = most;
       if (w > CCB_MAX_SLOTS / 2) w = CCB_MAX_SLOTS / 2;
       // overlapping calls alternate between the two halves of the flag rows: 4 waves each
-      if (c->call_overlap && c->nlocal == 1 && w > CCB_MAX_SLOTS / 4) w = CCB_MAX_SLOTS / 4;
+      if (overlaps(c) && w > CCB_MAX_SLOTS / 4) w = CCB_MAX_SLOTS / 4;
       if (w < 1) w = 1;
       pipe_waves = w;
       pipe_ctas = (int)(ctas ? ctas : 1);
@@ -1131,9 +1134,10 @@ static int reduce_launch(ccb_comm* c, const void* const* send, void* const* recv
     a.waves = pipe_waves;
     a.tile_warps = kWarps;
     a.link_warps = c->pipe_link_warps;
-    a.row_base = (c->call_overlap && c->nlocal == 1 && (a.c.epoch & 1u)) ? CCB_MAX_SLOTS / 2 : 0;
+    a.row_base = (overlaps(c) && (a.c.epoch & 1u)) ? CCB_MAX_SLOTS / 2 : 0;
     a.use_mc = (c->mc_arena && c->nlocal == 1 && c->pipe_mc) ? 1 : 0;
-    return launch(c, fn, pipe_ctas, &a, stream, pipe_kernel_threads(), true);
+    a.early = overlaps(c) ? 1 : 0;
+    return launch(c, fn, pipe_ctas, &a, stream, pipe_kernel_threads(), overlaps(c));
   }
   const int ctas = ctas_for(c, fn, shard_elems < count ? shard_elems : count, &a.tile_warps);
   // Each extra wave of the non-specialised kernel costs a pipeline drain (fence + flag

@@ -88,6 +88,7 @@ typedef struct ReduceArgs {
   int row_base;               /* pipelined two-shot: first flag row of this call (0, or 8 for odd epochs when calls may overlap) */
   int link_warps;             /* pipelined two-shot: warps that store over NVLink (the rest decode, one signals) */
   int use_mc;                 /* pipelined two-shot: phase 2 stores once to the NVLS multicast address */
+  int early;                  /* pipelined two-shot: what follows on the stream may begin before this call has ended */
 } ReduceArgs;
 enum { CCB_MODE_ALLREDUCE = 0, CCB_MODE_REDUCESCATTER = 1, CCB_MODE_REDUCE = 2 };
 

@@ -55,3 +55,29 @@ def test_a_chain_waits_for_what_it_reads(count):
         assert all(torch.equal(a, b) for a, b in zip(got, want))
     del graph
     comm.close()
+
+
+def test_a_call_behind_a_capped_one_leaves_the_other_sms_free():
+    """What is launched behind a collective of a few CTAs does not wait on the SMs that the cap leaves to other streams."""
+    comm, behind = Communicator.local(2, arena_bytes=1 << 30), Communicator.local(2, arena_bytes=32 << 20)
+    comm.set_pipeline(2)
+    comm.set_max_ctas(4)
+    xs = [torch.randn(48 << 20, device="cuda").bfloat16() for _ in range(2)]
+    ys, zs = [torch.empty_like(x) for x in xs], [torch.empty_like(x) for x in xs]
+    small = torch.zeros(1 << 16, device="cuda")
+    other = torch.cuda.Stream()
+    for _ in range(3):   # once to load the kernels
+        torch.cuda.synchronize()
+        start, done, end = (torch.cuda.Event(enable_timing=True) for _ in range(3))
+        start.record()
+        comm.all_reduce(xs, ys)
+        behind.all_reduce(xs, zs)   # more CTAs than fit
+        with torch.cuda.stream(other):
+            small += 1
+            done.record()
+        end.record()
+        torch.cuda.synchronize()
+    assert start.elapsed_time(end) > 1.0
+    assert start.elapsed_time(done) < 0.5 * start.elapsed_time(end)
+    comm.close()
+    behind.close()
