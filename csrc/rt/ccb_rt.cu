@@ -17,7 +17,6 @@
 #include <atomic>
 #include <map>
 #include <mutex>
-#include <set>
 #include <tuple>
 #include <string>
 #include <vector>
@@ -31,6 +30,7 @@
 #include "../kernels/ccb_ring.cuh"
 #include "ccb/ccb.h"
 #include "ccb_bootstrap.h"
+#include "ccb_overlap.h"
 #include "ccb_rt_internal.h"
 
 namespace ccb {
@@ -285,25 +285,24 @@ int grid_cap(ccb_comm* c, const void* kernel, int threads) {
   return cap < 1 ? 1 : cap;
 }
 
-// Streams whose last launch here was an overlapping one (see launch()). What comes next on them waits for more than
-// that kernel: the one before it, for which it did not wait, may still run. Rare, so that others look at a counter alone.
-static std::atomic<int> g_overlapped_count{0};
-static std::mutex g_overlapped_lock;
-static std::set<cudaStream_t> g_overlapped;
-static bool g_overlapped_all = false;   // too many streams to tell apart
-static void note_overlapped(cudaStream_t stream) {
-  std::lock_guard<std::mutex> hold(g_overlapped_lock);
-  if (g_overlapped.size() < 4096) g_overlapped.insert(stream);
-  else g_overlapped_all = true;
-  g_overlapped_count.store((int)g_overlapped.size());
+static OverlapNotes g_overlapped;
+// False where CUDA does not say, for instance of the default stream while another stream's capture forbids it. A stream
+// that captures must not be asked for its number: that ends the capture in an error.
+static bool launch_place(cudaStream_t stream, LaunchPlace& at) {
+  cudaStreamCaptureStatus status;
+  at.stream = at.capture = 0;
+  bool told = cudaGetDevice(&at.device) == cudaSuccess && cudaStreamGetCaptureInfo(stream, &status, &at.capture) == cudaSuccess;
+  if (told && status == cudaStreamCaptureStatusNone) {
+    at.capture = 0;
+    told = cudaStreamGetId(stream, &at.stream) == cudaSuccess;
+  }
+  if (!told) (void)cudaGetLastError();
+  return told;
 }
 static bool behind_overlapped(cudaStream_t stream) {
-  if (g_overlapped_count.load() == 0) return false;
-  std::lock_guard<std::mutex> hold(g_overlapped_lock);
-  if (g_overlapped_all) return true;
-  const bool hit = g_overlapped.erase(stream) != 0;
-  g_overlapped_count.store((int)g_overlapped.size());
-  return hit;
+  if (!g_overlapped.any()) return false;
+  LaunchPlace at;
+  return !launch_place(stream, at) || g_overlapped.behind(at);
 }
 
 cudaError_t launch_next(const void* kernel, dim3 grid, dim3 block, void** params, size_t shared, cudaStream_t stream) {
@@ -325,7 +324,7 @@ cudaError_t launch_next(const void* kernel, dim3 grid, dim3 block, void** params
 // Whether consecutive calls of this communicator's pipelined kernel may overlap: a rank a GPU, and the caller says so.
 static bool overlaps(const ccb_comm* c) { return c->call_overlap && c->nlocal == 1; }
 
-int launch(ccb_comm* c, const void* kernel, int ctas, void* args, cudaStream_t stream, int threads, bool overlapping) {
+int launch(ccb_comm* c, const void* kernel, int ctas, void* args, cudaStream_t stream, int threads, const LaunchPlace* overlapping) {
   dim3 grid((unsigned)ctas, (unsigned)c->nlocal, 1), block((unsigned)threads, 1, 1);
   void* params[] = {args};
   // Consecutive calls may overlap tail and head (ccb_comm_set_call_overlap): the launch is
@@ -351,7 +350,7 @@ int launch(ccb_comm* c, const void* kernel, int ctas, void* args, cudaStream_t s
       set_error("kernel launch failed: %s", cudaGetErrorString(e));
       return CCB_ERR_CUDA;
     }
-    note_overlapped(stream);
+    g_overlapped.note(*overlapping);
     count_launch();
     return CCB_OK;
   }
@@ -1136,8 +1135,10 @@ static int reduce_launch(ccb_comm* c, const void* const* send, void* const* recv
     a.link_warps = c->pipe_link_warps;
     a.row_base = (overlaps(c) && (a.c.epoch & 1u)) ? CCB_MAX_SLOTS / 2 : 0;
     a.use_mc = (c->mc_arena && c->nlocal == 1 && c->pipe_mc) ? 1 : 0;
-    a.early = overlaps(c) ? 1 : 0;
-    return launch(c, fn, pipe_ctas, &a, stream, pipe_kernel_threads(), overlaps(c));
+    LaunchPlace place;
+    const bool early = overlaps(c) && launch_place(stream, place);
+    a.early = early ? 1 : 0;
+    return launch(c, fn, pipe_ctas, &a, stream, pipe_kernel_threads(), early ? &place : nullptr);
   }
   const int ctas = ctas_for(c, fn, shard_elems < count ? shard_elems : count, &a.tile_warps);
   // Each extra wave of the non-specialised kernel costs a pipeline drain (fence + flag

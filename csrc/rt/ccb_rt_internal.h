@@ -7,13 +7,15 @@
 struct ccb_comm;
 
 namespace ccb {
+
+struct LaunchPlace;   // ccb_overlap.h
 void set_error(const char* fmt, ...);
 void count_launch();
 int sm_count();   // of the current device
 CommDev comm_dev(ccb_comm* c, uint32_t epoch);
 uint32_t next_epoch(ccb_comm* c);
 int grid_cap(ccb_comm* c, const void* kernel, int threads = 512);
-int launch(ccb_comm* c, const void* kernel, int ctas, void* args, cudaStream_t stream, int threads = 512, bool overlapping = false);
+int launch(ccb_comm* c, const void* kernel, int ctas, void* args, cudaStream_t stream, int threads = 512, const LaunchPlace* overlapping = nullptr);
 // A launch that is got ready while the kernel before it on the stream still runs: for kernels that begin with
 // after_kernel_before() (ccb_device.cuh). Kernels behind one another on a stream begin about 2 us sooner (B200, us, launched
 // plainly / so: three chunks of 3,000,001 values compressed, reduced and decompressed, five kernels, 30.7 / 20.5; a
