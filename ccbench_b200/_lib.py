@@ -8,12 +8,14 @@ from __future__ import annotations
 
 import ctypes
 import functools
+import hashlib
 import importlib.machinery
 import importlib.util
 import os
 import shutil
 import subprocess
 import sysconfig
+import warnings
 from pathlib import Path
 
 ROOT = Path(__file__).resolve().parent.parent
@@ -59,17 +61,38 @@ def build_native(force: bool = False, verbose: bool = False) -> Path:
     return LIBCCB
 
 
+def _calls_marks() -> list[str]:
+    """What the native side of the frequent calls is compiled with and has to hold: the torch and the Python whose objects it
+    reads by their layout, and its sources with the C API that it calls (where they are there to look at)."""
+    import torch
+
+    marks = [f"torch {torch.__version__} {torch.version.git_version} {importlib.machinery.EXTENSION_SUFFIXES[0]}"]
+    if CALLS_SOURCE.exists():
+        digest = hashlib.sha256()
+        for f in [CALLS_SOURCE, *sorted((ROOT / "include").rglob("*.h"))]:
+            digest.update(f.read_bytes())
+        marks.append(f"sources {digest.hexdigest()}")
+    return marks
+
+
+def _calls_fit() -> bool:
+    if not CALLS.exists():
+        return False
+    held = CALLS.read_bytes()
+    return all(mark.encode() in held for mark in _calls_marks())
+
+
 def build_calls(force: bool = False, verbose: bool = False) -> Path:
-    """Compile the native side of the frequent calls (csrc/py/ccb_calls.cpp) against the torch that is installed,
-    if it is missing or older than its sources. Processes that build at once each make their own file."""
+    """Compile the native side of the frequent calls (csrc/py/ccb_calls.cpp) against the torch that is installed, if it
+    is missing or made for another torch or of other sources. Processes that build at once each make their own file."""
     import torch
 
     NATIVE_DIR.mkdir(parents=True, exist_ok=True)
-    if force or _stale(CALLS, [CALLS_SOURCE, *(ROOT / "include").rglob("*.h")]):
+    if force or not _calls_fit():
         home, cuda = Path(torch.__file__).parent, Path(os.environ.get("CUDA_HOME", "/usr/local/cuda"))
         made = CALLS.with_name(f"{CALLS.name}.{os.getpid()}")
         include = [home / "include", home / "include/torch/csrc/api/include", sysconfig.get_paths()["include"], cuda / "include", ROOT / "include"]
-        cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", *(f"-I{i}" for i in include), str(CALLS_SOURCE), "-o", str(made), f"-L{home / 'lib'}",
+        cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", f'-DCCB_BUILT_FOR="{"; ".join(_calls_marks())}"', *(f"-I{i}" for i in include), str(CALLS_SOURCE), "-o", str(made), f"-L{home / 'lib'}",
                "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda", f"-L{cuda / 'lib64'}", "-lcudart"]
         if verbose:
             print(" ".join(cmd))
@@ -80,22 +103,24 @@ def build_calls(force: bool = False, verbose: bool = False) -> Path:
 
 @functools.cache
 def calls():
-    """The native side of the frequent calls, or None where it cannot be had (no compiler, another torch than it was
-    built with): every call has a way without it."""
+    """The native side of the frequent calls, or None where it cannot be had (made for another torch or of other
+    sources, and no compiler to make it again; a libccb.so without what it calls): every call has a way without it, slower
+    by some microseconds of the host. Said once."""
     import torch
 
     from . import constants as K
 
     try:
-        if not CALLS.exists():
+        if not _calls_fit():   # before it is loaded: it would read another torch's objects wrongly, not fail
             build_calls()
         spec = importlib.util.spec_from_file_location("ccb_calls", CALLS, loader=importlib.machinery.ExtensionFileLoader("ccb_calls", str(CALLS)))
         module = importlib.util.module_from_spec(spec)
         spec.loader.exec_module(module)
-    except (ImportError, OSError, subprocess.CalledProcessError):
+        L = lib()
+        where = {name: ctypes.cast(getattr(L, name), ctypes.c_void_p).value for name in module.names().split()}
+    except (ImportError, OSError, subprocess.CalledProcessError, AttributeError) as e:
+        warnings.warn(f"calls from Python take their slower way: {CALLS.name} cannot be used ({e})", RuntimeWarning, stacklevel=2)
         return None
-    L = lib()
-    where = {name: ctypes.cast(getattr(L, name), ctypes.c_void_p).value for name in module.names().split()}
     module.setup(where, K.OPS, K.CODECS, K.ALGOS, torch.nn.Parameter)
     return module
 

@@ -458,6 +458,9 @@ PyObject* setup(PyObject*, PyObject* args) {
   if (PyErr_Occurred()) return nullptr;
   Py_RETURN_NONE;
 }
+// What this file was compiled for, looked for in the built file before it is loaded: the objects above are read by
+// the layout that the headers of one torch give them.
+PyObject* built_for(PyObject*, PyObject*) { return PyUnicode_FromString(CCB_BUILT_FOR); }
 PyObject* names(PyObject*, PyObject*) {
 #define CCB_NAME(f) #f " "
   return PyUnicode_FromString(CCB_CALLS(CCB_NAME));
@@ -466,7 +469,7 @@ PyObject* names(PyObject*, PyObject*) {
 
 #define METHOD(f) {#f, (PyCFunction)(void (*)(void))f, METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {
-    {"setup", setup, METH_VARARGS, nullptr}, {"names", names, METH_NOARGS, nullptr},
+    {"setup", setup, METH_VARARGS, nullptr}, {"names", names, METH_NOARGS, nullptr}, {"built_for", built_for, METH_NOARGS, nullptr},
     METHOD(all_reduce), METHOD(reduce_scatter), METHOD(all_gather), METHOD(moe_dispatch), METHOD(moe_combine), METHOD(encode), METHOD(decode),
     METHOD(reduce_recode), METHOD(lossless_encode), METHOD(lossless_decode), METHOD(sz_compress), METHOD(sz_decompress), METHOD(sz_scan), METHOD(sz_open),
     METHOD(sz_pack), METHOD(sz_unpack), {nullptr, nullptr, 0, nullptr}};
