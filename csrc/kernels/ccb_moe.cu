@@ -255,8 +255,8 @@ __global__ void __launch_bounds__(kMoeLocalThreads, 12) moe_local_dispatch_kerne
 // shared memory, 4 KiB under way at once, where a row at a time in registers left a warp waiting for one row after
 // the other, 1 KiB each. An index outside its block (the entry of a dropped pair) contributes nothing.
 // (8 ranks, 8192 x 4096 bf16, top 2, fp8: 328 us a row at a time with 40 warps an SM, 267 so, of 246 that the memory
-// needs; 2048 x 4096 fp32, top 2, int8 162 and 131; top 1 of 4096 x 4096 62 and 47.5; top 4 of 2048 x 2048 in int8, bound by
-// its codec, 84 and 84. 36 warps an SM, 56 registers: with 40, which spill, 265 but 98 at top 4, with 32 276. B200.)
+// needs; top 4 of 2048 x 2048 in int8, bound by its codec, 84 and 84. 36 warps an SM, 56 registers: with 40, which spill, 265
+// but 98 at top 4, with 32 276. B200.)
 template <class T, class C>
 __global__ void __launch_bounds__(kMoeLocalThreads, 9) moe_local_combine_kernel(const __grid_constant__ MoeLocalArgs a) {
   after_kernel_before();

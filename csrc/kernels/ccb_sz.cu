@@ -1178,14 +1178,10 @@ __device__ __forceinline__ uint32_t pack_planes(const SzLocalArgs& a, unsigned c
 // A warp stages the whole of its tile, 8256 bytes at most, three CTAs an SM; with less of it, tiles that were larger
 // went through the codec a second time, to their places (512^3 values of white noise, bound 1e-5 of their range,
 // 470 us). Bound by instructions at 24 warps an SM: ncu, 384^3, 48.8 M of them, 221 a plane with all that a tile needs
-// besides, 73 % of the issue slots, 60 % of the pipe of logical operations. With planes loaded to registers one ahead
-// (moves of eight registers a plane), residuals one to a word, the masks of the bit transpose chosen at each use and planes
-// of 9 to 16 bits a row at a time it was 62.3 M. (B200, us, that / so: 512^3 field, bound 1e-4 of its range, 173 / 138;
-// 1e-3 168 / 132; 1e-5 190 / 166; with 30 added to its values 179 / 148; 300 x 300 x 404 55.6 / 49.4, x 403 68 / 61; 130
-// x 201 x 258 22.8 / 16; white noise 512^3, 1e-5 266 / 262, 1e-6 265 / 245, 1e-7, all raw, 239 / 206. An address computed
-// afresh for each piece that is staged 143; tiles begun again by the general way where a plane is not one for halves, 175 at
-// 1e-5. Two planes at a time, with one vote and their transposes interleaved, 135.5 at 1e-4 but 202 at 1e-5.) Operands of the
-// packed operations kept in registers, or given as pairs of arguments, changed nothing; one vote for both tests neither.
+// besides, 73 % of the issue slots, 60 % of the pipe of logical operations. With planes loaded to registers one ahead,
+// residuals one to a word and planes of 9 to 16 bits a row at a time it was 62.3 M (B200, us, that / so: 512^3 field, bound
+// 1e-4 of its range, 173 / 138; 1e-3 168 / 132; 1e-5 190 / 166; 300 x 300 x 404 55.6 / 49.4, x 403 68 / 61; 130 x 201 x 258
+// 22.8 / 16; white noise 512^3, 1e-6 265 / 245, 1e-7, all raw, 239 / 206). Two planes at a time 135.5 at 1e-4 but 202 at 1e-5.
 template <int kVec>
 __global__ void __launch_bounds__(kSzThreads, 3) sz_pack_kernel(const __grid_constant__ SzLocalArgs a) {
   after_kernel_before();
@@ -1438,16 +1434,12 @@ __device__ __forceinline__ void unpack_digits(PlaneOut<kAligned>& io, unsigned c
 // A warp brings a packed tile to shared memory, all of it under way at once or, above 2816 bytes, in two turns, and
 // takes its planes from there by the tensor cores; raw ones, and those with residuals of more than 15 bits, are read
 // where they are, from L2 where a prefetch puts them, and summed by shuffles. (B200, us, the whole by shuffles with
-// one plane requested ahead / so: 512^3 field, bound 1e-4 of its range, 163 / 111; 1e-3 154 / 105; 1e-5 183 / 129;
-// the first with 30 added to its values 165 / 118; 300 x 300 x 404 49.5 / 32, x 403 62 / 51; 512^3 of white noise,
-// 1e-6 190 / 173, 1e-5 277 / 258. Stages of 4608 bytes took as long on the fields and 12 us more on the noise at
-// 1e-6, of 3328 10 us more there; of 2304, with larger tiles by shuffles, a field at 3e-6, 1.3 bytes a value, 242
-// instead of 175, 256^3 white noise of 1.65 bytes a value 41 instead of 27, 256^3 at 1e-5 21.5 instead of 22.4 (one
-// loop for both kinds of wide tiles 23.1). Five CTAs of 48 registers spill and take 10 us more, three of 80 18. Lanes
-// that hold 32 bytes of a line: as fast at 512^3, 45 instead of 33 where lines lie on 16 bytes. Resident CTAs that
-// take groups in turn with the next tile under way: 209 instead of 119. Addresses moved on instead of computed,
-// values scaled in pairs: 119 and 111.) ncu, 384^3: 30.8 M instructions, 58.2 M by shuffles. What is left of the 94
-// us that the memory needs is the latency of a tile's size, then its words.
+// one plane requested ahead / so: 512^3 field, bound 1e-4 of its range, 163 / 111; 1e-3 154 / 105; 3e-6 242 / 175; 300 x 300
+// x 404 49.5 / 32, x 403 62 / 51; 512^3 of white noise, 1e-6 190 / 173. Stages of 3328 and 4608 bytes cost the noise 10 and
+// 12 us and give the fields nothing; five CTAs of 48 registers spill, +10, three of 80 +18; lanes that hold 32 bytes of a
+// line 45 instead of 33 where lines lie on 16; resident CTAs with the next tile under way 209 instead of 119.) ncu, 384^3:
+// 30.8 M instructions, 58.2 M by shuffles. What is left of the 94 us that the memory needs is the latency of a tile's size,
+// then its words.
 template <int kVec>
 __global__ void __launch_bounds__(kSzThreads, 4) sz_unpack_kernel(const __grid_constant__ SzLocalArgs a) {
   after_kernel_before();
@@ -1927,11 +1919,18 @@ static void launch_pack(const SzLocalArgs& a, cudaStream_t stream) {
   }
   launch_next(sz_pack_kernel<kVec>, a.ngroups, kSzThreads, kBytes, stream, a);
 }
-// Tiles up to which a CTA a tile unpacks a field faster than a warp a tile, us, CTA / warp, at bounds of 1e-4
-// and 1e-5 of the range (0.6 and 1 byte a value), B200. Lines on 16 bytes: 64^3 (128 tiles) 6.0 / 8.6 and
-// 5.9 / 13.8, 128 x 128 x 256 (2048) 10.6 / 10.4 and 10.6 / 14.7, 160 x 160 x 256 (3200) 14.7 / 10.6 and
-// 14.9 / 16.7. Lines anywhere: 130 x 130 x 258 (2601) 12.8 / 14.6 and 12.7 / 18.9, 176 x 176 x 258 (4356)
-// 18.8 / 16.7 and 19.2 / 20.8, 256 x 256 x 257 (9216) 35 / 29 and 37 / 34.
+// Tiles up to which a CTA a tile unpacks a field faster than a warp a tile, or loses less at loose bounds than it gains at
+// tight ones. B200, us, CTA / warp at bounds of 1e-4, 1e-5 and 1e-6 of the range (0.6, 1 and 2.1 bytes a value; 1e-3 as 1e-4, or
+// up to 2 us less for the warp):
+//   lines on 32 bytes  64 x 64 x 64 (128 tiles)   3.5 / 6.2   3.5 / 7.0   3.7 / 11.9
+//                      128 x 128 x 256 (2048)     8.7 / 8.0   9.1 / 9.2   10.0 / 10.2
+//                      144 x 136 x 256 (2448)     9.9 / 8.7   10.3 / 10.7 11.2 / 12.9
+//                      160 x 160 x 256 (3200)     12.2 / 8.8  12.7 / 11.5 13.7 / 14.9
+//   on 16              128 x 128 x 260 (2304)     9.8 / 7.5   10.2 / 8.7  10.9 / 10.1
+//                      144 x 136 x 260 (2754)     11.2 / 8.4  11.7 / 10.9 12.8 / 12.7
+//   anywhere           144 x 136 x 258 (2754)     11.4 / 11.7 11.9 / 14.0 12.6 / 15.5
+//                      176 x 200 x 258 (4950)     18.3 / 17.8 19.1 / 21.1 20.4 / 24.0
+//                      200 x 208 x 258 (5850)     21.2 / 18.2 22.0 / 23.4 23.4 / 26.1
 static unsigned int few_tiles(int width) { return width == 1 ? 5120u : 2560u; }
 static int launched(const char* what) {
   const cudaError_t e = cudaGetLastError();

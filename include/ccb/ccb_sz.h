@@ -26,7 +26,8 @@ int ccb_sz_launch_path(void);
  * and a buffer to be read on 4. `d_used` (device memory, optional) receives the number of compressed
  * bytes produced (those of the tiles, without the groups' size words). A tile of a damaged buffer whose
  * size words put it outside its group, or whose rows are wider than 32 bits, is decompressed to NaN;
- * what else a damaged buffer holds is decoded as it stands, from inside its slots. */
+ * what else a damaged buffer holds is decoded as it stands, from inside its slots, to values that may differ
+ * with the size and the alignment of the field. */
 int ccb_sz_compress(const float* in, int nx, int ny, int nz, float eb, void* out, unsigned long long* d_used,
                     ccb_stream_t stream);
 int ccb_sz_decompress(const void* in, int nx, int ny, int nz, float eb, float* out, ccb_stream_t stream);

@@ -1,5 +1,7 @@
 """Launches that are got ready while the kernel before them runs: a chain in which every kernel reads what the one
 before it wrote, ours and torch's in turn, on the default stream, on another, and as a graph."""
+import ctypes
+
 import pytest
 import torch
 
@@ -81,3 +83,29 @@ def test_a_call_behind_a_capped_one_leaves_the_other_sms_free():
     assert start.elapsed_time(done) < 0.5 * start.elapsed_time(end)
     comm.close()
     behind.close()
+
+
+@pytest.mark.parametrize("blocking", [False, True])
+def test_a_launch_waits_for_other_streams_that_its_own_waits_for(blocking):
+    """A kernel of ours, a long one of another stream behind it, and ours again, which reads what that wrote: ordered by an
+    event, or by the default stream's own rule for streams that block."""
+    stream, other = torch.cuda.current_stream(), torch.cuda.Stream()
+    if blocking:   # torch's own do not
+        made = ctypes.c_void_p()
+        assert ctypes.CDLL("libcudart.so.12").cudaStreamCreate(ctypes.byref(made)) == 0
+        other = torch.cuda.ExternalStream(made.value)
+    x = torch.zeros(1 << 20, device="cuda")
+    want = standalone.encode(torch.full_like(x, 7.0), "int8")
+    for _ in range(3):
+        x.zero_()
+        before = standalone.encode(x, "int8")
+        if not blocking:
+            other.wait_stream(stream)
+        with torch.cuda.stream(other):
+            torch.cuda._sleep(20_000_000)   # some 10 ms
+            x.fill_(7.0)
+        if not blocking:
+            stream.wait_stream(other)
+        got = standalone.encode(x, "int8")
+        torch.cuda.synchronize()
+        assert torch.equal(got, want) and not torch.equal(before, want)
