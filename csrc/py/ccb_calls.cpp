@@ -401,7 +401,7 @@ FUNCTION(sz_open, 2)
   if (!blob || blob->scalar_type() != at::kByte || !number(a[1], room) || !room || room >> 31) NOT_TAKEN;
   const cudaStream_t st = stream();
   if (capturing(st)) NOT_TAKEN;
-  const at::Tensor offsets = made({(int64_t)room + 2 + 7}, at::kLong, *blob), host = pinned(7);
+  const at::Tensor offsets = made({(int64_t)room + 2}, at::kLong, *blob), host = pinned(7);
   const void* in = blob->data_ptr();
   const uint64_t bytes = (uint64_t)blob->numel();
   unsigned long long* at = static_cast<unsigned long long*>(offsets.data_ptr());
